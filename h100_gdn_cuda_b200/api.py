@@ -29,6 +29,22 @@ Prefill, Decode, SpecVerify = InferenceMode.Prefill, InferenceMode.Decode, Infer
 
 _state = {"library_root": None, "cuda_home": None}
 
+# The per-call functions below hand their arguments straight to the C++ front end (csrc/torch_ext/fastcall.cpp) when
+# the extension is built: 3 - 6 us of host time a call where the ctypes bodies take 25 - 35, which for a decode step or
+# a short prompt was several times the GPU's own time.  The ctypes bodies serve installations of the library alone
+# and the private arguments of the tests and the benchmark.
+_ext = None
+
+
+def _load_ext():
+    global _ext
+    try:
+        from . import gdn_cuda
+        _ext = gdn_cuda
+    except ImportError:
+        _ext = False
+    return _ext
+
 
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
@@ -126,6 +142,9 @@ def fused_gdn_gating(A_log, dt_bias, a, b, is_var_len: bool = False) -> Tuple[to
 
     `A_log` may be the per-head vector (vh,) or, as in the reference, a tensor shaped like
     `a` whose first vh entries are the per-head values.  Output dtype = input dtype."""
+    ext = _ext if _ext is not None else _load_ext()
+    if ext:
+        return ext._fast_fused_gdn_gating(A_log, dt_bias, a, b)
     _require(a.is_cuda and b.is_cuda and A_log.is_cuda and dt_bias.is_cuda, "inputs must be CUDA tensors")
     _require(a.dtype == b.dtype == A_log.dtype == dt_bias.dtype, "A_log, dt_bias, a, b must share a dtype")
     vh = a.shape[-1]
@@ -200,6 +219,10 @@ def recurrent_forward(query, key, value, initial_state=None, beta=None, gate=Non
     `initial_state` is a pool of states (P, vh, dv, dk): sequence s uses slot state_indices[s], the new
     state is written back to the same slot (the pool is returned), and a negative slot marks a padding
     sequence that is skipped altogether."""
+    ext = _ext if _ext is not None else _load_ext()
+    if ext and _max_head_dim == 256:
+        return ext._fast_recurrent_forward(query, key, value, initial_state, beta, gate, cu_seqlens, num_accepted_tokens,
+                                           inference_mode, is_qk_norm, scale, inplace_state, gating, state_indices)
     if gating is not None:
         _require(beta is None and gate is None, "pass either gating=(A_log, dt_bias, a, b) or beta/gate, not both")
         g_A, g_dt, g_a, g_b = gating
@@ -320,6 +343,10 @@ def chunked_forward(query, key, value, beta, gate, scale: Optional[float] = None
     The default scale is d ** -0.5 with d the caller's (unpadded) head dimension.
     `is_qk_norm=True` (keyword-only extension; the reference lists it as future work) L2-normalises
     q and k per head inside the kernels, as recurrent_forward does."""
+    ext = _ext if _ext is not None else _load_ext()
+    if ext and _stage_events is None:
+        return ext._fast_chunked_forward(query, key, value, beta, gate, scale, initial_state, cu_seqlens, chunk_indices,
+                                         cu_chunks, total_chunks, is_qk_norm, _workspace)
     for t, n in ((query, "query"), (key, "key"), (value, "value")):
         _cuda_bf16(t, n)
     _require(gate is None or gate.dtype in (torch.float32, torch.bfloat16), "gate must be fp32 (or bf16)")
@@ -482,6 +509,9 @@ def causal_conv1d(x, weight, bias=None, initial_state=None, cu_seqlens=None, act
     each sequence (None: zeros).  Returns y, or (y, final_state) with the last W-1 inputs of every sequence
     when `return_final_state` (or when a `final_state` buffer is given; it may be `initial_state` itself for
     decode-sized calls)."""
+    ext = _ext if _ext is not None else _load_ext()
+    if ext:
+        return ext._fast_causal_conv1d(x, weight, bias, initial_state, cu_seqlens, activation, final_state, return_final_state)
     _cuda_bf16(x, "x")
     _cuda_bf16(weight, "weight")
     _require(x.stride(-1) == 1, "channels must be contiguous")
@@ -516,6 +546,9 @@ def causal_conv1d(x, weight, bias=None, initial_state=None, cu_seqlens=None, act
 def gated_rmsnorm(x, z, weight, eps: float = 1e-6):
     """y = x * rsqrt(mean(x^2) + eps) * weight * silu(z) over the last axis: the output norm that follows Gated
     DeltaNet (x: the layer's output, z: the gate projection, both (..., D) bf16; weight (D))."""
+    ext = _ext if _ext is not None else _load_ext()
+    if ext:
+        return ext._fast_gated_rmsnorm(x, z, weight, eps)
     _cuda_bf16(x, "x")
     _cuda_bf16(z, "z")
     _cuda_bf16(weight, "weight")

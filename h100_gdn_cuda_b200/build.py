@@ -85,7 +85,7 @@ def build_ext(force: bool = False) -> str:
     from torch.utils import cpp_extension
     lib = build(force=False)
     out = ext_path()
-    srcs = [os.path.join(EXT_DIR, f) for f in ("gdn_api.cpp", "python_api.cpp")]
+    srcs = [os.path.join(EXT_DIR, f) for f in ("gdn_api.cpp", "python_api.cpp", "fastcall.cpp")]
     newest = max(os.path.getmtime(f) for f in srcs + [os.path.join(EXT_DIR, "gdn_api.hpp"),
                                                        os.path.join(PKG, "..", "include", "gdn_b200.h")])
     if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
@@ -114,7 +114,7 @@ def build_ext(force: bool = False) -> str:
         return obj
 
     os.makedirs(OBJDIR, exist_ok=True)
-    with ThreadPoolExecutor(max_workers=2) as ex:
+    with ThreadPoolExecutor(max_workers=len(srcs)) as ex:
         objs = list(ex.map(cc, srcs))
     cmd = ["g++", "-shared", "-o", out + ".tmp", *objs, "-L", tlib, "-L", LIBDIR, "-lgdn_b200", "-ltorch", "-ltorch_cpu",
            "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-L", os.path.join(cuda_home, "lib64"), "-lcudart",

@@ -10,6 +10,8 @@
 #include "kernels/prefill_zp.cuh"
 #include "tma_host.hpp"
 
+#include <atomic>
+
 using namespace gdn;
 
 namespace {
@@ -90,9 +92,16 @@ int check_scalar(const GdnTokenScalar& t, const char* name, bool required) {
     return GDN_OK;
 }
 
-template <typename K>
-int set_smem(K kernel, int bytes) {
-    GDN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+// The kernel's dynamic shared-memory limit, raised once per device (the attribute call is a good part of a
+// microsecond, and a short prompt's call lasts a few).
+template <auto kKernel>
+int set_smem(int bytes) {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    GDN_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return GDN_OK;
+    GDN_CUDA(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return GDN_OK;
 }
 
@@ -120,20 +129,17 @@ int launch_uw(const GdnShape& s, const GdnTokenTensor& k, const GdnTokenTensor& 
     p.status = d->status;
     constexpr int smem = UWSmem<kD>::kBytes;
     const int grid = uw_grid(static_cast<long long>(nc) * s.num_v_heads, d->sms);
-    if (int rc = set_smem(gdn_uw_kernel<kD>, smem)) return rc;
+    if (int rc = set_smem<gdn_uw_kernel<kD>>(smem)) return rc;
     gdn_uw_kernel<kD><<<grid, 128, smem, st>>>(tmK, tmV, tmUo, tmWo, p);
     GDN_CUDA(cudaGetLastError());
     return GDN_OK;
 }
 
 // Chunk-parallel stage of the whole-layer path: Z and PT of every (chunk, v-head) into `blocks`.
-int launch_zp(const GdnShape& s, const GdnTokenTensor& q, const GdnTokenTensor& k, const GdnTokenScalar& beta,
+int launch_zp(const GdnShape& s, const CUtensorMap& tmQ, const CUtensorMap& tmK, const GdnTokenScalar& beta,
               const GdnTokenScalar& gate, void* blocks, float* norms, float p_scale, DeviceInfo* d, cudaStream_t st) {
     const int nc = num_chunks(s);
     if (nc == 0) return GDN_OK;
-    CUtensorMap tmK, tmQ;
-    if (int rc = make_token_map(&tmK, k, s, s.num_k_heads, "k", s.head_dim_k)) return rc;
-    if (int rc = make_token_map(&tmQ, q, s, s.num_k_heads, "q", s.head_dim_k)) return rc;
     ZPParams p{};
     p.map = chunk_map(s);
     p.beta = scalar_view(beta);
@@ -160,10 +166,10 @@ int launch_zp(const GdnShape& s, const GdnTokenTensor& q, const GdnTokenTensor& 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (norms) {
-        if (int rc = set_smem(gdn_zp_kernel<true>, smem)) return rc;
+        if (int rc = set_smem<gdn_zp_kernel<true>>(smem)) return rc;
         GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_zp_kernel<true>, tmK, tmQ, p));
     } else {
-        if (int rc = set_smem(gdn_zp_kernel<false>, smem)) return rc;
+        if (int rc = set_smem<gdn_zp_kernel<false>>(smem)) return rc;
         GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_zp_kernel<false>, tmK, tmQ, p));
     }
     return GDN_OK;
@@ -173,7 +179,7 @@ template <bool O, bool H, bool UN>
 int launch_seq_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmW, const CUtensorMap& tmU,
                  const SeqParams& p, dim3 grid, cudaStream_t st) {
     constexpr int smem = SeqSmem::kBytes;
-    if (int rc = set_smem(gdn_seq_kernel<O, H, UN>, smem)) return rc;
+    if (int rc = set_smem<gdn_seq_kernel<O, H, UN>>(smem)) return rc;
     gdn_seq_kernel<O, H, UN><<<grid, 256, smem, st>>>(tmQ, tmK, tmW, tmU, p);
     GDN_CUDA(cudaGetLastError());
     return GDN_OK;
@@ -279,7 +285,7 @@ int gdn_compute_o(const GdnComputeOArgs* a, gdn_stream_t stream) {
     p.scale = a->scale;
     p.status = d->status;
     constexpr int smem = OSmem::kBytes;
-    if (int rc = set_smem(gdn_o_kernel, smem)) return rc;
+    if (int rc = set_smem<gdn_o_kernel>(smem)) return rc;
     gdn_o_kernel<<<dim3(nc, s.num_v_heads), 128, smem, static_cast<cudaStream_t>(stream)>>>(tmQ, tmK, tmU, tmH, tmO, p);
     GDN_CUDA(cudaGetLastError());
     return GDN_OK;
@@ -413,17 +419,17 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     uint8_t* const ws_extra = ws + ws_blocks_bytes(nchunks, s.num_v_heads) + ws_norms_bytes(nchunks, s.num_k_heads);
     // Both kernels are prepared before the first is launched, so that the state kernel is in the stream
     // when the chunk-parallel kernel starts to drain.
+    CUtensorMap tmQ, tmK, tmV, tmO;
+    if (int rc = make_token_map(&tmQ, a->q, s, s.num_k_heads, "q", hd)) return rc;
+    if (int rc = make_token_map(&tmK, a->k, s, s.num_k_heads, "k", hd)) return rc;
+    if (int rc = make_token_map(&tmV, a->v, s, s.num_v_heads, "v", hd)) return rc;
+    if (int rc = make_token_map(&tmO, a->out, s, s.num_v_heads, "out", hd)) return rc;
     auto run_zp = [&]() -> int {
-        if (int rc = launch_zp(s, a->q, a->k, a->beta, a->gate, a->workspace, norms, a->scale, d, st)) return rc;
+        if (int rc = launch_zp(s, tmQ, tmK, a->beta, a->gate, a->workspace, norms, a->scale, d, st)) return rc;
         if (ev) GDN_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(ev[1]), st));
         return GDN_OK;
     };
     {
-        CUtensorMap tmQ, tmK, tmV, tmO;
-        if (int rc = make_token_map(&tmQ, a->q, s, s.num_k_heads, "q", hd)) return rc;
-        if (int rc = make_token_map(&tmK, a->k, s, s.num_k_heads, "k", hd)) return rc;
-        if (int rc = make_token_map(&tmV, a->v, s, s.num_v_heads, "v", hd)) return rc;
-        if (int rc = make_token_map(&tmO, a->out, s, s.num_v_heads, "out", hd)) return rc;
         FusedParams p{};
         p.d = hd;
         p.map = chunk_map(s);
@@ -442,7 +448,7 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
         p.blocks = static_cast<const uint8_t*>(a->workspace);
         p.norms = norms;
         constexpr int smem = FusedSmem::kBytes;
-        if (int rc = set_smem(gdn_fused_seq_kernel, smem)) return rc;
+        if (int rc = set_smem<gdn_fused_seq_kernel>(smem)) return rc;
         const long long chains = static_cast<long long>(s.batch) * s.num_v_heads;
         const SegmentPlan plan = segment_plan_of(s);
         if (plan.num_segments <= 1 && packed && s.batch > 1 && s.batch <= kMaxOrderedSeqs && chains > d->sms) {
@@ -467,7 +473,7 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
             p.seg_mn = seg_mn;
             p.seg_start = seg_start;
             p.mode = 1;
-            if (int rc = set_smem(gdn_seg_combine_kernel, SegCombineSmem::kBytes)) return rc;
+            if (int rc = set_smem<gdn_seg_combine_kernel>(SegCombineSmem::kBytes)) return rc;
             if (int rc = run_zp()) return rc;
             GDN_CUDA(launch_fused_after_zp(dim3(plan.slots, s.num_v_heads, 2), smem, st, tmQ, tmK, tmV, tmO, p));
             SegCombineParams cp{};

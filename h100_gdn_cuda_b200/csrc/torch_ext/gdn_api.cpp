@@ -41,6 +41,7 @@ GdnTokenTensor tok(const at::Tensor& t, bool packed) {
 GdnTokenScalar sca(const std::optional<at::Tensor>& o, bool packed, int64_t tokens) {
     if (!o.has_value()) return GdnTokenScalar{nullptr, 0, 0, 0, 0};
     at::Tensor t = o.value();
+    require(t.is_cuda(), "beta, gate and the gating projections must be CUDA tensors");
     if (t.size(-2) != tokens) t = t.narrow(-2, 0, tokens);  // MN-major views carry a padded token axis
     if (packed) {
         require(t.dim() == 2, "packed beta/gate are rank 2 (tokens, heads)");
@@ -75,6 +76,7 @@ at::Tensor pad_state(const at::Tensor& t, int64_t dv, int64_t dk) {
     if (t.size(-1) == dk && t.size(-2) == dv) return t;
     return at::constant_pad_nd(t, {0, dk - t.size(-1), 0, dv - t.size(-2)}, 0);
 }
+float default_scale(int64_t d) { return static_cast<float>(1.0 / std::sqrt(static_cast<double>(d))); }
 int64_t align64(int64_t d) { return (d + 63) / 64 * 64; }
 
 GdnShape make_shape(const at::Tensor& q, const at::Tensor& v, const std::optional<at::Tensor>& cu_seqlens,
@@ -110,6 +112,18 @@ std::pair<at::Tensor, at::Tensor> chunked_forward(at::Tensor& query, at::Tensor&
                                                   std::optional<at::Tensor>& cu_chunks,
                                                   std::optional<int> total_chunks, cudaStream_t stream,
                                                   bool is_qk_norm) {
+    return chunked_forward_ext(query, key, value, beta, gate, scale, initial_state, cu_seqlens, chunk_indices, cu_chunks,
+                               total_chunks, stream, is_qk_norm, std::nullopt);
+}
+
+std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, const at::Tensor& key, const at::Tensor& value,
+                                                      const at::Tensor& beta, const std::optional<at::Tensor>& gate,
+                                                      std::optional<float> scale, const std::optional<at::Tensor>& initial_state,
+                                                      const std::optional<at::Tensor>& cu_seqlens,
+                                                      const std::optional<at::Tensor>& chunk_indices,
+                                                      const std::optional<at::Tensor>& cu_chunks,
+                                                      std::optional<int> total_chunks, cudaStream_t stream, bool is_qk_norm,
+                                                      const std::optional<at::Tensor>& workspace) {
     cuda_bf16(query, "query");
     cuda_bf16(key, "key");
     cuda_bf16(value, "value");
@@ -148,9 +162,11 @@ std::pair<at::Tensor, at::Tensor> chunked_forward(at::Tensor& query, at::Tensor&
     a.gate = sca(gate, packed, tokens);
     a.initial_state = st(s_in);
     a.final_state = st(fin);
-    a.scale = scale.value_or(1.0f / std::sqrt(static_cast<float>(d)));
+    a.scale = scale.value_or(default_scale(d));
     const size_t ws_bytes = gdn_chunked_forward_workspace_bytes(&a.shape);
-    at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, v.options().dtype(at::kByte));
+    const bool given = workspace.has_value() && workspace->is_cuda() && workspace->scalar_type() == at::kByte &&
+                       static_cast<size_t>(workspace->numel()) >= ws_bytes;
+    at::Tensor ws = given ? *workspace : at::empty({static_cast<int64_t>(ws_bytes)}, v.options().dtype(at::kByte));
     a.workspace = ws.data_ptr();
     a.workspace_bytes = ws_bytes;
     a.stage_events = nullptr;
@@ -234,6 +250,8 @@ std::pair<at::Tensor, at::Tensor> recurrent_impl(at::Tensor& query, at::Tensor& 
         require(gating->a.scalar_type() == gating->b.scalar_type() && gating->a.scalar_type() == gating->A_log.scalar_type() &&
                     gating->a.scalar_type() == gating->dt_bias.scalar_type(),
                 "A_log, dt_bias, a, b must share a dtype");
+        require(gating->a.sizes() == gating->b.sizes() && gating->A_log.is_cuda() && gating->dt_bias.is_cuda(),
+                "gating: a and b are (B,T,vh) / (N,vh); A_log and dt_bias hold one entry per v-head");
         require(gating->A_log.numel() >= vh && gating->dt_bias.numel() >= vh, "A_log and dt_bias need one entry per head");
         Ac = gating->A_log.contiguous();
         dc = gating->dt_bias.contiguous();
@@ -248,7 +266,7 @@ std::pair<at::Tensor, at::Tensor> recurrent_impl(at::Tensor& query, at::Tensor& 
     }
     a.state_in = st(s_in);
     a.num_accepted_tokens = i32(num_accepted_tokens, "num_accepted_tokens");
-    a.scale = scale.value_or(1.0f / std::sqrt(static_cast<float>(d)));
+    a.scale = scale.value_or(default_scale(d));
     a.is_qk_norm = is_qk_norm ? 1 : 0;
     a.store_step_state = store_steps ? 1 : 0;
     check(gdn_recurrent_forward(&a, stream), "recurrent_forward");
@@ -525,7 +543,7 @@ void bf16_gdn_chunked_compute_O(at::Tensor& q, at::Tensor& state, at::Tensor& k,
         at::Tensor qp = pad_last(q, D), kp = pad_last(k, D), up = pad_last(u, D);
         at::Tensor sp = pad_state(state, D, D).contiguous();
         at::Tensor op = at::empty_like(up);
-        std::optional<float> sc = scale.value_or(1.0f / std::sqrt(static_cast<float>(d)));
+        std::optional<float> sc = scale.value_or(default_scale(d));
         bf16_gdn_chunked_compute_O(qp, sp, kp, up, op, gate, sc, "t", stream, cu_seqlens, chunk_indices, cu_chunks,
                                    std::nullopt, chunk_size);
         o.copy_(op.narrow(-1, 0, d));
@@ -542,7 +560,7 @@ void bf16_gdn_chunked_compute_O(at::Tensor& q, at::Tensor& state, at::Tensor& k,
     a.out = tok(o, packed);
     a.gate_cumsum = sca(gate, packed, tokens);
     a.chunk_states = state.data_ptr();
-    a.scale = scale.value_or(1.0f / std::sqrt(static_cast<float>(q.size(-1))));
+    a.scale = scale.value_or(default_scale(q.size(-1)));
     check(gdn_compute_o(&a, stream), "bf16_gdn_chunked_compute_O");
 }
 

@@ -25,6 +25,17 @@ std::pair<at::Tensor, at::Tensor> chunked_forward(at::Tensor& query, at::Tensor&
                                                   std::optional<int> total_chunks, cudaStream_t stream,
                                                   bool is_qk_norm = false);  // last argument: extension, see gdn_b200.h
 
+// chunked_forward with the gate optional (no decay without it) and, when `workspace` is large enough, that buffer
+// instead of one allocated for the call.
+std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, const at::Tensor& key, const at::Tensor& value,
+                                                      const at::Tensor& beta, const std::optional<at::Tensor>& gate,
+                                                      std::optional<float> scale, const std::optional<at::Tensor>& initial_state,
+                                                      const std::optional<at::Tensor>& cu_seqlens,
+                                                      const std::optional<at::Tensor>& chunk_indices,
+                                                      const std::optional<at::Tensor>& cu_chunks,
+                                                      std::optional<int> total_chunks, cudaStream_t stream, bool is_qk_norm,
+                                                      const std::optional<at::Tensor>& workspace);
+
 std::pair<at::Tensor, at::Tensor> recurrent_forward(at::Tensor& query, at::Tensor& key, at::Tensor& value,
                                                     std::optional<at::Tensor>& initial_state, at::Tensor& beta,
                                                     at::Tensor& gate, std::optional<at::Tensor>& cu_seqlens,

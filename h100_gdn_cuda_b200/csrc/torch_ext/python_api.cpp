@@ -10,6 +10,8 @@
 
 namespace py = pybind11;
 
+void add_fastcall_functions(PyObject* module);  // fastcall.cpp
+
 // Every call runs on the device of its first tensor and on that device's current torch stream.
 struct OnDevice {
     c10::cuda::CUDAGuard guard;
@@ -181,4 +183,6 @@ PYBIND11_MODULE(gdn_cuda, m) {
         .value("Decode", gdn_cuda::InferenceMode::Decode)
         .value("SpecVerify", gdn_cuda::InferenceMode::SpecVerify)
         .export_values();
+
+    add_fastcall_functions(m.ptr());  // what api.py calls
 }

@@ -1,0 +1,73 @@
+"""The package's per-call functions through the C++ front end and through the ctypes bodies: same library calls, so
+the same bits (and the same refusals)."""
+import pytest
+import torch
+
+from h100_gdn_cuda_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api():
+    from h100_gdn_cuda_b200 import api, build
+    build.build()
+    build.build_ext()
+    assert api._load_ext(), "the extension is built but does not load"
+    return api
+
+
+def _cuda(p):
+    return {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+
+
+def _flat(r):
+    return [t for t in (r if isinstance(r, tuple) else (r,)) if t is not None]
+
+
+def _calls(api):
+    d = _cuda(synthetic.decode_inputs(3, 2, 2, 4, 64, seed=1))
+    p = _cuda(synthetic.prefill_inputs(2, 97, 2, 4, 60, seed=2))
+    v = _cuda(synthetic.varlen_inputs([70, 0, 5], 2, 4, 128, seed=3))
+    gating = (d["A_log"], d["dt_bias"], d["a"], d["b"])
+    slots = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
+    conv_in, conv_w = d["v"].reshape(3, 2, 256), torch.randn(256, 4, device="cuda").bfloat16()
+    beta = torch.sigmoid(d["b"].float()).bfloat16()
+    return {
+        "gating": lambda: api.fused_gdn_gating(*gating),
+        "recurrent, gating inside": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], None, None, gating=gating,
+                                                                  is_qk_norm=True, inference_mode=2),
+        "recurrent, no gate, pool": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"].clone(), beta,
+                                                                  scale=0.3, state_indices=slots),
+        "recurrent, fp32, no state": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], None, beta, d["a"].float()),
+        "prefill, padded dims": lambda: api.chunked_forward(p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"]),
+        "prefill, no gate": lambda: api.chunked_forward(p["q"], p["k"], p["v"], p["beta"], None, is_qk_norm=True),
+        "prefill, packed": lambda: api.chunked_forward(v["q"], v["k"], v["v"], v["beta"], v["g"], 0.2, v["state"], v["cu_seqlens"],
+                                                       v["chunk_indices"], v["cu_chunks"]),
+        "conv": lambda: api.causal_conv1d(conv_in, conv_w, None, None, return_final_state=True),
+        "conv, y only": lambda: api.causal_conv1d(conv_in, conv_w, activation=False),
+        "norm": lambda: api.gated_rmsnorm(d["v"], d["v"], conv_w[:64, 0].contiguous()),
+    }
+
+
+def test_both_front_ends_give_the_same_bits(api, monkeypatch):
+    for name, call in _calls(api).items():
+        fast = _flat(call())
+        with monkeypatch.context() as m:
+            m.setattr(api, "_ext", False)
+            slow = _flat(call())
+        assert len(fast) == len(slow), name
+        for a, b in zip(fast, slow):
+            assert a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype and torch.equal(a, b), name
+
+
+def test_refusals(api):
+    d = _cuda(synthetic.decode_inputs(1, 1, 1, 1, 64, seed=1))
+    with pytest.raises(RuntimeError):
+        api.recurrent_forward(d["q"], d["k"], d["v"], d["state"])          # beta missing
+    with pytest.raises(RuntimeError):
+        api.recurrent_forward(d["q"].cpu(), d["k"], d["v"], d["state"], d["b"])
+    with pytest.raises(RuntimeError):
+        api.chunked_forward(d["q"], d["k"], d["v"], d["b"].cpu(), None)
+    with pytest.raises(RuntimeError):
+        api.gated_rmsnorm(d["v"], d["q"].float(), d["q"][0, 0, 0])
