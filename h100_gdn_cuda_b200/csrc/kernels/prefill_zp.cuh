@@ -20,6 +20,11 @@
 // TF32 warp MMAs), T and (diag(d) T)^T as bf16 tiles, then three M=64 MMAs (the two 64-column
 // halves of Z, and PT) and the bf16 epilogue into a staging area that leaves by two bulk copies.
 // Persistent CTAs, two per SM (85 KB of shared memory, 256 tensor-memory columns each).
+//
+// kWide: head dims 129 .. 256 on 256 columns (one CTA per SM, 512 tensor-memory columns).  Those head dims keep the
+// arithmetic of the fp32 token recurrence they ran on before: every matrix that is not one of the caller's bf16 inputs
+// (P, T, dT, and Z, PT for the state kernel) is carried as a sum of two bf16 terms, x = hi + lo (16 significand
+// bits), products as hi.hi + hi.lo + lo.hi, and the inverse takes its TF32 products in three terms the same way.
 #pragma once
 #include <cuda.h>
 
@@ -42,16 +47,18 @@ struct ZPParams {
     int* status;
 };
 
+template <bool kWide = false>
 struct ZPSmem {
+    static constexpr int kAtoms = kWide ? 4 : 2;  // 64-column swizzle atoms of a K or Q tile
     static constexpr int kLd = 68;  // fp32 row stride of A, conflict-free for the MMA fragment loads
     // K and Q tiles interleaved atom by atom: [K cols 0-63 | Q cols 0-63 | K cols 64-127 | Q cols 64-127],
     // 8 KB each, so that rows 0-127 of one atom pair are K stacked on Q (the M=128 A operand)
     static constexpr int kOffKQ = 0;
-    static constexpr int kTeam = 32768;                  // per-team area starts here, two of them
-    static constexpr int kOffA = 0;                      // A / X fp32 (17 KB), later T | (dT)^T, later the staged Z
-    static constexpr int kOffP = 64 * kLd * 4;           // 17408: P tile (8 KB), later the staged PT
-    static constexpr int kOffVec = kOffP + 8192;         // beta[64], g log2e[64], d[64], scan partials[64], column factors[32]
-    static constexpr int kTeamBytes = kOffVec + 2048;    // 27648 (multiple of 1024)
+    static constexpr int kTeam = kAtoms * 16384;         // per-team area starts here, two of them
+    static constexpr int kOffA = 0;                      // A / X fp32 (17 KB), later T | dT (kWide: T hi, dT hi, T lo, dT lo), later the staged Z
+    static constexpr int kOffP = kWide ? 32768 : 64 * kLd * 4;  // P tile (8 KB; kWide: hi, lo), later the staged PT
+    static constexpr int kOffVec = kOffP + (kWide ? 16384 : 8192);  // beta[64], g log2e[64], d[64], scan partials[64], column factors[32]
+    static constexpr int kTeamBytes = kOffVec + 2048;    // a multiple of 1024
     static constexpr int kOffNorm = kTeam + 2 * kTeamBytes;  // kNorm: inverse row norms of K [64] and Q [64], their log2 [128]
     static constexpr int kOffBar = kOffNorm + 1024;
     static constexpr int kBytes = kOffBar + 128 + 1024;
@@ -62,7 +69,52 @@ namespace zp {
 constexpr int kThreads = 256;
 constexpr uint32_t kTmKQ = 0;    // fp32 K K^T (lanes 0-63) and Q K^T (lanes 64-127), 64 columns
 constexpr uint32_t kTmPT = 64;   // PT of team 0 (lanes +0) and team 1 (lanes +16), 64 columns
-constexpr uint32_t kTmZ = 128;   // + 64 * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16)
+constexpr uint32_t kTmZ = 128;   // + 64 (kWide: 128) * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16), kWide: 128-255 in the next 64
+// TF32 operands of the inverse's block products; kSplit: with the rounding error as a second term, and three
+// products per block (what the second terms' product would add is below fp32's own rounding)
+template <bool kSplit, int N>
+struct Frag {
+    uint32_t hi[N], lo[kSplit ? N : 1];
+    __device__ __forceinline__ void set(int i, float x) {
+        hi[i] = uw::to_tf32(x);
+        if (kSplit) lo[i] = uw::to_tf32(x - __uint_as_float(hi[i]));
+    }
+};
+template <bool kSplit>
+__device__ __forceinline__ void mma_frag(float* d, const Frag<kSplit, 4>& a, const Frag<kSplit, 2>& b) {
+    uw::mma_tf32(d, a.hi, b.hi);
+    if (kSplit) {
+        uw::mma_tf32(d, a.lo, b.hi);
+        uw::mma_tf32(d, a.hi, b.lo);
+    }
+}
+// 16x8 fragment of `m` at [r0][k0] as the A operand (kRows 8: the lower half is zero), 8x8 at [k0][n0] as the B operand
+template <bool kSplit, int kRows = 16>
+__device__ __forceinline__ void load_a(Frag<kSplit, 4>& a, const float* m, int ld, int r0, int k0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    a.set(0, m[(r0 + g) * ld + k0 + t]);
+    a.set(1, kRows == 16 ? m[(r0 + g + 8) * ld + k0 + t] : 0.f);
+    a.set(2, m[(r0 + g) * ld + k0 + t + 4]);
+    a.set(3, kRows == 16 ? m[(r0 + g + 8) * ld + k0 + t + 4] : 0.f);
+}
+template <bool kSplit>
+__device__ __forceinline__ void load_b(Frag<kSplit, 2>& b, const float* m, int ld, int k0, int n0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    b.set(0, m[(k0 + t) * ld + n0 + g]);
+    b.set(1, m[(k0 + t + 4) * ld + n0 + g]);
+}
+template <bool kSplit, int kRows = 16>
+__device__ __forceinline__ void mma_blk(float* d, const float* am, int r0, int k0, const float* bm, int k0b, int n0, int ld, int lane) {
+    Frag<kSplit, 4> a;
+    Frag<kSplit, 2> b;
+    load_a<kSplit, kRows>(a, am, ld, r0, k0, lane);
+    load_b<kSplit>(b, bm, ld, k0b, n0, lane);
+    mma_frag<kSplit>(d, a, b);
+}
+// two bf16 terms of a pair: hi = bf16(x), lo = bf16(x - hi)
+__device__ __forceinline__ uint32_t pack_lo(float a, float b, uint32_t hi) {
+    return ptx::pack_bf16(a - ptx::bf16_lo(hi), b - ptx::bf16_hi(hi));
+}
 __device__ __forceinline__ void team_sync(int team) {
     if (team)
         asm volatile("bar.sync 2, 128;" ::: "memory");
@@ -75,15 +127,15 @@ __device__ __forceinline__ void team_sync(int team) {
 // (k_i.k_j) r_i r_j and (q_i.k_j) rq_i r_j enter through the row factor of the A / P pass and through
 // the column's gate (g_j - log2 r_j in the exponent), Z = (dT)^T diag(r) K through d_i r_i.  The
 // factors are also written to `norms` for the state kernel.
-template <bool kNorm>
-__global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_constant__ CUtensorMap tmK,
+template <bool kNorm, bool kWide = false>
+__global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                  const __grid_constant__ CUtensorMap tmQ,
                                                                  const ZPParams p) {
     using namespace ptx;
     using namespace uw;
     using namespace zp;
-    using L = ZPSmem;
-    constexpr int LD = L::kLd;
+    using L = ZPSmem<kWide>;
+    constexpr int LD = L::kLd, NA = L::kAtoms;
     extern __shared__ uint8_t smem_raw[];
     // aligned by an offset from the array itself, so that the compiler still knows the pointer is shared memory
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -118,7 +170,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
         mbar_init(&bar_mma[1], 1);
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(tmem_slot, 256);
+    if (warp == 0) tmem_alloc(tmem_slot, kWide ? 512 : 256);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -168,8 +220,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
         return u;
     };
     auto issue_loads = [&](const UnitPos& u) {  // one thread
-        mbar_arrive_expect_tx(bar_load, 4 * 8192);
-        for (int a = 0; a < 2; ++a) {
+        mbar_arrive_expect_tx(bar_load, NA * 16384);
+        for (int a = 0; a < NA; ++a) {
             tma_load_4d(sKQ + a * 16384, &tmK, bar_load, a * 64, u.khead, static_cast<int>(u.cp.tok0), u.cp.batch);
             tma_load_4d(sKQ + a * 16384 + 8192, &tmQ, bar_load, a * 64, u.khead, static_cast<int>(u.cp.tok0), u.cp.batch);
         }
@@ -235,13 +287,13 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             if (rd == 0) {
                 mbar_wait(bar_load, it & 1u, abort_flag);
                 if (kNorm) {
-                    // inverse L2 norm of every row of the stacked K | Q tile: two threads per row, 64 columns each
+                    // inverse L2 norm of every row of the stacked K | Q tile: two threads per row, half the columns each
                     const int r = tid >> 1, hf = tid & 1;
-                    const uint8_t* rowp = sKQ + hf * 16384 + (r >> 6) * 8192 + (r & 63) * 128;
+                    const uint8_t* rowp = sKQ + hf * (NA / 2) * 16384 + (r >> 6) * 8192 + (r & 63) * 128;
                     float ss = 0.f;
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 w = *reinterpret_cast<const uint4*>(rowp + 16 * c);
+                    for (int c = 0; c < 4 * NA; ++c) {
+                        const uint4 w = *reinterpret_cast<const uint4*>(rowp + (c >> 3) * 16384 + 16 * (c & 7));
                         const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
@@ -264,7 +316,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     constexpr uint32_t idesc = make_idesc_bf16(128, 64, false, false);
                     const uint64_t dkq = make_smem_desc_sw128(smem_u32(sKQ), 0, 1024);  // A: 128 rows, B: its first 64
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
+                    for (int ks = 0; ks < 4 * NA; ++ks) {
                         const uint32_t off = kmajor_step(ks, 16384);
                         if (ks == 0)
                             mma_ss_w<false>(tmem + kTmKQ, desc_advance(dkq, off), desc_advance(dkq, off), idesc);
@@ -343,9 +395,13 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                                     *reinterpret_cast<float4*>(&sA[i * LD + 32 * cb + j]) = make_float4(o[0], o[1], o[2], o[3]);
                                     *reinterpret_cast<float4*>(&sA[i * LD + 32 * cb + j + 4]) = make_float4(o[4], o[5], o[6], o[7]);
                                 } else {
-                                    *reinterpret_cast<uint4*>(sP + tile_off(i, (32 * cb + j) >> 3)) =
-                                        make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]),
-                                                   pack_bf16(o[6], o[7]));
+                                    const uint4 h = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]),
+                                                               pack_bf16(o[6], o[7]));
+                                    *reinterpret_cast<uint4*>(sP + tile_off(i, (32 * cb + j) >> 3)) = h;
+                                    if (kWide)
+                                        *reinterpret_cast<uint4*>(sP + 8192 + tile_off(i, (32 * cb + j) >> 3)) =
+                                            make_uint4(pack_lo(o[0], o[1], h.x), pack_lo(o[2], o[3], h.y), pack_lo(o[4], o[5], h.z),
+                                                       pack_lo(o[6], o[7], h.w));
                                 }
                             }
                         };
@@ -360,8 +416,10 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     }
                     if (is_p && rb == 0) {  // rows 0-31 of P: columns 32-63 lie above the diagonal
 #pragma unroll
-                        for (int c16 = 4; c16 < 8; ++c16)
+                        for (int c16 = 4; c16 < 8; ++c16) {
                             *reinterpret_cast<uint4*>(sP + tile_off(i, c16)) = make_uint4(0u, 0u, 0u, 0u);
+                            if (kWide) *reinterpret_cast<uint4*>(sP + 8192 + tile_off(i, c16)) = make_uint4(0u, 0u, 0u, 0u);
+                        }
                     }
                 }
                 if (rd + 1 < rounds) {
@@ -404,17 +462,20 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     // level 0 (8 -> 16)
                     const int i0 = 16 * b + 8, j0 = 16 * b;
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_block8(d, sA, LD, i0, j0, sA, LD, j0, j0, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
+                    mma_blk<kWide, 8>(d, sA, i0, j0, sA, j0, j0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
                     // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
                     const int g = lane >> 2, tq = lane & 3;
                     const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
                     const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
                     const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
                     const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
-                    uint32_t bfrag[2] = {to_tf32((g & 1) ? v01 : v00), to_tf32((g & 1) ? v11 : v10)};
-                    uint32_t afrag[4] = {to_tf32(sA[(i0 + g) * LD + i0 + tq]), 0u, to_tf32(sA[(i0 + g) * LD + i0 + tq + 4]), 0u};
+                    Frag<kWide, 2> bfrag;
+                    bfrag.set(0, (g & 1) ? v01 : v00);
+                    bfrag.set(1, (g & 1) ? v11 : v10);
+                    Frag<kWide, 4> afrag;
+                    load_a<kWide, 8>(afrag, sA, LD, i0, i0, lane);
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_tf32(e, afrag, bfrag);  // X_11 t
+                    mma_frag<kWide>(e, afrag, bfrag);  // X_11 t
                     *reinterpret_cast<float2*>(&sA[(i0 + g) * LD + j0 + 2 * tq]) = make_float2(-e[0], -e[1]);
                 }
                 team_sync(team);
@@ -425,12 +486,12 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     const int i0 = 16 * (2 * pr + 1), j0 = 16 * (2 * pr);
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_block(d, sA, LD, i0, j0 + 8 * ks, sA, LD, j0 + 8 * ks, j0 + n0, lane);
+                    for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(d, sA, i0, j0 + 8 * ks, sA, j0 + 8 * ks, j0 + n0, LD, lane);
                     store_block(d, 1.f, sA, LD, j0, i0 + n0, lane);
                     team_sync(team);
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_block(e, sA, LD, i0, i0 + 8 * ks, sA, LD, j0 + 8 * ks, i0 + n0, lane);
+                    for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
                     store_block(e, -1.f, sA, LD, i0, j0 + n0, lane);
                 }
                 team_sync(team);
@@ -442,12 +503,13 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         if (ks >= 2 * cb) {
-                            uint32_t af[4], bf[2];
-                            load_afrag(af, sA, LD, 32 + 16 * rb, 8 * ks, lane);  // shared by the two column tiles
+                            Frag<kWide, 4> af;
+                            Frag<kWide, 2> bf;
+                            load_a<kWide>(af, sA, LD, 32 + 16 * rb, 8 * ks, lane);  // shared by the two column tiles
 #pragma unroll
                             for (int nt = 0; nt < 2; ++nt) {
-                                load_bfrag(bf, sA, LD, 8 * ks, 16 * cb + 8 * nt, lane);
-                                mma_tf32(d[nt], af, bf);
+                                load_b<kWide>(bf, sA, LD, 8 * ks, 16 * cb + 8 * nt, lane);
+                                mma_frag<kWide>(d[nt], af, bf);
                             }
                         }
                     }
@@ -458,12 +520,13 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         if (ks < 2 * (rb + 1)) {
-                            uint32_t af[4], bf[2];
-                            load_afrag(af, sA, LD, 32 + 16 * rb, 32 + 8 * ks, lane);
+                            Frag<kWide, 4> af;
+                            Frag<kWide, 2> bf;
+                            load_a<kWide>(af, sA, LD, 32 + 16 * rb, 32 + 8 * ks, lane);
 #pragma unroll
                             for (int nt = 0; nt < 2; ++nt) {
-                                load_bfrag(bf, sA, LD, 8 * ks, 32 + 16 * cb + 8 * nt, lane);
-                                mma_tf32(e[nt], af, bf);
+                                load_b<kWide>(bf, sA, LD, 8 * ks, 32 + 16 * cb + 8 * nt, lane);
+                                mma_frag<kWide>(e[nt], af, bf);
                             }
                         }
                     }
@@ -498,10 +561,16 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                         unpk(mul2(t0, di2), w[0], w[1]); unpk(mul2(t1, di2), w[2], w[3]);
                         unpk(mul2(t2, di2), w[4], w[5]); unpk(mul2(t3, di2), w[6], w[7]);
                         const uint32_t off = sw128_offset(i, c0 + 8 * ch);
-                        *reinterpret_cast<uint4*>(sT + off) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]),
-                                                                         pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-                        *reinterpret_cast<uint4*>(sTd + off) = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]),
-                                                                          pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
+                        const uint4 hv = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                        const uint4 hw = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
+                        *reinterpret_cast<uint4*>(sT + off) = hv;
+                        *reinterpret_cast<uint4*>(sTd + off) = hw;
+                        if (kWide) {
+                            *reinterpret_cast<uint4*>(sT + 16384 + off) = make_uint4(pack_lo(v[0], v[1], hv.x), pack_lo(v[2], v[3], hv.y),
+                                                                                     pack_lo(v[4], v[5], hv.z), pack_lo(v[6], v[7], hv.w));
+                            *reinterpret_cast<uint4*>(sTd + 16384 + off) = make_uint4(pack_lo(w[0], w[1], hw.x), pack_lo(w[2], w[3], hw.y),
+                                                                                      pack_lo(w[4], w[5], hw.z), pack_lo(w[6], w[7], hw.w));
+                        }
                     }
                 }
                 fence_proxy_async_smem();
@@ -514,20 +583,32 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     const uint64_t dTd = make_smem_desc_sw128(smem_u32(sTd), 8192, 1024);       // A, read MN-major
                     const uint64_t dPa = make_smem_desc_sw128(smem_u32(sP), 0, 1024);           // A, K-major
                     const uint64_t dTb = make_smem_desc_sw128(smem_u32(sT), 8192, 1024);        // B, read MN-major
-                    const uint64_t dK0 = make_smem_desc_sw128(smem_u32(sKQ), 8192, 1024);       // B, K columns 0-63, MN-major
-                    const uint64_t dK1 = make_smem_desc_sw128(smem_u32(sKQ + 16384), 8192, 1024);
-                    const uint32_t tZ = tmem + kTmZ + 64u * team;
+                    const uint64_t dK = make_smem_desc_sw128(smem_u32(sKQ), 8192, 1024);        // B, K columns 0-63, MN-major
+                    const uint32_t tZ = tmem + kTmZ + (NA * 32u) * team;
                     const uint32_t tPT = tmem + kTmPT + (team ? (16u << 16) : 0u);
-                    mma_ss_w<false>(tZ, dTd, dK0, idescz);
 #pragma unroll
-                    for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tZ, desc_advance(dTd, ks * 2048), desc_advance(dK0, ks * 2048), idescz);
-                    mma_ss_w<false>(tZ + (16u << 16), dTd, dK1, idescz);
+                    for (int a = 0; a < NA; ++a) {  // 64 columns of Z each
+                        const uint32_t tz = tZ + (a >> 1) * 64u + ((a & 1) ? (16u << 16) : 0u);
+                        const uint64_t dk = desc_advance(dK, a * 16384);
+                        mma_ss_w<false>(tz, dTd, dk, idescz);
 #pragma unroll
-                    for (int ks = 1; ks < 4; ++ks)
-                        mma_ss_w<true>(tZ + (16u << 16), desc_advance(dTd, ks * 2048), desc_advance(dK1, ks * 2048), idescz);
+                        for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tz, desc_advance(dTd, ks * 2048), desc_advance(dk, ks * 2048), idescz);
+                        if (kWide) {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                mma_ss_w<true>(tz, desc_advance(dTd, 16384 + ks * 2048), desc_advance(dk, ks * 2048), idescz);
+                        }
+                    }
                     mma_ss_w<false>(tPT, dPa, dTb, idesc);
 #pragma unroll
                     for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tPT, desc_advance(dPa, ks * 32), desc_advance(dTb, ks * 2048), idesc);
+                    if (kWide) {
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks) {
+                            mma_ss_w<true>(tPT, desc_advance(dPa, 8192 + ks * 32), desc_advance(dTb, ks * 2048), idesc);
+                            mma_ss_w<true>(tPT, desc_advance(dPa, ks * 32), desc_advance(dTb, 16384 + ks * 2048), idesc);
+                        }
+                    }
                     mma_commit_w(&bar_mma[team]);
                 }
                 __syncwarp();
@@ -545,10 +626,44 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 }
             }
             if (active) {
-                // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> two bulk copies
-                uint8_t* stZ = tbase + L::kOffA;
                 const int row = 16 * tw + (lane & 15), hi = lane >> 4;
                 const uint32_t tl = static_cast<uint32_t>(32 * tw) << 16;
+                if constexpr (kWide) {
+                    // ---- accumulators -> two bf16 terms -> the unit's block, written where they belong (the four Z and
+                    //      two PT tiles of both teams would not fit beside K and Q, and this kernel is a small part of a wide call)
+                    uint8_t* dst = p.blocks + (static_cast<size_t>(chunk) * p.vh + head) * kWideBlockBytes;
+                    const bool healthy = *abort_flag == 0;
+                    auto emit = [&](const uint32_t* r, uint8_t* hi_tile, uint8_t* lo_tile, int c16) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            float f[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * q + e]);
+                            const uint4 h = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+                            *reinterpret_cast<uint4*>(hi_tile + tile_off(row, c16 + q)) = h;
+                            *reinterpret_cast<uint4*>(lo_tile + tile_off(row, c16 + q)) = make_uint4(
+                                pack_lo(f[0], f[1], h.x), pack_lo(f[2], f[3], h.y), pack_lo(f[4], f[5], h.z), pack_lo(f[6], f[7], h.w));
+                        }
+                    };
+#pragma unroll
+                    for (int cb = 0; cb < 4; ++cb) {  // 32 columns of every 64; lanes +16 hold the odd atoms
+                        uint32_t r[32];
+                        tmem_ld32(tmem + kTmZ + 128u * team + tl + 32 * cb, r);
+                        tmem_wait_ld();
+                        if (healthy) emit(r, dst, dst + 32768, 16 * (cb >> 1) + 8 * hi + 4 * (cb & 1));
+                    }
+#pragma unroll
+                    for (int cb = 0; cb < 2; ++cb) {
+                        uint32_t r[32];
+                        tmem_ld32(tmem + kTmPT + tl + 32 * cb, r);
+                        tmem_wait_ld();
+                        if (hi == team && healthy) emit(r, dst + 65536, dst + 65536 + 8192, 4 * cb);
+                    }
+                    tc_fence_before_sync();
+                    team_sync(team);  // T, dT and P are free for the next round
+                } else {
+                // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> two bulk copies
+                uint8_t* stZ = tbase + L::kOffA;
 #pragma unroll
                 for (int cb = 0; cb < 2; ++cb) {
                     uint32_t r[32];
@@ -589,13 +704,14 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     bulk_commit();
                 }
                 stores_pending = true;
+                }
             }
         }  // head pairs
     }      // units
     if (stores_pending && tt == 0) bulk_wait_read<0>();
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 256);
+    if (warp == 0) tmem_dealloc(tmem, kWide ? 512 : 256);
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 2);
 }
 
