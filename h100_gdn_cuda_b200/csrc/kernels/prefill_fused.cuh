@@ -232,11 +232,14 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         const int lq = warp & 3, hf = warp >> 2;
         const int row = 32 * lq + lane;
         const uint32_t tm_lane = static_cast<uint32_t>(32 * lq) << 16;
-        // element (token i, this row) of a swizzled 64 x 128 tile: i * 128 + uoff8[i & 7]
-        uint32_t uoff8[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            uoff8[k] = static_cast<uint32_t>((row >> 6) * 8192 + ((((row & 63) >> 3) ^ k) << 4) + (row & 7) * 2);
+        // R is handled in warp-MMA fragments (tmem_ld_frag32): 16 rows at a time, two tokens per register pair.  Then V^T comes
+        // by transposing matrix loads: lane 8m + r addresses token r of block m (8 rows x 8 tokens), block m = rows 8 (m & 1) ..
+        // of the 16, tokens 8 (m >> 1) .. of 16.  (Row-per-lane accesses took 32 two-byte loads and 16 packs per thread; the
+        // chain's passes and the epilogue share the schedulers and are bound by their instructions.)
+        const uint32_t vlane = static_cast<uint32_t>((lq >> 1) * 8192 + (32 * hf + 8 * (lane >> 4) + (lane & 7)) * 128);
+        const uint32_t vchunk = static_cast<uint32_t>(4 * (lq & 1) + ((lane >> 3) & 1));  // 16-byte piece of the first 16 rows
+        const uint32_t vsw0 = vlane + ((vchunk ^ (lane & 7)) << 4), vsw1 = vlane + (((vchunk + 2) ^ (lane & 7)) << 4);
+        const int t0 = 32 * hf + 2 * (lane & 3);  // first token of this lane's first pair; the others are 8 further on each
         float S[64];
         if (p.mode == 2) {
             grid_dep_wait();  // the start states come from the kernel launched just before this one
@@ -286,18 +289,21 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             const float* gb = gate_buf(c);
             mbar_wait(&bar_full[c & 1], static_cast<uint32_t>((c >> 1) & 1), abort_flag);  // gate values visible
             // ---- R = V^T - e^g .* (S K^T) -> bf16 operand copy in tensor memory
-            // This thread's 32 values of V^T come straight from the TMA tile (element (token, row)
-            // of the swizzled layout), packed two tokens per register while the MMA is running.
-            const uint8_t* sV = smem + (c & 1) * L::kStage + L::kOffV;
-            uint32_t vpk[16];
+            // This thread's values of V^T are fetched from the TMA tile while the MMA is running.
+            const uint32_t sV = smem_u32(smem + (c & 1) * L::kStage + L::kOffV);
+            uint32_t vpk[2][2][4];  // [16-row half][16 tokens][block]
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const int i0 = 32 * hf + 2 * e;
-                const uint32_t lo = *reinterpret_cast<const uint16_t*>(sV + i0 * 128 + uoff8[i0 & 7]);
-                const uint32_t hi = *reinterpret_cast<const uint16_t*>(sV + (i0 + 1) * 128 + uoff8[(i0 + 1) & 7]);
-                vpk[e] = zero_u ? 0u : (lo | (hi << 16));
+            for (int j = 0; j < 2; ++j) {
+                ldmatrix_x4_trans(sV + vsw0 + 2048 * j, vpk[0][j]);
+                ldmatrix_x4_trans(sV + vsw1 + 2048 * j, vpk[1][j]);
             }
-            const int nloc = n - 32 * hf;  // tokens of this half that exist
+            if (zero_u) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) vpk[j >> 3][(j >> 2) & 1][j & 3] = 0u;
+            }
+            f2 neg[4];  // -e^{g} of this lane's token pairs
+#pragma unroll
+            for (int i = 0; i < 4; ++i) neg[i] = *reinterpret_cast<const f2*>(gb + 64 + t0 + 8 * i);
             // The state warps now idle until D1 arrives: the window in which the output warps (which
             // share the schedulers) run the previous chunk's epilogue without slowing the chain down.
             __syncwarp();
@@ -305,31 +311,42 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             mbar_wait(bar_d1, par, abort_flag);
             tc_fence_after_sync();
             {
-                uint32_t r[32];
-                tmem_ld32(tmem + kTmD1 + tm_lane + 32 * hf, r);  // S K^T
-                float neg[32];                                    // -e^{g} of this half's tokens
-#pragma unroll
-                for (int e4 = 0; e4 < 8; ++e4) {
-                    const float4 t = *reinterpret_cast<const float4*>(gb + 64 + 32 * hf + 4 * e4);
-                    neg[4 * e4] = t.x; neg[4 * e4 + 1] = t.y; neg[4 * e4 + 2] = t.z; neg[4 * e4 + 3] = t.w;
-                }
+                uint32_t r[2][16];  // S K^T, 16 rows each
+                tmem_ld_frag32(tmem + kTmD1 + tm_lane + 32 * hf, r[0]);
+                tmem_ld_frag32(tmem + kTmD1 + tm_lane + (16u << 16) + 32 * hf, r[1]);
                 tmem_wait_ld();
-                uint32_t wa[16];
+                uint32_t wa[2][8];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    float r0, r1;
-                    unpk(fma2(pk(neg[2 * e], neg[2 * e + 1]), pk(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])),
-                              pk(bf16_lo(vpk[e]), bf16_hi(vpk[e]))),
-                         r0, r1);
-                    // rows past the end of a sequence meet zero rows of Z and zero columns of PT; they are
-                    // cleared all the same so that no stray Inf/NaN of a neighbouring sequence can enter
-                    if (nloc < 32) {
-                        if (2 * e >= nloc) r0 = 0.f;
-                        if (2 * e + 1 >= nloc) r1 = 0.f;
+                for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {  // 8 tokens
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {  // rows l/4 and l/4 + 8 of the 16
+                            const uint32_t v = vpk[h][i >> 1][2 * (i & 1) + a];
+                            float r0, r1;
+                            unpk(fma2(neg[i], pk(__uint_as_float(r[h][4 * i + 2 * a]), __uint_as_float(r[h][4 * i + 2 * a + 1])),
+                                      pk(bf16_lo(v), bf16_hi(v))),
+                                 r0, r1);
+                            wa[h][2 * i + a] = pack_bf16(r0, r1);
+                        }
                     }
-                    wa[e] = pack_bf16(r0, r1);
                 }
-                tmem_st16(tmem + kTmR + tm_lane + 16 * hf, wa);
+                // rows past the end of a sequence meet zero rows of Z and zero columns of PT; they are cleared all the same
+                // so that no stray Inf/NaN of a neighbouring sequence can enter.  (One branch for all of them: a branch per
+                // element was two thirds of this pass.)
+                if (n < kChunk) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t keep = (t0 + 8 * i < n ? 0xFFFFu : 0u) | (t0 + 8 * i + 1 < n ? 0xFFFF0000u : 0u);
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {
+                            wa[0][2 * i + a] &= keep;
+                            wa[1][2 * i + a] &= keep;
+                        }
+                    }
+                }
+                tmem_st_frag16(tmem + kTmR + tm_lane + 16 * hf, wa[0]);
+                tmem_st_frag16(tmem + kTmR + tm_lane + (16u << 16) + 16 * hf, wa[1]);
             }
             tmem_wait_st();
             tc_fence_before_sync();
@@ -392,14 +409,12 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // =============================================================== output warps
         reg_dec<88>();
         const int lq = warp & 3;
-        const int row = 32 * lq + lane;  // dv index = TMEM lane
         const int otid = tid - 256;
         const uint32_t tm_lane = static_cast<uint32_t>(32 * lq) << 16;
-        // element (token i, dv row) of the swizzled staging tile: i * 128 + off8[i & 7]
-        uint32_t off8[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            off8[k] = static_cast<uint32_t>((row >> 6) * 8192 + ((((row & 63) >> 3) ^ k) << 4) + (row & 7) * 2);
+        // fragments again: transposing matrix stores into the swizzled staging tile, lane 8m + r addressing token r of block m
+        const uint32_t olane = static_cast<uint32_t>((lq >> 1) * 8192 + (8 * (lane >> 4) + (lane & 7)) * 128);
+        const uint32_t ochunk = static_cast<uint32_t>(4 * (lq & 1) + ((lane >> 3) & 1));
+        const uint32_t osw0 = olane + ((ochunk ^ (lane & 7)) << 4), osw1 = olane + (((ochunk + 2) ^ (lane & 7)) << 4);
         const bool packed = p.map.cu_seqlens != nullptr;
         for (int c = 0; c < (emit_o ? nchunks : 0); ++c) {
             const uint32_t par = static_cast<uint32_t>(c & 1);
@@ -412,30 +427,35 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             mbar_wait_relaxed<100>(bar_o, par, abort_flag);
             mbar_wait_relaxed<50>(bar_go, static_cast<uint32_t>((c + 1) & 1), abort_flag);
             tc_fence_after_sync();
+            const uint32_t sOa = smem_u32(sO);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                uint32_t r1[16], r2[16];
-                tmem_ld16(tO1 + 16 * b, r1);
-                tmem_ld16(tO2 + 16 * b, r2);
-                // the gate factors of this batch are read before any store to the staging tile, so
-                // that the loads do not queue up behind the stores they might alias
-                float gv[16];
+            for (int b = 0; b < 2; ++b) {  // 32 tokens
+                f2 gv[4];
 #pragma unroll
-                for (int e4 = 0; e4 < 4; ++e4) {
-                    const float4 t = *reinterpret_cast<const float4*>(gb + 16 * b + 4 * e4);
-                    gv[4 * e4] = t.x; gv[4 * e4 + 1] = t.y; gv[4 * e4 + 2] = t.z; gv[4 * e4 + 3] = t.w;
-                }
-                tmem_wait_ld();
-                if (b == 3) {
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_ofree);  // accumulators consumed
-                }
+                for (int i = 0; i < 4; ++i) gv[i] = *reinterpret_cast<const f2*>(gb + 32 * b + 8 * i + 2 * (lane & 3));
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const int i = 16 * b + e;
-                    const float o = fmaf(gv[e], __uint_as_float(r1[e]), __uint_as_float(r2[e]));
-                    *reinterpret_cast<__nv_bfloat16*>(sO + i * 128 + off8[i & 7]) = __float2bfloat16(o);
+                for (int h = 0; h < 2; ++h) {  // 16 rows
+                    uint32_t r1[16], r2[16], w[8];
+                    const uint32_t at = (static_cast<uint32_t>(16 * h) << 16) + 32 * b;
+                    tmem_ld_frag32(tO1 + at, r1);
+                    tmem_ld_frag32(tO2 + at, r2);
+                    tmem_wait_ld();
+                    if (b == 1 && h == 1) {
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_ofree);  // accumulators consumed
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        float o0, o1;
+                        unpk(fma2(gv[i >> 1], pk(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1])),
+                                  pk(__uint_as_float(r2[2 * i]), __uint_as_float(r2[2 * i + 1]))),
+                             o0, o1);
+                        w[i] = pack_bf16(o0, o1);
+                    }
+                    const uint32_t so = sOa + (h ? osw1 : osw0) + 4096 * b;
+                    stmatrix_x4_trans(so, w[0], w[1], w[2], w[3]);
+                    stmatrix_x4_trans(so + 2048, w[4], w[5], w[6], w[7]);
                 }
             }
             const long long tok0 = seq_tok0 + static_cast<long long>(c) * kChunk;
