@@ -3,6 +3,7 @@
 // allocate outputs / workspace with torch, fill the C structs, call, throw on a non-zero status.
 #include "gdn_api.hpp"
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/constant_pad_nd.h>
 #include <gdn_b200.h>
 
@@ -14,16 +15,25 @@ namespace {
 
 constexpr int64_t kPrefillDim = 128;  // head dimension the tensor-core prefill kernels are built for
 
-void require(bool cond, const std::string& msg) {
+// Messages are put together only when they are needed: a call makes some thirty of these checks.
+void require(bool cond, const char* msg) {
     if (!cond) throw std::runtime_error(msg);
+}
+void require(bool cond, const char* name, const char* msg) {
+    if (!cond) throw std::runtime_error(std::string(name) + msg);
 }
 void check(int rc, const char* what) {
     if (rc != GDN_OK) throw std::runtime_error(std::string(what) + " failed: " + gdn_last_error());
 }
 void cuda_bf16(const at::Tensor& t, const char* name) {
-    require(t.is_cuda(), std::string(name) + " must be a CUDA tensor");
-    require(t.scalar_type() == at::kBFloat16, std::string(name) + " must be bf16");
+    require(t.is_cuda(), name, " must be a CUDA tensor");
+    require(t.scalar_type() == at::kBFloat16, name, " must be bf16");
 }
+// Uninitialised CUDA tensors without the dispatcher.
+at::Tensor empty(at::IntArrayRef sizes, const at::Tensor& like, at::ScalarType dtype) {
+    return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
+}
+at::Tensor empty_shaped_like(const at::Tensor& t) { return t.is_contiguous() ? empty(t.sizes(), t, t.scalar_type()) : at::empty_like(t); }
 int dtype_tag(const at::Tensor& t) {
     if (t.scalar_type() == at::kBFloat16) return GDN_BF16;
     if (t.scalar_type() == at::kFloat) return GDN_F32;
@@ -59,7 +69,7 @@ GdnState st(const std::optional<at::Tensor>& o) {
 const int32_t* i32(const std::optional<at::Tensor>& o, const char* name) {
     if (!o.has_value()) return nullptr;
     require(o->is_cuda() && o->scalar_type() == at::kInt && o->is_contiguous(),
-            std::string(name) + " must be a contiguous int32 CUDA tensor");
+            name, " must be a contiguous int32 CUDA tensor");
     return o->data_ptr<int32_t>();
 }
 // The prefill kernels read token tensors through TMA: 16-byte aligned base, contiguous head dim, every other
@@ -150,8 +160,8 @@ std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, c
     }
     GdnChunkedArgs a{};
     a.shape = make_shape(q, v, cu_seqlens, chunk_indices, cu_chunks, tc);
-    at::Tensor out = at::empty_like(v);
-    at::Tensor fin = at::empty({a.shape.batch, v.size(-2), D, D}, v.options());
+    at::Tensor out = empty_shaped_like(v);
+    at::Tensor fin = empty({a.shape.batch, v.size(-2), D, D}, v, at::kBFloat16);
     const int64_t tokens = packed ? q.size(0) : q.size(1);
     a.q = tok(q, packed);
     a.k = tok(k, packed);
@@ -165,7 +175,7 @@ std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, c
     const size_t ws_bytes = gdn_chunked_forward_workspace_bytes(&a.shape);
     const bool given = workspace.has_value() && workspace->is_cuda() && workspace->scalar_type() == at::kByte &&
                        static_cast<size_t>(workspace->numel()) >= ws_bytes;
-    at::Tensor ws = given ? *workspace : at::empty({static_cast<int64_t>(ws_bytes)}, v.options().dtype(at::kByte));
+    at::Tensor ws = given ? *workspace : empty({static_cast<int64_t>(ws_bytes)}, v, at::kByte);
     a.workspace = ws.data_ptr();
     a.workspace_bytes = ws_bytes;
     a.stage_events = nullptr;
@@ -203,12 +213,12 @@ std::pair<at::Tensor, at::Tensor> recurrent_impl(at::Tensor& query, at::Tensor& 
     // lies when the caller asks for that or passes a pool of states with one slot index per sequence
     const bool in_place = ext.inplace_state || ext.state_indices.has_value();
     std::optional<at::Tensor> s_in;
-    auto state_opts = v.options();
+    at::ScalarType state_type = at::kBFloat16;
     if (initial_state.has_value()) {
         const at::Tensor& s0 = *initial_state;
         require(s0.is_cuda() && (s0.scalar_type() == at::kBFloat16 || s0.scalar_type() == at::kFloat),
                 "initial_state must be a bf16 or fp32 CUDA tensor");
-        state_opts = s0.options();
+        state_type = s0.scalar_type();
         at::Tensor t = pad_state(s0, dv_al, d_al);
         if (!(t.stride(-1) == 1 && t.stride(-2) == d_al)) t = t.contiguous();
         // a padded or compacted copy would never reach the caller's tensor
@@ -219,22 +229,22 @@ std::pair<at::Tensor, at::Tensor> recurrent_impl(at::Tensor& query, at::Tensor& 
     GdnRecurrentArgs a{};
     a.shape = make_shape(q, v, cu_seqlens, std::nullopt, std::nullopt, 0);
     const int64_t vh = v.size(-2);
-    at::Tensor out = at::empty_like(v);
+    at::Tensor out = empty_shaped_like(v);
     at::Tensor s_out;
     if (store_steps) {
         require(!ext.state_indices.has_value(), "state_indices cannot be combined with per-token states");
-        s_out = packed ? at::empty({q.size(0), vh, dv_al, d_al}, state_opts)
-                       : at::empty({q.size(0), q.size(1), vh, dv_al, d_al}, state_opts);
+        s_out = packed ? empty({q.size(0), vh, dv_al, d_al}, v, state_type)
+                       : empty({q.size(0), q.size(1), vh, dv_al, d_al}, v, state_type);
         a.state_out = GdnState{s_out.data_ptr(), vh * dv_al * d_al, dv_al * d_al};
     } else if (in_place) {
         require(s_in.has_value(), "inplace_state / state_indices need an initial_state");
         s_out = *s_in;
         a.state_out = st(s_out);
     } else {
-        s_out = at::empty({a.shape.batch, vh, dv_al, d_al}, state_opts);
+        s_out = empty({a.shape.batch, vh, dv_al, d_al}, v, state_type);
         a.state_out = st(s_out);
     }
-    a.state_dtype = state_opts.dtype() == at::kFloat ? GDN_F32 : GDN_BF16;
+    a.state_dtype = state_type == at::kFloat ? GDN_F32 : GDN_BF16;
     if (ext.state_indices.has_value()) {
         require(ext.state_indices->numel() == a.shape.batch, "state_indices needs one entry per sequence");
         a.state_indices = i32(ext.state_indices, "state_indices");
@@ -327,7 +337,7 @@ std::pair<at::Tensor, std::optional<at::Tensor>> causal_conv1d(at::Tensor& x, at
     const int64_t C = weight.size(0), W = weight.size(1);
     require(packed ? x.dim() == 2 : x.dim() == 3, packed ? "packed input is (tokens, channels)" : "padded input is (batch, tokens, channels)");
     const int64_t batch = packed ? cu_seqlens->numel() - 1 : x.size(0);
-    at::Tensor y = at::empty(x.sizes(), x.options());
+    at::Tensor y = empty(x.sizes(), x, at::kBFloat16);
     at::Tensor w = weight.contiguous(), b, s_in;
     if (bias.has_value()) {
         cuda_bf16(*bias, "bias");
@@ -341,7 +351,7 @@ std::pair<at::Tensor, std::optional<at::Tensor>> causal_conv1d(at::Tensor& x, at
         s_in = initial_state->contiguous();
     }
     std::optional<at::Tensor> s_out = final_state;
-    if (!s_out.has_value() && return_final_state) s_out = at::empty({batch, W - 1, C}, x.options());
+    if (!s_out.has_value() && return_final_state) s_out = empty({batch, W - 1, C}, x, at::kBFloat16);
     if (s_out.has_value())
         require(s_out->is_contiguous() && s_out->dim() == 3 && s_out->size(0) == batch && s_out->size(1) == W - 1 &&
                     s_out->size(2) == C && s_out->scalar_type() == at::kBFloat16,
@@ -375,12 +385,12 @@ at::Tensor gated_rmsnorm(at::Tensor& x, at::Tensor& z, at::Tensor& weight, float
     require(x.sizes() == z.sizes() && x.size(-1) == weight.numel(),
             "x and z must have the same shape, weight one entry per column");
     const int64_t D = x.size(-1);
-    at::Tensor x2 = x.contiguous().view({-1, D}), z2 = z.contiguous().view({-1, D}), w = weight.contiguous();
-    at::Tensor y = at::empty(x2.sizes(), x.options());
-    check(gdn_gated_rmsnorm(x2.data_ptr(), z2.data_ptr(), y.data_ptr(), w.data_ptr(), x2.size(0), static_cast<int32_t>(D),
-                            x2.stride(0), z2.stride(0), y.stride(0), eps, stream),
+    const at::Tensor xc = x.contiguous(), zc = z.contiguous(), w = weight.contiguous();
+    at::Tensor y = empty(x.sizes(), x, at::kBFloat16);
+    check(gdn_gated_rmsnorm(xc.data_ptr(), zc.data_ptr(), y.data_ptr(), w.data_ptr(), x.numel() / D, static_cast<int32_t>(D),
+                            D, D, D, eps, stream),
           "gated_rmsnorm");
-    return y.view(x.sizes());
+    return y;
 }
 
 void bf16_gdn_recurrent(at::Tensor& q, at::Tensor& k, at::Tensor& v, std::optional<at::Tensor>& initial_state,
@@ -431,7 +441,7 @@ std::pair<at::Tensor, at::Tensor> fused_gdn_gating(at::Tensor& A_log, at::Tensor
     const int64_t vh = a.size(-1);
     require(A_log.numel() >= vh && dt_bias.numel() >= vh, "A_log and dt_bias need one entry per head");
     at::Tensor ac = a.contiguous(), bc = b.contiguous(), Ac = A_log.contiguous(), dc = dt_bias.contiguous();
-    at::Tensor beta = at::empty_like(bc), gate = at::empty_like(ac);
+    at::Tensor beta = empty_shaped_like(bc), gate = empty_shaped_like(ac);
     check(gdn_fused_gating(Ac.data_ptr(), dc.data_ptr(), ac.data_ptr(), bc.data_ptr(), beta.data_ptr(),
                            gate.data_ptr(), ac.numel() / vh, static_cast<int32_t>(vh), dtype_tag(ac), dtype_tag(gate),
                            stream),
