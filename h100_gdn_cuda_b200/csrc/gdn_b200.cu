@@ -7,6 +7,7 @@
 #include "kernels/helpers.cuh"
 #include "kernels/layer_adjacent.cuh"
 #include "kernels/recurrent.cuh"
+#include "kernels/recurrent_step.cuh"
 
 #include <atomic>
 
@@ -118,9 +119,40 @@ static int launch_recurrent(const RecurrentParams& p, int sms, cudaStream_t st, 
     return launch_recurrent_t<DK, false>(p, sms, st);
 }
 
+// Short padded runs (2 .. kStepTok tokens) on bf16 states of the head dims serving configurations use take
+// gdn_recurrent_step_kernel (recurrent_step.cuh), whatever the batch.
+static bool step_applies(const GdnShape& s, int state_dtype) {
+    return !s.cu_seqlens && s.seq_len >= 2 && s.seq_len <= kStepTok && state_dtype == GDN_BF16 && (s.head_dim_k == 64 || s.head_dim_k == 128) &&
+           s.head_dim_v % kStepRows == 0;
+}
+static StepParams step_plan(const RecurrentParams& r, int dk, int sms, unsigned* grid) {
+    StepParams p{};
+    p.r = r;
+    p.num_tiles = static_cast<long long>(r.batch) * r.vh * (r.dv / kStepRows);
+    const long long ctas = std::min<long long>(static_cast<long long>(sms) * kStepCtasPerSm, p.num_tiles);
+    p.stages = r.seq_len <= 6 ? 3 : 2;  // shared memory of a CTA: at most 100 KB
+    *grid = static_cast<unsigned>(ctas);
+    return p;
+}
+template <int DK>
+static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
+    unsigned grid = 0;
+    const StepParams p = step_plan(r, DK, sms, &grid);
+    static std::atomic<bool> attr_set[64];
+    int dev = 0;
+    GDN_CUDA(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_step_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        attr_set[dev & 63].store(true, std::memory_order_release);
+    }
+    GDN_CUDA(launch_dependent(gdn_recurrent_step_kernel<DK>, dim3(grid), kRecThreads,
+                              static_cast<size_t>(kStepWarps) * step_warp_bytes(DK, r.seq_len, p.stages), st, p));
+    return GDN_OK;
+}
+
 // Head dimensions without a prebuilt kernel (or every call when GDN_JIT_RECURRENT=1) go through
 // the run-time compiler: a three-line translation unit instantiates the kernel body for DK.
-static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaStream_t st, bool ring) {
+static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaStream_t st, bool ring, bool step = false) {
     const RecurrentConfig cfg = recurrent_config(dk, p.num_tiles, sms, ring);
     char src[512];
     snprintf(src, sizeof(src),
@@ -130,6 +162,23 @@ static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaS
              kRecThreads, cfg.ctas_per_sm, dk, ring ? "true" : "false");
     jit::LoadedKernel k;
     std::string err;
+    if (step) {
+        // the same kernel an ahead-of-time launch of this call would take
+        snprintf(src, sizeof(src),
+                 "#include \"kernels/recurrent_step.cuh\"\n"
+                 "extern \"C\" __global__ void __launch_bounds__(%d, %d) gdn_recurrent_jit(const gdn::StepParams p) {\n"
+                 "    gdn::gdn_recurrent_step_body<%d>(p);\n}\n",
+                 kRecThreads, kStepCtasPerSm, dk);
+        if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + ".step", src, "gdn_recurrent_jit", &k, &err)) return fail(rc, "%s", err.c_str());
+        unsigned grid = 0;
+        StepParams sp = step_plan(p, dk, sms, &grid);
+        const size_t smem = static_cast<size_t>(kStepWarps) * step_warp_bytes(dk, p.seq_len, sp.stages);
+        GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(smem)));
+        void* args[] = {&sp};
+        GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(kRecThreads), args, smem, st));
+        return GDN_OK;
+    }
     if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + (ring ? "_ring" : ""), src, "gdn_recurrent_jit", &k, &err))
         return fail(rc, "%s", err.c_str());
     GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -423,7 +472,9 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     // prepared tokens among them.  (Splitting the tiles of small decode batches over more CTAs as well was
     // tried: 3 % at B = 8, and the run-time unit decode it needs cost the large batches 2 %.)
     p.split_tiles = ring ? 1 : 0;
-    if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring);
+    const bool step = !ring && step_applies(s, a->state_dtype);
+    if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
+    if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
     if (a->state_dtype == GDN_F32) {
         // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
         if (s.head_dim_k == 128) return ring ? launch_recurrent_t<128, true, false, true>(p, d->sms, st) : launch_recurrent_t<128, false, false, true>(p, d->sms, st);

@@ -1,4 +1,5 @@
-// Recurrent Gated DeltaNet step (decode, speculative verify, short prefill).
+// Recurrent Gated DeltaNet step (decode, speculative verify, short prefill).  Padded runs of 2 .. 8 tokens on bf16 states of
+// head dims 64 and 128 take recurrent_step.cuh instead.
 //
 // Replaces the reference's fused_recurrent_gated_delta_rule_bf16
 // (gdn_cuda/include/gdn_cuda/kernels/sm90_bf16_gdn_recurrent.cuh:20-440) with the
