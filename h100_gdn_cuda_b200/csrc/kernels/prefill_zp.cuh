@@ -488,56 +488,58 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(d, sA, i0, j0 + 8 * ks, sA, j0 + 8 * ks, j0 + n0, LD, lane);
                     store_block(d, 1.f, sA, LD, j0, i0 + n0, lane);
-                    team_sync(team);
+                    __syncwarp();  // the 8 columns of the intermediate are this warp's alone
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
                     store_block(e, -1.f, sA, LD, i0, j0 + n0, lane);
                 }
                 team_sync(team);
-                // level 2 (32 -> 64): X_[2:4,0:2] = -X_[2:4,2:4] A_[2:4,0:2] X_[0:2,0:2]; warp = 16x16 block of the
-                // result; the intermediate goes to the unused upper-right quadrant
+                // level 2 (32 -> 64): X_[2:4,0:2] = -X_[2:4,2:4] A_[2:4,0:2] X_[0:2,0:2]; warp = 8 columns of the result, so
+                // that its part of the intermediate (parked in the unused upper-right quadrant) is its own as well
                 {
-                    const int rb = tw >> 1, cb = tw & 1;
+                    const int n0 = 8 * tw;
                     float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        if (ks >= 2 * cb) {
+                        if (ks >= tw) {  // (blocks of X above the diagonal are zero)
                             Frag<kWide, 4> af;
                             Frag<kWide, 2> bf;
-                            load_a<kWide>(af, sA, LD, 32 + 16 * rb, 8 * ks, lane);  // shared by the two column tiles
+                            load_b<kWide>(bf, sA, LD, 8 * ks, n0, lane);  // shared by the two row tiles
 #pragma unroll
-                            for (int nt = 0; nt < 2; ++nt) {
-                                load_b<kWide>(bf, sA, LD, 8 * ks, 16 * cb + 8 * nt, lane);
-                                mma_frag<kWide>(d[nt], af, bf);
+                            for (int mt = 0; mt < 2; ++mt) {
+                                load_a<kWide>(af, sA, LD, 32 + 16 * mt, 8 * ks, lane);
+                                mma_frag<kWide>(d[mt], af, bf);
                             }
                         }
                     }
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) store_block(d[nt], 1.f, sA, LD, 16 * rb, 32 + 16 * cb + 8 * nt, lane);
-                    team_sync(team);
+                    for (int mt = 0; mt < 2; ++mt) store_block(d[mt], 1.f, sA, LD, 16 * mt, 32 + n0, lane);
+                    __syncwarp();
                     float e[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        if (ks < 2 * (rb + 1)) {
-                            Frag<kWide, 4> af;
-                            Frag<kWide, 2> bf;
-                            load_a<kWide>(af, sA, LD, 32 + 16 * rb, 32 + 8 * ks, lane);
+                        Frag<kWide, 4> af;
+                        Frag<kWide, 2> bf;
+                        load_b<kWide>(bf, sA, LD, 8 * ks, 32 + n0, lane);
 #pragma unroll
-                            for (int nt = 0; nt < 2; ++nt) {
-                                load_b<kWide>(bf, sA, LD, 8 * ks, 32 + 16 * cb + 8 * nt, lane);
-                                mma_frag<kWide>(e[nt], af, bf);
+                        for (int mt = 0; mt < 2; ++mt) {
+                            if (ks < 2 * (mt + 1)) {
+                                load_a<kWide>(af, sA, LD, 32 + 16 * mt, 32 + 8 * ks, lane);
+                                mma_frag<kWide>(e[mt], af, bf);
                             }
                         }
                     }
+                    team_sync(team);  // every warp has read A_[2:4,0:2]
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) store_block(e[nt], -1.f, sA, LD, 32 + 16 * rb, 16 * cb + 8 * nt, lane);
+                    for (int mt = 0; mt < 2; ++mt) store_block(e[mt], -1.f, sA, LD, 32 + 16 * mt, n0, lane);
                 }
                 team_sync(team);
                 // ---- T = X diag(beta) and dT = diag(d) T as bf16 swizzled tiles (row = token i, 64 columns j) over X;
                 //      every thread first pulls its 32 values of X into registers
                 {
-                    const int i = tt >> 1, c0 = (tt & 1) * 32;
+                    // (16 rows and both halves per warp: eight rows per phase of a 16-byte access, no bank conflicts)
+                    const int i = 16 * tw + (lane & 15), c0 = (lane >> 4) * 32;
                     float xs[32];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
