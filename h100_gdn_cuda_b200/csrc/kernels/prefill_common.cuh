@@ -25,6 +25,13 @@ struct ScalarView {
         return is_f32 ? __ldg(reinterpret_cast<const float*>(ptr) + o)
                       : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(ptr)[o]);
     }
+    // The entry as its bits, for loads issued ahead of their use: converting at the load would wait for it there.
+    __device__ __forceinline__ uint32_t load_bits(long long b, long long t, int h) const {
+        const long long o = b * sb + t * st + static_cast<long long>(h) * sh;
+        return is_f32 ? __ldg(reinterpret_cast<const uint32_t*>(ptr) + o)
+                      : static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(ptr) + o));
+    }
+    __device__ __forceinline__ float value(uint32_t bits) const { return __uint_as_float(is_f32 ? bits : bits << 16); }
 };
 
 struct TokenView {

@@ -483,18 +483,18 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // =============================================================== producer
         // Raw gate values are fetched two chunks ahead into registers (lane l holds tokens l and
         // l + 32), so that when a stage frees up only the TMA issue remains to be done.
-        auto load_raw = [&](int c, float& a0, float& a1) {
-            a0 = 0.f;
-            a1 = 0.f;
+        auto load_raw = [&](int c, uint32_t& a0, uint32_t& a1) {
+            a0 = 0u;
+            a1 = 0u;
             if (p.gate.ptr && c < nchunks) {
                 const long long t0 = static_cast<long long>(c) * kChunk + lane;
-                if (t0 < seq_tokens) a0 = p.gate.load(batch, seq_tok0 + t0, head);
-                if (t0 + 32 < seq_tokens) a1 = p.gate.load(batch, seq_tok0 + t0 + 32, head);
+                if (t0 < seq_tokens) a0 = p.gate.load_bits(batch, seq_tok0 + t0, head);
+                if (t0 + 32 < seq_tokens) a1 = p.gate.load_bits(batch, seq_tok0 + t0 + 32, head);
             }
         };
         // the Z, PT blocks and the V tiles are read exactly once: first in line for eviction from L2
         const uint64_t once = l2_policy_evict_first();
-        float ra0, ra1, rb0, rb1;  // raw gates of chunks c and c + 1
+        uint32_t ra0, ra1, rb0, rb1;  // raw gates of chunks c and c + 1, as bits
         load_raw(0, ra0, ra1);
         load_raw(1, rb0, rb1);
         // Everything up to here (and the state warps' load of the initial state) touches only the caller's
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         for (int c = 0; c < nchunks; ++c) {
             const int s = c & 1;
             const int n = chunk_n(c);
-            float g0 = ra0, g1 = ra1;
+            float g0 = p.gate.value(ra0), g1 = p.gate.value(ra1);
             ra0 = rb0;
             ra1 = rb1;
             load_raw(c + 2, rb0, rb1);

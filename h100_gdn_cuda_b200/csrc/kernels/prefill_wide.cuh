@@ -349,14 +349,14 @@ __global__ void __launch_bounds__(wide::kThreads, 1)
     }
     if (warp == 13) {
         // =============================================================== producer
-        float ra0 = 0.f, ra1 = 0.f;  // raw gates of the coming chunk
+        uint32_t ra0 = 0u, ra1 = 0u;  // raw gates of the coming chunk, as bits
         auto load_raw = [&](int c) {
-            ra0 = 0.f;
-            ra1 = 0.f;
+            ra0 = 0u;
+            ra1 = 0u;
             if (p.gate.ptr && c < nchunks) {
                 const long long t0 = static_cast<long long>(c) * kChunk + lane;
-                if (t0 < seq_tokens) ra0 = p.gate.load(batch, seq_tok0 + t0, head);
-                if (t0 + 32 < seq_tokens) ra1 = p.gate.load(batch, seq_tok0 + t0 + 32, head);
+                if (t0 < seq_tokens) ra0 = p.gate.load_bits(batch, seq_tok0 + t0, head);
+                if (t0 + 32 < seq_tokens) ra1 = p.gate.load_bits(batch, seq_tok0 + t0 + 32, head);
             }
         };
         auto token_of = [&](int c) { return static_cast<int>(seq_tok0 + static_cast<long long>(c) * kChunk); };
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(wide::kThreads, 1)
         // K, V and the gate vectors of chunk c, whose raw gates are in ra0, ra1; fetches those of the next chunk
         auto load_kv = [&](int c) {
             const int n = chunk_n(c);
-            float g0 = ra0, g1 = ra1;
+            float g0 = p.gate.value(ra0), g1 = p.gate.value(ra1);
             load_raw(c + 1);
             float rk0 = 1.f, rk1 = 1.f, rq0 = 1.f, rq1 = 1.f;
             if (p.norms) {

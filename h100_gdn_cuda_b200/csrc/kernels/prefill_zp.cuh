@@ -231,18 +231,18 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
 
     // beta and the raw gate of this thread's token for (unit, round): fetched one round ahead, so that
     // their DRAM latency is not in front of every unit
-    auto fetch_scalars = [&](const UnitPos& u, int rd, float& b, float& g) {
-        b = 0.f;
-        g = 0.f;
+    auto fetch_scalars = [&](const UnitPos& u, int rd, uint32_t& b, uint32_t& g) {
+        b = 0u;
+        g = 0u;
         const int hloc = 2 * rd + team;
         if (!u.valid || hloc >= rep) return;
         if (tt < u.cp.n) {
             const int head = u.khead * rep + hloc;
-            b = p.beta.load(u.cp.batch, u.cp.tok0 + tt, head);
-            if (p.gate.ptr) g = p.gate.load(u.cp.batch, u.cp.tok0 + tt, head);
+            b = p.beta.load_bits(u.cp.batch, u.cp.tok0 + tt, head);
+            if (p.gate.ptr) g = p.gate.load_bits(u.cp.batch, u.cp.tok0 + tt, head);
         }
     };
-    float b_next, g_next;
+    uint32_t b_next, g_next;  // bits, see ScalarView::load_bits
     fetch_scalars(cur, 0, b_next, g_next);
 
     uint32_t it = 0;      // units done by this CTA (parity of bar_load and bar_kq)
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                 nxt = decode_unit(unit + gridDim.x);
                 fetch_scalars(nxt, 0, b_next, g_next);
             } else {
-                const float b_mine = b_next, g_mine = g_next;
+                const float b_mine = p.beta.value(b_next), g_mine = p.gate.value(g_next);
                 if (tt < 64) {
                     float g = g_mine;
 #pragma unroll
