@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     float ss = 0.f;
 #pragma unroll
                     for (int c = 0; c < 4 * NA; ++c) {
-                        const uint4 w = *reinterpret_cast<const uint4*>(rowp + (c >> 3) * 16384 + 16 * (c & 7));
+                        // (every row starts with another piece: rows are 128 bytes apart, all in the same banks)
+                        const uint4 w = *reinterpret_cast<const uint4*>(rowp + (c >> 3) * 16384 + 16 * ((c + r + 4 * hf) & 7));
                         const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
