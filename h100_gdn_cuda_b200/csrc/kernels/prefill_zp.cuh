@@ -61,7 +61,9 @@ struct ZPSmem {
     static constexpr int kTeamBytes = kOffVec + 2048;    // a multiple of 1024
     static constexpr int kOffNorm = kTeam + 2 * kTeamBytes;  // kNorm: inverse row norms of K [64] and Q [64], their log2 [128]
     static constexpr int kOffBar = kOffNorm + 1024;
-    static constexpr int kBytes = kOffBar + 128 + 1024;
+    static constexpr int kUnits = 256;                   // coordinates of this CTA's coming work units, 16 bytes each
+    static constexpr int kOffUnits = kOffBar + 128;
+    static constexpr int kBytes = kOffUnits + 16 * kUnits + 1024;
     static_assert(kOffP % 1024 == 0 && kTeamBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 };
 
@@ -70,6 +72,8 @@ constexpr int kThreads = 256;
 constexpr uint32_t kTmKQ = 0;    // fp32 K K^T (lanes 0-63) and Q K^T (lanes 64-127), 64 columns
 constexpr uint32_t kTmPT = 64;   // PT of team 0 (lanes +0) and team 1 (lanes +16), 64 columns
 constexpr uint32_t kTmZ = 128;   // + 64 (kWide: 128) * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16), kWide: 128-255 in the next 64
+// two neighbouring warps of a team
+__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(3 + pair) : "memory"); }
 // TF32 operands of the inverse's block products; kSplit: with the rounding error as a second term, and three
 // products per block (what the second terms' product would add is below fp32's own rounding)
 template <bool kSplit, int N>
@@ -204,29 +208,48 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
             khead = unit - chunk * p.kh;
         }
     };
-    // A unit's coordinates are worked out once (a handful of integer divisions) and carried along.
+    // Coordinates of a unit.  They are worked out for 256 of this CTA's units at a time, one thread each, and looked up in
+    // shared memory: done in every unit by every thread, the integer divisions (padded) or the two dependent loads (packed)
+    // stood in the middle of the unit's chain.
     struct UnitPos {
-        int chunk, khead;
-        ChunkPos cp;
+        int chunk, khead, n, tok0, batch;
         bool valid;
     };
-    auto decode_unit = [&](int unit) {
-        UnitPos u{};
-        u.valid = unit < total_units;
-        if (u.valid) {
-            unit_chunk(unit, u.chunk, u.khead);
-            u.cp = locate_chunk(p.map, u.chunk);
+    int4* const sUnits = reinterpret_cast<int4*>(smem + L::kOffUnits);
+    auto fill_units = [&](int unit0) {  // all threads; entry i: unit0 + i * gridDim.x
+        const long long unit = unit0 + static_cast<long long>(tid) * gridDim.x;
+        int4 e = make_int4(0, 0, 0, 0);
+        if (unit < total_units) {
+            int chunk, khead;
+            unit_chunk(static_cast<int>(unit), chunk, khead);
+            const ChunkPos cp = locate_chunk(p.map, chunk);
+            e = make_int4(chunk, khead | (cp.n << 16), static_cast<int>(cp.tok0), cp.batch);
         }
+        sUnits[tid] = e;
+    };
+    static_assert(L::kUnits == kThreads, "one entry per thread");
+    auto unit_at = [&](int i) {
+        const int4 e = sUnits[i];
+        UnitPos u;
+        u.chunk = e.x;
+        u.khead = e.y & 0xFFFF;
+        u.n = e.y >> 16;
+        u.tok0 = e.z;
+        u.batch = e.w;
+        u.valid = u.n > 0;
         return u;
     };
+    fill_units(static_cast<int>(blockIdx.x));
+    __syncthreads();
     auto issue_loads = [&](const UnitPos& u) {  // one thread
         mbar_arrive_expect_tx(bar_load, NA * 16384);
         for (int a = 0; a < NA; ++a) {
-            tma_load_4d(sKQ + a * 16384, &tmK, bar_load, a * 64, u.khead, static_cast<int>(u.cp.tok0), u.cp.batch);
-            tma_load_4d(sKQ + a * 16384 + 8192, &tmQ, bar_load, a * 64, u.khead, static_cast<int>(u.cp.tok0), u.cp.batch);
+            tma_load_4d(sKQ + a * 16384, &tmK, bar_load, a * 64, u.khead, u.tok0, u.batch);
+            tma_load_4d(sKQ + a * 16384 + 8192, &tmQ, bar_load, a * 64, u.khead, u.tok0, u.batch);
         }
     };
-    UnitPos cur = decode_unit(blockIdx.x), nxt{};
+    UnitPos cur = unit_at(0), nxt{};
+    int table = 0;  // entry of the present unit
     if (tid == 0 && cur.valid) issue_loads(cur);
 
     // beta and the raw gate of this thread's token for (unit, round): fetched one round ahead, so that
@@ -236,10 +259,10 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
         g = 0u;
         const int hloc = 2 * rd + team;
         if (!u.valid || hloc >= rep) return;
-        if (tt < u.cp.n) {
+        if (tt < u.n) {
             const int head = u.khead * rep + hloc;
-            b = p.beta.load_bits(u.cp.batch, u.cp.tok0 + tt, head);
-            if (p.gate.ptr) g = p.gate.load_bits(u.cp.batch, u.cp.tok0 + tt, head);
+            b = p.beta.load_bits(u.batch, u.tok0 + tt, head);
+            if (p.gate.ptr) g = p.gate.load_bits(u.batch, u.tok0 + tt, head);
         }
     };
     uint32_t b_next, g_next;  // bits, see ScalarView::load_bits
@@ -250,15 +273,20 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
     bool stores_pending = false;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x, ++it, cur = nxt) {
         const int chunk = cur.chunk, khead = cur.khead;
-        const ChunkPos cp = cur.cp;
-        const int n = cp.n;
+        const int n = cur.n;
+        if (++table == L::kUnits) {  // the next unit is past the table
+            __syncthreads();
+            fill_units(unit + static_cast<int>(gridDim.x));
+            __syncthreads();
+            table = 0;
+        }
         for (int rd = 0; rd < rounds; ++rd) {
             const int hloc = 2 * rd + team;
             const bool active = hloc < rep;  // team-uniform
             const int head = khead * rep + hloc;
             // ---- beta, chunk-local cumulative gate, decay to the chunk's last token
             if (!active) {  // (odd number of v-heads per k-head: team 1 sits the last round out)
-                nxt = decode_unit(unit + gridDim.x);
+                nxt = unit_at(table);
                 fetch_scalars(nxt, 0, b_next, g_next);
             } else {
                 const float b_mine = p.beta.value(b_next), g_mine = p.gate.value(g_next);
@@ -426,7 +454,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                 if (rd + 1 < rounds) {
                     fetch_scalars(cur, rd + 1, b_next, g_next);
                 } else {
-                    nxt = decode_unit(unit + gridDim.x);
+                    nxt = unit_at(table);
                     fetch_scalars(nxt, 0, b_next, g_next);
                 }
                 tc_fence_before_sync();
@@ -493,6 +521,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
+                    pair_sync(2 * team + pr);  // both warps of the pair have read A_10
                     store_block(e, -1.f, sA, LD, i0, j0 + n0, lane);
                 }
                 team_sync(team);

@@ -1,0 +1,37 @@
+"""The chunk-parallel prefill kernel works out the coordinates of its work units 256 per CTA at a time.  More units than
+that (76 800 = 300 sequences x 8 chunks x 32 k-heads on 296 CTAs, 260 each): every sequence must come out with the bits it
+has in a call of its own.  Padded, and packed with ragged lengths."""
+import pytest
+import torch
+
+from h100_gdn_cuda_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_more_units_than_one_table(packed):
+    import h100_gdn_cuda_b200 as gdn
+    B, T, H, d = 300, 512, 32, 16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k = (torch.nn.functional.normalize(r(B * T, H, d), dim=-1).bfloat16() for _ in range(2))
+    v, beta = r(B * T, H, d).bfloat16(), torch.sigmoid(r(B * T, H)).bfloat16()
+    gate, s0 = -torch.nn.functional.softplus(r(B * T, H)), (r(B, H, d, d) * 0.02).bfloat16()
+    if packed:
+        lens = [T - 1 if i % 2 else T + 1 for i in range(B)]  # 8 and 9 chunks
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        meta = [torch.tensor(x, dtype=torch.int32, device="cuda")
+                for x in (cu, synthetic.prepare_chunk_indices(cu), synthetic.prepare_cu_chunks(cu))]
+        o, s = gdn.chunked_forward(q, k, v, beta, gate, None, s0, *meta)
+    else:
+        cu = [i * T for i in range(B + 1)]
+        x4 = lambda x: x.view(B, T, *x.shape[1:])
+        o, s = gdn.chunked_forward(x4(q), x4(k), x4(v), x4(beta), x4(gate), None, s0)
+        o = o.view(B * T, H, d)
+    for i in (0, 1, 149, 290, 297, 299):
+        sl = slice(cu[i], cu[i + 1])
+        oi, si = gdn.chunked_forward(q[None, sl], k[None, sl], v[None, sl], beta[None, sl], gate[None, sl], None, s0[i:i + 1])
+        assert torch.equal(oi[0], o[sl]) and torch.equal(si[0], s[i])
