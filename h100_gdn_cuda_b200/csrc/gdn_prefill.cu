@@ -6,6 +6,7 @@
 #include "kernels/prefill_o.cuh"
 #include "kernels/prefill_seq.cuh"
 #include "kernels/prefill_segments.cuh"
+#include "kernels/prefill_transition.cuh"
 #include "kernels/prefill_uw.cuh"
 #include "kernels/prefill_wide.cuh"
 #include "kernels/prefill_zp.cuh"
@@ -454,10 +455,22 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
             p.num_seqs = s.batch;
             p.seg_mn = seg_mn;
             p.seg_start = seg_start;
-            p.mode = 1;
+            if (int rc = set_smem<gdn_seg_transition_kernel>(TransitionSmem::kBytes)) return rc;
             if (int rc = set_smem<gdn_seg_combine_kernel>(SegCombineSmem::kBytes)) return rc;
             if (int rc = run_zp()) return rc;
-            if (int rc = run_seq(dim3(plan.slots, s.num_v_heads, 2))) return rc;
+            // the launches of the segmented path, each a programmatic dependent of the one before it (every one of them waits
+            // before its first access to what that one wrote)
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.stream = st;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            cfg.gridDim = dim3(static_cast<unsigned>(plan.slots), static_cast<unsigned>(s.num_v_heads));
+            cfg.blockDim = dim3(transition::kThreads);
+            cfg.dynamicSmemBytes = TransitionSmem::kBytes;
+            GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_transition_kernel, tmK, tmV, p));
             SegCombineParams cp{};
             cp.seg_mn = seg_mn;
             cp.seg_start = seg_start;
@@ -470,20 +483,10 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
             cp.map = p.map;
             cp.seg_chunks = plan.seg_chunks;
             cp.status = d->status;
-            {
-                // a programmatic dependent of the composite-transition launch (it waits before its first global access)
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3(static_cast<unsigned>(chains), kD / SegCombineSmem::R);
-                cfg.blockDim = dim3(128);
-                cfg.dynamicSmemBytes = SegCombineSmem::kBytes;
-                cfg.stream = st;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_combine_kernel, cp));
-            }
+            cfg.gridDim = dim3(static_cast<unsigned>(chains), kD / SegCombineSmem::R);
+            cfg.blockDim = dim3(SegCombineSmem::kThreads);
+            cfg.dynamicSmemBytes = SegCombineSmem::kBytes;
+            GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_combine_kernel, cp));
             p.mode = 2;
             if (int rc = run_seq(dim3(plan.slots, s.num_v_heads))) return rc;
         }

@@ -39,9 +39,9 @@ inline PrefillConfig prefill_config() { return PrefillConfig{4, 512}; }
 // Segmented state propagation for few long sequences.  The state kernel is a serial chain
 // per (sequence, v-head); with fewer chains than SMs most of the GPU idles.  The chain obeys
 // S' = S M_c + N_c per chunk, so a sequence is cut into segments: one launch finds every
-// segment's composite (M, N) (two CTAs per chain and segment), a small kernel chains them into the
-// segments' start states, and a second launch of the state kernel produces the output of all
-// segments at once.  Three passes instead of one, many segments wide.
+// segment's composite (M, N) (one CTA per chain and segment runs both), a small kernel chains them into the
+// segments' start states, and a launch of the state kernel produces the output of all
+// segments at once.  Two passes and a quarter instead of one, many segments wide.
 // The plan must not depend on the device (the scratch size is computed without one), so it is
 // made for the 148 SMs of a B200.
 struct SegmentPlan {
@@ -53,10 +53,11 @@ struct SegmentPlan {
 namespace plan_detail {
 constexpr long long kSms = 148;
 // Cost model fitted to measurements (B=1..2, T=4096..131072, 4..32 v-heads), in units of "one
-// chunk of the state kernel": a CTA costs its chunks plus about 3 for start-up and pipeline
-// fill; a launch costs that times its CTA waves.  Plans whose second launch needs more than
-// one wave, or whose first needs more than two, measured worse than the model and are not made.
+// chunk of the state kernel" (1.25 us): a CTA costs its chunks plus about 3 for start-up and pipeline
+// fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Plans whose launches need more
+// than one wave measured worse than the model and are not made.
 constexpr int kFixed = 3, kMinSegment = 32;
+constexpr double kPasses = 2.2;
 inline long long waves(long long ctas) { return (ctas + kSms - 1) / kSms; }
 }  // namespace plan_detail
 
@@ -66,10 +67,9 @@ inline SegmentPlan prefill_segments(long long chains, int chunks_per_seq, bool p
     if (packed || chains <= 0) return plan;
     double best = 0.8 * static_cast<double>(waves(chains) * (chunks_per_seq + kFixed));
     for (int P = 2; P <= 32 && chunks_per_seq / P >= kMinSegment; ++P) {
-        const long long w1 = waves(2 * chains * P), w3 = waves(chains * P);
-        if (w3 > 1 || w1 > 2) break;
+        if (waves(chains * P) > 1) break;
         const int len = (chunks_per_seq + P - 1) / P;
-        const double cost = static_cast<double>((w1 + w3) * (len + kFixed));
+        const double cost = kPasses * (len + kFixed);
         if (cost < best) {
             best = cost;
             plan.num_segments = P;
@@ -99,9 +99,8 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
         // hold work when the sequences are about equally long: every sequence end but the last may add one
         // short segment
         const long long work = (total_chunks + len - 1) / len + num_seqs - 1;
-        const long long w1 = waves(2 * work * num_v_heads), w3 = waves(work * num_v_heads);
-        if (w3 > 1 || w1 > 2) break;
-        const double cost = static_cast<double>((w1 + w3) * (len + kFixed));
+        if (waves(work * num_v_heads) > 1) break;
+        const double cost = kPasses * (len + kFixed);
         if (cost < best) {
             best = cost;
             plan.num_segments = P;

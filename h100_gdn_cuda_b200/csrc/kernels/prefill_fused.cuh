@@ -47,12 +47,9 @@ struct FusedParams {
     // norms (written by gdn_zp_kernel); they enter through the two per-token factors of a chunk
     const float* norms;
     // Segmented runs (few long sequences; see gdn_chunked_forward).  The state obeys
-    // S' = S M_c + N_c per chunk, so a segment of chunks has a composite (M, N) as well.
+    // S' = S M_c + N_c per chunk, so a segment of chunks has a composite (M, N) as well; gdn_seg_transition_kernel
+    // leaves them in fp32 in seg_mn[(slot * vh + head) * 2 + {N, M}], slot = a (sequence, segment) pair (locate_segment).
     //   mode 0: one CTA walks the whole sequence (grid = sequences x heads, or heads x ranks with seq_order).
-    //   mode 1: grid = (slots, heads, 2); blockIdx.x = slot of a (sequence, segment) pair (locate_segment),
-    //           blockIdx.z = kind; no output.  kind 0 starts from S = 0 and ends with N of the segment;
-    //           kind 1 starts from S = I with V taken as 0 and ends with M.
-    //           Both are written in fp32 to seg_mn[(slot * vh + head) * 2 + kind].
     //   mode 2: grid = (slots, heads); starts from seg_start[slot * vh + head] (fp32), writes the
     //           output of its chunks; the last segment of a sequence writes the final state.
     int mode, seg_chunks, num_segments, num_seqs;
@@ -162,8 +159,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     const int seq = p.mode != 0 ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
     const int head = p.mode == 0 && p.seq_order ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
     const int segment = sp.segment, seq_nseg = sp.nseg;
-    const int seg_kind = p.mode == 1 ? static_cast<int>(blockIdx.z) : 0;
-    const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;  // modes 1, 2
+    const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;  // mode 2
     const int khead = head / (p.vh / p.kh);
 
     int batch, gchunk0;
@@ -182,8 +178,6 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     }
     int nchunks = static_cast<int>((seq_tokens + kChunk - 1) / kChunk);
     // A segment is handled as a sequence of its own: shift the token and chunk origins.
-    const bool emit_o = p.mode != 1;
-    const bool zero_u = p.mode == 1 && seg_kind == 1;
     if (p.mode != 0) {
         const int c0 = min(segment * p.seg_chunks, nchunks);
         const int c1 = min(c0 + p.seg_chunks, nchunks);
@@ -250,9 +244,6 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
                 const float4 v = __ldg(src + q);
                 S[4 * q] = v.x; S[4 * q + 1] = v.y; S[4 * q + 2] = v.z; S[4 * q + 3] = v.w;
             }
-        } else if (p.mode == 1) {
-#pragma unroll
-            for (int q = 0; q < 64; ++q) S[q] = (seg_kind == 1 && row == 64 * hf + q) ? 1.f : 0.f;
         } else if (p.state_in) {
             const uint4* src = reinterpret_cast<const uint4*>(p.state_in + seq * p.si_ss + head * p.si_sh +
                                                               static_cast<long long>(row) * p.d + 64 * hf);
@@ -296,10 +287,6 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             for (int j = 0; j < 2; ++j) {
                 ldmatrix_x4_trans(sV + vsw0 + 2048 * j, vpk[0][j]);
                 ldmatrix_x4_trans(sV + vsw1 + 2048 * j, vpk[1][j]);
-            }
-            if (zero_u) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) vpk[j >> 3][(j >> 2) & 1][j & 3] = 0u;
             }
             f2 neg[4];  // -e^{g} of this lane's token pairs
 #pragma unroll
@@ -387,11 +374,6 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // nothing is written once a wait of this CTA has given up (the results would be garbage)
         const bool healthy = *abort_flag == 0;
         if (!healthy) {
-        } else if (p.mode == 1) {
-            float4* d4 = reinterpret_cast<float4*>(p.seg_mn + (seg_idx * 2 + seg_kind) * (D * D) +
-                                                   static_cast<long long>(row) * D + 64 * hf);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) d4[q] = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
         } else if (p.state_out && (p.mode == 0 || segment == seq_nseg - 1)) {
             uint4* d4 = reinterpret_cast<uint4*>(p.state_out + seq * p.so_ss + head * p.so_sh +
                                                  static_cast<long long>(row) * p.d + 64 * hf);
@@ -416,7 +398,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         const uint32_t ochunk = static_cast<uint32_t>(4 * (lq & 1) + ((lane >> 3) & 1));
         const uint32_t osw0 = olane + ((ochunk ^ (lane & 7)) << 4), osw1 = olane + (((ochunk + 2) ^ (lane & 7)) << 4);
         const bool packed = p.map.cu_seqlens != nullptr;
-        for (int c = 0; c < (emit_o ? nchunks : 0); ++c) {
+        for (int c = 0; c < nchunks; ++c) {
             const uint32_t par = static_cast<uint32_t>(c & 1);
             const int n = chunk_n(c);
             const float* gb = gate_buf(c);
@@ -551,15 +533,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
                 for (int a = 0; a < 2; ++a) tma_load_4d_w(st + L::kOffK + a * 8192, &tmK, &bar_full[s], a * 64, khead, tok, batch);
 #pragma unroll
                 for (int a = 0; a < 2; ++a) tma_load_4d_hint_w(st + L::kOffV + a * 8192, &tmV, &bar_full[s], a * 64, head, tok, batch, once);
-                if (emit_o) {
-                    mbar_arrive_expect_tx_w(&bar_full2[s], L::kTile + kZPBlockBytes);
-                    bulk_load_hint_w(st + L::kOffZ, blk, kZPBlockBytes, &bar_full2[s], once);
+                mbar_arrive_expect_tx_w(&bar_full2[s], L::kTile + kZPBlockBytes);
+                bulk_load_hint_w(st + L::kOffZ, blk, kZPBlockBytes, &bar_full2[s], once);
 #pragma unroll
-                    for (int a = 0; a < 2; ++a) tma_load_4d_w(st + L::kOffQ + a * 8192, &tmQ, &bar_full2[s], a * 64, khead, tok, batch);
-                } else {
-                    mbar_arrive_expect_tx_w(&bar_full2[s], L::kTile);  // no output: Z is all the second group needs
-                    bulk_load_hint_w(st + L::kOffZ, blk, L::kTile, &bar_full2[s], once);
-                }
+                for (int a = 0; a < 2; ++a) tma_load_4d_w(st + L::kOffQ + a * 8192, &tmQ, &bar_full2[s], a * 64, khead, tok, batch);
                 if (lane == 0) *issued = c + 1;
             }
         }
@@ -583,9 +560,9 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
                     if (a * 64 >= p.d) break;  // nothing in memory behind the second half of a small head
                     tma_prefetch_4d(&tmK, a * 64, khead, tok, batch);
                     tma_prefetch_4d(&tmV, a * 64, head, tok, batch);
-                    if (emit_o) tma_prefetch_4d(&tmQ, a * 64, khead, tok, batch);
+                    tma_prefetch_4d(&tmQ, a * 64, khead, tok, batch);
                 }
-                bulk_prefetch_l2(blk, emit_o ? kZPBlockBytes : L::kTile);
+                bulk_prefetch_l2(blk, kZPBlockBytes);
             }
         }
     } else if (warp == 13) {
@@ -620,24 +597,19 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
                 // O1 = S_bf Q^T
                 mbar_wait(&bar_full2[s], static_cast<uint32_t>((c >> 1) & 1), abort_flag);
                 tc_fence_after_sync();
-                if (emit_o) {
-                    const uint32_t tO1 = tmem + ((c & 1) ? kTmO1b : kTmO1a);
-                    mma_ts_k128_w<false>(tO1, tS, q, id_sq);
-                }
+                mma_ts_k128_w<false>(tmem + ((c & 1) ? kTmO1b : kTmO1a), tS, q, id_sq);
                 mbar_wait(bar_un, par, abort_flag);
                 tc_fence_after_sync();
                 // dS = R Z
                 mma_ts_k64_w<false, 128>(tDS, tR, z, id_ds);
                 mma_commit_w(bar_ds);
                 // O2 = R PT^T (its accumulator must have been drained by the previous epilogue)
-                if (emit_o) {
-                    if (c > 0) {
-                        mbar_wait(bar_ofree, static_cast<uint32_t>((c - 1) & 1), abort_flag);
-                        tc_fence_after_sync();
-                    }
-                    mma_ts_k64_w<false, 2>(tO2, tR, pp, id_sq);
-                    mma_commit_w(bar_o);
+                if (c > 0) {
+                    mbar_wait(bar_ofree, static_cast<uint32_t>((c - 1) & 1), abort_flag);
+                    tc_fence_after_sync();
                 }
+                mma_ts_k64_w<false, 2>(tO2, tR, pp, id_sq);
+                mma_commit_w(bar_o);
                 mma_commit_w(&bar_empty[s]);
             }
         }
