@@ -56,8 +56,11 @@ constexpr long long kSms = 148;
 // chunk of the state kernel" (1.25 us): a CTA costs its chunks plus about 3 for start-up and pipeline
 // fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Plans whose launches need more
 // than one wave measured worse than the model and are not made.
-constexpr int kFixed = 3, kMinSegment = 32;
+constexpr int kFixed = 3;
 constexpr double kPasses = 2.2;
+// Shortest segments: below, the two extra launches and the serial chaining of the start states eat the gain.  Packed
+// sequences of unequal lengths each end in a shorter one, hence the larger figure there.
+constexpr int kMinSegment = 25, kMinSegmentPacked = 32;
 inline long long waves(long long ctas) { return (ctas + kSms - 1) / kSms; }
 }  // namespace plan_detail
 
@@ -92,7 +95,7 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
     const long long chains = static_cast<long long>(num_seqs) * num_v_heads;
     const long long even = (total_chunks + num_seqs - 1) / num_seqs;
     double best = 0.8 * static_cast<double>(waves(chains) * (even + kFixed));
-    for (int P = 2; P <= 128 && total_chunks / P >= kMinSegment; ++P) {
+    for (int P = 2; P <= 128 && total_chunks / P >= kMinSegmentPacked; ++P) {
         const int len = static_cast<int>((total_chunks + P - 1) / P);
         const long long slots = total_chunks / len + num_seqs;  // launched (and given scratch): the upper bound
         // CTAs of surplus slots leave at once and free their SM, so the waves are counted for the slots that
