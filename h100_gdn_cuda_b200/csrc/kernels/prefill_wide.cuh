@@ -212,12 +212,17 @@ __global__ void __launch_bounds__(wide::kThreads, 1)
                     unpk(fma2(pk(neg.x, neg.y), pk(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])),
                               pk(bf16_lo(v8[e]), bf16_hi(v8[e]))),
                          r0, r1);
-                    if (nloc < 32) {  // rows past the end may hold a neighbouring sequence's values
-                        if (i >= nloc) r0 = 0.f;
-                        if (i + 1 >= nloc) r1 = 0.f;
-                    }
                     h[e] = pack_bf16(r0, r1);
                     l[e] = pack_bf16(r0 - bf16_lo(h[e]), r1 - bf16_hi(h[e]));
+                }
+                if (nloc < 32) {  // rows past the end may hold a neighbouring sequence's values (one branch for all of them)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int i = 16 * b + 2 * e;
+                        const uint32_t keep = (i < nloc ? 0xFFFFu : 0u) | (i + 1 < nloc ? 0xFFFF0000u : 0u);
+                        h[e] &= keep;
+                        l[e] &= keep;
+                    }
                 }
                 tmem_st8(tX + 16 * b, h);
                 tmem_st8(tX + 16 * b + 8, l);

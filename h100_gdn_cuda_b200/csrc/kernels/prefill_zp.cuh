@@ -661,38 +661,66 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                 const int row = 16 * tw + (lane & 15), hi = lane >> 4;
                 const uint32_t tl = static_cast<uint32_t>(32 * tw) << 16;
                 if constexpr (kWide) {
-                    // ---- accumulators -> two bf16 terms -> the unit's block, written where they belong (the four Z and
-                    //      two PT tiles of both teams would not fit beside K and Q, and this kernel is a small part of a wide call)
+                    // ---- accumulators -> two bf16 terms -> staged tiles -> bulk copies: first Z hi (over T, dT) and both terms
+                    //      of PT (over P), then Z lo over Z hi once that has been read out.  (Written to global memory from
+                    //      registers, 16 bytes of a row per lane, this was 12 of a unit's 25 thousand cycles.)
                     uint8_t* dst = p.blocks + (static_cast<size_t>(chunk) * p.vh + head) * kWideBlockBytes;
-                    const bool healthy = *abort_flag == 0;
-                    auto emit = [&](const uint32_t* r, uint8_t* hi_tile, uint8_t* lo_tile, int c16) {
+                    uint8_t* stZ = tbase + L::kOffA;
+                    const uint64_t keep = l2_policy_evict_last();
+                    auto hi_of = [&](const uint32_t* r) {
+                        return make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
+                                          pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
+                    };
+                    auto lo_of = [&](const uint32_t* r, const uint4& h) {
+                        return make_uint4(pack_lo(__uint_as_float(r[0]), __uint_as_float(r[1]), h.x), pack_lo(__uint_as_float(r[2]), __uint_as_float(r[3]), h.y),
+                                          pack_lo(__uint_as_float(r[4]), __uint_as_float(r[5]), h.z), pack_lo(__uint_as_float(r[6]), __uint_as_float(r[7]), h.w));
+                    };
+                    auto stage_z = [&](bool lo) {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            float f[8];
+                        for (int cb = 0; cb < 4; ++cb) {  // 32 columns of every 64; lanes +16 hold the odd atoms
+                            uint32_t r[32];
+                            tmem_ld32(tmem + kTmZ + 128u * team + tl + 32 * cb, r);
+                            tmem_wait_ld();
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * q + e]);
-                            const uint4 h = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-                            *reinterpret_cast<uint4*>(hi_tile + tile_off(row, c16 + q)) = h;
-                            *reinterpret_cast<uint4*>(lo_tile + tile_off(row, c16 + q)) = make_uint4(
-                                pack_lo(f[0], f[1], h.x), pack_lo(f[2], f[3], h.y), pack_lo(f[4], f[5], h.z), pack_lo(f[6], f[7], h.w));
+                            for (int q = 0; q < 4; ++q) {
+                                const uint4 h = hi_of(r + 8 * q);
+                                *reinterpret_cast<uint4*>(stZ + tile_off(row, 16 * (cb >> 1) + 8 * hi + 4 * (cb & 1) + q)) = lo ? lo_of(r + 8 * q, h) : h;
+                            }
                         }
                     };
-#pragma unroll
-                    for (int cb = 0; cb < 4; ++cb) {  // 32 columns of every 64; lanes +16 hold the odd atoms
-                        uint32_t r[32];
-                        tmem_ld32(tmem + kTmZ + 128u * team + tl + 32 * cb, r);
-                        tmem_wait_ld();
-                        if (healthy) emit(r, dst, dst + 32768, 16 * (cb >> 1) + 8 * hi + 4 * (cb & 1));
-                    }
+                    stage_z(false);
 #pragma unroll
                     for (int cb = 0; cb < 2; ++cb) {
                         uint32_t r[32];
                         tmem_ld32(tmem + kTmPT + tl + 32 * cb, r);
                         tmem_wait_ld();
-                        if (hi == team && healthy) emit(r, dst + 65536, dst + 65536 + 8192, 4 * cb);
+                        if (hi == team) {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                const uint4 h = hi_of(r + 8 * q);
+                                *reinterpret_cast<uint4*>(sP + tile_off(row, 4 * cb + q)) = h;
+                                *reinterpret_cast<uint4*>(sP + 8192 + tile_off(row, 4 * cb + q)) = lo_of(r + 8 * q, h);
+                            }
+                        }
                     }
+                    fence_proxy_async_smem();
+                    team_sync(team);
+                    if (tt == 0 && *abort_flag == 0) {  // nothing is written once a wait has given up
+                        bulk_store_hint(dst, stZ, 32768, keep);
+                        bulk_store_hint(dst + 65536, sP, 16384, keep);
+                        bulk_commit();
+                        bulk_wait_read<0>();
+                    }
+                    team_sync(team);
+                    stage_z(true);
+                    fence_proxy_async_smem();
                     tc_fence_before_sync();
-                    team_sync(team);  // T, dT and P are free for the next round
+                    team_sync(team);
+                    if (tt == 0 && *abort_flag == 0) {
+                        bulk_store_hint(dst + 32768, stZ, 32768, keep);
+                        bulk_commit();
+                    }
+                    stores_pending = true;
                 } else {
                 // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> two bulk copies
                 uint8_t* stZ = tbase + L::kOffA;
