@@ -469,9 +469,12 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
                                    : (s.seq_len > ring_min);
     // Work units: the ring instance (long token runs) makes every 32-row tile a unit of its own; the decode
     // instance keeps the tiles of a (sequence, v-head) together, which shares the q/k normalisation and the
-    // prepared tokens among them.  (Splitting the tiles of small decode batches over more CTAs as well was
-    // tried: 3 % at B = 8, and the run-time unit decode it needs cost the large batches 2 %.)
+    // prepared tokens among them.  One-token batches with a CTA slot for every tile are split as well (B=1 with 32 v-heads
+    // of 128 rows: 5.3 -> 3.8 us, B=4 6.0 -> 4.8); with two tiles or more per slot a tile's own copies and norms cost more
+    // than the finer grain gives (B=8 6.9 -> 7.6 us, B=24 13.2 -> 17.4).
     p.split_tiles = ring ? 1 : 0;
+    const int slots_per_sm = s.head_dim_k > 128 ? 2 : (a->state_dtype == GDN_F32 && s.head_dim_k > 64 ? 3 : 4);
+    if (!ring && !s.cu_seqlens && s.seq_len == 1) p.split_tiles = p.num_tiles <= static_cast<long long>(d->sms) * slots_per_sm;
     const bool step = !ring && step_applies(s, a->state_dtype);
     if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
     if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
@@ -481,7 +484,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
         if (s.head_dim_k == 64) return ring ? launch_recurrent_t<64, true, false, true>(p, d->sms, st) : launch_recurrent_t<64, false, false, true>(p, d->sms, st);
         return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: fp32 states are built for dk = 64 and 128 (got %d)", s.head_dim_k);
     }
-    const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx;
+    const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx && !p.split_tiles;
     switch (s.head_dim_k) {
         case 64: return launch_recurrent<64>(p, d->sms, st, ring, lean);
         case 128: return launch_recurrent<128>(p, d->sms, st, ring, lean);

@@ -58,7 +58,7 @@ struct RecurrentParams {
     int fused_gating, gating_param_f32;
     const void* A_log;
     const void* dt_bias;
-    int split_tiles;  // 1: every 32-row tile is a work unit (multi-token runs of the ring instance); 0: a unit = all tiles of a (sequence, v-head)
+    int split_tiles;  // 1: every 32-row tile is a work unit (ring instance, small decode batches); 0: a unit = all tiles of a (sequence, v-head)
     long long num_tiles;
     int* status;
 };
@@ -201,8 +201,9 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     const bool has_in = kLean || p.state_in != nullptr;
     const bool store_step = !kLean && p.store_step != 0;
     const int rep = p.vh / p.kh;
-    const int tpu = (kRing && p.split_tiles) ? 1 : rblocks;  // tiles per work unit
+    const int tpu = (!kLean && p.split_tiles) ? 1 : rblocks;  // tiles per work unit
     const int upg = rblocks / tpu;                // work units per (sequence, v-head)
+    const int upg_shift = (upg & (upg - 1)) == 0 ? __ffs(upg) - 1 : -1;
     const int num_units = static_cast<int>(p.num_tiles / tpu);
     const int stride = static_cast<int>(gridDim.x);
 
@@ -239,7 +240,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
         int sh = unit;
         t.rb0 = 0;
         if (upg != 1) {
-            sh = unit / upg;
+            sh = upg_shift >= 0 ? unit >> upg_shift : unit / upg;
             t.rb0 = (unit - sh * upg) * tpu;
         }
         if (vh_shift >= 0) {
@@ -292,19 +293,21 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                       &full[stage]);
         }
     };
-    auto load_scalars = [&](const Unit& t, int tk, float& bt, float& gt) {
+    // beta and the gate of a token as their bits, to be converted where they are used: a conversion at the load waits for it
+    auto load_scalars = [&](const Unit& t, int tk, uint32_t& bt, uint32_t& gt) {
         const long long tok = t.tok0 + tk;
         const long long bo = t.bidx * p.beta_sb + tok * p.beta_st + t.head * p.beta_sh;
-        bt = p.beta_f32 ? __ldg(reinterpret_cast<const float*>(p.beta) + bo)
-                        : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.beta)[bo]);
+        bt = p.beta_f32 ? __ldg(reinterpret_cast<const uint32_t*>(p.beta) + bo)
+                        : static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(p.beta) + bo));
+        gt = 0u;
         if (p.gate) {
             const long long go = t.bidx * p.gate_sb + tok * p.gate_st + t.head * p.gate_sh;
-            gt = p.gate_f32 ? __ldg(reinterpret_cast<const float*>(p.gate) + go)
-                            : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.gate)[go]);
-        } else {
-            gt = 0.f;
+            gt = p.gate_f32 ? __ldg(reinterpret_cast<const uint32_t*>(p.gate) + go)
+                            : static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(p.gate) + go));
         }
     };
+    auto beta_of = [&](uint32_t bits) { return __uint_as_float(p.beta_f32 ? bits : bits << 16); };
+    auto gate_of = [&](uint32_t bits) { return __uint_as_float(p.gate_f32 ? bits : bits << 16); };
 
     // raw projections (b, a) of a token of v-head `head` -> (beta, gate)
     auto apply_gating = [&](int head, float& bt, float& gt) {
@@ -351,11 +354,11 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
         for (int s = 0; s < kStages - 1; ++s) produce_one();
     }
 
-    float beta_first = 0.f, g_first = 0.f;  // scalars of the first token of the current unit
+    uint32_t beta_bits = 0u, g_bits = 0u;  // scalars of the first token of the current unit
     if (static_cast<int>(blockIdx.x) < num_units) {
         const Unit t0 = decode(blockIdx.x);
         const int tk = kRing ? lane : 0;  // multi-token instance: lane l holds the scalars of token l
-        if (tk < t0.ntok) load_scalars(t0, tk, beta_first, g_first);
+        if (tk < t0.ntok) load_scalars(t0, tk, beta_bits, g_bits);
     }
 
     int it = 0;
@@ -364,7 +367,8 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     if (static_cast<int>(blockIdx.x) < num_units) T_carry = decode(blockIdx.x);
     for (int unit = blockIdx.x; unit < num_units; unit += stride) {
         const Unit T = T_carry;
-        float beta_next = 0.f, g_next = 0.f;
+        float beta_first = beta_of(beta_bits), g_first = gate_of(g_bits);
+        uint32_t beta_next = 0u, g_next = 0u;
         if (unit + stride < num_units) {
             T_carry = decode(unit + stride);
             const int tk = kRing ? lane : 0;
@@ -431,8 +435,9 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                         kk[pc] = __ldg(reinterpret_cast<const uint2*>(kp + pc * 64 + l16 * 4));
                         qq[pc] = __ldg(reinterpret_cast<const uint2*>(qp + pc * 64 + l16 * 4));
                     }
-                    float bt, gt;
-                    load_scalars(T, t, bt, gt);
+                    uint32_t btb, gtb;
+                    load_scalars(T, t, btb, gtb);
+                    float bt = beta_of(btb), gt = gate_of(gtb);
                     if (p.fused_gating) apply_gating(T.head, bt, gt);
                     prep_kq(kk, qq);
                     if (half == 0) {
@@ -507,7 +512,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
             __syncthreads();  // every thread has read this stage: it may be refilled
 
             // ---- token loop (inputs of token t+1 are fetched from global while token t is computed)
-            auto load_token = [&](int t, uint2* kk, uint2* qq, float* vv, float& bt, float& gt) {
+            auto load_token = [&](int t, uint2* kk, uint2* qq, float* vv, uint32_t& bt, uint32_t& gt) {
                 const long long tok = T.tok0 + t;
                 const __nv_bfloat16* kp = p.k + T.bidx * p.k_sb + tok * p.k_st + T.khead * p.k_sh;
                 const __nv_bfloat16* qp = p.q + T.bidx * p.q_sb + tok * p.q_st + T.khead * p.q_sh;
@@ -645,17 +650,18 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                 }
                 // beta and gate: lane l holds those of token 32 * group + l (group 0 was fetched during
                 // the previous unit), the next group is fetched one group ahead
-                float bsc = beta_first, gsc = g_first, bsn = 0.f, gsn = 0.f;
+                float bsc = beta_first, gsc = g_first;
+                uint32_t bsn = 0u, gsn = 0u;
                 for (int blk = 0; blk < nblk; ++blk) {
                     if ((blk & 3) == 0) {
                         if (blk > 0) {
-                            bsc = bsn;
-                            gsc = gsn;
+                            bsc = beta_of(bsn);
+                            gsc = gate_of(gsn);
                             if (p.fused_gating) apply_gating(T.head, bsc, gsc);  // one lane per token
                         }
                         const int tn = (blk + 4) * TB + lane;
-                        bsn = 0.f;
-                        gsn = 0.f;
+                        bsn = 0u;
+                        gsn = 0u;
                         if (tn < T.ntok) load_scalars(T, tn, bsn, gsn);
                     }
                     const uint8_t* ts;
@@ -720,7 +726,8 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
             } else
             for (int t = 0; t < T.ntok; ++t) {
                 uint2 kn[NQ / 2], qn[NQ / 2];
-                float vn[4], beta_n = 0.f, g_n = 0.f;
+                float vn[4];
+                uint32_t beta_n = 0u, g_n = 0u;
                 if (t + 1 < T.ntok) load_token(t + 1, kn, qn, vn, beta_n, g_n);
                 if (t > 0 || fresh_qk) prep_kq(kw, qw);
                 token_step(t, vr, beta_t, g_t);
@@ -731,8 +738,8 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) vr[j] = vn[j];
-                beta_t = beta_n;
-                g_t = g_n;
+                beta_t = beta_of(beta_n);
+                g_t = gate_of(g_n);
                 if (p.fused_gating && t + 1 < T.ntok) apply_gating(T.head, beta_t, g_t);
             }
 
@@ -759,8 +766,8 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                 }
             }
         }
-        beta_first = beta_next;
-        g_first = g_next;
+        beta_bits = beta_next;
+        g_bits = g_next;
     }
     if (tid == 0 && abort_flag && p.status) atomicExch(p.status, 1);
 }

@@ -85,3 +85,15 @@ def test_no_state_no_gate(gdn):
     o, s = gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], None, bb.cuda(), None, is_qk_norm=True)
     close(o, o_ref, "o")
     close(s, s_ref, "state")
+
+
+@pytest.mark.parametrize("B", [1, 4, 5])
+def test_one_token_tiles_apart_or_together(gdn, B):
+    """one token per sequence: up to 592 tiles of 32 rows (B=4 with 32 v-heads of 128 rows is 512) every tile is a work unit,
+    above that the tiles of a head stay together"""
+    p, pd, beta, g = problem(B, 1, 16, 32, 128, seed=40 + B)
+    bb = beta.bfloat16()
+    o_ref, s_ref = O.recurrent_ref(p["q"].float(), p["k"].float(), p["v"].float(), bb.float(), g, p["state"].float(), is_qk_norm=True)
+    o, s = gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], pd["state"], bb.cuda(), g.cuda(), inference_mode=gdn.Decode, is_qk_norm=True)
+    close(o, o_ref, "o")
+    close(s, s_ref, "state")
