@@ -584,7 +584,7 @@ def main():
                     "eager_us_per_step": 1e3 * ms_small_eager / gsteps,
                     "eager_pybind_us_per_step": None if ms_small_ext is None else 1e3 * ms_small_ext / gsteps,
                     "cuda_graph_us_per_step": 1e3 * ms_small_graph / gsteps,
-                    "note": "eager: one Python call per step through the ctypes / the pybind front end; graph: the same launches replayed"}
+                    "note": "eager: one Python call per step through the package / the module gdn_cuda; graph: the same launches replayed"}
     del small_graph, g_state
 
     # ---------------- speculative verify (B=64, T=4, accepted-token caps ~ U{1..4}, one state per sequence out)

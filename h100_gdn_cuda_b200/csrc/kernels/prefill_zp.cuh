@@ -16,10 +16,10 @@
 // (one M=128 tcgen05 MMA group whose A operand is K stacked on Q) for all the v-heads of the
 // k-head group; only beta and the gate differ between them.  A CTA of 256 threads is two teams of
 // four warps, each team taking one v-head of the group at a time: A / P pass from tensor memory,
-// in-place inverse (fp32 forward substitution on 16x16 blocks, two levels of recursive doubling on
+// in-place inverse (fp32 forward substitution on 8x8 blocks, three levels of recursive doubling on
 // TF32 warp MMAs), T and (diag(d) T)^T as bf16 tiles, then three M=64 MMAs (the two 64-column
 // halves of Z, and PT) and the bf16 epilogue into a staging area that leaves by two bulk copies.
-// Persistent CTAs, two per SM (85 KB of shared memory, 256 tensor-memory columns each).
+// Persistent CTAs, two per SM (92 KB of shared memory, 256 tensor-memory columns each).
 //
 // kWide: head dims 129 .. 256 on 256 columns (one CTA per SM, 512 tensor-memory columns).  Those head dims keep the
 // arithmetic of the fp32 token recurrence they ran on before: every matrix that is not one of the caller's bf16 inputs
