@@ -23,7 +23,8 @@
 //
 // What bounds it: the chain S -> D1 -> R -> dS -> S of each CTA, 8 500 cycles a chunk (D1 1 300 and dS 3 000 of them with
 // the state passes between the quarters, R 1 200); the MMAs alone are 4 000.  B=2, T=1500, 8 v-heads, d=256 (32 CTAs of
-// 24 chunks): 104 us after 39 us of gdn_zp_kernel, where the token recurrence took 1 006 us; same error against fp32.
+// 24 chunks): 104 us after 34 us of gdn_zp_kernel (121 us together, the set-up overlapped), where the token recurrence took
+// 1 006 us; same error against fp32.
 #pragma once
 #include <cuda.h>
 

@@ -187,7 +187,11 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
     // after its own grid_dep_wait.  The release comes AFTER the wait above: the state kernel loads its initial
     // state (which the work before this kernel may have produced: a state handed over from the previous call)
     // without waiting, so it must not be able to start before that work has completed.
-    if (tid == 0) grid_dep_launch();
+    // The wide instance releases it only behind the MMAs of its last unit.  With one CTA per SM a last wave that is not full
+    // leaves SMs empty for a whole unit, and the chains, placed there as these come free, crowd into a few GPCs, where each
+    // takes a quarter longer (B=2, T=1500, 8 v-heads, d=256: 154 -> 121 us; released at the start of the last unit 150).
+    // At head dims up to 128 the early release is the better one by 1 to 2 us.
+    if (!kWide && tid == 0) grid_dep_launch();
 
     const int rep = p.vh / p.kh;               // v-heads per k-head
     const int rounds = (rep + 1) >> 1;         // head pairs per unit
@@ -648,6 +652,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                 ++mma_it;
                 tc_fence_after_sync();
             }
+            if (kWide && tid == 0 && rd == rounds - 1 && unit + static_cast<int>(gridDim.x) >= total_units) grid_dep_launch();
             if (rd == rounds - 1 && tt == 0) {
                 // This team's MMAs have read the K tile (or it sat the round out).  The team that gets here second
                 // knows that both are done with the tiles and requests the next unit's, which land while the
