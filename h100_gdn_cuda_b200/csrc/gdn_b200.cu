@@ -352,7 +352,9 @@ int gdn_causal_conv1d(const GdnConvArgs* a, gdn_stream_t stream) {
     p.batch = a->batch; p.seq_len = a->seq_len; p.channels = a->channels; p.width = a->width; p.silu = a->silu;
     p.total_tokens = a->total_tokens;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const long long tblocks = (tokens + kConvTokBlock - 1) / kConvTokBlock;
+    const long long cblocks = (a->channels / 8 + 127) / 128 * static_cast<long long>(packed ? 1 : a->batch);
+    p.tok_block = tokens <= kConvTokBlock ? kConvTokBlock : conv_tok_block(tokens, cblocks, d->sms);
+    const long long tblocks = (tokens + p.tok_block - 1) / p.tok_block;
     GDN_REQUIRE(tblocks <= 65535 && a->batch <= 65535, "gdn_causal_conv1d: too many token blocks or sequences for one launch");
     if (tblocks > 0) {
         dim3 grid(static_cast<unsigned>((a->channels / 8 + 127) / 128), static_cast<unsigned>(tblocks), packed ? 1u : static_cast<unsigned>(a->batch));

@@ -125,4 +125,24 @@ inline int zp_grid(long long units, int sms, int per_sm) {
     return static_cast<int>(std::min<long long>(units, static_cast<long long>(sms) * per_sm));
 }
 
+// Tokens per thread of the causal convolution.  A CTA streams a block of tokens; what counts is how long the fullest SM is
+// busy.  Fitted to sweeps of the block (B x T from 100 to 32768 tokens, 2048 and 8192 channels): a CTA costs its tokens plus
+// about 9 for its start (weights, the first loads, width - 1 tokens of halo), n CTAs side by side take n + 2 parts where
+// one takes 3, and five fit.  With 32 tokens always, short inputs left most of the GPU idle and long ones its last wave.
+inline int conv_tok_block(long long tokens, long long blocks_per_token_block, int sms) {
+    constexpr int kStart = 9, kPerSm = 5;
+    int best = 32;
+    long long best_cost = -1;
+    for (int t = 4; t <= 64; ++t) {
+        const long long ctas = (tokens + t - 1) / t * blocks_per_token_block;
+        const long long n = (ctas + sms - 1) / sms, rest = n % kPerSm;
+        const long long cost = (n / kPerSm * (kPerSm + 2) + (rest ? rest + 2 : 0)) * (t + kStart);
+        if (best_cost < 0 || cost <= best_cost) {
+            best = t;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 }  // namespace gdn

@@ -10,7 +10,7 @@
 
 namespace gdn {
 
-constexpr int kConvTokBlock = 32;  // tokens per thread along the sequence
+constexpr int kConvTokBlock = 32;  // sequences of up to this many tokens are one block of tokens, whatever the launch's block
 constexpr int kConvMaxWidth = 4;
 constexpr int kConvRing = 8;       // tokens requested ahead per thread
 
@@ -24,6 +24,7 @@ struct ConvParams {
     long long x_sb, x_st, y_sb, y_st;
     const int* cu_seqlens;  // packed mode or NULL
     int batch, seq_len, channels, width, silu;
+    int tok_block;  // tokens per thread along the sequence
     long long total_tokens;
 };
 
@@ -88,12 +89,12 @@ __device__ __forceinline__ uint4 pack8(const f2* f) {
 }
 }  // namespace la
 
-// One thread: 8 adjacent channels, kConvTokBlock consecutive tokens; the last width - 1 inputs slide
+// One thread: 8 adjacent channels, tok_block consecutive tokens; the last width - 1 inputs slide
 // along in registers, so every input is loaded once (plus width - 1 tokens of halo per block).
 // blockIdx.x: channel groups, blockIdx.y: token blocks, blockIdx.z: batch entry (padded mode).
 // Token positions inside the kernel are 32-bit offsets from the block's first token and addresses advance
 // by pointer increments: the kernel is bound by instruction issue, and 64-bit index arithmetic per token was a
-// good part of it.  (Unrolling all 32 tokens, which makes ring slots constants, is slower: 3 k instructions
+// good part of it.  (Unrolling 32 tokens, which makes ring slots constants, is slower: 3 k instructions
 // per thread no longer sit in the instruction cache.)
 template <int W>
 __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvParams p) {
@@ -103,21 +104,12 @@ __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvPar
     const int cg = blockIdx.x * blockDim.x + threadIdx.x;
     if (cg * 8 >= p.channels) return;
     const int c0 = cg * 8;
-    f2 wt[W][4], bs[4];  // channel pairs
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        bs[e] = p.bias ? pk(__bfloat162float(p.bias[c0 + 2 * e]), __bfloat162float(p.bias[c0 + 2 * e + 1])) : pk(0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < W; ++i)
-            wt[i][e] = pk(__bfloat162float(p.w[static_cast<long long>(c0 + 2 * e) * W + i]),
-                          __bfloat162float(p.w[static_cast<long long>(c0 + 2 * e + 1) * W + i]));
-    }
     // the thread's token block [t0, t0 + n_tok) and the sequence it starts in
     const bool packed = p.cu_seqlens != nullptr;
-    const long long t0 = static_cast<long long>(blockIdx.y) * kConvTokBlock;
+    const long long t0 = static_cast<long long>(blockIdx.y) * p.tok_block;
     const long long limit = packed ? p.total_tokens : static_cast<long long>(p.seq_len);
     if (t0 >= limit) return;
-    const int n_tok = static_cast<int>(min(static_cast<long long>(kConvTokBlock), limit - t0));
+    const int n_tok = static_cast<int>(min(static_cast<long long>(p.tok_block), limit - t0));
     int seq;
     const __nv_bfloat16* xb;
     __nv_bfloat16* yb;
@@ -176,6 +168,15 @@ __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvPar
     };
 #pragma unroll
     for (int u = 0; u < kConvRing; ++u) request(u);
+    f2 wt[W][4], bs[4];  // channel pairs (read behind the first requests, so that the two latencies overlap)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        bs[e] = p.bias ? pk(__bfloat162float(p.bias[c0 + 2 * e]), __bfloat162float(p.bias[c0 + 2 * e + 1])) : pk(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            wt[i][e] = pk(__bfloat162float(p.w[static_cast<long long>(c0 + 2 * e) * W + i]),
+                          __bfloat162float(p.w[static_cast<long long>(c0 + 2 * e + 1) * W + i]));
+    }
     // The last W inputs are kept unpacked in W register sets used as a ring: step R of every W consecutive
     // tokens finds tap i in set (R + i) % W and puts the new token into set (R + W - 1) % W, so nothing is
     // ever moved or unpacked twice.
@@ -221,9 +222,9 @@ __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvPar
 #pragma unroll 1
     for (int j = 0; j < n_tok; j += W) {
         step(std::integral_constant<int, 0>{}, j);
-        if (j + 1 < n_tok && j + 1 < kConvTokBlock) step(std::integral_constant<int, 1 % W>{}, j + 1);
-        if (W > 2 && j + 2 < n_tok && j + 2 < kConvTokBlock) step(std::integral_constant<int, 2 % W>{}, j + 2);
-        if (W > 3 && j + 3 < n_tok && j + 3 < kConvTokBlock) step(std::integral_constant<int, 3 % W>{}, j + 3);
+        if (j + 1 < n_tok) step(std::integral_constant<int, 1 % W>{}, j + 1);
+        if (W > 2 && j + 2 < n_tok) step(std::integral_constant<int, 2 % W>{}, j + 2);
+        if (W > 3 && j + 3 < n_tok) step(std::integral_constant<int, 3 % W>{}, j + 3);
     }
 }
 

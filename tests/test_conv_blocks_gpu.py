@@ -1,0 +1,43 @@
+"""causal_conv1d where the launch picks its tokens per thread: just above one block, blocks below and above 32 tokens, a last
+block of one token, packed sequences whose ends fall anywhere in a block."""
+import pytest
+import torch
+
+from oracle import gdn_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# bf16 output: half a unit in the last place is at most 2^-9 of a value; SiLU's hardware tanh adds 2^-11 on a factor of
+# (1 + tanh) / 2: together below 2^-8
+TOL = 2.0 ** -8
+
+
+@pytest.fixture(scope="module")
+def gdn():
+    import h100_gdn_cuda_b200 as g
+    return g
+
+
+@pytest.mark.parametrize("B,T,C_,W", [(1, 33, 64, 4), (2, 37, 8, 3), (1, 505, 2048, 2), (3, 1000, 1032, 3), (1, 4097, 8192, 4)])
+def test_conv_padded_blocks(gdn, B, T, C_, W):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(B, T, C_, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(C_, W, generator=gen, device="cuda") * 0.5).bfloat16()
+    s0 = torch.randn(B, W - 1, C_, generator=gen, device="cuda").bfloat16()
+    y, fin = gdn.api.causal_conv1d(x, w, None, s0, return_final_state=True)
+    y_ref, fin_ref = O.causal_conv1d_ref(x.cpu(), w.cpu(), None, s0.cpu())
+    assert O.rel_fro(y.cpu(), y_ref) < TOL
+    assert torch.equal(fin.float().cpu(), fin_ref)
+
+
+def test_conv_packed_blocks(gdn):
+    lens = [5, 0, 61, 1, 1, 130, 7, 64, 300]
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    gen = torch.Generator().manual_seed(9)
+    x = torch.randn(sum(lens), 520, generator=gen).bfloat16()
+    w = (torch.randn(520, 4, generator=gen) * 0.5).bfloat16()
+    s0 = torch.randn(len(lens), 3, 520, generator=gen).bfloat16()
+    y, fin = gdn.api.causal_conv1d(x.cuda(), w.cuda(), None, s0.cuda(), cu_seqlens=cu.cuda(), return_final_state=True)
+    y_ref, fin_ref = O.causal_conv1d_ref(x, w, None, s0, cu_seqlens=cu.tolist())
+    assert O.rel_fro(y.cpu(), y_ref) < TOL
+    assert torch.equal(fin.float().cpu(), fin_ref)
