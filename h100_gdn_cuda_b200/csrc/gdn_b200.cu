@@ -386,15 +386,19 @@ int gdn_gated_rmsnorm(const void* x, const void* z, void* y, const void* weight,
     // lanes per row: the smallest power of two (4 .. 32) whose 16-byte pieces cover the row in one pass
     int lpr = 4;
     while (lpr < 32 && lpr * 8 < dim) lpr *= 2;
-    const long long rows_per_block = 8ll * (32 / lpr) * (lpr == 32 ? 1 : 2);  // 8 warps, rows in flight per lane group as in the kernel
+    const int passes = dim <= 256 ? 1 : dim <= 512 ? 2 : 4;  // of 256 elements
+    const long long rows_per_block = 8ll * (32 / lpr) * norm_unroll(passes);  // 8 warps, rows in flight per lane group
     const long long blocks = (rows + rows_per_block - 1) / rows_per_block;
     GDN_REQUIRE(blocks < (1ll << 31), "gdn_gated_rmsnorm: too many rows");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (lpr) {
-        case 4: GDN_CUDA(launch_dependent(gdn_gated_rmsnorm_kernel<4>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p)); break;
-        case 8: GDN_CUDA(launch_dependent(gdn_gated_rmsnorm_kernel<8>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p)); break;
-        case 16: GDN_CUDA(launch_dependent(gdn_gated_rmsnorm_kernel<16>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p)); break;
-        default: GDN_CUDA(launch_dependent(gdn_gated_rmsnorm_kernel<32>, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p)); break;
+    auto launch = [&](auto kernel) { return launch_dependent(kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, st, p); };
+    switch (lpr * passes) {
+        case 4: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<4, 1>)); break;
+        case 8: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<8, 1>)); break;
+        case 16: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<16, 1>)); break;
+        case 32: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<32, 1>)); break;
+        case 64: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<32, 2>)); break;
+        default: GDN_CUDA(launch(gdn_gated_rmsnorm_kernel<32, 4>)); break;
     }
     return GDN_OK;
 }
