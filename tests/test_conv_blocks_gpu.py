@@ -41,3 +41,13 @@ def test_conv_packed_blocks(gdn):
     y_ref, fin_ref = O.causal_conv1d_ref(x, w, None, s0, cu_seqlens=cu.tolist())
     assert O.rel_fro(y.cpu(), y_ref) < TOL
     assert torch.equal(fin.float().cpu(), fin_ref)
+
+
+@pytest.mark.parametrize("W", [2, 3, 4])
+def test_conv_weight_alignment(gdn, W):
+    """The taps are read 16 bytes at a time where the weight allows it: a weight at an odd element gives the same bits."""
+    gen = torch.Generator(device="cuda").manual_seed(W)
+    x = torch.randn(2, 70, 72, generator=gen, device="cuda").bfloat16()
+    flat = torch.randn(72 * W + 1, generator=gen, device="cuda").bfloat16()
+    w = flat[1:].view(72, W)
+    assert torch.equal(gdn.api.causal_conv1d(x, w), gdn.api.causal_conv1d(x, w.clone()))
