@@ -317,7 +317,7 @@ def _check_head_dim(d: int):
     _require(0 < d <= _PREFILL_D, "chunked kernels support head dims up to %d (got %d)" % (_PREFILL_D, d))
 
 
-_PREFILL_D_MAX = 256  # chunked_forward takes head dims up to here
+_PREFILL_D_MAX = 256  # chunked_forward takes head dims up to here (above 128: the token-recurrent kernel)
 
 
 def chunked_forward_workspace_bytes(batch: int, seq_len: int, num_v_heads: int, total_tokens: int = 0,
@@ -356,9 +356,10 @@ def chunked_forward(query, key, value, beta, gate, scale: Optional[float] = None
     _require(0 < d <= _PREFILL_D_MAX, "chunked_forward supports head dims up to %d (got %d)" % (_PREFILL_D_MAX, d))
     if scale is None:
         scale = 1.0 / math.sqrt(d)
-    # The kernels compute on 128 columns, above that on 256.  A head dim that is a multiple of 8 goes in as it is
-    # (the library's tensor maps supply the zero columns, nothing is copied); any other is zero-padded here.
-    D = d if d % 8 == 0 else (_PREFILL_D if d <= _PREFILL_D else _PREFILL_D_MAX)
+    # up to 128: the tensor-core kernels, which compute on 128 columns.  A head dim that is a multiple of 8
+    # goes in as it is (the library's tensor maps supply the zero columns, nothing is copied); any other is
+    # zero-padded to 128 here.  129..256: the library runs the token recurrence on 192 or 256 columns instead.
+    D = (d if d % 8 == 0 else _PREFILL_D) if d <= _PREFILL_D else _aligned_dim(d)
     q, k, v = (_tma_ready(_pad_last(t, D)) for t in (query, key, value))
     s_in = _pad_state(initial_state, D)
     if s_in is not None:

@@ -8,7 +8,6 @@
 #include "kernels/prefill_segments.cuh"
 #include "kernels/prefill_transition.cuh"
 #include "kernels/prefill_uw.cuh"
-#include "kernels/prefill_wide.cuh"
 #include "kernels/prefill_zp.cuh"
 #include "tma_host.hpp"
 
@@ -153,9 +152,8 @@ int launch_zp(const GdnShape& s, const CUtensorMap& tmQ, const CUtensorMap& tmK,
     p.vh = s.num_v_heads;
     p.num_chunks = nc;
     p.status = d->status;
-    const bool wide = s.head_dim_k > kD;
-    const int smem = wide ? ZPSmem<true>::kBytes : ZPSmem<false>::kBytes;
-    const int grid = zp_grid(static_cast<long long>(nc) * s.num_k_heads, d->sms, wide ? 1 : 2);
+    constexpr int smem = ZPSmem::kBytes;
+    const int grid = zp_grid(static_cast<long long>(nc) * s.num_k_heads, d->sms);
     // launched as a programmatic dependent of the preceding work in the stream (the kernel waits before its
     // first global read): its launch and set-up overlap that work's tail
     cudaLaunchConfig_t cfg{};
@@ -168,14 +166,13 @@ int launch_zp(const GdnShape& s, const CUtensorMap& tmQ, const CUtensorMap& tmK,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    auto launch = [&](auto norm_tag, auto wide_tag) -> int {
-        constexpr auto kernel = gdn_zp_kernel<decltype(norm_tag)::value, decltype(wide_tag)::value>;
+    auto launch = [&](auto norm_tag) -> int {
+        constexpr auto kernel = gdn_zp_kernel<decltype(norm_tag)::value>;
         if (int rc = set_smem<kernel>(smem)) return rc;
         GDN_CUDA(cudaLaunchKernelEx(&cfg, kernel, tmK, tmQ, p));
         return GDN_OK;
     };
-    if (wide) return norms ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{});
-    return norms ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{});
+    return norms ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 template <bool O, bool H, bool UN>
@@ -191,20 +188,19 @@ int launch_seq_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorM
 // Launch of the state kernel right after the chunk-parallel kernel in the same stream, with
 // programmatic stream serialization: its CTAs may be placed (each takes a whole SM) and set up while
 // that kernel drains; the kernel waits (grid_dep_wait) before it reads that kernel's results.
-template <typename Kernel>
-cudaError_t launch_after_zp(Kernel* kernel, dim3 grid, int threads, int smem, cudaStream_t st, const CUtensorMap& tmQ,
-                                   const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmO, const FusedParams& p) {
+cudaError_t launch_fused_after_zp(dim3 grid, cudaStream_t st, const CUtensorMap& tmQ, const CUtensorMap& tmK,
+                                  const CUtensorMap& tmV, const CUtensorMap& tmO, const FusedParams& p) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.blockDim = dim3(fused::kThreads);
+    cfg.dynamicSmemBytes = FusedSmem::kBytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, tmQ, tmK, tmV, tmO, p);
+    return cudaLaunchKernelEx(&cfg, gdn_fused_seq_kernel, tmQ, tmK, tmV, tmO, p);
 }
 
 }  // namespace
@@ -313,19 +309,49 @@ int gdn_compute_o(const GdnComputeOArgs* a, gdn_stream_t stream) {
     return GDN_OK;
 }
 
-// Head dims above 128 (up to 256, which the reference's chunked kernels accept:
-// sm90_bf16_gdn_compute_u_w.cuh:169) run on 256 columns (prefill_wide.cuh).
+// Head dims above the 128 the tensor-core kernels are built for (192 and 256, which the
+// reference's chunked kernels accept: sm90_bf16_gdn_compute_u_w.cuh:169) take the token-recurrent
+// kernel: the same layer semantics with the state and all intermediates in fp32 from the first token to the
+// last, no scratch, one launch.  (A chunked form on 256 columns whose operands were sums of two bf16 terms, 16
+// significand bits, took 129 us where this takes 1 006, B=2 T=1500 8 v-heads d=256, but stood further from the
+// 64-bit result: 0.1 to 0.55 % of the bf16 outputs rounded the other way against 0.003 to 0.16 %.)
 static bool wide_heads(const GdnShape& s) { return s.head_dim_k > kD || s.head_dim_v > kD; }
 
-// Workspace layout of gdn_chunked_forward: [Z, PT blocks][q/k norm factors][segment states | sequence order]
-static size_t ws_blocks_bytes(size_t chunks, const GdnShape& s) {
-    return (chunks * static_cast<size_t>(s.num_v_heads) * (wide_heads(s) ? kWideBlockBytes : kZPBlockBytes) + 255) / 256 * 256;
+static int chunked_forward_wide(const GdnChunkedArgs* a, gdn_stream_t stream) {
+    const GdnShape& s = a->shape;
+    GDN_REQUIRE(s.head_dim_k == s.head_dim_v && s.head_dim_k % 64 == 0 && s.head_dim_k <= 256,
+                "gdn_chunked_forward: head dims above 128 must be dk = dv = 192 or 256 (got %d, %d); pad with zeros",
+                s.head_dim_k, s.head_dim_v);
+    GDN_REQUIRE(a->final_state.ptr != nullptr, "gdn_chunked_forward: head dims above 128 need a final_state buffer");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    void* const* ev = a->stage_events;
+    if (ev) {
+        GDN_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(ev[0]), st));
+        GDN_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(ev[1]), st));
+    }
+    GdnRecurrentArgs r{};
+    r.shape = s;
+    r.q = a->q;
+    r.k = a->k;
+    r.v = a->v;
+    r.out = a->out;
+    r.beta = a->beta;
+    r.gate = a->gate;
+    r.state_in = a->initial_state;
+    r.state_out = a->final_state;
+    r.scale = a->scale;
+    r.is_qk_norm = a->is_qk_norm;
+    if (int rc = gdn_recurrent_forward(&r, stream)) return rc;
+    if (ev) GDN_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(ev[2]), st));
+    return GDN_OK;
 }
+
+// Workspace layout of gdn_chunked_forward: [Z, PT blocks][q/k norm factors][segment states | sequence order]
+static size_t ws_blocks_bytes(size_t chunks, int vh) { return (chunks * static_cast<size_t>(vh) * kZPBlockBytes + 255) / 256 * 256; }
 static size_t ws_norms_bytes(size_t chunks, int kh) { return (chunks * static_cast<size_t>(kh) * 128 * sizeof(float) + 255) / 256 * 256; }
 
 // The segment plan of a problem (heuristics.hpp); num_segments == 1: not segmented.
 static SegmentPlan segment_plan_of(const GdnShape& s) {
-    if (wide_heads(s)) return SegmentPlan{1, 0, 0};
     if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, s.total_chunks > 0 ? s.total_chunks : 0);
     SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, (s.seq_len + kChunk - 1) / kChunk, false);
     plan.slots = s.batch * plan.num_segments;
@@ -334,11 +360,12 @@ static SegmentPlan segment_plan_of(const GdnShape& s) {
 
 size_t gdn_chunked_forward_workspace_bytes(const GdnShape* s) {
     if (!s) return 0;
+    if (wide_heads(*s)) return 0;
     const size_t chunks = s->cu_seqlens ? static_cast<size_t>(s->total_chunks > 0 ? s->total_chunks : 0)
                                         : static_cast<size_t>(s->batch) * static_cast<size_t>((s->seq_len + kChunk - 1) / kChunk);
-    // one block of Z (64 x 128 bf16) and PT (64 x 64 bf16) per (chunk, v-head), two terms of 256 columns for wide heads; for a
+    // one block of Z (64 x 128 bf16) and PT (64 x 64 bf16) per (chunk, v-head); for a
     // segmented run (few long sequences) three fp32 states per v-head and segment slot on top
-    size_t bytes = ws_blocks_bytes(chunks, *s) + ws_norms_bytes(chunks, s->num_k_heads) + 256;
+    size_t bytes = ws_blocks_bytes(chunks, s->num_v_heads) + ws_norms_bytes(chunks, s->num_k_heads) + 256;
     const SegmentPlan plan = segment_plan_of(*s);
     if (plan.num_segments > 1)
         bytes += static_cast<size_t>(plan.slots) * s->num_v_heads * 3 * kD * kD * sizeof(float) + 256;
@@ -351,14 +378,14 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     GDN_REQUIRE(a != nullptr, "gdn_chunked_forward: args is NULL");
     const GdnShape& s = a->shape;
     if (int rc = check_shape(s, true)) return rc;
-    // The kernels are built for dk = dv = 128 and 256.  A smaller head dim that is a multiple of 8 (the 16-byte
+    if (wide_heads(s)) return chunked_forward_wide(a, stream);
+    // The kernels are built for dk = dv = 128.  A smaller head dim that is a multiple of 8 (the 16-byte
     // rule of the copies) runs on them as it is: the tensor maps deliver zero columns past it and the state
     // is read and written with a column predicate, which is the zero-padded problem without padded copies.
     const int hd = s.head_dim_k;
-    const bool wide = wide_heads(s);
-    if (s.head_dim_k != s.head_dim_v || hd % 8 != 0 || hd > 256)
+    if (s.head_dim_k != s.head_dim_v || hd % 8 != 0)
         return fail(GDN_ERR_UNSUPPORTED,
-                    "gdn_chunked_forward: head dims must be dk = dv, a multiple of 8 up to 256 (got %d, %d); "
+                    "gdn_chunked_forward: head dims must be dk = dv, a multiple of 8 up to 128, or 192 / 256 (got %d, %d); "
                     "pad the head dimension with zeros (the Python and C++ wrappers do)", s.head_dim_k, s.head_dim_v);
     if (int rc = check_token_tensor(a->q, "q", hd)) return rc;
     if (int rc = check_token_tensor(a->k, "k", hd)) return rc;
@@ -368,7 +395,7 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     if (int rc = check_scalar(a->gate, "gate", false)) return rc;
     if (int rc = check_state(a->initial_state, "initial_state")) return rc;
     if (int rc = check_state(a->final_state, "final_state")) return rc;
-    GDN_REQUIRE(s.num_v_heads <= (wide ? 32767 : 65535), "too many heads");
+    GDN_REQUIRE(s.num_v_heads <= 65535, "too many heads");
     const size_t need = gdn_chunked_forward_workspace_bytes(&s);
     if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 255u))
         return fail(GDN_ERR_WORKSPACE, "gdn_chunked_forward: workspace of %zu bytes (256-byte aligned) required, got %zu",
@@ -390,8 +417,8 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     }
     uint8_t* const ws = static_cast<uint8_t*>(a->workspace);
     const size_t nchunks = static_cast<size_t>(num_chunks(s));
-    float* const norms = a->is_qk_norm ? reinterpret_cast<float*>(ws + ws_blocks_bytes(nchunks, s)) : nullptr;
-    uint8_t* const ws_extra = ws + ws_blocks_bytes(nchunks, s) + ws_norms_bytes(nchunks, s.num_k_heads);
+    float* const norms = a->is_qk_norm ? reinterpret_cast<float*>(ws + ws_blocks_bytes(nchunks, s.num_v_heads)) : nullptr;
+    uint8_t* const ws_extra = ws + ws_blocks_bytes(nchunks, s.num_v_heads) + ws_norms_bytes(nchunks, s.num_k_heads);
     // Both kernels are prepared before the first is launched, so that the state kernel is in the stream
     // when the chunk-parallel kernel starts to drain.
     CUtensorMap tmQ, tmK, tmV, tmO;
@@ -422,15 +449,10 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
         p.status = d->status;
         p.blocks = static_cast<const uint8_t*>(a->workspace);
         p.norms = norms;
-        const int smem = wide ? WideSmem::kBytes : FusedSmem::kBytes;
-        if (int rc = wide ? set_smem<gdn_wide_seq_kernel>(smem) : set_smem<gdn_fused_seq_kernel>(smem)) return rc;
-        const int per_seq = wide ? 2 * s.num_v_heads : s.num_v_heads;  // CTAs of the state kernel per sequence
-        const long long chains = static_cast<long long>(s.batch) * per_seq;
+        if (int rc = set_smem<gdn_fused_seq_kernel>(FusedSmem::kBytes)) return rc;
+        const long long chains = static_cast<long long>(s.batch) * s.num_v_heads;
         auto run_seq = [&](dim3 grid) -> int {
-            if (wide)
-                GDN_CUDA(launch_after_zp(gdn_wide_seq_kernel, grid, wide::kThreads, smem, st, tmQ, tmK, tmV, tmO, p));
-            else
-                GDN_CUDA(launch_after_zp(gdn_fused_seq_kernel, grid, fused::kThreads, smem, st, tmQ, tmK, tmV, tmO, p));
+            GDN_CUDA(launch_fused_after_zp(grid, st, tmQ, tmK, tmV, tmO, p));
             return GDN_OK;
         };
         const SegmentPlan plan = segment_plan_of(s);
@@ -441,10 +463,10 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
             GDN_CUDA(cudaGetLastError());
             p.seq_order = order;
             if (int rc = run_zp()) return rc;
-            if (int rc = run_seq(dim3(per_seq, s.batch))) return rc;
+            if (int rc = run_seq(dim3(s.num_v_heads, s.batch))) return rc;
         } else if (plan.num_segments <= 1) {
             if (int rc = run_zp()) return rc;
-            if (int rc = run_seq(dim3(s.batch, per_seq))) return rc;
+            if (int rc = run_seq(dim3(s.batch, s.num_v_heads))) return rc;
         } else {
             // composite transitions of all segments, their start states, then all segments at once
             float* seg_mn = reinterpret_cast<float*>(ws_extra);

@@ -120,9 +120,9 @@ inline int uw_grid(long long units, int sms) {
 }
 
 // Grid of the persistent chunk-parallel kernel of the whole-layer path (units = chunks x k-heads,
-// two CTAs of 256 threads per SM, one for head dims above 128).
-inline int zp_grid(long long units, int sms, int per_sm) {
-    return static_cast<int>(std::min<long long>(units, static_cast<long long>(sms) * per_sm));
+// two CTAs of 256 threads per SM).
+inline int zp_grid(long long units, int sms) {
+    return static_cast<int>(std::min<long long>(units, static_cast<long long>(sms) * 2));
 }
 
 // Tokens per thread of the causal convolution.  A CTA streams a block of tokens; what counts is how long the fullest SM is

@@ -11,9 +11,6 @@ constexpr int kChunk = 64;
 // prefill_zp.cuh): per (global chunk, v-head) unit Z (64 x 128 bf16 as two 64 x 64 swizzled atoms, the
 // shared-memory image of an MN-major B operand) and then PT (64 x 64, one atom).
 constexpr int kZPBlockBytes = kChunk * 128 * 2 + kChunk * kChunk * 2;
-// Head dims above 128 run on 256 columns with every matrix as a sum of two bf16 terms: Z hi, Z lo (four atoms each),
-// PT hi, PT lo.
-constexpr int kWideBlockBytes = 2 * (kChunk * 256 * 2 + kChunk * kChunk * 2);
 
 // per-token scalar tensor (beta or gate) as the kernels see it
 struct ScalarView {

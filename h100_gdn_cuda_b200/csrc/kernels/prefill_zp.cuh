@@ -20,11 +20,6 @@
 // TF32 warp MMAs), T and (diag(d) T)^T as bf16 tiles, then three M=64 MMAs (the two 64-column
 // halves of Z, and PT) and the bf16 epilogue into a staging area that leaves by two bulk copies.
 // Persistent CTAs, two per SM (92 KB of shared memory, 256 tensor-memory columns each).
-//
-// kWide: head dims 129 .. 256 on 256 columns (one CTA per SM, 512 tensor-memory columns).  Those head dims keep the
-// arithmetic of the fp32 token recurrence they ran on before: every matrix that is not one of the caller's bf16 inputs
-// (P, T, dT, and Z, PT for the state kernel) is carried as a sum of two bf16 terms, x = hi + lo (16 significand
-// bits), products as hi.hi + hi.lo + lo.hi, and the inverse takes its TF32 products in three terms the same way.
 #pragma once
 #include <cuda.h>
 
@@ -47,17 +42,16 @@ struct ZPParams {
     int* status;
 };
 
-template <bool kWide = false>
 struct ZPSmem {
-    static constexpr int kAtoms = kWide ? 4 : 2;  // 64-column swizzle atoms of a K or Q tile
+    static constexpr int kAtoms = 2;  // 64-column swizzle atoms of a K or Q tile
     static constexpr int kLd = 68;  // fp32 row stride of A, conflict-free for the MMA fragment loads
     // K and Q tiles interleaved atom by atom: [K cols 0-63 | Q cols 0-63 | K cols 64-127 | Q cols 64-127],
     // 8 KB each, so that rows 0-127 of one atom pair are K stacked on Q (the M=128 A operand)
     static constexpr int kOffKQ = 0;
     static constexpr int kTeam = kAtoms * 16384;         // per-team area starts here, two of them
-    static constexpr int kOffA = 0;                      // A / X fp32 (17 KB), later T | dT (kWide: T hi, dT hi, T lo, dT lo), later the staged Z
-    static constexpr int kOffP = kWide ? 32768 : 64 * kLd * 4;  // P tile (8 KB; kWide: hi, lo), later the staged PT
-    static constexpr int kOffVec = kOffP + (kWide ? 16384 : 8192);  // beta[64], g log2e[64], d[64], scan partials[64], column factors[32]
+    static constexpr int kOffA = 0;                      // A / X fp32 (17 KB), later T | dT, later the staged Z
+    static constexpr int kOffP = 64 * kLd * 4;           // 17408: P tile (8 KB), later the staged PT
+    static constexpr int kOffVec = kOffP + 8192;         // beta[64], g log2e[64], d[64], scan partials[64], column factors[32]
     static constexpr int kTeamBytes = kOffVec + 2048;    // a multiple of 1024
     static constexpr int kOffNorm = kTeam + 2 * kTeamBytes;  // kNorm: inverse row norms of K [64] and Q [64], their log2 [128]
     static constexpr int kOffBar = kOffNorm + 1024;
@@ -71,53 +65,30 @@ namespace zp {
 constexpr int kThreads = 256;
 constexpr uint32_t kTmKQ = 0;    // fp32 K K^T (lanes 0-63) and Q K^T (lanes 64-127), 64 columns
 constexpr uint32_t kTmPT = 64;   // PT of team 0 (lanes +0) and team 1 (lanes +16), 64 columns
-constexpr uint32_t kTmZ = 128;   // + 64 (kWide: 128) * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16), kWide: 128-255 in the next 64
+constexpr uint32_t kTmZ = 128;   // + 64 * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16)
 // two neighbouring warps of a team
 __device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(3 + pair) : "memory"); }
-// TF32 operands of the inverse's block products; kSplit: with the rounding error as a second term, and three
-// products per block (what the second terms' product would add is below fp32's own rounding)
-template <bool kSplit, int N>
-struct Frag {
-    uint32_t hi[N], lo[kSplit ? N : 1];
-    __device__ __forceinline__ void set(int i, float x) {
-        hi[i] = uw::to_tf32(x);
-        if (kSplit) lo[i] = uw::to_tf32(x - __uint_as_float(hi[i]));
-    }
-};
-template <bool kSplit>
-__device__ __forceinline__ void mma_frag(float* d, const Frag<kSplit, 4>& a, const Frag<kSplit, 2>& b) {
-    uw::mma_tf32(d, a.hi, b.hi);
-    if (kSplit) {
-        uw::mma_tf32(d, a.lo, b.hi);
-        uw::mma_tf32(d, a.hi, b.lo);
-    }
-}
-// 16x8 fragment of `m` at [r0][k0] as the A operand (kRows 8: the lower half is zero), 8x8 at [k0][n0] as the B operand
-template <bool kSplit, int kRows = 16>
-__device__ __forceinline__ void load_a(Frag<kSplit, 4>& a, const float* m, int ld, int r0, int k0, int lane) {
+// TF32 operands of the inverse's block products: 16x8 fragment of `m` at [r0][k0] as the A operand (kRows 8: the lower
+// half is zero), 8x8 at [k0][n0] as the B operand
+template <int kRows = 16>
+__device__ __forceinline__ void load_a(uint32_t* a, const float* m, int ld, int r0, int k0, int lane) {
     const int g = lane >> 2, t = lane & 3;
-    a.set(0, m[(r0 + g) * ld + k0 + t]);
-    a.set(1, kRows == 16 ? m[(r0 + g + 8) * ld + k0 + t] : 0.f);
-    a.set(2, m[(r0 + g) * ld + k0 + t + 4]);
-    a.set(3, kRows == 16 ? m[(r0 + g + 8) * ld + k0 + t + 4] : 0.f);
+    a[0] = uw::to_tf32(m[(r0 + g) * ld + k0 + t]);
+    a[1] = kRows == 16 ? uw::to_tf32(m[(r0 + g + 8) * ld + k0 + t]) : 0u;
+    a[2] = uw::to_tf32(m[(r0 + g) * ld + k0 + t + 4]);
+    a[3] = kRows == 16 ? uw::to_tf32(m[(r0 + g + 8) * ld + k0 + t + 4]) : 0u;
 }
-template <bool kSplit>
-__device__ __forceinline__ void load_b(Frag<kSplit, 2>& b, const float* m, int ld, int k0, int n0, int lane) {
+__device__ __forceinline__ void load_b(uint32_t* b, const float* m, int ld, int k0, int n0, int lane) {
     const int g = lane >> 2, t = lane & 3;
-    b.set(0, m[(k0 + t) * ld + n0 + g]);
-    b.set(1, m[(k0 + t + 4) * ld + n0 + g]);
+    b[0] = uw::to_tf32(m[(k0 + t) * ld + n0 + g]);
+    b[1] = uw::to_tf32(m[(k0 + t + 4) * ld + n0 + g]);
 }
-template <bool kSplit, int kRows = 16>
+template <int kRows = 16>
 __device__ __forceinline__ void mma_blk(float* d, const float* am, int r0, int k0, const float* bm, int k0b, int n0, int ld, int lane) {
-    Frag<kSplit, 4> a;
-    Frag<kSplit, 2> b;
-    load_a<kSplit, kRows>(a, am, ld, r0, k0, lane);
-    load_b<kSplit>(b, bm, ld, k0b, n0, lane);
-    mma_frag<kSplit>(d, a, b);
-}
-// two bf16 terms of a pair: hi = bf16(x), lo = bf16(x - hi)
-__device__ __forceinline__ uint32_t pack_lo(float a, float b, uint32_t hi) {
-    return ptx::pack_bf16(a - ptx::bf16_lo(hi), b - ptx::bf16_hi(hi));
+    uint32_t a[4], b[2];
+    load_a<kRows>(a, am, ld, r0, k0, lane);
+    load_b(b, bm, ld, k0b, n0, lane);
+    uw::mma_tf32(d, a, b);
 }
 __device__ __forceinline__ void team_sync(int team) {
     if (team)
@@ -131,14 +102,14 @@ __device__ __forceinline__ void team_sync(int team) {
 // (k_i.k_j) r_i r_j and (q_i.k_j) rq_i r_j enter through the row factor of the A / P pass and through
 // the column's gate (g_j - log2 r_j in the exponent), Z = (dT)^T diag(r) K through d_i r_i.  The
 // factors are also written to `norms` for the state kernel.
-template <bool kNorm, bool kWide = false>
-__global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(const __grid_constant__ CUtensorMap tmK,
+template <bool kNorm>
+__global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                  const __grid_constant__ CUtensorMap tmQ,
                                                                  const ZPParams p) {
     using namespace ptx;
     using namespace uw;
     using namespace zp;
-    using L = ZPSmem<kWide>;
+    using L = ZPSmem;
     constexpr int LD = L::kLd, NA = L::kAtoms;
     extern __shared__ uint8_t smem_raw[];
     // aligned by an offset from the array itself, so that the compiler still knows the pointer is shared memory
@@ -174,7 +145,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
         mbar_init(&bar_mma[1], 1);
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(tmem_slot, kWide ? 512 : 256);
+    if (warp == 0) tmem_alloc(tmem_slot, 256);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -187,11 +158,7 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
     // after its own grid_dep_wait.  The release comes AFTER the wait above: the state kernel loads its initial
     // state (which the work before this kernel may have produced: a state handed over from the previous call)
     // without waiting, so it must not be able to start before that work has completed.
-    // The wide instance releases it only behind the MMAs of its last unit.  With one CTA per SM a last wave that is not full
-    // leaves SMs empty for a whole unit, and the chains, placed there as these come free, crowd into a few GPCs, where each
-    // takes a quarter longer (B=2, T=1500, 8 v-heads, d=256: 154 -> 121 us; released at the start of the last unit 150).
-    // At head dims up to 128 the early release is the better one by 1 to 2 us.
-    if (!kWide && tid == 0) grid_dep_launch();
+    if (tid == 0) grid_dep_launch();
 
     const int rep = p.vh / p.kh;               // v-heads per k-head
     const int rounds = (rep + 1) >> 1;         // head pairs per unit
@@ -431,10 +398,6 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                                     const uint4 h = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]),
                                                                pack_bf16(o[6], o[7]));
                                     *reinterpret_cast<uint4*>(sP + tile_off(i, (32 * cb + j) >> 3)) = h;
-                                    if (kWide)
-                                        *reinterpret_cast<uint4*>(sP + 8192 + tile_off(i, (32 * cb + j) >> 3)) =
-                                            make_uint4(pack_lo(o[0], o[1], h.x), pack_lo(o[2], o[3], h.y), pack_lo(o[4], o[5], h.z),
-                                                       pack_lo(o[6], o[7], h.w));
                                 }
                             }
                         };
@@ -449,10 +412,8 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     }
                     if (is_p && rb == 0) {  // rows 0-31 of P: columns 32-63 lie above the diagonal
 #pragma unroll
-                        for (int c16 = 4; c16 < 8; ++c16) {
+                        for (int c16 = 4; c16 < 8; ++c16)
                             *reinterpret_cast<uint4*>(sP + tile_off(i, c16)) = make_uint4(0u, 0u, 0u, 0u);
-                            if (kWide) *reinterpret_cast<uint4*>(sP + 8192 + tile_off(i, c16)) = make_uint4(0u, 0u, 0u, 0u);
-                        }
                     }
                 }
                 if (rd + 1 < rounds) {
@@ -495,20 +456,17 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     // level 0 (8 -> 16)
                     const int i0 = 16 * b + 8, j0 = 16 * b;
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_blk<kWide, 8>(d, sA, i0, j0, sA, j0, j0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
+                    mma_blk<8>(d, sA, i0, j0, sA, j0, j0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
                     // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
                     const int g = lane >> 2, tq = lane & 3;
                     const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
                     const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
                     const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
                     const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
-                    Frag<kWide, 2> bfrag;
-                    bfrag.set(0, (g & 1) ? v01 : v00);
-                    bfrag.set(1, (g & 1) ? v11 : v10);
-                    Frag<kWide, 4> afrag;
-                    load_a<kWide, 8>(afrag, sA, LD, i0, i0, lane);
+                    uint32_t bfrag[2] = {to_tf32((g & 1) ? v01 : v00), to_tf32((g & 1) ? v11 : v10)}, afrag[4];
+                    load_a<8>(afrag, sA, LD, i0, i0, lane);
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_frag<kWide>(e, afrag, bfrag);  // X_11 t
+                    mma_tf32(e, afrag, bfrag);  // X_11 t
                     *reinterpret_cast<float2*>(&sA[(i0 + g) * LD + j0 + 2 * tq]) = make_float2(-e[0], -e[1]);
                 }
                 team_sync(team);
@@ -519,12 +477,12 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     const int i0 = 16 * (2 * pr + 1), j0 = 16 * (2 * pr);
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(d, sA, i0, j0 + 8 * ks, sA, j0 + 8 * ks, j0 + n0, LD, lane);
+                    for (int ks = 0; ks < 2; ++ks) mma_blk(d, sA, i0, j0 + 8 * ks, sA, j0 + 8 * ks, j0 + n0, LD, lane);
                     store_block(d, 1.f, sA, LD, j0, i0 + n0, lane);
                     __syncwarp();  // the 8 columns of the intermediate are this warp's alone
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_blk<kWide>(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
+                    for (int ks = 0; ks < 2; ++ks) mma_blk(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
                     pair_sync(2 * team + pr);  // both warps of the pair have read A_10
                     store_block(e, -1.f, sA, LD, i0, j0 + n0, lane);
                 }
@@ -537,13 +495,12 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
                         if (ks >= tw) {  // (blocks of X above the diagonal are zero)
-                            Frag<kWide, 4> af;
-                            Frag<kWide, 2> bf;
-                            load_b<kWide>(bf, sA, LD, 8 * ks, n0, lane);  // shared by the two row tiles
+                            uint32_t af[4], bf[2];
+                            load_b(bf, sA, LD, 8 * ks, n0, lane);  // shared by the two row tiles
 #pragma unroll
                             for (int mt = 0; mt < 2; ++mt) {
-                                load_a<kWide>(af, sA, LD, 32 + 16 * mt, 8 * ks, lane);
-                                mma_frag<kWide>(d[mt], af, bf);
+                                load_a(af, sA, LD, 32 + 16 * mt, 8 * ks, lane);
+                                mma_tf32(d[mt], af, bf);
                             }
                         }
                     }
@@ -553,14 +510,13 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     float e[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        Frag<kWide, 4> af;
-                        Frag<kWide, 2> bf;
-                        load_b<kWide>(bf, sA, LD, 8 * ks, 32 + n0, lane);
+                        uint32_t af[4], bf[2];
+                        load_b(bf, sA, LD, 8 * ks, 32 + n0, lane);
 #pragma unroll
                         for (int mt = 0; mt < 2; ++mt) {
                             if (ks < 2 * (mt + 1)) {
-                                load_a<kWide>(af, sA, LD, 32 + 16 * mt, 32 + 8 * ks, lane);
-                                mma_frag<kWide>(e[mt], af, bf);
+                                load_a(af, sA, LD, 32 + 16 * mt, 32 + 8 * ks, lane);
+                                mma_tf32(e[mt], af, bf);
                             }
                         }
                     }
@@ -601,12 +557,6 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                         const uint4 hw = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
                         *reinterpret_cast<uint4*>(sT + off) = hv;
                         *reinterpret_cast<uint4*>(sTd + off) = hw;
-                        if (kWide) {
-                            *reinterpret_cast<uint4*>(sT + 16384 + off) = make_uint4(pack_lo(v[0], v[1], hv.x), pack_lo(v[2], v[3], hv.y),
-                                                                                     pack_lo(v[4], v[5], hv.z), pack_lo(v[6], v[7], hv.w));
-                            *reinterpret_cast<uint4*>(sTd + 16384 + off) = make_uint4(pack_lo(w[0], w[1], hw.x), pack_lo(w[2], w[3], hw.y),
-                                                                                      pack_lo(w[4], w[5], hw.z), pack_lo(w[6], w[7], hw.w));
-                        }
                     }
                 }
                 fence_proxy_async_smem();
@@ -620,31 +570,19 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     const uint64_t dPa = make_smem_desc_sw128(smem_u32(sP), 0, 1024);           // A, K-major
                     const uint64_t dTb = make_smem_desc_sw128(smem_u32(sT), 8192, 1024);        // B, read MN-major
                     const uint64_t dK = make_smem_desc_sw128(smem_u32(sKQ), 8192, 1024);        // B, K columns 0-63, MN-major
-                    const uint32_t tZ = tmem + kTmZ + (NA * 32u) * team;
+                    const uint32_t tZ = tmem + kTmZ + 64u * team;
                     const uint32_t tPT = tmem + kTmPT + (team ? (16u << 16) : 0u);
 #pragma unroll
                     for (int a = 0; a < NA; ++a) {  // 64 columns of Z each
-                        const uint32_t tz = tZ + (a >> 1) * 64u + ((a & 1) ? (16u << 16) : 0u);
+                        const uint32_t tz = tZ + (a ? (16u << 16) : 0u);
                         const uint64_t dk = desc_advance(dK, a * 16384);
                         mma_ss_w<false>(tz, dTd, dk, idescz);
 #pragma unroll
                         for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tz, desc_advance(dTd, ks * 2048), desc_advance(dk, ks * 2048), idescz);
-                        if (kWide) {
-#pragma unroll
-                            for (int ks = 0; ks < 4; ++ks)
-                                mma_ss_w<true>(tz, desc_advance(dTd, 16384 + ks * 2048), desc_advance(dk, ks * 2048), idescz);
-                        }
                     }
                     mma_ss_w<false>(tPT, dPa, dTb, idesc);
 #pragma unroll
                     for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tPT, desc_advance(dPa, ks * 32), desc_advance(dTb, ks * 2048), idesc);
-                    if (kWide) {
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            mma_ss_w<true>(tPT, desc_advance(dPa, 8192 + ks * 32), desc_advance(dTb, ks * 2048), idesc);
-                            mma_ss_w<true>(tPT, desc_advance(dPa, ks * 32), desc_advance(dTb, 16384 + ks * 2048), idesc);
-                        }
-                    }
                     mma_commit_w(&bar_mma[team]);
                 }
                 __syncwarp();
@@ -652,7 +590,6 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                 ++mma_it;
                 tc_fence_after_sync();
             }
-            if (kWide && tid == 0 && rd == rounds - 1 && unit + static_cast<int>(gridDim.x) >= total_units) grid_dep_launch();
             if (rd == rounds - 1 && tt == 0) {
                 // This team's MMAs have read the K tile (or it sat the round out).  The team that gets here second
                 // knows that both are done with the tiles and requests the next unit's, which land while the
@@ -665,68 +602,6 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
             if (active) {
                 const int row = 16 * tw + (lane & 15), hi = lane >> 4;
                 const uint32_t tl = static_cast<uint32_t>(32 * tw) << 16;
-                if constexpr (kWide) {
-                    // ---- accumulators -> two bf16 terms -> staged tiles -> bulk copies: first Z hi (over T, dT) and both terms
-                    //      of PT (over P), then Z lo over Z hi once that has been read out.  (Written to global memory from
-                    //      registers, 16 bytes of a row per lane, this was 12 of a unit's 25 thousand cycles.)
-                    uint8_t* dst = p.blocks + (static_cast<size_t>(chunk) * p.vh + head) * kWideBlockBytes;
-                    uint8_t* stZ = tbase + L::kOffA;
-                    const uint64_t keep = l2_policy_evict_last();
-                    auto hi_of = [&](const uint32_t* r) {
-                        return make_uint4(pack_bf16(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16(__uint_as_float(r[2]), __uint_as_float(r[3])),
-                                          pack_bf16(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16(__uint_as_float(r[6]), __uint_as_float(r[7])));
-                    };
-                    auto lo_of = [&](const uint32_t* r, const uint4& h) {
-                        return make_uint4(pack_lo(__uint_as_float(r[0]), __uint_as_float(r[1]), h.x), pack_lo(__uint_as_float(r[2]), __uint_as_float(r[3]), h.y),
-                                          pack_lo(__uint_as_float(r[4]), __uint_as_float(r[5]), h.z), pack_lo(__uint_as_float(r[6]), __uint_as_float(r[7]), h.w));
-                    };
-                    auto stage_z = [&](bool lo) {
-#pragma unroll
-                        for (int cb = 0; cb < 4; ++cb) {  // 32 columns of every 64; lanes +16 hold the odd atoms
-                            uint32_t r[32];
-                            tmem_ld32(tmem + kTmZ + 128u * team + tl + 32 * cb, r);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const uint4 h = hi_of(r + 8 * q);
-                                *reinterpret_cast<uint4*>(stZ + tile_off(row, 16 * (cb >> 1) + 8 * hi + 4 * (cb & 1) + q)) = lo ? lo_of(r + 8 * q, h) : h;
-                            }
-                        }
-                    };
-                    stage_z(false);
-#pragma unroll
-                    for (int cb = 0; cb < 2; ++cb) {
-                        uint32_t r[32];
-                        tmem_ld32(tmem + kTmPT + tl + 32 * cb, r);
-                        tmem_wait_ld();
-                        if (hi == team) {
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const uint4 h = hi_of(r + 8 * q);
-                                *reinterpret_cast<uint4*>(sP + tile_off(row, 4 * cb + q)) = h;
-                                *reinterpret_cast<uint4*>(sP + 8192 + tile_off(row, 4 * cb + q)) = lo_of(r + 8 * q, h);
-                            }
-                        }
-                    }
-                    fence_proxy_async_smem();
-                    team_sync(team);
-                    if (tt == 0 && *abort_flag == 0) {  // nothing is written once a wait has given up
-                        bulk_store_hint(dst, stZ, 32768, keep);
-                        bulk_store_hint(dst + 65536, sP, 16384, keep);
-                        bulk_commit();
-                        bulk_wait_read<0>();
-                    }
-                    team_sync(team);
-                    stage_z(true);
-                    fence_proxy_async_smem();
-                    tc_fence_before_sync();
-                    team_sync(team);
-                    if (tt == 0 && *abort_flag == 0) {
-                        bulk_store_hint(dst + 32768, stZ, 32768, keep);
-                        bulk_commit();
-                    }
-                    stores_pending = true;
-                } else {
                 // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> two bulk copies
                 uint8_t* stZ = tbase + L::kOffA;
 #pragma unroll
@@ -769,14 +644,13 @@ __global__ void __launch_bounds__(zp::kThreads, kWide ? 1 : 2) gdn_zp_kernel(con
                     bulk_commit();
                 }
                 stores_pending = true;
-                }
             }
         }  // head pairs
     }      // units
     if (stores_pending && tt == 0) bulk_wait_read<0>();
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kWide ? 512 : 256);
+    if (warp == 0) tmem_dealloc(tmem, 256);
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 2);
 }
 

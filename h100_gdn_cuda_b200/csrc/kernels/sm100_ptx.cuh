@@ -521,8 +521,8 @@ GDN_DEVICE void mma_ts_k128_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
         : "memory");
 }
 // Four K-steps (K = 64) the same way; the B descriptor advances by `kStep16` 16-byte units per step
-// (2 for a K-major tile, 128 for an MN-major one), A by `kStepA` tensor-memory columns.
-template <bool kAccumulateFirst, int kStep16, int kStepA = 8>
+// (2 for a K-major tile, 128 for an MN-major one).
+template <bool kAccumulateFirst, int kStep16>
 GDN_DEVICE void mma_ts_k64_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred pe;\n\t.reg .pred pa;\n\t.reg .pred pt;\n\t.reg .b32 ta;\n\t.reg .b64 bd;\n\t"
@@ -530,14 +530,14 @@ GDN_DEVICE void mma_ts_k64_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, 
         "setp.ne.b32 pa, %4, 0;\n\t"
         "setp.eq.b32 pt, 0, 0;\n\t"
         "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pa;\n\t"
-        "add.u32 ta, %1, %8;\n\tadd.u64 bd, %2, %5;\n\t"
+        "add.u32 ta, %1, 8;\n\tadd.u64 bd, %2, %5;\n\t"
         "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], bd, %3, pt;\n\t"
-        "add.u32 ta, %1, %9;\n\tadd.u64 bd, %2, %6;\n\t"
+        "add.u32 ta, %1, 16;\n\tadd.u64 bd, %2, %6;\n\t"
         "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], bd, %3, pt;\n\t"
-        "add.u32 ta, %1, %10;\n\tadd.u64 bd, %2, %7;\n\t"
+        "add.u32 ta, %1, 24;\n\tadd.u64 bd, %2, %7;\n\t"
         "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], bd, %3, pt;\n\t}\n" ::"r"(d_tmem),
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(kAccumulateFirst ? 1 : 0), "n"(kStep16), "n"(2 * kStep16),
-        "n"(3 * kStep16), "n"(kStepA), "n"(2 * kStepA), "n"(3 * kStepA)
+        "n"(3 * kStep16)
         : "memory");
 }
 GDN_DEVICE void mma_commit_w(uint64_t* bar) {

@@ -72,3 +72,25 @@ def test_static_scratch_refuses_oversize():
     a.shape = shape
     rc = lib.gdn_chunked_forward_static_scratch(C.byref(a), None)
     assert rc == -4 and b"built-in" in lib.gdn_last_error()
+
+
+def test_static_scratch_wide_heads_need_none():
+    """Head dims 192 and 256 run without scratch, so the size of the array is no limit for them (65536 tokens x v-heads
+    here; in blocks of 256 columns it would hold some 40000)."""
+    from h100_gdn_cuda_b200 import _cabi as cabi, api, build
+    build.build()
+    lib = cabi.load()
+    stream = torch.cuda.current_stream().cuda_stream
+    B, T, kh, vh, d = 1, 2048, 16, 32, 256
+    assert lib.gdn_chunked_forward_workspace_bytes(C.byref(api._shape(B, T, B * T, kh, vh, d, d))) == 0
+    p = {k: (v.cuda() if torch.is_tensor(v) else v)
+         for k, v in synthetic.prefill_inputs(B, T, kh, vh, d, seed=7, mild_gate=True).items()}
+    outs = []
+    for fn in (lib.gdn_chunked_forward, lib.gdn_chunked_forward_static_scratch):
+        out, final = torch.full_like(p["v"], float("nan")), torch.full_like(p["state"], float("nan"))
+        rc = fn(C.byref(_args(api, cabi, p, out, final, None, 0)), stream)
+        assert rc == 0, lib.gdn_last_error()
+        torch.cuda.synchronize()
+        outs.append((out, final))
+    assert torch.isfinite(outs[1][0].float()).all() and torch.isfinite(outs[1][1].float()).all()
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
