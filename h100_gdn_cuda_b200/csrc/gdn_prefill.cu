@@ -350,34 +350,42 @@ static int chunked_forward_wide(const GdnChunkedArgs* a, gdn_stream_t stream) {
 static size_t ws_blocks_bytes(size_t chunks, int vh) { return (chunks * static_cast<size_t>(vh) * kZPBlockBytes + 255) / 256 * 256; }
 static size_t ws_norms_bytes(size_t chunks, int kh) { return (chunks * static_cast<size_t>(kh) * 128 * sizeof(float) + 255) / 256 * 256; }
 
+static constexpr size_t kSegUnitBytes = 3 * kD * kD * sizeof(float);  // N, M and the start state of a (slot, v-head)
+
+// Scratch without the segment states: one block of Z (64 x 128 bf16) and PT (64 x 64 bf16) per (chunk, v-head), and the
+// q/k norm factors.
+static size_t ws_base_bytes(const GdnShape& s) {
+    const size_t chunks = s.cu_seqlens ? static_cast<size_t>(s.total_chunks > 0 ? s.total_chunks : 0)
+                                       : static_cast<size_t>(s.batch) * static_cast<size_t>((s.seq_len + kChunk - 1) / kChunk);
+    return ws_blocks_bytes(chunks, s.num_v_heads) + ws_norms_bytes(chunks, s.num_k_heads) + 256;
+}
+
 // The segment plan of a problem (heuristics.hpp); num_segments == 1: not segmented.
-static SegmentPlan segment_plan_of(const GdnShape& s) {
-    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, s.total_chunks > 0 ? s.total_chunks : 0);
-    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, (s.seq_len + kChunk - 1) / kChunk, false);
+static SegmentPlan segment_plan_of(const GdnShape& s, long long max_units = plan_detail::kNoLimit) {
+    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, s.total_chunks > 0 ? s.total_chunks : 0, max_units);
+    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, (s.seq_len + kChunk - 1) / kChunk, false, max_units);
     plan.slots = s.batch * plan.num_segments;
     return plan;
+}
+
+// Scratch of a run on `plan`: for a segmented one (few long sequences) three fp32 states per v-head and segment slot.
+static size_t ws_bytes(const GdnShape& s, const SegmentPlan& plan) {
+    size_t bytes = ws_base_bytes(s);
+    if (plan.num_segments > 1)
+        bytes += static_cast<size_t>(plan.slots) * s.num_v_heads * kSegUnitBytes + 256;
+    else if (s.cu_seqlens && s.batch > 1 && s.batch <= kMaxOrderedSeqs)
+        bytes += (static_cast<size_t>(s.batch) * sizeof(int) + 255) / 256 * 256;  // sequences by length
+    return bytes;
 }
 
 size_t gdn_chunked_forward_workspace_bytes(const GdnShape* s) {
     if (!s) return 0;
     if (wide_heads(*s)) return 0;
-    const size_t chunks = s->cu_seqlens ? static_cast<size_t>(s->total_chunks > 0 ? s->total_chunks : 0)
-                                        : static_cast<size_t>(s->batch) * static_cast<size_t>((s->seq_len + kChunk - 1) / kChunk);
-    // one block of Z (64 x 128 bf16) and PT (64 x 64 bf16) per (chunk, v-head); for a
-    // segmented run (few long sequences) three fp32 states per v-head and segment slot on top
-    size_t bytes = ws_blocks_bytes(chunks, s->num_v_heads) + ws_norms_bytes(chunks, s->num_k_heads) + 256;
-    const SegmentPlan plan = segment_plan_of(*s);
-    if (plan.num_segments > 1)
-        bytes += static_cast<size_t>(plan.slots) * s->num_v_heads * 3 * kD * kD * sizeof(float) + 256;
-    else if (s->cu_seqlens && s->batch > 1 && s->batch <= kMaxOrderedSeqs)
-        bytes += (static_cast<size_t>(s->batch) * sizeof(int) + 255) / 256 * 256;  // sequences by length
-    return bytes;
+    return ws_bytes(*s, segment_plan_of(*s));
 }
 
-int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
-    GDN_REQUIRE(a != nullptr, "gdn_chunked_forward: args is NULL");
+static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, gdn_stream_t stream) {
     const GdnShape& s = a->shape;
-    if (int rc = check_shape(s, true)) return rc;
     if (wide_heads(s)) return chunked_forward_wide(a, stream);
     // The kernels are built for dk = dv = 128.  A smaller head dim that is a multiple of 8 (the 16-byte
     // rule of the copies) runs on them as it is: the tensor maps deliver zero columns past it and the state
@@ -396,7 +404,7 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     if (int rc = check_state(a->initial_state, "initial_state")) return rc;
     if (int rc = check_state(a->final_state, "final_state")) return rc;
     GDN_REQUIRE(s.num_v_heads <= 65535, "too many heads");
-    const size_t need = gdn_chunked_forward_workspace_bytes(&s);
+    const size_t need = ws_bytes(s, plan);
     if (!a->workspace || a->workspace_bytes < need || (reinterpret_cast<uintptr_t>(a->workspace) & 255u))
         return fail(GDN_ERR_WORKSPACE, "gdn_chunked_forward: workspace of %zu bytes (256-byte aligned) required, got %zu",
                     need, a->workspace_bytes);
@@ -455,7 +463,6 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
             GDN_CUDA(launch_fused_after_zp(grid, st, tmQ, tmK, tmV, tmO, p));
             return GDN_OK;
         };
-        const SegmentPlan plan = segment_plan_of(s);
         if (plan.num_segments <= 1 && packed && s.batch > 1 && s.batch <= kMaxOrderedSeqs && chains > d->sms) {
             // more chains than SMs and unequal lengths: dispatch the longest sequences first
             int* order = reinterpret_cast<int*>(ws_extra);
@@ -517,6 +524,12 @@ int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     return GDN_OK;
 }
 
+int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
+    GDN_REQUIRE(a != nullptr, "gdn_chunked_forward: args is NULL");
+    if (int rc = check_shape(a->shape, true)) return rc;
+    return chunked_forward_on(a, segment_plan_of(a->shape), stream);
+}
+
 // ------------------------------------------------------------------ prefill on built-in scratch
 // Scratch for callers that cannot allocate device memory (see include/gdn_b200.h).  The array
 // lives in the library image; in host code its name is only a handle for the runtime, so the
@@ -528,7 +541,11 @@ static std::mutex g_static_scratch_mutex;
 int gdn_chunked_forward_static_scratch(const GdnChunkedArgs* a, gdn_stream_t stream) {
     GDN_REQUIRE(a != nullptr, "gdn_chunked_forward_static_scratch: args is NULL");
     if (int rc = check_shape(a->shape, true)) return rc;
-    const size_t need = gdn_chunked_forward_workspace_bytes(&a->shape);
+    // The plan that is the fastest with all the scratch it wants may not fit where fewer segments, or none, do.
+    const size_t base = ws_base_bytes(a->shape) + 256;
+    const SegmentPlan plan = segment_plan_of(
+        a->shape, base < GDN_STATIC_SCRATCH_BYTES ? static_cast<long long>((GDN_STATIC_SCRATCH_BYTES - base) / kSegUnitBytes) : 0);
+    const size_t need = wide_heads(a->shape) ? 0 : ws_bytes(a->shape, plan);
     if (need > GDN_STATIC_SCRATCH_BYTES)
         return fail(GDN_ERR_WORKSPACE,
                     "gdn_chunked_forward_static_scratch: this problem needs %zu bytes of scratch but the built-in "
@@ -553,7 +570,7 @@ int gdn_chunked_forward_static_scratch(const GdnChunkedArgs* a, gdn_stream_t str
     GdnChunkedArgs b = *a;
     b.workspace = scratch;
     b.workspace_bytes = GDN_STATIC_SCRATCH_BYTES;
-    return gdn_chunked_forward(&b, stream);
+    return chunked_forward_on(&b, plan, stream);
 }
 
 }  // extern "C"

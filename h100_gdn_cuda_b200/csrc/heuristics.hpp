@@ -6,6 +6,7 @@
 #pragma once
 #include <algorithm>
 #include <cstdlib>
+#include <limits>
 
 namespace gdn {
 
@@ -43,7 +44,8 @@ inline PrefillConfig prefill_config() { return PrefillConfig{4, 512}; }
 // segments' start states, and a launch of the state kernel produces the output of all
 // segments at once.  Two passes and a quarter instead of one, many segments wide.
 // The plan must not depend on the device (the scratch size is computed without one), so it is
-// made for the 148 SMs of a B200.
+// made for the 148 SMs of a B200.  `max_units`: (slot, v-head) pairs whose segment states the scratch has room for; a plan
+// with more is not made, the best one that fits is.
 struct SegmentPlan {
     int num_segments;  // padded mode: segments per sequence; 1: not segmented
     int seg_chunks;    // chunks per segment
@@ -52,6 +54,7 @@ struct SegmentPlan {
 };
 namespace plan_detail {
 constexpr long long kSms = 148;
+constexpr long long kNoLimit = std::numeric_limits<long long>::max();
 // Cost model fitted to measurements (B=1..2, T=4096..131072, 4..32 v-heads), in units of "one
 // chunk of the state kernel" (1.25 us): a CTA costs its chunks plus about 3 for start-up and pipeline
 // fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Plans whose launches need more
@@ -64,13 +67,13 @@ constexpr int kMinSegment = 25, kMinSegmentPacked = 32;
 inline long long waves(long long ctas) { return (ctas + kSms - 1) / kSms; }
 }  // namespace plan_detail
 
-inline SegmentPlan prefill_segments(long long chains, int chunks_per_seq, bool packed) {
+inline SegmentPlan prefill_segments(long long chains, int chunks_per_seq, bool packed, long long max_units = plan_detail::kNoLimit) {
     using namespace plan_detail;
     SegmentPlan plan{1, chunks_per_seq, 0};
     if (packed || chains <= 0) return plan;
     double best = 0.8 * static_cast<double>(waves(chains) * (chunks_per_seq + kFixed));
     for (int P = 2; P <= 32 && chunks_per_seq / P >= kMinSegment; ++P) {
-        if (waves(chains * P) > 1) break;
+        if (waves(chains * P) > 1 || chains * P > max_units) break;
         const int len = (chunks_per_seq + P - 1) / P;
         const double cost = kPasses * (len + kFixed);
         if (cost < best) {
@@ -88,7 +91,8 @@ inline SegmentPlan prefill_segments(long long chains, int chunks_per_seq, bool p
 // CTAs leave at once.  The unsegmented run is costed as if all sequences were equally long (its
 // best case), so unequal lengths only make the segmented plan better than assumed.
 constexpr int kMaxSegmentedSeqs = 64;
-inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long long total_chunks) {
+inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long long total_chunks,
+                                           long long max_units = plan_detail::kNoLimit) {
     using namespace plan_detail;
     SegmentPlan plan{1, static_cast<int>(std::min<long long>(total_chunks, 1 << 30)), 0};
     if (num_seqs <= 0 || num_seqs > kMaxSegmentedSeqs || num_v_heads <= 0 || total_chunks <= 0 || total_chunks > (1 << 30)) return plan;
@@ -103,6 +107,7 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
         // short segment
         const long long work = (total_chunks + len - 1) / len + num_seqs - 1;
         if (waves(work * num_v_heads) > 1) break;
+        if (slots * num_v_heads > max_units) continue;
         const double cost = kPasses * (len + kFixed);
         if (cost < best) {
             best = cost;

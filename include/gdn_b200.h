@@ -286,11 +286,13 @@ int gdn_chunked_forward(const GdnChunkedArgs* args, gdn_stream_t stream);
  * library, held until the process exits).  `workspace` and `workspace_bytes` in `args` are
  * ignored; inputs and outputs are passed as usual.
  *
- *   - Limit: gdn_chunked_forward_workspace_bytes(&args->shape) must not exceed
- *     GDN_STATIC_SCRATCH_BYTES (49 MiB + 8.5 KiB).  The scratch holds 24 KiB per 64-token
- *     chunk and v-head (384 bytes per token and v-head) plus 512 bytes per chunk and k-head,
- *     so with whole chunks that is tokens * num_v_heads <= 131072, for example 4096
- *     tokens of 32 v-heads (less where long sequences of few heads add their segment states).
+ *   - Limit: the scratch must fit GDN_STATIC_SCRATCH_BYTES (49 MiB + 8.5 KiB).  It holds
+ *     24 KiB per 64-token chunk and v-head (384 bytes per token and v-head) plus 512 bytes per
+ *     chunk and k-head, so with whole chunks that is tokens * num_v_heads <= 131072, for example
+ *     4096 tokens of 32 v-heads.  Long sequences of few heads run in as many segments as the rest
+ *     of the array has room for (fewer than with a workspace of
+ *     gdn_chunked_forward_workspace_bytes(&args->shape) bytes where that is more).  Head dims 192
+ *     and 256 need no scratch and have no limit.
  *     Larger problems are refused with GDN_ERR_WORKSPACE and a message.
  *   - It calls no cudaMalloc / cudaFree and no allocating library routine.
  *   - The first call on each device looks up the array's device address; make that first

@@ -135,6 +135,22 @@ def test_segment_plan_heuristic():
     assert rows[13][0] == 1              # four equal sequences would already run side by side
 
 
+@pytest.mark.parametrize("B,T,vh,packed", [(1, 50048, 2, False), (1, 65536, 2, False), (1, 16384, 8, False), (4, 8000, 4, True)])
+def test_static_scratch_takes_fewer_segments(lib, B, T, vh, packed):
+    """What fits the built-in scratch array without segment states is not refused because the preferred segment plan
+    does not fit.  (The call then stops at the device lookup or at the missing tensors, before any device work.)"""
+    from h100_gdn_cuda_b200 import _cabi as cabi, api
+    a = cabi.ChunkedArgs()
+    chunks = B * ((T + 63) // 64)
+    a.shape = cabi.Shape(B, 0 if packed else T, B * T, vh, vh, 128, 128, 0x1000 if packed else None, 0x1000 if packed else None,
+                         0x1000 if packed else None, chunks if packed else 0)
+    assert chunks * vh * (24576 + 512) + 1024 <= (49 << 20) + 8704
+    assert lib.gdn_chunked_forward_workspace_bytes(ctypes.byref(a.shape)) > (49 << 20) + 8704
+    assert lib.gdn_chunked_forward_static_scratch(ctypes.byref(a), None) in (-1, -3)
+    a.shape = cabi.Shape(1, 131072 // vh + 64, 131072 // vh + 64, vh, vh, 128, 128, None, None, None, 0)
+    assert lib.gdn_chunked_forward_static_scratch(ctypes.byref(a), None) == -4
+
+
 def test_state_alignment_is_checked_on_the_host(lib):
     """States are accessed 16 bytes at a time: a misaligned pointer or a stride that is not a multiple of
     8 elements is refused with GDN_ERR_INVALID before anything touches a device."""

@@ -74,6 +74,29 @@ def test_static_scratch_refuses_oversize():
     assert rc == -4 and b"built-in" in lib.gdn_last_error()
 
 
+def test_static_scratch_runs_in_the_segments_that_fit():
+    """2 v-heads of 50048 tokens: the states of 31 segments on top of the blocks do not fit the array, those of 29 do.  Other
+    segments, other roundings of the state between them: both within the prefill tests' tolerance of each other."""
+    from h100_gdn_cuda_b200 import _cabi as cabi, api, build
+    build.build()
+    lib = cabi.load()
+    stream = torch.cuda.current_stream().cuda_stream
+    B, T, vh, d = 1, 50048, 2, 128
+    n = lib.gdn_chunked_forward_workspace_bytes(C.byref(api._shape(B, T, B * T, vh, vh, d, d)))
+    assert n > (49 << 20) + 8704
+    p = {k: (v.cuda() if torch.is_tensor(v) else v)
+         for k, v in synthetic.prefill_inputs(B, T, vh, vh, d, seed=8, mild_gate=True).items()}
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    outs = []
+    for fn, args in ((lib.gdn_chunked_forward, (ws.data_ptr(), n)), (lib.gdn_chunked_forward_static_scratch, (None, 0))):
+        out, final = torch.full_like(p["v"], float("nan")), torch.full_like(p["state"], float("nan"))
+        assert fn(C.byref(_args(api, cabi, p, out, final, *args)), stream) == 0, lib.gdn_last_error()
+        torch.cuda.synchronize()
+        outs.append((out.float(), final.float()))
+    for a, b in zip(*outs):
+        assert torch.isfinite(b).all() and ((a - b).norm() / a.norm()).item() <= 1e-2
+
+
 def test_static_scratch_wide_heads_need_none():
     """Head dims 192 and 256 run without scratch, so the size of the array is no limit for them (65536 tokens x v-heads
     here; in blocks of 256 columns it would hold some 40000)."""
