@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             int chunk, khead;
             unit_chunk(static_cast<int>(unit), chunk, khead);
             const ChunkPos cp = locate_chunk(p.map, chunk);
-            e = make_int4(chunk, khead | (cp.n << 16), static_cast<int>(cp.tok0), cp.batch);
+            // (an entry of chunk_indices may name an empty chunk: the unit is walked all the same, its block is never read)
+            e = make_int4(chunk, khead | (max(cp.n, 0) << 16) | (1 << 30), static_cast<int>(cp.tok0), cp.batch);
         }
         sUnits[tid] = e;
     };
@@ -204,10 +205,10 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
         UnitPos u;
         u.chunk = e.x;
         u.khead = e.y & 0xFFFF;
-        u.n = e.y >> 16;
+        u.n = (e.y >> 16) & 0x7F;
         u.tok0 = e.z;
         u.batch = e.w;
-        u.valid = u.n > 0;
+        u.valid = (e.y >> 30) != 0;
         return u;
     };
     fill_units(static_cast<int>(blockIdx.x));
@@ -274,7 +275,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 if (tt < 64) {
                     // tokens past the end had a raw gate of 0: they carry the last valid value
                     const float g = sPart[tt] + (tt >= 32 ? sPart[31] : 0.f);
-                    const float gl = sPart[n - 1] + (n - 1 >= 32 ? sPart[31] : 0.f);
+                    const int last = max(n, 1) - 1;
+                    const float gl = sPart[last] + (last >= 32 ? sPart[31] : 0.f);
                     sBeta[tt] = b_mine;
                     sG[tt] = g * 1.4426950408889634f;  // times log2(e): decay factors are ex2 of differences
                     sD[tt] = __expf(gl - g);

@@ -35,3 +35,19 @@ def test_more_units_than_one_table(packed):
         sl = slice(cu[i], cu[i + 1])
         oi, si = gdn.chunked_forward(q[None, sl], k[None, sl], v[None, sl], beta[None, sl], gate[None, sl], None, s0[i:i + 1])
         assert torch.equal(oi[0], o[sl]) and torch.equal(si[0], s[i])
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_chunk_entries_without_tokens(norm):
+    """chunk_indices may hold entries that name no token (a chunk for an empty sequence, counted in cu_chunks; chunks past a
+    sequence's end behind the last one, as a caller with buffers of a fixed size has them): the bits of the exact lists."""
+    import h100_gdn_cuda_b200 as gdn
+    lens = [70, 0, 130, 0, 1]
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.varlen_inputs(lens, 2, 4, 128, seed=4, mild_gate=True).items()}
+    args = (p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], p["cu_seqlens"])
+    o_ref, s_ref = gdn.chunked_forward(*args, p["chunk_indices"], p["cu_chunks"], is_qk_norm=norm)
+    ci = [0, 0, 0, 1, 1, 0, 2, 0, 2, 1, 2, 2, 3, 0, 4, 0] + [4, 1, 3, 0, 0, 2]
+    cc = [0, 2, 3, 6, 7, 8]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    o, s = gdn.chunked_forward(*args, i32(ci), i32(cc), is_qk_norm=norm)
+    assert torch.equal(o, o_ref) and torch.equal(s, s_ref)
