@@ -54,7 +54,12 @@ __global__ void __launch_bounds__(transition::kThreads, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const SegPos sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
-    if (sp.seq < 0 || sp.segment == sp.nseg - 1) return;  // surplus slot; nothing follows a sequence's last segment
+    if (sp.seq < 0 || sp.segment == sp.nseg - 1) {  // surplus slot; nothing follows a sequence's last segment
+        // The launches behind this one wait for this grid alone, so it must not complete before the chunk-parallel kernel
+        // has: every CTA waits for that, the ones without work too (all of them, where no sequence has a second segment).
+        grid_dep_wait();
+        return;
+    }
     const int head = static_cast<int>(blockIdx.y), khead = head / (p.vh / p.kh);
     const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;
     int batch = sp.seq, gchunk0 = sp.seq * p.map.chunks_per_seq;

@@ -51,3 +51,19 @@ def test_chunk_entries_without_tokens(norm):
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
     o, s = gdn.chunked_forward(*args, i32(ci), i32(cc), is_qk_norm=norm)
     assert torch.equal(o, o_ref) and torch.equal(s, s_ref)
+
+
+def test_segmented_launches_without_a_second_segment():
+    """chunk_indices padded to a fixed number of chunks: the segment plan is made for that number, and no sequence is longer
+    than one segment.  The output launch must still find the chunk-parallel kernel's blocks complete: the bits of the exact
+    lists (one segment per sequence is the unsegmented run)."""
+    import h100_gdn_cuda_b200 as gdn
+    lens = [1100, 700]
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.varlen_inputs(lens, 2, 4, 128, seed=6, mild_gate=True).items()}
+    args = (p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], p["cu_seqlens"])
+    o_ref, s_ref = gdn.chunked_forward(*args, p["chunk_indices"], p["cu_chunks"])
+    ci = torch.zeros(4096, 2, dtype=torch.int32, device="cuda")  # the surplus entries repeat the first chunk
+    ci[:p["total_chunks"]] = p["chunk_indices"].view(-1, 2)
+    for _ in range(20):
+        o, s = gdn.chunked_forward(*args, ci.flatten(), p["cu_chunks"])
+        assert torch.equal(o, o_ref) and torch.equal(s, s_ref)
