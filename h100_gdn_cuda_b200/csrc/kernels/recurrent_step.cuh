@@ -365,13 +365,15 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                 }
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    R[0][e] = fmaf(cb, e ? bf16_hi(v0) : bf16_lo(v0), -ck * d0[e]);
-                    R[1][e] = fmaf(cb, e ? bf16_hi(v1) : bf16_lo(v1), -ck * d1[e]);
+                    // (rows of tokens that do not exist are zero, whatever the state holds)
+                    R[0][e] = g < ntok ? fmaf(cb, e ? bf16_hi(v0) : bf16_lo(v0), -ck * d0[e]) : 0.f;
+                    R[1][e] = g < ntok ? fmaf(cb, e ? bf16_hi(v1) : bf16_lo(v1), -ck * d1[e]) : 0.f;
                     O[0][e] = cq * d0[2 + e];
                     O[1][e] = cq * d1[2 + e];
                 }
             }
-            // ---- c and o
+            // ---- c and o (selected, not multiplied by the zeros of s_ap: an infinite or undefined value of a later token
+            //      must not reach an earlier one)
 #pragma unroll 1
             for (int s = 0; s < ntok; ++s) {
                 const float2 ap = s_ap[warp][s][g];
@@ -379,8 +381,8 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                 for (int i = 0; i < 4; ++i) {
                     float& Ri = R[i >> 1][i & 1];
                     const float c = __shfl_sync(0xffffffffu, Ri, 4 * s + t);
-                    Ri = fmaf(-ap.x, c, Ri);
-                    O[i >> 1][i & 1] = fmaf(ap.y, c, O[i >> 1][i & 1]);
+                    Ri = s < g ? fmaf(-ap.x, c, Ri) : Ri;
+                    O[i >> 1][i & 1] = s <= g ? fmaf(ap.y, c, O[i >> 1][i & 1]) : O[i >> 1][i & 1];
                 }
             }
             {
@@ -391,7 +393,10 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                 }
                 out_ptr += kStepRows / 2;
             }
-            // ---- S_tau = G_tau S_0 + sum_s (Gamma_{tau,s} r_s c_s) k_s^T: the last token's state, or every token's
+            // ---- S_tau = G_tau S_0 + sum_s (Gamma_{tau,s} r_s c_s) k_s^T: the last token's state, or every token's.  Both factors
+            //      of a token after tau are zero: either alone would turn the other's infinite or undefined value into a NaN.
+            //      (These selects cost 0.4 us of 31.2 at B=64, T=4 and 0.35 of 20.25 at B=13, T=5 with step states; a second copy of
+            //      the update for the tiles that need them, behind a vote, costs 0.9 and 0.1.)
             if (slot >= 0) {
                 const int last = max(ntok - 1, 0);
 #pragma unroll 1
@@ -401,15 +406,20 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                     const float f = s_w[warp][tau][g];
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        float x0 = f * R[h][0], x1 = f * R[h][1];
+                        float x0 = g <= tau ? f * R[h][0] : 0.f, x1 = g <= tau ? f * R[h][1] : 0.f;
 #pragma unroll
                         for (int i = 0; i < 3; ++i) {
                             const uint32_t b = pack_bf16(x0, x1);
                             x0 -= bf16_lo(b);
                             x1 -= bf16_hi(b);
+                            if (i == 0) {  // inf - inf: any finite number (fmaxf drops a NaN), the first term outweighs it
+                                x0 = fmaxf(x0, -3.0e38f);
+                                x1 = fmaxf(x1, -3.0e38f);
+                            }
                             w[h][i] = transpose8(b);
                         }
                     }
+                    const uint32_t ktok = (2 * t <= tau ? 0xFFFFu : 0u) | (2 * t + 1 <= tau ? 0xFFFF0000u : 0u);
                     __nv_bfloat16* d = steps ? dst + tau * p.so_ss : dst;
 #pragma unroll
                     for (int j = 0; j < NJ; ++j) {
@@ -423,8 +433,9 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                             float c[4];
                             c[0] = G * bf16_lo(wa[e]); c[1] = G * bf16_hi(wa[e]);
                             c[2] = G * bf16_lo(wb[e]); c[3] = G * bf16_hi(wb[e]);
-                            mma16(c, w[0][0], w[1][0], w[0][1], w[1][1], kt[4 * j + e], kt[4 * j + e]);
-                            mma8(c, w[0][2], w[1][2], kt[4 * j + e]);
+                            const uint32_t kk = kt[4 * j + e] & ktok;
+                            mma16(c, w[0][0], w[1][0], w[0][1], w[1][1], kk, kk);
+                            mma8(c, w[0][2], w[1][2], kk);
                             na[e] = pack_bf16(c[0], c[1]);
                             nb[e] = pack_bf16(c[2], c[3]);
                         }

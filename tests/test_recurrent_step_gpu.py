@@ -97,3 +97,50 @@ def test_one_token_tiles_apart_or_together(gdn, B):
     o, s = gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], pd["state"], bb.cuda(), g.cuda(), inference_mode=gdn.Decode, is_qk_norm=True)
     close(o, o_ref, "o")
     close(s, s_ref, "state")
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("where", ["q", "k", "v", "beta", "gate"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_undefined_values_stay_behind_their_token(gdn, d, where, bad):
+    """An undefined or infinite input of one token reaches no earlier token's output or state, as in the recurrence."""
+    B, T, kh, vh, t = 2, 6, 2, 4, 3
+    p, pd, beta, g = problem(B, T, kh, vh, d, seed=3 * d)
+    x = dict(q=pd["q"], k=pd["k"], v=pd["v"], beta=beta.bfloat16().cuda(), gate=g.cuda())
+    call = lambda: gdn.recurrent_forward(x["q"], x["k"], x["v"], pd["state"], x["beta"], x["gate"], inference_mode=gdn.SpecVerify, is_qk_norm=True)
+    o_ref, s_ref = call()
+    x[where] = x[where].clone()
+    x[where][0, t].flatten()[0] = bad  # k-head 0 or v-head 0 of sequence 0
+    o, s = call()
+    assert torch.equal(o[:, :t], o_ref[:, :t]) and torch.equal(s[:, :t], s_ref[:, :t])
+    assert torch.equal(o[1], o_ref[1]) and torch.equal(s[1], s_ref[1]) and torch.equal(o[0, :, 2:], o_ref[0, :, 2:])
+    assert not torch.isfinite(o[0, t:, 0]).all()
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("steps", [False, True])
+def test_infinite_value_gives_an_infinite_row(gdn, sign, steps):
+    """v infinite in one row: that row of the token's state is infinite with the sign of v k, the others are untouched"""
+    T, d, t = 2, 128, 1
+    p, pd, beta, g = problem(1, T, 1, 1, d, seed=12)
+    args = lambda v: (pd["q"], pd["k"], v, pd["state"], beta.bfloat16().cuda(), g.cuda())
+    kw = dict(inference_mode=gdn.SpecVerify if steps else gdn.Decode, is_qk_norm=True)
+    last = lambda s: s[0, t, 0] if steps else s[0, 0]
+    s_ref = last(gdn.recurrent_forward(*args(pd["v"]), **kw)[1])
+    v = pd["v"].clone()
+    v[0, t, 0, 37] = sign * float("inf")
+    s = last(gdn.recurrent_forward(*args(v), **kw)[1])
+    rows = [r for r in range(d) if r != 37]
+    assert torch.equal(s[rows], s_ref[rows])
+    k = pd["k"][0, t, 0].float()
+    assert (k != 0).all() and torch.equal(s[37].float(), torch.where(k * sign > 0, float("inf"), float("-inf")))
+
+
+@pytest.mark.parametrize("T", [2, 8])
+def test_no_token_accepted_passes_any_state(gdn, T):
+    p, pd, beta, g = problem(2, T, 1, 2, 128, seed=T)
+    s0 = pd["state"].clone()
+    s0[0, 0, 5, 7], s0[0, 1, 0, 0], s0[1, 1, 127, 127] = float("inf"), float("nan"), float("-inf")
+    acc = torch.zeros(2, dtype=torch.int32, device="cuda")
+    _, s = gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], s0, beta.bfloat16().cuda(), g.cuda(), None, acc, gdn.Decode, True)
+    assert torch.equal(s.nan_to_num(12345.0), s0.nan_to_num(12345.0)) and torch.equal(s.isnan(), s0.isnan())
