@@ -335,7 +335,8 @@ int gdn_causal_conv1d(const GdnConvArgs* a, gdn_stream_t stream) {
     GDN_REQUIRE(tokens >= 0, "gdn_causal_conv1d: negative token count");
     if (a->state_out && a->state_out == a->state_in)
         GDN_REQUIRE(packed ? a->total_tokens <= a->batch : a->seq_len <= kConvTokBlock,
-                    "gdn_causal_conv1d: state_out may alias state_in only when no sequence spans more than one %d-token block",
+                    "gdn_causal_conv1d: state_out may alias state_in only for padded sequences of up to %d tokens and for packed "
+                    "inputs with no more tokens than sequences",
                     kConvTokBlock);
     DeviceInfo* d = nullptr;
     if (int rc = get_device_info(&d)) return rc;
@@ -354,14 +355,16 @@ int gdn_causal_conv1d(const GdnConvArgs* a, gdn_stream_t stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long cblocks = (a->channels / 8 + 127) / 128 * static_cast<long long>(packed ? 1 : a->batch);
     p.tok_block = tokens <= kConvTokBlock ? kConvTokBlock : conv_tok_block(tokens, cblocks, d->sms);
+    const bool whole = packed && p.state_out && p.state_out == p.state_in;
     const long long tblocks = (tokens + p.tok_block - 1) / p.tok_block;
     GDN_REQUIRE(tblocks <= 65535 && a->batch <= 65535, "gdn_causal_conv1d: too many token blocks or sequences for one launch");
     if (tblocks > 0) {
         dim3 grid(static_cast<unsigned>((a->channels / 8 + 127) / 128), static_cast<unsigned>(tblocks), packed ? 1u : static_cast<unsigned>(a->batch));
+        auto launch = [&](auto kernel, auto whole_kernel) { return launch_dependent(whole ? whole_kernel : kernel, grid, 128, 0, st, p); };
         switch (a->width) {
-            case 2: GDN_CUDA(launch_dependent(gdn_causal_conv1d_kernel<2>, grid, 128, 0, st, p)); break;
-            case 3: GDN_CUDA(launch_dependent(gdn_causal_conv1d_kernel<3>, grid, 128, 0, st, p)); break;
-            default: GDN_CUDA(launch_dependent(gdn_causal_conv1d_kernel<4>, grid, 128, 0, st, p)); break;
+            case 2: GDN_CUDA(launch(gdn_causal_conv1d_kernel<2>, gdn_causal_conv1d_kernel<2, true>)); break;
+            case 3: GDN_CUDA(launch(gdn_causal_conv1d_kernel<3>, gdn_causal_conv1d_kernel<3, true>)); break;
+            default: GDN_CUDA(launch(gdn_causal_conv1d_kernel<4>, gdn_causal_conv1d_kernel<4, true>)); break;
         }
     }
     if (packed && p.state_out && p.state_in && p.state_out != p.state_in) {

@@ -10,7 +10,7 @@
 
 namespace gdn {
 
-constexpr int kConvTokBlock = 32;  // sequences of up to this many tokens are one block of tokens, whatever the launch's block
+constexpr int kConvTokBlock = 32;  // an input of up to this many tokens (per sequence; packed: in all) is one block of tokens
 constexpr int kConvMaxWidth = 4;
 constexpr int kConvRing = 8;       // tokens requested ahead per thread
 
@@ -96,7 +96,9 @@ __device__ __forceinline__ uint4 pack8(const f2* f) {
 // by pointer increments: the kernel is bound by instruction issue, and 64-bit index arithmetic per token was a
 // good part of it.  (Unrolling 32 tokens, which makes ring slots constants, is slower: 3 k instructions
 // per thread no longer sit in the instruction cache.)
-template <int W>
+// kWhole (packed, state_out == state_in): a thread takes the whole sequences that start in its block.  The block that ends a
+// sequence would otherwise overwrite the state that the block it starts in may still have to read.
+template <int W, bool kWhole = false>
 __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvParams p) {
     static_assert(W >= 2 && W <= kConvMaxWidth, "filter widths 2 .. 4");
     using namespace la;
@@ -106,10 +108,23 @@ __global__ void __launch_bounds__(128, 5) gdn_causal_conv1d_kernel(const ConvPar
     const int c0 = cg * 8;
     // the thread's token block [t0, t0 + n_tok) and the sequence it starts in
     const bool packed = p.cu_seqlens != nullptr;
-    const long long t0 = static_cast<long long>(blockIdx.y) * p.tok_block;
+    long long t0 = static_cast<long long>(blockIdx.y) * p.tok_block;
     const long long limit = packed ? p.total_tokens : static_cast<long long>(p.seq_len);
-    if (t0 >= limit) return;
-    const int n_tok = static_cast<int>(min(static_cast<long long>(p.tok_block), limit - t0));
+    long long t1 = min(t0 + p.tok_block, limit);
+    if (kWhole) {
+        auto first_start = [&](long long t) {  // the first start of a sequence at or behind t, or the end
+            int lo = 0, hi = p.batch;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (p.cu_seqlens[mid] < t) lo = mid + 1; else hi = mid;
+            }
+            return lo < p.batch ? min(static_cast<long long>(p.cu_seqlens[lo]), limit) : limit;
+        };
+        t0 = first_start(t0);
+        t1 = first_start(t1);
+    }
+    if (t0 >= t1) return;
+    const int n_tok = static_cast<int>(t1 - t0);
     int seq;
     const __nv_bfloat16* xb;
     __nv_bfloat16* yb;

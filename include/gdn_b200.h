@@ -320,9 +320,9 @@ int gdn_chunked_forward_static_scratch(const GdnChunkedArgs* args, gdn_stream_t 
  * NULL; width 2 .. 4; channels a multiple of 8.  Inputs before a sequence's first token come from
  * state_in (sequences, width-1, channels; row width-2 is the input right before the sequence) or are zero
  * when it is NULL; state_out (same shape, or NULL) receives the sequence's last width-1 inputs, so that a
- * later call continues it (decode).  state_out may be the same buffer as state_in only when no sequence
- * spans more than one 32-token block: padded mode with seq_len <= 32, packed mode with one token per
- * sequence at most (total_tokens <= batch). */
+ * later call continues it (decode).  state_out may be the same buffer as state_in for short runs: padded
+ * mode with seq_len <= 32, packed mode with no more tokens than sequences (total_tokens <= batch; meant for
+ * one token each, a longer sequence is walked by one thread per 8 channels). */
 typedef struct {
     const void* x;
     void* y;

@@ -43,6 +43,23 @@ def test_conv_packed_blocks(gdn):
     assert torch.equal(fin.float().cpu(), fin_ref)
 
 
+@pytest.mark.parametrize("lens", [[1] * 70, [3, 0, 0, 1, 9, 0, 0, 0] * 8 + [0] * 80, [0, 40, 1, 2] + [0] * 60, [0] * 64 + [64]])
+@pytest.mark.parametrize("C_,W", [(8192, 4), (520, 2)])
+def test_conv_packed_state_in_place(gdn, lens, C_, W):
+    """No more tokens than sequences, but sequences of any length (8192 channels: blocks of 4 tokens, which they span): the
+    state updated where it lies, the same bits as into a buffer of its own."""
+    assert sum(lens) <= len(lens)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(len(lens))
+    x = torch.randn(sum(lens), C_, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(C_, W, generator=gen, device="cuda") * 0.5).bfloat16()
+    s0 = torch.randn(len(lens), W - 1, C_, generator=gen, device="cuda").bfloat16()
+    y_ref, s_ref = gdn.api.causal_conv1d(x, w, None, s0, cu_seqlens=cu, return_final_state=True)
+    y, s = gdn.api.causal_conv1d(x, w, None, s0, cu_seqlens=cu, final_state=s0)
+    assert s.data_ptr() == s0.data_ptr()
+    assert torch.equal(y, y_ref) and torch.equal(s, s_ref)
+
+
 @pytest.mark.parametrize("W", [2, 3, 4])
 def test_conv_weight_alignment(gdn, W):
     """The taps are read 16 bytes at a time where the weight allows it: a weight at an odd element gives the same bits."""
