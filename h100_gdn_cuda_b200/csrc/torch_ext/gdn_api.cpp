@@ -386,6 +386,7 @@ at::Tensor gated_rmsnorm(at::Tensor& x, at::Tensor& z, at::Tensor& weight, float
     require(x.sizes() == z.sizes() && x.size(-1) == weight.numel(),
             "x and z must have the same shape, weight one entry per column");
     const int64_t D = x.size(-1);
+    require(D > 0, "gated_rmsnorm: rows of no columns");
     const at::Tensor xc = x.contiguous(), zc = z.contiguous(), w = weight.contiguous();
     at::Tensor y = empty(x.sizes(), x, at::kBFloat16);
     check(gdn_gated_rmsnorm(xc.data_ptr(), zc.data_ptr(), y.data_ptr(), w.data_ptr(), x.numel() / D, static_cast<int32_t>(D),
@@ -440,6 +441,7 @@ std::pair<at::Tensor, at::Tensor> fused_gdn_gating(at::Tensor& A_log, at::Tensor
                 a.scalar_type() == dt_bias.scalar_type(),
             "A_log, dt_bias, a, b must share a dtype");
     const int64_t vh = a.size(-1);
+    require(vh > 0, "fused_gdn_gating: no heads");
     require(A_log.numel() >= vh && dt_bias.numel() >= vh, "A_log and dt_bias need one entry per head");
     at::Tensor ac = a.contiguous(), bc = b.contiguous(), Ac = A_log.contiguous(), dc = dt_bias.contiguous();
     at::Tensor beta = empty_shaped_like(bc), gate = empty_shaped_like(ac);

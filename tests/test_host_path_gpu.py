@@ -71,3 +71,12 @@ def test_refusals(api):
         api.chunked_forward(d["q"], d["k"], d["v"], d["b"].cpu(), None)
     with pytest.raises(RuntimeError):
         api.gated_rmsnorm(d["v"], d["q"].float(), d["q"][0, 0, 0])
+
+
+def test_empty_last_axis_is_refused(api):
+    """The row count of these calls is the size divided by the last axis: an empty one raises and does not divide."""
+    e = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(RuntimeError):
+        api.gated_rmsnorm(e(3, 0), e(3, 0), e(0))
+    with pytest.raises(RuntimeError):
+        api.fused_gdn_gating(e(0), e(0), e(3, 0), e(3, 0))
