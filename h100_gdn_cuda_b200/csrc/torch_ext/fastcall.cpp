@@ -2,6 +2,8 @@
 // A decode step or a short prompt lasts a few microseconds on the GPU, so the host path is what such a call
 // costs: filling the C structs through ctypes took 25 - 35 us a call and the keyword dispatch of the pybind
 // functions takes about 2.  Here an argument is a pointer check, and the work below is namespace gdn_cuda's.
+// That work runs without the interpreter lock: a launch waits while the stream's queue is full, and other Python threads
+// must not wait with it.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
@@ -61,6 +63,13 @@ struct OnDevice {
     cudaStream_t stream() const { return at::cuda::getCurrentCUDAStream().stream(); }
 };
 
+// `work()` without the interpreter lock (an exception takes it back on its way out).
+template <typename F>
+auto unlocked(F&& work) {
+    pybind11::gil_scoped_release release;
+    return work();
+}
+
 // query, key, value, initial_state, beta, gate, cu_seqlens, num_accepted_tokens, inference_mode, is_qk_norm, scale,
 // inplace_state, gating, state_indices
 PyObject* recurrent_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -81,10 +90,13 @@ PyObject* recurrent_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     gdn_cuda::RecurrentExtensions ext;
     ext.inplace_state = truth(a[11]);
     ext.state_indices = optional_tensor(a[13], "state_indices");
+    const auto mode = static_cast<gdn_cuda::InferenceMode>(integer(a[8]));
+    const bool norm = truth(a[9]);
+    const auto scale = optional_real(a[10]);
     OnDevice dev(q, "query");
-    const auto r = gdn_cuda::recurrent_forward_ext(q, k, v, state, beta, gate, gating, cu, accepted,
-                                                   static_cast<gdn_cuda::InferenceMode>(integer(a[8])), dev.stream(), truth(a[9]),
-                                                   optional_real(a[10]), ext);
+    const auto r = unlocked([&] {
+        return gdn_cuda::recurrent_forward_ext(q, k, v, state, beta, gate, gating, cu, accepted, mode, dev.stream(), norm, scale, ext);
+    });
     return pair(r.first, r.second);
     END_HANDLE_TH_ERRORS
 }
@@ -99,9 +111,12 @@ PyObject* chunked_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     std::optional<int> chunks;
     if (a[10] != Py_None) chunks = static_cast<int>(integer(a[10]));
     auto workspace = optional_tensor(a[12], "workspace");
+    const auto scale = optional_real(a[5]);
+    const bool norm = truth(a[11]);
     OnDevice dev(q, "query");
-    const auto r = gdn_cuda::chunked_forward_ext(q, k, v, beta, gate, optional_real(a[5]), state, cu, ci, cc, chunks, dev.stream(),
-                                                 truth(a[11]), workspace);
+    const auto r = unlocked([&] {
+        return gdn_cuda::chunked_forward_ext(q, k, v, beta, gate, scale, state, cu, ci, cc, chunks, dev.stream(), norm, workspace);
+    });
     return pair(r.first, r.second);
     END_HANDLE_TH_ERRORS
 }
@@ -112,7 +127,7 @@ PyObject* fused_gdn_gating(PyObject*, PyObject* const* a, Py_ssize_t n) {
     require(n == 4, "fused_gdn_gating takes 4 positional arguments");
     at::Tensor A = tensor(a[0], "A_log"), dt = tensor(a[1], "dt_bias"), x = tensor(a[2], "a"), b = tensor(a[3], "b");
     OnDevice dev(x, "a");
-    const auto r = gdn_cuda::fused_gdn_gating(A, dt, x, b, false, dev.stream());
+    const auto r = unlocked([&] { return gdn_cuda::fused_gdn_gating(A, dt, x, b, false, dev.stream()); });
     return pair(r.first, r.second);
     END_HANDLE_TH_ERRORS
 }
@@ -124,8 +139,9 @@ PyObject* causal_conv1d(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::Tensor x = tensor(a[0], "x"), w = tensor(a[1], "weight");
     auto bias = optional_tensor(a[2], "bias"), s_in = optional_tensor(a[3], "initial_state"), cu = optional_tensor(a[4], "cu_seqlens");
     auto s_out = optional_tensor(a[6], "final_state");
+    const bool silu = truth(a[5]), want_state = truth(a[7]);
     OnDevice dev(x, "x");
-    const auto r = gdn_cuda::causal_conv1d(x, w, bias, s_in, cu, truth(a[5]), s_out, truth(a[7]), dev.stream());
+    const auto r = unlocked([&] { return gdn_cuda::causal_conv1d(x, w, bias, s_in, cu, silu, s_out, want_state, dev.stream()); });
     return r.second.has_value() ? pair(r.first, *r.second) : THPVariable_Wrap(r.first);
     END_HANDLE_TH_ERRORS
 }
@@ -135,8 +151,9 @@ PyObject* gated_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     require(n == 4, "gated_rmsnorm takes 4 positional arguments");
     at::Tensor x = tensor(a[0], "x"), z = tensor(a[1], "z"), w = tensor(a[2], "weight");
+    const float eps = static_cast<float>(real(a[3]));
     OnDevice dev(x, "x");
-    return THPVariable_Wrap(gdn_cuda::gated_rmsnorm(x, z, w, static_cast<float>(real(a[3])), dev.stream()));
+    return THPVariable_Wrap(unlocked([&] { return gdn_cuda::gated_rmsnorm(x, z, w, eps, dev.stream()); }));
     END_HANDLE_TH_ERRORS
 }
 

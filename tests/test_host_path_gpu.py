@@ -1,5 +1,8 @@
 """The package's per-call functions through the C++ front end and through the ctypes bodies: same library calls, so
 the same bits (and the same refusals)."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -80,3 +83,38 @@ def test_empty_last_axis_is_refused(api):
         api.gated_rmsnorm(e(3, 0), e(3, 0), e(0))
     with pytest.raises(RuntimeError):
         api.fused_gdn_gating(e(0), e(0), e(3, 0), e(3, 0))
+
+
+def test_a_full_queue_does_not_stop_other_threads(api):
+    """A launch blocks while the stream's queue is full (some 1000 launches, here behind a kernel of about half a second):
+    another Python thread goes on meanwhile."""
+    d = _cuda(synthetic.decode_inputs(1, 1, 1, 1, 64, seed=1))
+    x = torch.randn(8, 64, device="cuda").bfloat16()
+    calls = [lambda: api.fused_gdn_gating(d["A_log"], d["dt_bias"], d["a"], d["b"]), lambda: api.gated_rmsnorm(x, x, x[0]),
+             lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], d["b"]),
+             lambda: api.causal_conv1d(x[None], x[:4].T.contiguous()),
+             lambda: api.chunked_forward(d["q"], d["k"], d["v"], d["b"], None)]
+    for call in calls:
+        call()
+        torch.cuda.synchronize()
+        beats, done = [], threading.Event()
+
+        def beat():
+            while not done.is_set():
+                beats.append(time.perf_counter())
+                time.sleep(0.002)
+        t = threading.Thread(target=beat)
+        t.start()
+        torch.cuda._sleep(900_000_000)
+        t0, longest = time.perf_counter(), 0.0
+        for _ in range(2500):
+            t1 = time.perf_counter()
+            call()
+            longest = max(longest, time.perf_counter() - t1)
+        t1 = time.perf_counter()
+        done.set()
+        t.join()
+        torch.cuda.synchronize()
+        during = [t0] + [b for b in beats if t0 <= b <= t1] + [t1]
+        assert longest > 0.1, "no launch had to wait"
+        assert max(b - a for a, b in zip(during, during[1:])) < longest / 2
