@@ -31,7 +31,13 @@ bool truth(PyObject* o) {
     if (r < 0) throw python_error();
     return r != 0;
 }
-long integer(PyObject* o) {
+long integer(PyObject* o) {  // whatever int() takes
+    THPObjectPtr converted;
+    if (!PyLong_Check(o)) {
+        converted = PyNumber_Long(o);
+        if (!converted) throw python_error();
+        o = converted.get();
+    }
     const long r = PyLong_AsLong(o);
     if (r == -1 && PyErr_Occurred()) throw python_error();
     return r;

@@ -118,3 +118,14 @@ def test_a_full_queue_does_not_stop_other_threads(api):
         during = [t0] + [b for b in beats if t0 <= b <= t1] + [t1]
         assert longest > 0.1, "no launch had to wait"
         assert max(b - a for a, b in zip(during, during[1:])) < longest / 2
+
+
+def test_counts_and_modes_as_int_takes_them(api):
+    v = _cuda(synthetic.varlen_inputs([70, 5], 1, 1, 64, seed=3))
+    args = (v["q"], v["k"], v["v"], v["beta"], v["g"], None, None, v["cu_seqlens"], v["chunk_indices"], v["cu_chunks"])
+    ref = api.chunked_forward(*args, v["total_chunks"])
+    for chunks in (float(v["total_chunks"]), torch.tensor(v["total_chunks"]), torch.tensor(float(v["total_chunks"]), device="cuda")):
+        assert torch.equal(api.chunked_forward(*args, chunks)[0], ref[0])
+    d = _cuda(synthetic.decode_inputs(1, 2, 1, 1, 64, seed=1))
+    for mode in (2.0, torch.tensor(2), api.SpecVerify):
+        assert api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], d["b"], inference_mode=mode)[1].dim() == 5
