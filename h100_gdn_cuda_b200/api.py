@@ -9,6 +9,8 @@ from __future__ import annotations
 import ctypes as C
 import enum
 import math
+import os
+import warnings
 from typing import Optional, Tuple
 
 import torch
@@ -30,19 +32,31 @@ Prefill, Decode, SpecVerify = InferenceMode.Prefill, InferenceMode.Decode, Infer
 _state = {"library_root": None, "cuda_home": None}
 
 # The per-call functions below hand their arguments straight to the C++ front end (csrc/torch_ext/fastcall.cpp) when
-# the extension is built: 3 - 6 us of host time a call where the ctypes bodies take 25 - 35, which for a decode step or
+# the extension is built: 3 - 7 us of host time a call where the ctypes bodies take 25 - 35, which for a decode step or
 # a short prompt was several times the GPU's own time.  The ctypes bodies serve installations of the library alone
 # and the private arguments of the tests and the benchmark.
 _ext = None
+_FAST = ("_fast_recurrent_forward", "_fast_chunked_forward", "_fast_fused_gdn_gating", "_fast_causal_conv1d", "_fast_gated_rmsnorm")
 
 
 def _load_ext():
+    """The extension module, or False: not built (no word of it), or built but unusable (one warning, the calls are slower)."""
     global _ext
+    _ext, why = False, None
     try:
         from . import gdn_cuda
-        _ext = gdn_cuda
-    except ImportError:
-        _ext = False
+    except ImportError as e:
+        why = str(e)
+    else:
+        if all(hasattr(gdn_cuda, name) for name in _FAST):
+            _ext = gdn_cuda
+        else:
+            why = "it is older than this package"
+    if why is not None:
+        from . import build
+        if os.path.exists(build.ext_path()):
+            warnings.warn("%s is not used (%s); calls go through ctypes.  Rebuild it with python -m h100_gdn_cuda_b200.build --ext"
+                          % (build.ext_path(), why), RuntimeWarning, stacklevel=3)
     return _ext
 
 
