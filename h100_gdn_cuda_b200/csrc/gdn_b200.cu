@@ -121,11 +121,11 @@ static int launch_recurrent(const RecurrentParams& p, int sms, cudaStream_t st, 
 
 // Short padded runs (2 .. kStepTok tokens) on bf16 states of the head dims serving configurations use take
 // gdn_recurrent_step_kernel (recurrent_step.cuh), whatever the batch.
-static bool step_applies(const GdnShape& s, int state_dtype) {
+static bool step_takes(const GdnShape& s, int state_dtype) {
     return !s.cu_seqlens && s.seq_len >= 2 && s.seq_len <= kStepTok && state_dtype == GDN_BF16 && (s.head_dim_k == 64 || s.head_dim_k == 128) &&
-           s.head_dim_v % kStepRows == 0;
+           step_applies(s.head_dim_v);
 }
-static StepParams step_plan(const RecurrentParams& r, int dk, int sms, unsigned* grid) {
+static StepParams step_plan(const RecurrentParams& r, int sms, unsigned* grid) {
     StepParams p{};
     p.r = r;
     p.num_tiles = static_cast<long long>(r.batch) * r.vh * (r.dv / kStepRows);
@@ -137,7 +137,7 @@ static StepParams step_plan(const RecurrentParams& r, int dk, int sms, unsigned*
 template <int DK>
 static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
     unsigned grid = 0;
-    const StepParams p = step_plan(r, DK, sms, &grid);
+    const StepParams p = step_plan(r, sms, &grid);
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     GDN_CUDA(cudaGetDevice(&dev));
@@ -171,7 +171,7 @@ static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaS
                  kRecThreads, kStepCtasPerSm, dk);
         if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + ".step", src, "gdn_recurrent_jit", &k, &err)) return fail(rc, "%s", err.c_str());
         unsigned grid = 0;
-        StepParams sp = step_plan(p, dk, sms, &grid);
+        StepParams sp = step_plan(p, sms, &grid);
         const size_t smem = static_cast<size_t>(kStepWarps) * step_warp_bytes(dk, p.seq_len, sp.stages);
         GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
@@ -484,7 +484,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     p.split_tiles = ring ? 1 : 0;
     const int slots_per_sm = s.head_dim_k > 128 ? 2 : (a->state_dtype == GDN_F32 && s.head_dim_k > 64 ? 3 : 4);
     if (!ring && !s.cu_seqlens && s.seq_len == 1) p.split_tiles = p.num_tiles <= static_cast<long long>(d->sms) * slots_per_sm;
-    const bool step = !ring && step_applies(s, a->state_dtype);
+    const bool step = !ring && step_takes(s, a->state_dtype);
     if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
     if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
     if (a->state_dtype == GDN_F32) {

@@ -1,5 +1,5 @@
 // Recurrent Gated DeltaNet step on warp matrix instructions: padded inputs of 2 .. 8 tokens per sequence, bf16 states,
-// dk = 64 or 128, dv a multiple of 16 (speculative verify, short runs).  Same recurrence as recurrent.cuh:
+// dk = 64 or 128, dv a multiple of 32 (speculative verify, short runs).  Same recurrence as recurrent.cuh:
 //     S_t = a_t S_{t-1} + c_t k_t^T,   c_t = beta_t (v_t - a_t S_{t-1} k_t),   o_t = scale S_t q_t,   a_t = e^{g_t}
 // rewritten over the state S_0 the call starts from, with G_t = a_1 .. a_t and Gamma_ts = a_{s+1} .. a_t:
 //     c_t = beta_t v_t - beta_t G_t (S_0 k_t) - sum_{s<t} beta_t Gamma_ts (k_s.k_t) c_s
@@ -34,8 +34,14 @@ namespace gdn {
 constexpr int kStepTok = 8;      // tokens an item can have
 constexpr int kStepRows = 16;    // state rows per tile
 constexpr int kStepWarps = kRecThreads / 32;
-constexpr int kStepMaxStages = 4;
+constexpr int kStepMaxStages = 3;
 constexpr int kStepCtasPerSm = 2;  // 234 registers a thread; spilled to fit three, the update's stores to local memory cost more
+
+// The k, q of item i sit in slot i % stages until the item's first tile has been taken in, and at that moment the tile `stages`
+// further on is requested.  That one must belong to an item before i + stages: so at least two tiles per unit (only the two
+// ends of a warp's range, its first item and its last, can have fewer).
+__host__ __device__ constexpr bool step_applies(int dv) { return dv % (2 * kStepRows) == 0; }
+static_assert(step_applies(2 * kStepRows) && !step_applies(kStepRows), "one tile per unit would overwrite its k and q");
 
 // shared memory of one warp: the stages, the present item's k, q as MMA operands (16 rows), then for each stage room for the
 // k and q of an item's tokens
