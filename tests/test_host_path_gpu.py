@@ -36,7 +36,21 @@ def _calls(api):
     slots = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
     conv_in, conv_w = d["v"].reshape(3, 2, 256), torch.randn(256, 4, device="cuda").bfloat16()
     beta = torch.sigmoid(d["b"].float()).bfloat16()
+    wide = _cuda(synthetic.prefill_inputs(1, 70, 1, 2, 200, seed=4))
+    caps = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
+    conv_s, cu = torch.randn(3, 3, 256, device="cuda").bfloat16(), torch.tensor([0, 1, 5, 6], dtype=torch.int32, device="cuda")
+    bias, packed_in = torch.randn(256, device="cuda").bfloat16(), conv_in.reshape(6, 256)
+    ones = torch.tensor([0, 1, 2, 3], dtype=torch.int32, device="cuda")
     return {
+        "recurrent, caps": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], beta, d["a"], None, caps, 1, True)[1],
+        "recurrent, step states": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], beta, d["a"], inference_mode=2),
+        "recurrent, in place": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"].clone(), beta, d["a"], inplace_state=True),
+        "recurrent, fp32 state": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"].float(), beta, d["a"]),
+        "recurrent, packed": lambda: api.recurrent_forward(v["q"], v["k"], v["v"], v["state"], v["beta"], v["g"], v["cu_seqlens"]),
+        "prefill, d=200": lambda: api.chunked_forward(wide["q"], wide["k"], wide["v"], wide["beta"], wide["g"], None, wide["state"]),
+        "conv, bias and state": lambda: api.causal_conv1d(conv_in, conv_w, bias, conv_s, return_final_state=True),
+        "conv, packed": lambda: api.causal_conv1d(packed_in, conv_w, bias, conv_s, cu, return_final_state=True),
+        "conv, packed in place": lambda: (lambda s: api.causal_conv1d(packed_in[:3], conv_w, None, s, ones, final_state=s))(conv_s.clone()),
         "gating": lambda: api.fused_gdn_gating(*gating),
         "recurrent, gating inside": lambda: api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], None, None, gating=gating,
                                                                   is_qk_norm=True, inference_mode=2),

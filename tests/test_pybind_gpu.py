@@ -1,5 +1,6 @@
 """The C++/pybind11 `gdn_cuda` extension (same module surface as the reference's
-csrc/python_api.cpp) gives the same bits as the ctypes mirror, and raises RuntimeError."""
+csrc/python_api.cpp) gives the same bits as the ctypes mirror (the package with its native front end put aside: with it,
+both sides would be the same C++ functions), and raises RuntimeError."""
 import pytest
 import torch
 
@@ -16,6 +17,12 @@ def mods():
     build.build_ext()
     from h100_gdn_cuda_b200 import gdn_cuda as ext
     return py, ext
+
+
+@pytest.fixture(autouse=True)
+def ctypes_bodies(monkeypatch):
+    from h100_gdn_cuda_b200 import api
+    monkeypatch.setattr(api, "_ext", False)
 
 
 def dev(d):
