@@ -57,12 +57,18 @@ constexpr long long kSms = 148;
 constexpr long long kNoLimit = std::numeric_limits<long long>::max();
 // Cost model fitted to measurements (B=1..2, T=4096..131072, 4..32 v-heads), in units of "one
 // chunk of the state kernel" (1.25 us): a CTA costs its chunks plus about 3 for start-up and pipeline
-// fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Plans whose launches need more
-// than one wave measured worse than the model and are not made.
+// fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Every boundary between two segments of a chain
+// costs kBoundary on top: its composite and start state move 0.4 MB, and it is one more product of a kernel that runs 9 chains
+// at a time.  Without that term 20 to 48 chains of 75 to 200 chunks were cut although it cost time (B=1, d=128: 48 v-heads
+// of 100 chunks 200 us against 179 uncut, 32 of 75 130 against 121); with it all shapes measured (2 to 72 chains, 75 to 400
+// chunks, padded and packed) are within the noise of the better of cut and uncut.  Plans whose launches need more than one wave measured worse
+// than the model and are not made.
 constexpr int kFixed = 3;
-constexpr double kPasses = 2.2;
-// Shortest segments: below, the two extra launches and the serial chaining of the start states eat the gain.  Packed
-// sequences of unequal lengths each end in a shorter one, hence the larger figure there.
+constexpr double kPasses = 2.2, kBoundary = 0.15, kMargin = 0.85;
+// Shortest segments.  With 16 chains of 90, 100, 125 chunks at least 20 gives 103, 103, 113 us, 25 117, 112, 119 and 32 121, 128,
+// 151; but 66 chunks are slower cut in three (94 us against 92), 32 chains of 66 by 11 %.  Packed sequences of unequal
+// lengths each end in a shorter one, hence the larger figure there (equal ones gain from 25: one of 100 chunks on 16 heads 129
+// -> 112 us).
 constexpr int kMinSegment = 25, kMinSegmentPacked = 32;
 inline long long waves(long long ctas) { return (ctas + kSms - 1) / kSms; }
 }  // namespace plan_detail
@@ -71,11 +77,11 @@ inline SegmentPlan prefill_segments(long long chains, int chunks_per_seq, bool p
     using namespace plan_detail;
     SegmentPlan plan{1, chunks_per_seq, 0};
     if (packed || chains <= 0) return plan;
-    double best = 0.8 * static_cast<double>(waves(chains) * (chunks_per_seq + kFixed));
+    double best = kMargin * static_cast<double>(waves(chains) * (chunks_per_seq + kFixed));
     for (int P = 2; P <= 32 && chunks_per_seq / P >= kMinSegment; ++P) {
         if (waves(chains * P) > 1 || chains * P > max_units) break;
         const int len = (chunks_per_seq + P - 1) / P;
-        const double cost = kPasses * (len + kFixed);
+        const double cost = kPasses * (len + kFixed) + kBoundary * static_cast<double>(chains * (P - 1));
         if (cost < best) {
             best = cost;
             plan.num_segments = P;
@@ -98,7 +104,7 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
     if (num_seqs <= 0 || num_seqs > kMaxSegmentedSeqs || num_v_heads <= 0 || total_chunks <= 0 || total_chunks > (1 << 30)) return plan;
     const long long chains = static_cast<long long>(num_seqs) * num_v_heads;
     const long long even = (total_chunks + num_seqs - 1) / num_seqs;
-    double best = 0.8 * static_cast<double>(waves(chains) * (even + kFixed));
+    double best = kMargin * static_cast<double>(waves(chains) * (even + kFixed));
     for (int P = 2; P <= 128 && total_chunks / P >= kMinSegmentPacked; ++P) {
         const int len = static_cast<int>((total_chunks + P - 1) / P);
         const long long slots = total_chunks / len + num_seqs;  // launched (and given scratch): the upper bound
@@ -108,7 +114,7 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
         const long long work = (total_chunks + len - 1) / len + num_seqs - 1;
         if (waves(work * num_v_heads) > 1) break;
         if (slots * num_v_heads > max_units) continue;
-        const double cost = kPasses * (len + kFixed);
+        const double cost = kPasses * (len + kFixed) + kBoundary * static_cast<double>((work - num_seqs) * num_v_heads);
         if (cost < best) {
             best = cost;
             plan.num_segments = P;

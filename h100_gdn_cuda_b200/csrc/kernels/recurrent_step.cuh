@@ -11,8 +11,9 @@
 // which is all 24 bits of them.
 //
 // Why: on FMAs (recurrent.cuh) a warp spends 240 instructions per token and 8 rows of state, and the step is bound by
-// their issue.  Here it is some 500 per 16 rows for any number of tokens: B=64, T=4, accepted caps 1..4, 32 v-heads, d=128
-// 52.5 -> 31.5 us (140 MB: 21.5 us at the measured copy bandwidth), B=13, T=5 with a state per token 25.4 -> 20.8 us.
+// their issue.  Here it is 750 per 16 rows for four tokens and the last state, where that would be 1 920 (counted by
+// ncu, per-item work included), and 2 390 with five states: B=64, T=4, accepted caps 1..4, 32 v-heads, d=128 52.5 -> 31.7 us
+// (140 MB: 21.5 us at the measured copy bandwidth), B=13, T=5 with a state per token 25.4 -> 20.6 us.
 // (For ONE token per sequence the FMA kernel is already bound by HBM and stays: 88.7 us at B=256 against 92 - 102 this way.)
 //
 // Every warp works by itself on items of whole (sequence, v-head) units, dealt round by round; what does not fill a last
@@ -20,8 +21,8 @@
 // the cut a seventh of the GPU idles in the fourth round; with ranges for everything the warps' streams are spread over all
 // of memory at once).  Each warp has a ring of stages of its own, filled by bulk copies (a tile is 16 x dk
 // contiguous; the item's k, q come with its first tile).  A tile is taken into registers at once and its stage requested again, so all stages are in flight
-// while the warp computes, and no warp waits for another.  (Tiles of 64 rows shared by the four warps of a CTA, with the
-// per-item work repeated by each: 724 instead of about 350 instructions per 16 rows.)  
+// while the warp computes, and no warp waits for another.  (With tiles of 64 rows shared by
+// the four warps of a CTA each of them would repeat the per-item work.)
 // Products: [k; q] (tokens 0-7 and 8-15 of M) times S^T (8 state rows of N), so that a 16-byte piece of a state row is two B
 // operands as it lies; the contraction index may be permuted freely, and lane (g, t) takes the pieces t, t + 4, .. of rows g
 // and g + 8.  Their result has token g, rows 2t, 2t + 1 in lane (g, t), which is how v is read and o written.  Update: rows

@@ -135,6 +135,29 @@ def test_segment_plan_heuristic():
     assert rows[13][0] == 1              # four equal sequences would already run side by side
 
 
+def test_short_sequences_of_many_chains_stay_whole():
+    """24 to 48 chains: measured uncut at 75 .. 100 chunks (cut it took up to 16 % longer), cut at 400."""
+    import subprocess, tempfile, textwrap
+    src = textwrap.dedent('''
+        #include <cstdio>
+        #include "heuristics.hpp"
+        int main() {
+            for (int chains : {24, 32, 40, 48})
+                for (int chunks : {75, 90, 400})
+                    std::printf("%d %d\\n", gdn::prefill_segments(chains, chunks, false).num_segments,
+                                gdn::prefill_segments_packed(1, chains, chunks).num_segments);
+            return 0;
+        }''')
+    with tempfile.TemporaryDirectory() as d:
+        c = os.path.join(d, "h.cpp")
+        open(c, "w").write(src)
+        exe = os.path.join(d, "h")
+        subprocess.check_call(["g++", "-std=c++17", "-I", os.path.join(ROOT, "h100_gdn_cuda_b200", "csrc"), c, "-o", exe])
+        rows = [l.split() for l in subprocess.check_output([exe]).decode().splitlines()]
+    for i, row in enumerate(rows):
+        assert all((int(n) > 1) == (i % 3 == 2) for n in row), (i, row)
+
+
 @pytest.mark.parametrize("B,T,vh,packed", [(1, 50048, 2, False), (1, 65536, 2, False), (1, 16384, 8, False), (4, 8000, 4, True)])
 def test_static_scratch_takes_fewer_segments(lib, B, T, vh, packed):
     """What fits the built-in scratch array without segment states is not refused because the preferred segment plan
