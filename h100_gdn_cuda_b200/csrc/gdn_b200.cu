@@ -93,19 +93,19 @@ static cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, int threads, s
     return cudaLaunchKernelEx(&cfg, kernel, params);
 }
 
-template <int DK, bool kRing, bool kLean = false, bool kF32 = false>
+template <int DK, bool kRing, bool kLean = false, bool kF32 = false, bool kSplit = false>
 static int launch_recurrent_t(const RecurrentParams& p, int sms, cudaStream_t st) {
     constexpr int smem = recurrent_smem_bytes<DK, kRing, kF32>();
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev]) {
-        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_kernel<DK, kRing, kLean, kF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_kernel<DK, kRing, kLean, kF32, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev] = true;
     }
     const int per_sm = recurrent_ctas_per_sm<DK, kRing, kF32>();
     const long long grid = std::min<long long>(p.num_tiles, static_cast<long long>(sms) * per_sm);
-    GDN_CUDA(launch_dependent(gdn_recurrent_kernel<DK, kRing, kLean, kF32>, dim3(static_cast<unsigned>(grid)), kRecThreads, smem, st, p));
+    GDN_CUDA(launch_dependent(gdn_recurrent_kernel<DK, kRing, kLean, kF32, kSplit>, dim3(static_cast<unsigned>(grid)), kRecThreads, smem, st, p));
     return GDN_OK;
 }
 
@@ -116,7 +116,15 @@ template <int DK>
 static int launch_recurrent(const RecurrentParams& p, int sms, cudaStream_t st, bool ring, bool lean) {
     if (ring) return launch_recurrent_t<DK, true>(p, sms, st);
     if (lean) return launch_recurrent_t<DK, false, true>(p, sms, st);
+    if (p.split_tiles) return launch_recurrent_t<DK, false, false, false, true>(p, sms, st);
     return launch_recurrent_t<DK, false>(p, sms, st);
+}
+
+template <int DK>
+static int launch_recurrent_f32(const RecurrentParams& p, int sms, cudaStream_t st, bool ring) {
+    if (ring) return launch_recurrent_t<DK, true, false, true>(p, sms, st);
+    if (p.split_tiles) return launch_recurrent_t<DK, false, false, true, true>(p, sms, st);
+    return launch_recurrent_t<DK, false, false, true>(p, sms, st);
 }
 
 // Short padded runs (2 .. kStepTok tokens) on bf16 states of the head dims serving configurations use take
@@ -158,8 +166,8 @@ static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaS
     snprintf(src, sizeof(src),
              "#include \"kernels/recurrent.cuh\"\n"
              "extern \"C\" __global__ void __launch_bounds__(%d, %d) gdn_recurrent_jit(const gdn::RecurrentParams p) {\n"
-             "    gdn::gdn_recurrent_body<%d, %s>(p);\n}\n",
-             kRecThreads, cfg.ctas_per_sm, dk, ring ? "true" : "false");
+             "    gdn::gdn_recurrent_body<%d, %s, false, false, %s>(p);\n}\n",
+             kRecThreads, cfg.ctas_per_sm, dk, ring ? "true" : "false", !ring && p.split_tiles ? "true" : "false");
     jit::LoadedKernel k;
     std::string err;
     if (step) {
@@ -179,7 +187,7 @@ static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaS
         GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(kRecThreads), args, smem, st));
         return GDN_OK;
     }
-    if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + (ring ? "_ring" : ""), src, "gdn_recurrent_jit", &k, &err))
+    if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + (ring ? "_ring" : p.split_tiles ? "_split" : ""), src, "gdn_recurrent_jit", &k, &err))
         return fail(rc, "%s", err.c_str());
     GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   cfg.smem_bytes));
@@ -489,8 +497,8 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
     if (a->state_dtype == GDN_F32) {
         // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
-        if (s.head_dim_k == 128) return ring ? launch_recurrent_t<128, true, false, true>(p, d->sms, st) : launch_recurrent_t<128, false, false, true>(p, d->sms, st);
-        if (s.head_dim_k == 64) return ring ? launch_recurrent_t<64, true, false, true>(p, d->sms, st) : launch_recurrent_t<64, false, false, true>(p, d->sms, st);
+        if (s.head_dim_k == 128) return launch_recurrent_f32<128>(p, d->sms, st, ring);
+        if (s.head_dim_k == 64) return launch_recurrent_f32<64>(p, d->sms, st, ring);
         return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: fp32 states are built for dk = 64 and 128 (got %d)", s.head_dim_k);
     }
     const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx && !p.split_tiles;
