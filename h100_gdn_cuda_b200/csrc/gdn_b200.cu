@@ -128,9 +128,19 @@ static int launch_recurrent_f32(const RecurrentParams& p, int sms, cudaStream_t 
 }
 
 // Short padded runs (2 .. kStepTok tokens) on bf16 states of the head dims serving configurations use take
-// gdn_recurrent_step_kernel (recurrent_step.cuh), whatever the batch.
-static bool step_takes(const GdnShape& s, int state_dtype) {
-    return !s.cu_seqlens && s.seq_len >= 2 && s.seq_len <= kStepTok && state_dtype == GDN_BF16 && (s.head_dim_k == 64 || s.head_dim_k == 128) &&
+// gdn_recurrent_step_kernel (recurrent_step.cuh).  Not where the (sequence, v-head) units are one nearly full wave of the FMA
+// kernel's CTA slots and the tokens few: its slots then take a unit each, while the tiles a warp has here are 3.2 to 4 (at d=64
+// 1.3 to 2) of them, rounded up.  With 32 v-heads and a state per token, FMA against this: d=128, T=2 B=14 13.2 : 13.8 us, B=16
+// 13.8 : 15.7, B=18 14.1 : 16.0, B=20 (two waves) 17.9 : 16.1; T=4 B=16 20.8 : 22.1; T=5 24.9 : 25.8 but B=14 4 % the other way;
+// d=64, T=2 B=10 1 % apart, B=12 7.0 : 7.7, B=18 7.4 : 8.1; T=4 B=16 9.8 : 10.2.  With the last state alone only d=64, T=2 is
+// (6.7 : 7.1 at B=12; d=128 within 3 % of each other at B=16, 18).
+static bool fma_wave(const GdnShape& s, bool steps, int sms) {
+    const long long units = static_cast<long long>(s.batch) * s.num_v_heads, slots = 4ll * sms;
+    const bool narrow = s.head_dim_k == 64;
+    return s.head_dim_k == s.head_dim_v && s.seq_len <= (steps ? 4 : narrow ? 2 : 0) && units <= slots && 10 * units >= (narrow ? 6 : 8) * slots;
+}
+static bool step_takes(const GdnShape& s, int state_dtype, bool steps, int sms) {
+    return !s.cu_seqlens && !fma_wave(s, steps, sms) && s.seq_len >= 2 && s.seq_len <= kStepTok && state_dtype == GDN_BF16 && (s.head_dim_k == 64 || s.head_dim_k == 128) &&
            step_applies(s.head_dim_v);
 }
 static StepParams step_plan(const RecurrentParams& r, int sms, unsigned* grid) {
@@ -492,7 +502,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     p.split_tiles = ring ? 1 : 0;
     const int slots_per_sm = s.head_dim_k > 128 ? 2 : (a->state_dtype == GDN_F32 && s.head_dim_k > 64 ? 3 : 4);
     if (!ring && !s.cu_seqlens && s.seq_len == 1) p.split_tiles = p.num_tiles <= static_cast<long long>(d->sms) * slots_per_sm;
-    const bool step = !ring && step_takes(s, a->state_dtype);
+    const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
     if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
     if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
     if (a->state_dtype == GDN_F32) {

@@ -87,6 +87,19 @@ def test_no_state_no_gate(gdn):
     close(s, s_ref, "state")
 
 
+@pytest.mark.parametrize("B,T,vh,d", [(14, 2, 32, 128), (15, 2, 32, 128), (18, 4, 32, 128), (37, 3, 16, 128), (38, 2, 16, 128), (16, 5, 32, 128),
+                                      (11, 2, 32, 64), (12, 3, 32, 64), (37, 4, 16, 64)])
+@pytest.mark.parametrize("steps", [False, True])
+def test_one_wave_of_units(gdn, B, T, vh, d, steps):
+    """on either side of the band of units (474 to 592 at d=128, 356 to 592 at d=64) where short runs stay with the FMA kernel"""
+    p, pd, beta, g = problem(B, T, vh // 2, vh, d, seed=B + T)
+    bb = beta.bfloat16()
+    o_ref, s_ref = O.recurrent_ref(p["q"].float(), p["k"].float(), p["v"].float(), bb.float(), g, p["state"].float(), is_qk_norm=True, store_step_state=True)
+    o, s = gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], pd["state"], bb.cuda(), g.cuda(), inference_mode=gdn.SpecVerify if steps else gdn.Decode, is_qk_norm=True)
+    close(o, o_ref, "o")
+    close(s, s_ref if steps else s_ref[:, -1], "states")
+
+
 @pytest.mark.parametrize("B", [1, 4, 5])
 def test_one_token_tiles_apart_or_together(gdn, B):
     """one token per sequence: up to 592 tiles of 32 rows (B=4 with 32 v-heads of 128 rows is 512) every tile is a work unit,
