@@ -32,7 +32,7 @@ Prefill, Decode, SpecVerify = InferenceMode.Prefill, InferenceMode.Decode, Infer
 _state = {"library_root": None, "cuda_home": None}
 
 # The per-call functions below hand their arguments straight to the C++ front end (csrc/torch_ext/fastcall.cpp) when
-# the extension is built: 3 - 7 us of host time a call where the ctypes bodies take 25 - 35, which for a decode step or
+# the extension is built: 4 - 9 us of host time a call where the ctypes bodies take 25 - 35, which for a decode step or
 # a short prompt was several times the GPU's own time.  The ctypes bodies serve installations of the library alone
 # and the private arguments of the tests and the benchmark.
 _ext = None

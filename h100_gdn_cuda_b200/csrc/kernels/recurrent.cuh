@@ -1,5 +1,5 @@
 // Recurrent Gated DeltaNet step (decode, speculative verify, short prefill).  Padded runs of 2 .. 8 tokens on bf16 states of
-// head dims 64 and 128 take recurrent_step.cuh instead.
+// head dims 64 and 128 take recurrent_step.cuh instead, but for those where one wave of units fits here (fma_wave, gdn_b200.cu).
 //
 // Replaces the reference's fused_recurrent_gated_delta_rule_bf16
 // (gdn_cuda/include/gdn_cuda/kernels/sm90_bf16_gdn_recurrent.cuh:20-440) with the

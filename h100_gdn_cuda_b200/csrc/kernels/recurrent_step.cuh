@@ -36,7 +36,7 @@ constexpr int kStepTok = 8;      // tokens an item can have
 constexpr int kStepRows = 16;    // state rows per tile
 constexpr int kStepWarps = kRecThreads / 32;
 constexpr int kStepMaxStages = 3;
-constexpr int kStepCtasPerSm = 2;  // 234 registers a thread; spilled to fit three, the update's stores to local memory cost more
+constexpr int kStepCtasPerSm = 2;  // 249 registers a thread; spilled to fit three, the update's stores to local memory cost more
 
 // The k, q of item i sit in slot i % stages until the item's first tile has been taken in, and at that moment the tile `stages`
 // further on is requested.  That one must belong to an item before i + stages: so at least two tiles per unit (only the two
