@@ -7,6 +7,7 @@
 #include "kernels/helpers.cuh"
 #include "kernels/layer_adjacent.cuh"
 #include "kernels/recurrent.cuh"
+#include "kernels/recurrent_block.cuh"
 #include "kernels/recurrent_step.cuh"
 
 #include <atomic>
@@ -165,6 +166,33 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
     }
     GDN_CUDA(launch_dependent(gdn_recurrent_step_kernel<DK>, dim3(grid), kRecThreads,
                               static_cast<size_t>(kStepWarps) * step_warp_bytes(DK, r.seq_len, p.stages), st, p));
+    return GDN_OK;
+}
+
+// Long runs of tokens whose last state alone is wanted: blocks of tokens on warp matrix instructions (recurrent_block.cuh),
+// unless the runs are but one token longer than a block and the CTAs are many: a block with one token takes as long as one with
+// 16, and the token recurrence fills the GPU then.  Token recurrence against this, 32 v-heads: d=128, T=17 B=64 316 : 342 us, B=8
+// 48 : 45, B=1 (one wave of CTAs) 14.2 : 8.1; T=24 B=64 430 : 343; d=64, T=17 B=64 105 : 143, B=8 17.2 : 21.5, T=24 138 : 144, T=40
+// 222 : 187; d=256, 8 v-heads, T=17 B=16 59 : 60, T=32 102 : 61.
+static bool block_takes(const GdnShape& s, bool steps, int sms) {
+    if (steps || (s.head_dim_k != 64 && s.head_dim_k != 128 && s.head_dim_k != 192 && s.head_dim_k != 256)) return false;
+    const long long tokens = s.cu_seqlens ? s.total_tokens : static_cast<long long>(s.seq_len) * s.batch;
+    const long long ctas = static_cast<long long>(s.batch) * s.num_v_heads * (s.head_dim_v / kBlkRows);
+    return ctas <= 2ll * sms || tokens >= (s.head_dim_k == 64 ? 26ll : 20ll) * s.batch;
+}
+template <int DK, bool kF32 = false>
+static int launch_block_t(const RecurrentParams& p, cudaStream_t st) {
+    constexpr int smem = BlockSmem<DK>::kBytes;
+    static std::atomic<bool> attr_set[64];
+    int dev = 0;
+    GDN_CUDA(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_set[dev & 63].store(true, std::memory_order_release);
+    }
+    const long long grid = static_cast<long long>(p.batch) * p.vh * (p.dv / kBlkRows);
+    GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
+    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kF32>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
     return GDN_OK;
 }
 
@@ -505,6 +533,16 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
     if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
     if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
+    if (ring && block_takes(s, p.store_step != 0, d->sms)) {
+        switch (s.head_dim_k * (a->state_dtype == GDN_F32 ? -1 : 1)) {
+            case 64: return launch_block_t<64>(p, st);
+            case 128: return launch_block_t<128>(p, st);
+            case 192: return launch_block_t<192>(p, st);
+            case 256: return launch_block_t<256>(p, st);
+            case -64: return launch_block_t<64, true>(p, st);
+            case -128: return launch_block_t<128, true>(p, st);
+        }
+    }
     if (a->state_dtype == GDN_F32) {
         // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
         if (s.head_dim_k == 128) return launch_recurrent_f32<128>(p, d->sms, st, ring);

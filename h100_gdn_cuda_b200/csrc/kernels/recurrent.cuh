@@ -18,7 +18,7 @@
 // The eight row sums are reduced over 16 lanes with a transposing butterfly (8 shuffles
 // instead of 32).  For single-token decode q/k normalisation and k.q are computed once per
 // unit, not per tile.  New states leave through coalesced 8-byte stores from registers.
-// Long runs of tokens (short prefill, head dims the chunked kernels do not cover) take a second
+// Long runs of tokens take recurrent_block.cuh, or where that is no better, or a state per token is wanted, a second
 // instance of the kernel (kRing), chosen by the host when the sequences average more than
 // kRecTokRingMin tokens: every tile is a work unit of its own, so that a few long sequences
 // still spread over all CTAs, and k, q, v arrive 8 tokens at a time by bulk copies: the first

@@ -1,0 +1,556 @@
+// Recurrent Gated DeltaNet over long runs of tokens (short prefill through recurrent_forward, head dims above 128 in
+// chunked_forward): blocks of 16 tokens on warp matrix instructions.  Same recurrence as recurrent.cuh, rewritten over the
+// state S_0 a block starts from as in recurrent_step.cuh, with G_t = a_1 .. a_t and Gamma_ts = a_{s+1} .. a_t:
+//     c_t = beta_t v_t - beta_t G_t (S_0 k_t) - sum_{s<t} A_ts c_s,   A_ts = beta_t Gamma_ts (k_s.k_t)
+//     o_t = scale G_t (S_0 q_t) + sum_{s<=t} P_ts c_s,                P_ts = scale Gamma_ts (k_s.q_t)
+//     S  <- G_n S_0 + sum_s (Gamma_ns c_s) k_s^T
+// Precision is that of fp32 arithmetic.  The state stays in fp32 registers from the first token to the last; it enters
+// S_0 [k; q] as three bf16 terms, which is all 24 bits of it, and so do the coefficients of the update; k and q are the bf16
+// values they are (their norms are fp32 factors of the results).  Products of bf16 values are exact, their sums are fp32; the
+// solve and the outputs are fp32 FMAs; the update is added to the decayed state by one fp32 FMA per element and BLOCK, where
+// the token recurrence rounds the state at every token.
+//
+// Why: the token recurrence (recurrent.cuh, ring instance) is a chain of about 1 250 cycles per token, and a sequence of a
+// few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of products (1 000
+// cycles), sums and a triangular solve (850), the update (500) and the outputs (400): B=2, T=1500, 8 v-heads, d=256 996 -> 256 us,
+// T=700, 4 v-heads, d=192 401 -> 73, T=65 42 -> 12.5; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.75 ms.  With two CTAs per SM
+// the matrix instructions set the pace (16 cycles each, 84 per scheduler, block and CTA: 2 700 of 4 450 cycles), with one the
+// chain.  Against 64 bits an fp32 state is off by 2.6e-7 instead of 2.9e-7 after 1500 tokens of weak decay, 1.2e-7 instead of
+// 3.4e-7 without decay, 5.7e-8 instead of 5.8e-8 with a strong one (d=128, relative 2-norm).
+//
+// A CTA owns 16 state rows (M of the products) of one (sequence, v-head) and walks its blocks:
+//   warps 0-3   a quarter of the columns each, kept as accumulator fragments, which are the A operands of the product
+//               S_0 [k; q]^T as they lie.  The four partial products meet in shared memory; then EVERY warp sums them and
+//               solves for c (lane r + 16 h: row r, tokens 8 h .. 8 h + 7), which costs less than a second barrier and a
+//               trip through shared memory, and updates its own columns.  Each warp writes a quarter of the tokens' outputs.
+//   warps 4-7   prepare blocks in turn (warp 4 + j: blocks j, j + 4, ..), up to four ahead: copies of k, q, v, the Gram matrices
+//               k k^T and q k^T on matrix instructions, decay products, norms, and from them the matrices A and P.
+//               (Four of them, so that their work is spread over the four schedulers.)
+// Two CTAs per SM at dk = 256: one's chain fills the gaps of the other.
+#pragma once
+#include <type_traits>
+
+#include "recurrent_step.cuh"
+
+namespace gdn {
+
+constexpr int kBlkTok = 16;   // tokens per block
+constexpr int kBlkRows = 16;  // state rows per CTA
+constexpr int kBlkThreads = 256;
+
+template <int DK>
+struct BlockSmem {
+    // rows of k and q are 16 bytes longer than the data: eight rows at one column lie in different banks
+    static constexpr int kRow = DK * 2 + 16;
+    static constexpr int kOffQ = kBlkTok * kRow, kOffV = 2 * kBlkTok * kRow;
+    static constexpr int kStage = kOffV + kBlkTok * kBlkRows * 2;
+    static constexpr int kStages = 4;  // one per preparing warp
+    // what a block's solve needs, floats: A as [s][t], P as [t][s], beta v as [row][t] (before that: decay products), factors
+    static constexpr int kA = 0, kP = 256, kR0 = 512, kLdR = 20, kCk = kR0 + 16 * kLdR, kCq = kCk + 16, kW = kCq + 16, kG = kW + 16;
+    static constexpr int kPrepFloats = kG + 4;
+    static constexpr int kOffPrep = kStages * kStage;
+    static constexpr int kLdD = 36;  // partial products of a warp: 16 rows x (16 k tokens, 16 q tokens)
+    static constexpr int kOffD = kOffPrep + kStages * kPrepFloats * 4;
+    static constexpr int kOffC = kOffD + 2 * 4 * kBlkRows * kLdD * 4;  // coefficients as operands: [warp][term][row], 48-byte rows
+    static constexpr int kRowC = 48;
+    static constexpr int kBytes = kOffC + 4 * 3 * kBlkRows * kRowC;
+    static_assert(kStage % 16 == 0 && kOffPrep % 16 == 0 && (kPrepFloats * 4) % 16 == 0 && kOffD % 16 == 0 && kOffC % 16 == 0, "alignment");
+};
+
+namespace blk {
+using ptx::smem_u32;
+__device__ __forceinline__ void ldmatrix_x4(uint32_t saddr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(saddr)
+                 : "memory");
+}
+// Two fp32 values as three bf16 terms each, cut off at 8 significand bits (so that the terms add up to the value exactly).
+// kSafe: an infinity is its own first term; otherwise the rest of it, inf - inf, is undefined.
+template <bool kSafe>
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const uint32_t u0 = __float_as_uint(x0), u1 = __float_as_uint(x1);
+    hi = __byte_perm(u0, u1, 0x7632);
+    float r0 = x0 - __uint_as_float(u0 & 0xFFFF0000u), r1 = x1 - __uint_as_float(u1 & 0xFFFF0000u);
+    if (kSafe) {
+        r0 = r0 == r0 ? r0 : 0.f;
+        r1 = r1 == r1 ? r1 : 0.f;
+    }
+    const uint32_t w0 = __float_as_uint(r0), w1 = __float_as_uint(r1);
+    mid = __byte_perm(w0, w1, 0x7632);
+    lo = __byte_perm(__float_as_uint(r0 - __uint_as_float(w0 & 0xFFFF0000u)), __float_as_uint(r1 - __uint_as_float(w1 & 0xFFFF0000u)), 0x7632);
+}
+// (not volatile: results of their operands alone, to be scheduled freely)
+__device__ __forceinline__ void mma16f(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes below 16: zeros for the rest
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
+}
+// this thread's arrival at `bar` once all its copies so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+}  // namespace blk
+
+template <int DK, bool kF32>
+__device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& p) {
+    using namespace ptx;
+    using namespace step;
+    using namespace blk;
+    using L = BlockSmem<DK>;
+    constexpr int NK = DK / 64;  // K-steps of 16 columns per warp
+    static_assert(DK % 64 == 0, "four warps with whole K-steps each");
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t full[4], ready[4], done[4];  // k, q, v have landed / the block is prepared / its buffers have been read
+    __shared__ int abort_flag;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&full[i], 32);
+            mbar_init(&ready[i], 1);
+            mbar_init(&done[i], 4);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    // a programmatic dependent of the work before it; every kernel launched that way waits for the whole of its predecessor
+    grid_dep_wait();
+    grid_dep_launch();
+
+    const int rblocks = p.dv / kBlkRows;
+    const int unit = static_cast<int>(blockIdx.x) / rblocks, rb = static_cast<int>(blockIdx.x) - unit * rblocks;
+    const int seq = unit / p.vh, head = unit - seq * p.vh, khead = head / (p.vh / p.kh);
+    long long tok0 = 0, bidx = seq;
+    int ntok = p.seq_len;
+    if (p.cu_seqlens) {
+        tok0 = p.cu_seqlens[seq];
+        ntok = p.cu_seqlens[seq + 1] - static_cast<int>(tok0);
+        bidx = 0;
+    }
+    if (p.num_accepted) ntok = min(ntok, p.num_accepted[seq]);
+    const int slot = p.state_idx ? p.state_idx[seq] : seq;
+    if (slot < 0) return;  // padding sequence: no tokens, no state
+    const int nblk = ntok > 0 ? (ntok + kBlkTok - 1) / kBlkTok : 0;
+    // ldmatrix: lane l addresses row l & 7 of 8x8 matrix l >> 3; matrices 1 and 3 are rows 8 .. 15, matrices 2 and 3 columns 8 .. 15
+    const int lm_row = lane & 15, lm_col = 8 * (lane >> 4);
+    auto prep_of = [&](int b) { return reinterpret_cast<float*>(smem + L::kOffPrep) + (b & 3) * L::kPrepFloats; };
+
+    if (warp >= 4) {
+        // =============================================================== preparation
+        const int j = warp - 4;
+        uint8_t* const st = smem + j * L::kStage;
+        float* const pr = prep_of(j);
+        float* const X = pr + L::kR0;  // [t][s] = Gamma_ts, [t][16] = G_t, [t][17], [t][18] = inverse norms of k_t, q_t
+        const __nv_bfloat16* const kp = p.k + bidx * p.k_sb + tok0 * p.k_st + khead * p.k_sh;
+        const __nv_bfloat16* const qp = p.q + bidx * p.q_sb + tok0 * p.q_st + khead * p.q_sh;
+        const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * kBlkRows;
+        float al = 0.f, db = 0.f;
+        if (p.fused_gating) {
+            al = __expf(from_bits(ld_bits(p.A_log, p.gating_param_f32, head), p.gating_param_f32));
+            db = from_bits(ld_bits(p.dt_bias, p.gating_param_f32, head), p.gating_param_f32);
+        }
+        uint32_t b_next = 0u, g_next = 0u;  // bits of beta and the gate (or of the raw projections) of token `lane` of the next block
+        auto fetch = [&](int b) {
+            b_next = g_next = 0u;
+            const long long i = static_cast<long long>(b) * kBlkTok + lane;
+            if (lane < kBlkTok && i < ntok) {
+                b_next = ld_bits(p.beta, p.beta_f32, bidx * p.beta_sb + (tok0 + i) * p.beta_st + head * p.beta_sh);
+                if (p.gate) g_next = ld_bits(p.gate, p.gate_f32, bidx * p.gate_sb + (tok0 + i) * p.gate_st + head * p.gate_sh);
+            }
+        };
+        fetch(j);
+        for (int b = j; b < nblk; b += 4) {
+            const uint32_t it = static_cast<uint32_t>(b >> 2);
+            if (b >= 4 && !mbar_wait(&done[j], (it - 1) & 1u, &abort_flag)) break;
+            const int n = min(kBlkTok, ntok - b * kBlkTok);
+            {
+                // rows past the end of the sequence are filled with zeros (their address is that of the last row)
+                constexpr int kPieces = DK / 8;
+                const uint32_t dst = smem_u32(st);
+#pragma unroll 4
+                for (int i = lane; i < kBlkTok * kPieces; i += 32) {
+                    const int row = i / kPieces, c = i % kPieces;
+                    const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
+                    const uint32_t bytes = row < n ? 16u : 0u;
+                    cp_async16(dst + row * L::kRow + 16 * c, kp + at * p.k_st + 8 * c, bytes);
+                    cp_async16(dst + L::kOffQ + row * L::kRow + 16 * c, qp + at * p.q_st + 8 * c, bytes);
+                }
+                {
+                    const int row = lane >> 1;
+                    const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
+                    cp_async16(dst + L::kOffV + 16 * lane, vp + at * p.v_st + 8 * (lane & 1), row < n ? 16u : 0u);
+                }
+                cp_async_arrive(&full[j]);
+            }
+            // ---- scalars; tokens past the end: beta 0, decay 1
+            float beta = from_bits(b_next, p.beta_f32), gate = from_bits(g_next, p.gate_f32);
+            if (p.fused_gating) {
+                // softplus and sigmoid on the fast exponential, logarithm and reciprocal, as in recurrent.cuh
+                const float x = gate + db, e = __expf(x);
+                gate = -al * (x > 20.f ? x : (x < -15.f ? e : __logf(1.f + e)));
+                beta = __fdividef(1.f, 1.f + __expf(-beta));
+            }
+            const bool real = lane < n;
+            const float a = real ? __expf(gate) : 1.f;
+            if (!real) beta = 0.f;
+            fetch(b + 4);
+            float run = 1.f;
+#pragma unroll
+            for (int i = 0; i < kBlkTok; ++i) {
+                const float ai = __shfl_sync(0xffffffffu, a, i);
+                if (lane == 16 || lane < i) run *= ai;
+                if (lane <= 16) X[i * L::kLdR + lane] = run;  // (entries s > t are not used)
+            }
+            if (!mbar_wait(&full[j], it & 1u, &abort_flag)) break;  // not handed on: the other warps' waits end with it
+            // ---- Gram matrices.  kk, qk: tokens 0 .. 15 against tokens 0 .. 7 of k; hh: tokens 8 .. 15 of k and of q against tokens
+            //      8 .. 15 of k; qq: the diagonals of q q^T.  The matrix instructions cut their sums off, so only two follow one another.
+            float kk[4] = {}, qk[4] = {}, hh[4] = {}, qq0[4] = {}, qq1[4] = {};
+            const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + lm_col * 2, qaddr = kaddr + L::kOffQ;
+#pragma unroll 2
+            for (int ks = 0; ks < DK / 16; ks += 2) {
+                uint32_t x[2][4], y[2][4];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    ldmatrix_x4(kaddr + 32 * (ks + e), x[e]);
+                    ldmatrix_x4(qaddr + 32 * (ks + e), y[e]);
+                }
+                float s0[4] = {}, s1[4] = {}, s2[4] = {};
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const uint32_t h[4] = {x[e][1], y[e][1], x[e][3], y[e][3]};
+                    mma16f(s0, x[e], x[e][0], x[e][2]);
+                    mma16f(s1, y[e], x[e][0], x[e][2]);
+                    mma16f(s2, h, x[e][1], x[e][3]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    kk[e] += s0[e];
+                    qk[e] += s1[e];
+                    hh[e] += s2[e];
+                }
+                if (p.is_qk_norm) {
+                    float s3[4] = {}, s4[4] = {};
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        mma16f(s3, y[e], y[e][0], y[e][2]);
+                        mma16f(s4, y[e], y[e][1], y[e][3]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        qq0[e] += s3[e];
+                        qq1[e] += s4[e];
+                    }
+                }
+            }
+            if (t == (g >> 1)) {  // this lane holds the diagonal entries of tokens g and g + 8
+                float r0 = 1.f, r1 = 1.f, r2 = 1.f, r3 = 1.f;
+                if (p.is_qk_norm) {
+                    r0 = rsqrtf(((g & 1) ? kk[1] : kk[0]) + 1e-6f);
+                    r1 = rsqrtf(((g & 1) ? hh[1] : hh[0]) + 1e-6f);
+                    r2 = rsqrtf(((g & 1) ? qq0[1] : qq0[0]) + 1e-6f);
+                    r3 = rsqrtf(((g & 1) ? qq1[3] : qq1[2]) + 1e-6f);
+                }
+                X[g * L::kLdR + 17] = r0;
+                X[(g + 8) * L::kLdR + 17] = r1;
+                X[g * L::kLdR + 18] = r2;
+                X[(g + 8) * L::kLdR + 18] = r3;
+            }
+            __syncwarp();
+            const float beta_g = __shfl_sync(0xffffffffu, beta, g), beta_h = __shfl_sync(0xffffffffu, beta, g + 8);
+            const float rk_g = X[g * L::kLdR + 17], rk_h = X[(g + 8) * L::kLdR + 17];
+            const float rq_g = p.scale * X[g * L::kLdR + 18], rq_h = p.scale * X[(g + 8) * L::kLdR + 18];
+            // [s][t] = beta_t Gamma_ts k_s.k_t  and  [t][s] = scale Gamma_ts k_s.q_t (entries s >= t and s > t are not read)
+            auto put = [&](int ti, int si, float kkv, float qkv, float bt, float rq) {
+                const float w = X[ti * L::kLdR + si] * X[si * L::kLdR + 17];
+                pr[L::kA + si * 16 + ti] = bt * w * kkv;
+                pr[L::kP + ti * 16 + si] = rq * w * qkv;
+            };
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int s0 = 2 * t + e;
+                put(g, s0, kk[e], qk[e], beta_g * rk_g, rq_g);
+                put(g + 8, s0, kk[2 + e], qk[2 + e], beta_h * rk_h, rq_h);
+                put(g + 8, s0 + 8, hh[e], hh[2 + e], beta_h * rk_h, rq_h);
+            }
+            if (lane < kBlkTok) {
+                const float G = X[lane * L::kLdR + 16], rk = X[lane * L::kLdR + 17], rq = X[lane * L::kLdR + 18];
+                pr[L::kCk + lane] = beta * G * rk;
+                pr[L::kCq + lane] = p.scale * G * rq;
+                pr[L::kW + lane] = real ? X[(n - 1) * L::kLdR + lane] * rk : 0.f;
+                if (lane == n - 1) pr[L::kG] = G;
+            }
+            __syncwarp();
+            // ---- beta v over the decay products
+            {
+                const int tk = lane & 15;
+                const uint4 v = *reinterpret_cast<const uint4*>(st + L::kOffV + tk * kBlkRows * 2 + 16 * (lane >> 4));
+                const float bt = __shfl_sync(0xffffffffu, beta, tk);
+                float* const R = X + 8 * (lane >> 4) * L::kLdR + tk;
+                const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
+                    R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[j]);
+        }
+    } else {
+        // =============================================================== state
+        const int col0 = warp * (DK / 4);
+        const int r = lane & 15, h = lane >> 4;  // in the solve: row r, tokens 8 h .. 8 h + 7
+        float S[2 * NK][4];  // 8 columns each: rows g (0, 1) and g + 8 (2, 3), columns 2t, 2t + 1
+        const long long srow = static_cast<long long>(rb * kBlkRows + g) * DK + col0 + 2 * t;
+        if (p.state_in) {
+            const long long base = static_cast<long long>(slot) * p.si_ss + head * p.si_sh + srow;
+#pragma unroll
+            for (int i = 0; i < 2 * NK; ++i) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (kF32) {
+                        const float2 w = *reinterpret_cast<const float2*>(static_cast<const float*>(p.state_in) + base + 8 * e * DK + 8 * i);
+                        S[i][2 * e] = w.x;
+                        S[i][2 * e + 1] = w.y;
+                    } else {
+                        const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.state_in) + base + 8 * e * DK + 8 * i);
+                        S[i][2 * e] = bf16_lo(w);
+                        S[i][2 * e + 1] = bf16_hi(w);
+                    }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
+        }
+        __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
+        uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
+        bool ok = true;  // false once a wait has given up: nothing is stored from then on
+        for (int b = 0; b < nblk; ++b) {
+            ok = mbar_wait(&ready[b & 3], static_cast<uint32_t>((b >> 2) & 1), &abort_flag) && ok;
+            const int n = min(kBlkTok, ntok - b * kBlkTok);
+            const float* const pr = prep_of(b);
+            const uint32_t kaddr = smem_u32(smem + (b & 3) * L::kStage) + lm_row * L::kRow + (col0 + lm_col) * 2;
+            float* const D = reinterpret_cast<float*>(smem + L::kOffD) + (b & 1) * (4 * kBlkRows * L::kLdD);
+            // ---- this warp's columns of S_0 [k; q]^T: tokens 0 - 7 and 8 - 15 of k, then of q.  The first terms have sums of their own:
+            //      they are the long ones, and the chains are shorter.
+            {
+                float dh[4][4], dl[4][4];
+                auto products = [&](auto safe_tag) {
+                    constexpr bool kSafe = decltype(safe_tag)::value;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) dh[i][e] = dl[i][e] = 0.f;
+                    uint32_t x[2][4], y[2][4];
+                    ldmatrix_x4(kaddr, x[0]);
+                    ldmatrix_x4(kaddr + L::kOffQ, y[0]);
+#pragma unroll
+                    for (int kc = 0; kc < NK; ++kc) {
+                        if (kc + 1 < NK) {
+                            ldmatrix_x4(kaddr + 32 * (kc + 1), x[(kc + 1) & 1]);
+                            ldmatrix_x4(kaddr + L::kOffQ + 32 * (kc + 1), y[(kc + 1) & 1]);
+                        }
+                        const uint32_t* const xk = x[kc & 1];
+                        const uint32_t* const yk = y[kc & 1];
+                        uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float* s = &S[2 * kc + (e >> 1)][2 * (e & 1)];
+                            split3<kSafe>(s[0], s[1], hi[e], mid[e], lo[e]);
+                        }
+                        mma16f(dl[0], lo, xk[0], xk[2]);
+                        mma16f(dl[1], lo, xk[1], xk[3]);
+                        mma16f(dl[2], lo, yk[0], yk[2]);
+                        mma16f(dl[3], lo, yk[1], yk[3]);
+                        mma16f(dh[0], hi, xk[0], xk[2]);
+                        mma16f(dh[1], hi, xk[1], xk[3]);
+                        mma16f(dh[2], hi, yk[0], yk[2]);
+                        mma16f(dh[3], hi, yk[1], yk[3]);
+                        mma16f(dl[0], mid, xk[0], xk[2]);
+                        mma16f(dl[1], mid, xk[1], xk[3]);
+                        mma16f(dl[2], mid, yk[0], yk[2]);
+                        mma16f(dl[3], mid, yk[1], yk[3]);
+                    }
+                };
+                products(std::false_type{});
+                // a row of the state with an infinity has undefined low terms in every column: taken again with care
+                const float chk = dl[0][0] + dl[0][2];
+                if (__any_sync(0xffffffffu, chk != chk)) products(std::true_type{});
+                float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    *reinterpret_cast<float2*>(d + 8 * i) = make_float2(dh[i][0] + dl[i][0], dh[i][1] + dl[i][1]);
+                    *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
+                }
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            // ---- c of row r, tokens 8 h ..: right-hand sides, then forward substitution, first half of the tokens before the second
+            float c[8];
+            {
+                const float* const d = D + r * L::kLdD + 8 * h;
+                float sum[8];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    float4 x[4];
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float4*>(d + w * (kBlkRows * L::kLdD) + 4 * q);
+                    sum[4 * q] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
+                    sum[4 * q + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+                    sum[4 * q + 2] = (x[0].z + x[1].z) + (x[2].z + x[3].z);
+                    sum[4 * q + 3] = (x[0].w + x[1].w) + (x[2].w + x[3].w);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + r * L::kLdR + 8 * h + 4 * q);
+                    const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
+                    c[4 * q] = fmaf(-ck.x, sum[4 * q], bv.x);
+                    c[4 * q + 1] = fmaf(-ck.y, sum[4 * q + 1], bv.y);
+                    c[4 * q + 2] = fmaf(-ck.z, sum[4 * q + 2], bv.z);
+                    c[4 * q + 3] = fmaf(-ck.w, sum[4 * q + 3], bv.w);
+                }
+            }
+            // column s of A, tokens 8 th .. 8 th + 7
+            auto col_of = [&](int s, int th, float* x) {
+                const float4 u = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th);
+                const float4 v = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th + 4);
+                x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+            };
+            // (what a token gets from the tokens before it is summed apart from its own, larger, term)
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            auto substitute = [&](int half) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    c[s] -= acc[s];
+                    if (s == 7) break;
+                    float x[8];
+                    col_of(8 * half + s, half, x);
+#pragma unroll
+                    for (int i = s + 1; i < 8; ++i) acc[i] = fmaf(x[i], c[s], acc[i]);
+                }
+            };
+            if (h == 0) substitute(0);
+            __syncwarp();
+            float c0[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) c0[i] = __shfl_sync(0xffffffffu, c[i], r);
+            if (h == 1) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    float x[8];
+                    col_of(s, 1, x);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[i] = fmaf(x[i], c0[s], acc[i]);
+                }
+                substitute(1);
+            }
+            if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
+#pragma unroll
+                for (int i = 0; i < 8; ++i) c[i] = 8 * h + i < n ? c[i] : 0.f;
+            }
+            __syncwarp();
+            // ---- S <- G S + sum_s (Gamma_ns r_s c_s) k_s^T
+            {
+                uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 w = *reinterpret_cast<const float4*>(pr + L::kW + 8 * h + 4 * q);
+                    split3<true>(w.x * c[4 * q], w.y * c[4 * q + 1], hi[2 * q], mid[2 * q], lo[2 * q]);
+                    split3<true>(w.z * c[4 * q + 2], w.w * c[4 * q + 3], hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1]);
+                }
+                uint8_t* const o = sc + r * L::kRowC + 16 * h;
+                *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(o + kBlkRows * L::kRowC) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+                *reinterpret_cast<uint4*>(o + 2 * kBlkRows * L::kRowC) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                __syncwarp();
+                const uint32_t caddr = smem_u32(sc) + lm_row * L::kRowC + lm_col * 2;
+                ldmatrix_x4(caddr, hi);
+                ldmatrix_x4(caddr + kBlkRows * L::kRowC, mid);
+                ldmatrix_x4(caddr + 2 * kBlkRows * L::kRowC, lo);
+                const float G = pr[L::kG];
+#pragma unroll
+                for (int kc = 0; kc < NK; ++kc) {
+                    uint32_t x[4];
+                    ldmatrix_x4_trans(kaddr + 32 * kc, x);  // tokens of k in pairs, columns 0 - 7 and 8 - 15
+                    // first terms and the others apart: the matrix instructions cut their sums off, which the short sums of first
+                    // terms lose next to nothing by, and an fp32 addition rounds
+                    float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f}, f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma16f(e0, lo, x[0], x[1]);
+                    mma16f(e1, lo, x[2], x[3]);
+                    mma16f(f0, hi, x[0], x[1]);
+                    mma16f(f1, hi, x[2], x[3]);
+                    mma16f(e0, mid, x[0], x[1]);
+                    mma16f(e1, mid, x[2], x[3]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        S[2 * kc][e] = fmaf(G, S[2 * kc][e], f0[e] + e0[e]);
+                        S[2 * kc + 1][e] = fmaf(G, S[2 * kc + 1][e], f1[e] + e1[e]);
+                    }
+                }
+            }
+            // ---- outputs of row r, tokens 4 warp + 2 h and the next.  Coefficients of later tokens are left out, not multiplied by
+            //      zero: an infinite or undefined value stays behind its token.
+            {
+                float c1[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) c1[i] = __shfl_sync(0xffffffffu, c[i], r + 16);
+                const int t0 = 4 * warp + 2 * h;
+                const float* const d = D + r * L::kLdD + 16 + t0;
+                float2 x[4];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
+                const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t0);
+                float o0 = cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), o1 = cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y));
+                const float* const P = pr + L::kP + t0 * 16;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (q > warp) break;
+                    const float4 pa = *reinterpret_cast<const float4*>(P + 4 * q), pb = *reinterpret_cast<const float4*>(P + 16 + 4 * q);
+                    const float* const cc = (q < 2 ? c0 : c1) + 4 * (q & 1);
+                    o0 = fmaf(pa.x, cc[0], o0);
+                    o1 = fmaf(pb.x, cc[0], o1);
+                    o1 = fmaf(pb.y, cc[1], o1);
+                    if (q < warp || h) {  // q == warp: tokens 4 q + 2 h and + 1
+                        o0 = fmaf(pa.y, cc[1], o0);
+                        o0 = fmaf(pa.z, cc[2], o0);
+                        o1 = fmaf(pb.z, cc[2], o1);
+                        o1 = fmaf(pb.w, cc[3], o1);
+                    }
+                    if (q < warp) o0 = fmaf(pa.w, cc[3], o0);
+                }
+                const long long i = static_cast<long long>(b) * kBlkTok + t0;
+                if (ok && t0 < n) out[i * p.o_st] = __float2bfloat16(o0);
+                if (ok && t0 + 1 < n) out[(i + 1) * p.o_st] = __float2bfloat16(o1);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&done[b & 3]);
+        }
+        if (ok) {
+            const long long base = static_cast<long long>(slot) * p.so_ss + head * p.so_sh + srow;
+#pragma unroll
+            for (int i = 0; i < 2 * NK; ++i) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (kF32)
+                        *reinterpret_cast<float2*>(static_cast<float*>(p.state_out) + base + 8 * e * DK + 8 * i) = make_float2(S[i][2 * e], S[i][2 * e + 1]);
+                    else
+                        *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.state_out) + base + 8 * e * DK + 8 * i) = pack_bf16(S[i][2 * e], S[i][2 * e + 1]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && abort_flag && p.status) atomicExch(p.status, 1);
+}
+
+template <int DK, bool kF32 = false>
+__global__ void __launch_bounds__(kBlkThreads, 2) gdn_recurrent_block_kernel(const RecurrentParams p) {
+    gdn_recurrent_block_body<DK, kF32>(p);
+}
+
+}  // namespace gdn

@@ -1,0 +1,108 @@
+"""Long runs of tokens through recurrent_forward (blocks of 16 tokens, the state in fp32 from the first token to the last)
+against the fp32 oracle.  bf16 results are off by their rounding, 2^-9 relative per element at most; the rest are sums of at
+most 256 products in fp32, 64 terms of 2^-17 in the worst direction: 2^-9 + 2^-11.  An fp32 state has no rounding to bf16:
+sums of 256 products rounded to 2^-24 each, added up over the tokens a state remembers, 2^-24 * 256 = 2^-16.
+"""
+import pytest
+import torch
+
+from oracle import gdn_oracle as O
+from h100_gdn_cuda_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+REL, REL32 = 2.0 ** -9 + 2.0 ** -11, 2.0 ** -16
+
+
+@pytest.fixture(scope="module")
+def gdn():
+    import h100_gdn_cuda_b200 as g
+    from h100_gdn_cuda_b200 import build
+    build.build()
+    return g
+
+
+def close(x, ref, tol, what):
+    x = x.float().cpu()
+    assert torch.isfinite(x).all(), what
+    assert O.rel_fro(x, ref) <= tol, "%s: rel_fro %.3e" % (what, O.rel_fro(x, ref))
+
+
+def inputs(B, T, kh, vh, d, norm, seed):
+    p = synthetic.prefill_inputs(B, T, kh, vh, d, seed=seed, with_state=True, mild_gate=True, normalize=not norm)
+    return p, {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+
+
+# around whole blocks, around the turn of the four preparing warps, one CTA and several waves of them
+@pytest.mark.parametrize("B,T,kh,vh,d", [(1, 17, 1, 1, 64), (2, 31, 1, 2, 128), (1, 32, 2, 2, 192), (1, 33, 1, 1, 256), (3, 63, 1, 3, 64),
+                                         (1, 64, 2, 4, 128), (1, 65, 1, 2, 256), (40, 47, 2, 8, 128), (24, 40, 2, 8, 64)])
+@pytest.mark.parametrize("norm,f32,state", [(True, False, True), (False, True, True), (True, True, False)])
+def test_padded(gdn, B, T, kh, vh, d, norm, f32, state):
+    if f32 and d > 128:
+        pytest.skip("fp32 states are built for dk 64 and 128")
+    p, c = inputs(B, T, kh, vh, d, norm, 7 * T + d)
+    s0 = (c["state"].float() if f32 else c["state"]) if state else None
+    if f32 and not state:
+        s0 = torch.zeros_like(c["state"], dtype=torch.float32)
+    o, s = gdn.recurrent_forward(c["q"], c["k"], c["v"], s0, c["beta"], c["g"], inference_mode=gdn.Decode, is_qk_norm=norm)
+    o_ref, s_ref = O.recurrent_ref(p["q"].float(), p["k"].float(), p["v"].float(), p["beta"].float(), p["g"],
+                                   p["state"].float() if state else None, is_qk_norm=norm)
+    assert s.dtype == (torch.float32 if f32 else torch.bfloat16)
+    close(o, o_ref, REL, "O")
+    close(s, s_ref, REL32 if f32 else REL, "state")
+
+
+def test_caps_pool_and_gating(gdn):
+    """sequences that end inside a block, before the first token and at the last one, their states in a pool with a padding
+    sequence, beta and the gate made inside"""
+    B, T, kh, vh, d = 6, 50, 1, 2, 128
+    p, c = inputs(B, T, kh, vh, d, True, 3)
+    gen = torch.Generator().manual_seed(4)
+    A_log, dt_bias = torch.rand(vh, generator=gen).bfloat16(), torch.randn(vh, generator=gen).bfloat16()
+    a, b = torch.randn(B, T, vh, generator=gen).bfloat16(), torch.randn(B, T, vh, generator=gen).bfloat16()
+    nat = torch.tensor([50, 0, 17, 33, 48, 1], dtype=torch.int32)
+    slots = torch.tensor([4, 0, 6, -1, 2, 1], dtype=torch.int32)
+    pool = (torch.randn(8, vh, d, d, generator=gen) * 0.02).bfloat16()
+    beta, g = O.gating_ref(A_log, dt_bias, a, b)
+    got = pool.cuda()
+    o, _ = gdn.recurrent_forward(c["q"], c["k"], c["v"], got, None, None, None, nat.cuda(), gdn.Decode, True,
+                                 gating=(A_log.cuda(), dt_bias.cuda(), a.cuda(), b.cuda()), state_indices=slots.cuda())
+    want = pool.clone()
+    for i in range(B):
+        n, sl = int(nat[i]), int(slots[i])
+        if sl < 0:
+            continue
+        if n:
+            o_ref, s_ref = O.recurrent_ref(p["q"][i:i + 1, :n].float(), p["k"][i:i + 1, :n].float(), p["v"][i:i + 1, :n].float(),
+                                           beta[i:i + 1, :n].float(), g[i:i + 1, :n], pool[sl:sl + 1].float(), is_qk_norm=True)
+            close(o[i:i + 1, :n], o_ref, REL, "O of sequence %d" % i)
+            want[sl] = s_ref[0].bfloat16()
+    close(got, want.float(), REL, "pool")
+    for sl in (0, 3, 5, 7):
+        assert torch.equal(got[sl].cpu(), pool[sl])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", ["v", "k", "state"])
+def test_undefined_values_stay_behind_their_token(gdn, what, bad):
+    B, T, kh, vh, d, at = 1, 60, 1, 1, 128, 21
+    p, c = inputs(B, T, kh, vh, d, False, 5)
+    run = lambda: gdn.recurrent_forward(c["q"], c["k"], c["v"], c["state"], c["beta"], c["g"], inference_mode=gdn.Decode)
+    o0, s0 = run()
+    if what == "state":  # one row of the state: the others are untouched
+        c["state"] = c["state"].clone()
+        c["state"][0, 0, 5, 7] = bad
+        o1, s1 = run()
+        rows = [r for r in range(d) if r != 5]
+        assert torch.equal(o0[..., rows], o1[..., rows]) and torch.equal(s0[:, :, rows], s1[:, :, rows])
+        assert not torch.isfinite(s1[0, 0, 5]).any() and not torch.isfinite(o1[0, :, 0, 5]).any()
+    else:
+        c[what] = c[what].clone()
+        c[what][0, at, 0, 9] = bad
+        o1, s1 = run()
+        assert torch.equal(o0[:, :at], o1[:, :at])
+        if what == "v":
+            rows = [r for r in range(d) if r != 9]
+            assert torch.equal(o0[..., rows], o1[..., rows]) and torch.equal(s0[:, :, rows], s1[:, :, rows])
+            assert not torch.isfinite(o1[0, at:, 0, 9]).any()
+        else:
+            assert not torch.isfinite(o1[:, at:]).any()
