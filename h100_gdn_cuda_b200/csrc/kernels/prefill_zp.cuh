@@ -15,11 +15,19 @@
 // Work unit = (chunk, k-head): the K and Q tiles are loaded once and K K^T, Q K^T are computed once
 // (one M=128 tcgen05 MMA group whose A operand is K stacked on Q) for all the v-heads of the
 // k-head group; only beta and the gate differ between them.  A CTA of 256 threads is two teams of
-// four warps, each team taking one v-head of the group at a time: A / P pass from tensor memory,
-// in-place inverse (fp32 forward substitution on 8x8 blocks, three levels of recursive doubling on
-// TF32 warp MMAs), T and (diag(d) T)^T as bf16 tiles, then three M=64 MMAs (the two 64-column
-// halves of Z, and PT) and the bf16 epilogue into a staging area that leaves by two bulk copies.
-// Persistent CTAs, two per SM (92 KB of shared memory, 256 tensor-memory columns each).
+// four warps, each team taking one v-head of the group at a time: A / P pass from tensor memory, inverse row block by row
+// block in registers, T and (diag(d) T)^T as bf16 tiles, then M=64 MMAs (Z, and PT) and the bf16 epilogue into a staging
+// area that leaves by one bulk copy.
+// The inverse: 16x16 diagonal blocks in fp32 (8x8 forward substitution and one TF32 doubling step).  Then warp r owns row
+// block r of X and walks it from the diagonal to the left, X_rc = -(sum_{c<m<=r} X_rm A_mc) inv_cc, which needs nothing of
+// the other row blocks: the blocks of X stay accumulator fragments, which are the A operands of the next products as they
+// lie; A and the inverses are B operands in shared memory.  All of them enter the products as two bf16 terms (16
+// significand bits; a doubling scheme on TF32, 11 bits, was here before).
+// What bounds it: the latency of a unit's dependent phases (11 200 cycles with four teams per SM, 8 700 with two; before
+// 12 100).  The doubling scheme had ten barriers per unit (five now), 5 660 warp instructions and 1 808 wavefronts of
+// shared-memory accesses, besides some 900 of MMA operands and copies, of the 3 000 cycles a unit took an SM.
+// B=4 T=4096, 32 v-heads, whole step 214.7 -> 204.0 us; 16 packed sequences of 32768 tokens 458 -> 423; B=2 T=131072, 4 v-heads 618 -> 578.
+// Persistent CTAs, two per SM (111 KB of shared memory, 256 tensor-memory columns each).
 #pragma once
 #include <cuda.h>
 
@@ -44,30 +52,36 @@ struct ZPParams {
 
 struct ZPSmem {
     static constexpr int kAtoms = 2;  // 64-column swizzle atoms of a K or Q tile
-    static constexpr int kLd = 68;  // fp32 row stride of A, conflict-free for the MMA fragment loads
     // K and Q tiles interleaved atom by atom: [K cols 0-63 | Q cols 0-63 | K cols 64-127 | Q cols 64-127],
     // 8 KB each, so that rows 0-127 of one atom pair are K stacked on Q (the M=128 A operand)
     static constexpr int kOffKQ = 0;
     static constexpr int kTeam = kAtoms * 16384;         // per-team area starts here, two of them
-    static constexpr int kOffA = 0;                      // A / X fp32 (17 KB), later T | dT, later the staged Z
-    static constexpr int kOffP = 64 * kLd * 4;           // 17408: P tile (8 KB), later the staged PT
-    static constexpr int kOffVec = kOffP + 8192;         // beta[64], g log2e[64], d[64], scan partials[64], column factors[32]
-    static constexpr int kTeamBytes = kOffVec + 2048;    // a multiple of 1024
-    static constexpr int kOffNorm = kTeam + 2 * kTeamBytes;  // kNorm: inverse row norms of K [64] and Q [64], their log2 [128]
-    static constexpr int kOffBar = kOffNorm + 1024;
-    static constexpr int kUnits = 256;                   // coordinates of this CTA's coming work units, 16 bytes each
+    static constexpr int kOffT = 0, kOffTd = 8192;       // T and dT (8 KB each), later the staged Z
+    static constexpr int kOffP = 16384;                  // P tile (8 KB), later the staged PT
+    // 16x16 blocks of A below the diagonal, block (r, c) at r (r - 1) / 2 + c, as two bf16 terms: see blk_off
+    static constexpr int kOffA = kOffP + 8192;
+    // diagonal blocks of A in fp32, 20 floats per row; each makes way for its inverse as two bf16 terms
+    static constexpr int kLdD = 20, kDiag = 16 * kLdD * 4;
+    static constexpr int kOffDiag = kOffA + 6 * 1024;
+    static constexpr int kOffVec = kOffDiag + 4 * kDiag;  // beta[64], d[64], then per warp g log2e[64] and column factors[80]
+    static constexpr int kTeamBytes = kOffVec + 3072;    // a multiple of 1024
+    static constexpr int kOffNorm = kTeam + 2 * kTeamBytes;  // kNorm: inverse row norms of K [64] and Q [64]
+    static constexpr int kOffBar = kOffNorm + 512;
+    static constexpr int kUnits = 64;                    // coordinates of this CTA's coming work units, 16 bytes each
     static constexpr int kOffUnits = kOffBar + 128;
     static constexpr int kBytes = kOffUnits + 16 * kUnits + 1024;
-    static_assert(kOffP % 1024 == 0 && kTeamBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+    static_assert(kTeamBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+    static_assert(kDiag >= 1024 && kDiag % 128 == 0, "the inverse of a diagonal block fits over it");
 };
 
 namespace zp {
+using namespace ptx;
 constexpr int kThreads = 256;
 constexpr uint32_t kTmKQ = 0;    // fp32 K K^T (lanes 0-63) and Q K^T (lanes 64-127), 64 columns
 constexpr uint32_t kTmPT = 64;   // PT of team 0 (lanes +0) and team 1 (lanes +16), 64 columns
-constexpr uint32_t kTmZ = 128;   // + 64 * team: Z columns 0-63 (lanes +0) and 64-127 (lanes +16)
-// two neighbouring warps of a team
-__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(3 + pair) : "memory"); }
+constexpr uint32_t kTmZ = 128;   // Z, 128 columns (lanes +0: team 0, +16: team 1)
+// the two warps of a team that write P
+__device__ __forceinline__ void pair_sync(int team) { asm volatile("bar.sync %0, 64;" ::"r"(3 + team) : "memory"); }
 // TF32 operands of the inverse's block products: 16x8 fragment of `m` at [r0][k0] as the A operand (kRows 8: the lower
 // half is zero), 8x8 at [k0][n0] as the B operand
 template <int kRows = 16>
@@ -96,12 +110,61 @@ __device__ __forceinline__ void team_sync(int team) {
     else
         asm volatile("bar.sync 1, 128;" ::: "memory");
 }
+// A 16x16 block as two bf16 terms: 16 rows of 64 bytes, 16-byte pieces { first terms of columns 0-7, 8-15, second terms of
+// the same }, swizzled so that one piece of eight rows covers all banks.
+__device__ __forceinline__ uint32_t blk_off(int row, int piece) { return static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)); }
+// two fp32 values as two bf16 terms each
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+    hi = pack_bf16(x0, x1);
+    lo = pack_bf16(x0 - bf16_lo(hi), x1 - bf16_hi(hi));
+}
+// a 16x16 accumulator fragment (two halves of 8 columns) as the A operand of the next product, two terms
+__device__ __forceinline__ void split_frag(const float (*x)[4], uint32_t* hi, uint32_t* lo) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split2(x[i >> 1][2 * (i & 1)], x[i >> 1][2 * (i & 1) + 1], hi[i], lo[i]);
+}
+__device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// acc += X B for 16x16 blocks: X as fragments of two terms, B in shared memory (blk_off); the product of the second terms is
+// below 2^-16 of the result
+__device__ __forceinline__ void mma_blk16(float (*acc)[4], const uint32_t* xh, const uint32_t* xl, uint32_t b_saddr, int lane) {
+    uint32_t bh[4], bl[4];  // { columns 0-7: rows 0-7, 8-15; columns 8-15: the same }
+    ldmatrix_x4_trans(b_saddr + blk_off(lane & 15, lane >> 4), bh);
+    ldmatrix_x4_trans(b_saddr + blk_off(lane & 15, 2 + (lane >> 4)), bl);
+    mma_bf16(acc[0], xl, bh[0], bh[1]);
+    mma_bf16(acc[1], xl, bh[2], bh[3]);
+    mma_bf16(acc[0], xh, bl[0], bl[1]);
+    mma_bf16(acc[1], xh, bl[2], bl[3]);
+    mma_bf16(acc[0], xh, bh[0], bh[1]);
+    mma_bf16(acc[1], xh, bh[2], bh[3]);
+}
+// Row block R of X = (I + A)^-1 from its diagonal block on, right to left.  x: fragments of the blocks X_R0 .. X_RR.
+template <int R>
+__device__ __forceinline__ void row_blocks(float (*x)[2][4], uint32_t a_saddr, uint32_t inv_saddr, int lane) {
+    uint32_t xh[4][4], xl[4][4];
+    if (R > 0) split_frag(x[R], xh[R], xl[R]);
+#pragma unroll
+    for (int c = R - 1; c >= 0; --c) {
+        float s[2][4] = {};
+#pragma unroll
+        for (int m = R; m > c; --m) mma_blk16(s, xh[m], xl[m], a_saddr + (m * (m - 1) / 2 + c) * 1024, lane);
+        uint32_t sh[4], sl[4];
+        split_frag(s, sh, sl);
+        float y[2][4] = {};
+        mma_blk16(y, sh, sl, inv_saddr + c * ZPSmem::kDiag, lane);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[c][i >> 2][i & 3] = -y[i >> 2][i & 3];
+        if (c > 0) split_frag(x[c], xh[c], xl[c]);
+    }
+}
 }  // namespace zp
 
 // kNorm: q and k are L2-normalised per head (x * rsqrt(sum x^2 + 1e-6)) without touching the tiles:
-// (k_i.k_j) r_i r_j and (q_i.k_j) rq_i r_j enter through the row factor of the A / P pass and through
-// the column's gate (g_j - log2 r_j in the exponent), Z = (dT)^T diag(r) K through d_i r_i.  The
-// factors are also written to `norms` for the state kernel.
+// (k_i.k_j) r_i r_j and (q_i.k_j) rq_i r_j enter through a row and a column factor of the A / P pass,
+// Z = (dT)^T diag(r) K through d_i r_i.  The factors are also written to `norms` for the state kernel.
 template <bool kNorm>
 __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                  const __grid_constant__ CUtensorMap tmQ,
@@ -110,7 +173,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
     using namespace uw;
     using namespace zp;
     using L = ZPSmem;
-    constexpr int LD = L::kLd, NA = L::kAtoms;
+    constexpr int NA = L::kAtoms;
     extern __shared__ uint8_t smem_raw[];
     // aligned by an offset from the array itself, so that the compiler still knows the pointer is shared memory
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -118,17 +181,14 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
     const int team = warp >> 2, tw = warp & 3, tt = tid & 127;
     uint8_t* sKQ = smem + L::kOffKQ;
     uint8_t* tbase = smem + L::kTeam + team * L::kTeamBytes;
-    float* sA = reinterpret_cast<float*>(tbase + L::kOffA);
-    uint8_t* sT = tbase + L::kOffA;           // T   = X diag(beta), rows i (128 B), columns j
-    uint8_t* sTd = tbase + L::kOffA + 8192;   // dT  = diag(d) T, same layout; read MN-major as (dT)^T
+    uint8_t* sT = tbase + L::kOffT;    // T   = X diag(beta), rows i (128 B), columns j
+    uint8_t* sTd = tbase + L::kOffTd;  // dT  = diag(d) T, same layout; read MN-major as (dT)^T
     uint8_t* sP = tbase + L::kOffP;
     float* sBeta = reinterpret_cast<float*>(tbase + L::kOffVec);
-    float* sG = sBeta + 64;
-    float* sD = sG + 64;
-    float* sPart = sD + 64;   // 64 floats: partial sums of the gate scan (each half of the chunk on its own)
-    float* sC = sPart + 64;    // 32 floats: e^{g_32 - g_j} for the columns j < 32 of the block below the diagonal
+    float* sD = sBeta + 64;
+    float* sG = sD + 64 + 144 * tw;  // this warp's own copy
+    float* sC = sG + 64;  // decay to the first token of this warp's two row blocks: e^{g_32 - g_j} [32], e^{g_48 - g_j} [48] (tw & 1), or e^{g_16 - g_j} [16]
     float* sRn = reinterpret_cast<float*>(smem + L::kOffNorm);  // [128] inverse norms (K rows, then Q rows)
-    float* sLr = sRn + 128;                                      // [128] their log2
     uint64_t* bar_load = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
     uint64_t* bar_kq = bar_load + 1;
     uint64_t* bar_mma = bar_load + 2;  // [2], one per team
@@ -179,7 +239,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             khead = unit - chunk * p.kh;
         }
     };
-    // Coordinates of a unit.  They are worked out for 256 of this CTA's units at a time, one thread each, and looked up in
+    // Coordinates of a unit.  They are worked out for 64 of this CTA's units at a time, one thread each, and looked up in
     // shared memory: done in every unit by every thread, the integer divisions (padded) or the two dependent loads (packed)
     // stood in the middle of the unit's chain.
     struct UnitPos {
@@ -187,7 +247,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
         bool valid;
     };
     int4* const sUnits = reinterpret_cast<int4*>(smem + L::kOffUnits);
-    auto fill_units = [&](int unit0) {  // all threads; entry i: unit0 + i * gridDim.x
+    auto fill_units = [&](int unit0) {  // entry i: unit0 + i * gridDim.x
+        if (tid >= L::kUnits) return;
         const long long unit = unit0 + static_cast<long long>(tid) * gridDim.x;
         int4 e = make_int4(0, 0, 0, 0);
         if (unit < total_units) {
@@ -199,7 +260,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
         }
         sUnits[tid] = e;
     };
-    static_assert(L::kUnits == kThreads, "one entry per thread");
+    static_assert(L::kUnits <= kThreads, "one entry per thread");
     auto unit_at = [&](int i) {
         const int4 e = sUnits[i];
         UnitPos u;
@@ -224,20 +285,23 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
     int table = 0;  // entry of the present unit
     if (tid == 0 && cur.valid) issue_loads(cur);
 
-    // beta and the raw gate of this thread's token for (unit, round): fetched one round ahead, so that
+    // beta and the raw gate of the tokens `lane` and `lane + 32` for (unit, round), fetched one round ahead, so that
     // their DRAM latency is not in front of every unit
-    auto fetch_scalars = [&](const UnitPos& u, int rd, uint32_t& b, uint32_t& g) {
-        b = 0u;
-        g = 0u;
+    auto fetch_scalars = [&](const UnitPos& u, int rd, uint32_t* b, uint32_t* g) {
+        b[0] = b[1] = g[0] = g[1] = 0u;
         const int hloc = 2 * rd + team;
         if (!u.valid || hloc >= rep) return;
-        if (tt < u.n) {
-            const int head = u.khead * rep + hloc;
-            b = p.beta.load_bits(u.batch, u.tok0 + tt, head);
-            if (p.gate.ptr) g = p.gate.load_bits(u.batch, u.tok0 + tt, head);
+        const int head = u.khead * rep + hloc;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int t = lane + 32 * i;
+            if (t < u.n) {
+                if (tw < 2) b[i] = p.beta.load_bits(u.batch, u.tok0 + t, head);
+                if (p.gate.ptr) g[i] = p.gate.load_bits(u.batch, u.tok0 + t, head);
+            }
         }
     };
-    uint32_t b_next, g_next;  // bits, see ScalarView::load_bits
+    uint32_t b_next[2], g_next[2];  // bits, see ScalarView::load_bits
     fetch_scalars(cur, 0, b_next, g_next);
 
     uint32_t it = 0;      // units done by this CTA (parity of bar_load and bar_kq)
@@ -257,32 +321,48 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             const bool active = hloc < rep;  // team-uniform
             const int head = khead * rep + hloc;
             // ---- beta, chunk-local cumulative gate, decay to the chunk's last token
+            float b_mine[2] = {0.f, 0.f}, g_mine = 0.f;
             if (!active) {  // (odd number of v-heads per k-head: team 1 sits the last round out)
                 nxt = unit_at(table);
                 fetch_scalars(nxt, 0, b_next, g_next);
             } else {
-                const float b_mine = p.beta.value(b_next), g_mine = p.gate.value(g_next);
-                if (tt < 64) {
-                    float g = g_mine;
+                // (every warp scans the whole chunk for itself: no barrier)
+                b_mine[0] = p.beta.value(b_next[0]);
+                b_mine[1] = p.beta.value(b_next[1]);
+                float g0 = p.gate.value(g_next[0]), g1 = p.gate.value(g_next[1]);
 #pragma unroll
-                    for (int m = 1; m < 32; m <<= 1) {
-                        const float y = __shfl_up_sync(0xffffffffu, g, m);
-                        if (lane >= m) g += y;
+                for (int m = 1; m < 32; m <<= 1) {
+                    const float y0 = __shfl_up_sync(0xffffffffu, g0, m), y1 = __shfl_up_sync(0xffffffffu, g1, m);
+                    if (lane >= m) {
+                        g0 += y0;
+                        g1 += y1;
                     }
-                    sPart[tt] = g;  // cumulative sum within each half of the chunk
                 }
-                team_sync(team);
-                if (tt < 64) {
+                g1 += __shfl_sync(0xffffffffu, g0, 31);
+                g0 *= 1.4426950408889634f;  // times log2(e): decay factors are ex2 of differences
+                g1 *= 1.4426950408889634f;
+                g_mine = (tw & 1) ? g1 : g0;
+                sG[lane] = g0;
+                sG[lane + 32] = g1;
+                if (tw & 1) {
+                    const float r2 = __shfl_sync(0xffffffffu, g1, 0), r3 = __shfl_sync(0xffffffffu, g1, 16);
+                    sC[lane] = ex2(r2 - g0);
+                    sC[32 + lane] = ex2(r3 - g0);
+                    if (lane < 16) sC[64 + lane] = ex2(r3 - g1);
+                } else {
+                    const float r1 = __shfl_sync(0xffffffffu, g0, 16);
+                    if (lane < 16) sC[lane] = ex2(r1 - g0);
+                }
+                if (tw == 0) {
+                    sBeta[lane] = b_mine[0];
+                    sBeta[lane + 32] = b_mine[1];
+                } else if (tw == 2) {
                     // tokens past the end had a raw gate of 0: they carry the last valid value
-                    const float g = sPart[tt] + (tt >= 32 ? sPart[31] : 0.f);
-                    const int last = max(n, 1) - 1;
-                    const float gl = sPart[last] + (last >= 32 ? sPart[31] : 0.f);
-                    sBeta[tt] = b_mine;
-                    sG[tt] = g * 1.4426950408889634f;  // times log2(e): decay factors are ex2 of differences
-                    sD[tt] = __expf(gl - g);
-                    if (tt < 32) sC[tt] = __expf(sPart[32] + sPart[31] - g);  // g_32 is the first entry of the second scan plus the first half's total
+                    const float gl = __shfl_sync(0xffffffffu, g1, 31);
+                    sD[lane] = ex2(gl - g0);
+                    sD[lane + 32] = ex2(gl - g1);
                 }
-                team_sync(team);
+                __syncwarp();
             }
             // ---- K K^T (lanes 0-63) and Q K^T (lanes 64-127): once per unit, shared by its v-heads
             if (rd == 0) {
@@ -308,7 +388,6 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     const float rinv = rsqrtf(ss + 1e-6f);
                     if (hf == 0) {
                         sRn[r] = rinv;
-                        sLr[r] = log2f(rinv);
                         if (*abort_flag == 0) p.norms[(static_cast<size_t>(chunk) * p.kh + khead) * 128 + r] = rinv;
                     }
                     __syncthreads();
@@ -332,109 +411,128 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 tc_fence_after_sync();
             }
             if (active) {
-                if (stores_pending) {
-                    // the previous round's staged Z and PT must have been read out before A and P are rewritten;
-                    // by now that has long happened and the wait costs nothing
-                    if (tt == 0) bulk_wait_read<0>();
-                    stores_pending = false;
-                    team_sync(team);
+                if (stores_pending && tw >= 2) {
+                    // the previous round's staged Z and PT must have been read out before P (here) and T (past the next
+                    // barrier) are written; by now that has long happened and the wait costs nothing
+                    if (tt == 64) bulk_wait_read<0>();
+                    pair_sync(team);
                 }
-                // ---- A = tril(beta_i (k_i.k_j) e^{g_i-g_j}, -1) in fp32 (warps 0, 1 of the team) and
-                //      P = scale tril((q_i.k_j) e^{g_i-g_j}) as a bf16 tile (warps 2, 3); thread = row
+                // ---- A = tril(beta_i (k_i.k_j) e^{g_i-g_j}, -1) (warps 0, 1 of the team) and P = scale tril((q_i.k_j) e^{g_i-g_j})
+                //      as a bf16 tile (warps 2, 3), 16x16 block by block as accumulator fragments: a warp has two rows of blocks and
+                //      nothing of what lies above the diagonal is touched.  A: the diagonal blocks in fp32, the others as two bf16 terms.
+                //      In a block below the diagonal e^{g_i-g_j} = e^{g_i-g_r} e^{g_r-g_j} with r the first of its rows, both factors
+                //      <= 1 (the cumulative gate only falls): the column factors come from a table, no ex2 is left per element.
                 {
                     const bool is_p = tw >= 2;
-                    const int rb = tw & 1;
-                    const int i = 32 * rb + lane;
-                    const float gi = sG[i];
-                    float f = is_p ? p.p_scale : sBeta[i];
-                    if (kNorm) f *= sRn[is_p ? 64 + i : i];
-                    const f2 fv = pk(f, f);
-                    const int lim = (i < n) ? (is_p ? i : i - 1) : -1;  // columns kept: col <= lim
-                    for (int cb = 0; cb <= rb; ++cb) {
-                        uint32_t r[32];
-                        tmem_ld32(tmem + kTmKQ + (static_cast<uint32_t>(32 * tw) << 16) + 32 * cb, r);
+                    const int g = lane >> 2, tq = lane & 3;
+                    const uint32_t pt = smem_u32(sP);
+                    auto row_block = [&](auto rb_tag, auto h_tag) {
+                        constexpr int rb = decltype(rb_tag)::value, h = decltype(h_tag)::value, r = 2 * rb + h;
+                        const uint32_t ta = tmem + kTmKQ + (static_cast<uint32_t>(32 * tw + 16 * h) << 16);
+                        uint32_t kq[2][16];
+                        tmem_ld_frag32(ta, kq[0]);
+                        if (rb) tmem_ld_frag32(ta + 32, kq[1]);
+                        float gi[2], f[2];  // rows g and g + 8 of the block
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) {
+                            gi[a] = __shfl_sync(0xffffffffu, g_mine, 16 * h + g + 8 * a);
+                            f[a] = __shfl_sync(0xffffffffu, rb ? b_mine[1] : b_mine[0], 16 * h + g + 8 * a);
+                            if (is_p) f[a] = p.p_scale;
+                            if (kNorm) f[a] *= sRn[(is_p ? 64 : 0) + 16 * r + g + 8 * a];
+                        }
+                        const float gr = sG[16 * r];
+                        const float w0 = f[0] * ex2(gi[0] - gr), w1 = f[1] * ex2(gi[1] - gr);
+                        const f2 fo[2] = {pk(w0, w0), pk(w1, w1)}, fd[2] = {pk(f[0], f[0]), pk(f[1], f[1])};
                         tmem_wait_ld();
-                        // kMode 0: the block meets the diagonal (or the chunk is ragged): every element masked.
-                        // kMode 1: a block entirely below the diagonal of a full chunk: every element kept.
-                        // kMode 2: the same, with the decay of the block factored: for rows i >= 32 and columns j < 32
-                        //          e^{g_i-g_j} = e^{g_i-g_32} e^{g_32-g_j}, both factors <= 1 (the cumulative gate only
-                        //          falls), so the column factors come from a table and no ex2 is left per element.
-                        auto block = [&](auto mode_tag) {
-                            constexpr int kMode = decltype(mode_tag)::value;
-                            constexpr bool kMask = kMode == 0;
-                            f2 fvr = fv;
-                            if (kMode == 2) {
-                                const float ri = ex2(gi - sG[32]);
-                                fvr = mul2(fv, pk(ri, ri));
+                        // one block; `v`: its products
+                        auto block = [&](int c, const uint32_t* v, auto diag_tag) {
+                            constexpr bool kDiagonal = decltype(diag_tag)::value;
+                            float o[2][4];  // [8 columns][row g: two columns, row g + 8: two]
+#pragma unroll
+                            for (int nt = 0; nt < 2; ++nt) {
+                                const int cl = 8 * nt + 2 * tq;  // column within the block
+                                float2 rn = make_float2(1.f, 1.f);
+                                if (kNorm) rn = *reinterpret_cast<const float2*>(sRn + 16 * c + cl);  // the key's norm
+                                const float2 cf = *reinterpret_cast<const float2*>(kDiagonal ? sG + 16 * c + cl : sC + (rb ? 32 * h : 0) + 16 * c + cl);
+#pragma unroll
+                                for (int a = 0; a < 2; ++a) {
+                                    f2 x = pk(__uint_as_float(v[4 * nt + 2 * a]), __uint_as_float(v[4 * nt + 2 * a + 1]));
+                                    if (kNorm) x = mul2(x, pk(rn.x, rn.y));
+                                    if (kDiagonal) {
+                                        const int lim = g + 8 * a - (is_p ? 0 : 1);  // columns kept: cl <= lim
+                                        const float e0 = ex2(gi[a] - cf.x), e1 = ex2(gi[a] - cf.y);
+                                        unpk(mul2(mul2(x, fd[a]), pk(e0, e1)), o[nt][2 * a], o[nt][2 * a + 1]);
+                                        if (cl > lim) o[nt][2 * a] = 0.f;
+                                        if (cl + 1 > lim) o[nt][2 * a + 1] = 0.f;
+                                    } else {
+                                        unpk(mul2(mul2(x, fo[a]), pk(cf.x, cf.y)), o[nt][2 * a], o[nt][2 * a + 1]);
+                                    }
+                                }
                             }
+                            if (n < kChunk) {  // rows past the end: nothing, whatever lies there
 #pragma unroll
-                            for (int j = 0; j < 32; j += 8) {
-                                float o[8];
+                                for (int i = 0; i < 8; ++i)
+                                    if (16 * r + g + 8 * ((i >> 1) & 1) >= n) o[i >> 2][i & 3] = 0.f;
+                            }
+                            if (is_p) {
+                                stmatrix_x4(pt + tile_off(16 * r + (lane & 15), 2 * c + (lane >> 4)), pack_bf16(o[0][0], o[0][1]),
+                                            pack_bf16(o[0][2], o[0][3]), pack_bf16(o[1][0], o[1][1]), pack_bf16(o[1][2], o[1][3]));
+                            } else if (kDiagonal) {
+                                float* const o2 = reinterpret_cast<float*>(tbase + L::kOffDiag + r * L::kDiag) + g * L::kLdD + 2 * tq;
 #pragma unroll
-                                for (int e4 = 0; e4 < 2; ++e4) {
-                                    const float4 gc = *reinterpret_cast<const float4*>((kMode == 2 ? sC : sG) + 32 * cb + j + 4 * e4);
-                                    float gcv[4] = {gc.x, gc.y, gc.z, gc.w};
-                                    if (kNorm) {  // the column's key norm enters through the exponent
-                                        const float4 lr = *reinterpret_cast<const float4*>(sLr + 32 * cb + j + 4 * e4);
-                                        gcv[0] -= lr.x; gcv[1] -= lr.y; gcv[2] -= lr.z; gcv[3] -= lr.w;
-                                    }
-#pragma unroll
-                                    for (int e = 0; e < 4; e += 2) {
-                                        const int col = 32 * cb + j + 4 * e4 + e, k = j + 4 * e4 + e;
-                                        float d0, d1;
-                                        if (kMode == 2) {
-                                            d0 = gcv[e];
-                                            d1 = gcv[e + 1];
-                                        } else {
-                                            d0 = (!kMask || col <= lim) ? ex2(gi - gcv[e]) : 0.f;
-                                            d1 = (!kMask || col + 1 <= lim) ? ex2(gi - gcv[e + 1]) : 0.f;
-                                        }
-                                        unpk(mul2(mul2(pk(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), fvr), pk(d0, d1)),
-                                             o[4 * e4 + e], o[4 * e4 + e + 1]);
-                                    }
-                                }
-                                if (!is_p) {
-                                    *reinterpret_cast<float4*>(&sA[i * LD + 32 * cb + j]) = make_float4(o[0], o[1], o[2], o[3]);
-                                    *reinterpret_cast<float4*>(&sA[i * LD + 32 * cb + j + 4]) = make_float4(o[4], o[5], o[6], o[7]);
-                                } else {
-                                    const uint4 h = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]),
-                                                               pack_bf16(o[6], o[7]));
-                                    *reinterpret_cast<uint4*>(sP + tile_off(i, (32 * cb + j) >> 3)) = h;
-                                }
+                                for (int i = 0; i < 4; ++i)
+                                    *reinterpret_cast<float2*>(o2 + (i & 1) * 8 * L::kLdD + 8 * (i >> 1)) = make_float2(o[i >> 1][2 * (i & 1)], o[i >> 1][2 * (i & 1) + 1]);
+                            } else {
+                                uint32_t hi[4], lo[4];
+                                split_frag(o, hi, lo);
+                                const uint32_t ob = smem_u32(tbase + L::kOffA + (r * (r - 1) / 2 + c) * 1024);
+                                stmatrix_x4(ob + blk_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+                                stmatrix_x4(ob + blk_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
                             }
                         };
-                        if (cb < rb && n == kChunk) {
-                            if (kNorm)
-                                block(std::integral_constant<int, 1>{});
-                            else
-                                block(std::integral_constant<int, 2>{});
-                        } else {
-                            block(std::integral_constant<int, 0>{});
+                        constexpr std::false_type below{};
+                        constexpr std::true_type diagonal{};
+                        if (rb) {
+                            block(0, kq[0], below);
+                            block(1, kq[0] + 8, below);
+                            if (h) block(2, kq[1], below);
+                        } else if (h) {
+                            block(0, kq[0], below);
                         }
-                    }
-                    if (is_p && rb == 0) {  // rows 0-31 of P: columns 32-63 lie above the diagonal
+                        block(r, h == 0 ? (rb ? kq[1] : kq[0]) : (rb ? kq[1] + 8 : kq[0] + 8), diagonal);
+                        if (is_p) {  // the blocks above the diagonal: zeros
 #pragma unroll
-                        for (int c16 = 4; c16 < 8; ++c16)
-                            *reinterpret_cast<uint4*>(sP + tile_off(i, c16)) = make_uint4(0u, 0u, 0u, 0u);
+                            for (int c = 1; c < 4; ++c)
+                                if (c > r) stmatrix_x4(pt + tile_off(16 * r + (lane & 15), 2 * c + (lane >> 4)), 0u, 0u, 0u, 0u);
+                        }
+                    };
+                    using I0 = std::integral_constant<int, 0>;
+                    using I1 = std::integral_constant<int, 1>;
+                    if (tw & 1) {
+                        row_block(I1{}, I0{});
+                        row_block(I1{}, I1{});
+                    } else {
+                        row_block(I0{}, I0{});
+                        row_block(I0{}, I1{});
                     }
-                }
-                if (rd + 1 < rounds) {
-                    fetch_scalars(cur, rd + 1, b_next, g_next);
-                } else {
-                    nxt = unit_at(table);
-                    fetch_scalars(nxt, 0, b_next, g_next);
                 }
                 tc_fence_before_sync();
                 team_sync(team);
-                // ---- X = (I + A)^-1 in place.  Every warp owns one 16x16 diagonal block: its two 8x8 diagonal
-                //      blocks by forward substitution in fp32 (one column per lane, 16 lanes), then
-                //      X_10 = -X_11 A_10 X_00 with two TF32 warp MMAs (the intermediate stays in registers).
+                // ---- X = (I + A)^-1.  Every warp owns a 16-row block (team 1 in reverse order: the last one is the longest, and warps w of
+                //      both teams share a scheduler).  Its diagonal block first: the two 8x8 diagonal blocks by forward substitution in
+                //      fp32 (one column per lane, 16 lanes), then X_10 = -X_11 A_10 X_00 with two TF32 warp MMAs (the intermediate
+                //      stays in registers).
+                const int rblk = team ? 3 - tw : tw;
+                const int g = lane >> 2, tq = lane & 3;
+                float x[4][2][4], xd[2][4];  // blocks X_r0 .. X_rr of the row block and its diagonal block, as accumulator fragments
                 {
-                    const int b = tw, hb = (lane >> 3) & 1, j = lane & 7;
-                    const int o = 16 * b + 8 * hb;  // first row / column of this lane's 8x8 block
-                    float x[8];
+                    constexpr int LD = L::kLdD;
+                    float* const sA = reinterpret_cast<float*>(tbase + L::kOffDiag + rblk * L::kDiag);
+                    const int hb = (lane >> 3) & 1, j = lane & 7;
+                    const int o = 8 * hb;  // first row / column of this lane's 8x8 block
+                    float xc[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) x[i] = (i == j) ? 1.f : 0.f;
+                    for (int i = 0; i < 8; ++i) xc[i] = (i == j) ? 1.f : 0.f;
                     // x_j = 1, x_i = -sum_{m<i} A_im x_m
 #pragma unroll
                     for (int i = 1; i < 8; ++i) {
@@ -446,148 +544,107 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                         }
                         float acc = 0.f;
 #pragma unroll
-                        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[m], x[m], acc);
-                        if (i > j) x[i] = -fmaf(a[i - 1], x[i - 1], acc);
+                        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[m], xc[m], acc);
+                        if (i > j) xc[i] = -fmaf(a[i - 1], xc[i - 1], acc);
                     }
                     __syncwarp();  // the block is private to this warp: every lane has read it
                     if (lane < 16) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) sA[(o + i) * LD + o + j] = x[i];
+                        for (int i = 0; i < 8; ++i) sA[(o + i) * LD + o + j] = xc[i];
                     }
                     __syncwarp();
-                    // level 0 (8 -> 16)
-                    const int i0 = 16 * b + 8, j0 = 16 * b;
+                    // 8 -> 16
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_blk<8>(d, sA, i0, j0, sA, j0, j0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
+                    mma_blk<8>(d, sA, 8, 0, sA, 0, 0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
                     // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
-                    const int g = lane >> 2, tq = lane & 3;
                     const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
                     const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
                     const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
                     const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
                     uint32_t bfrag[2] = {to_tf32((g & 1) ? v01 : v00), to_tf32((g & 1) ? v11 : v10)}, afrag[4];
-                    load_a<8>(afrag, sA, LD, i0, i0, lane);
+                    load_a<8>(afrag, sA, LD, 8, 8, lane);
+                    const float2 c00 = *reinterpret_cast<const float2*>(&sA[g * LD + 2 * tq]);
+                    const float2 c11 = *reinterpret_cast<const float2*>(&sA[(8 + g) * LD + 8 + 2 * tq]);
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
                     mma_tf32(e, afrag, bfrag);  // X_11 t
-                    *reinterpret_cast<float2*>(&sA[(i0 + g) * LD + j0 + 2 * tq]) = make_float2(-e[0], -e[1]);
+                    xd[0][0] = c00.x; xd[0][1] = c00.y; xd[0][2] = -e[0]; xd[0][3] = -e[1];
+                    xd[1][0] = 0.f; xd[1][1] = 0.f; xd[1][2] = c11.x; xd[1][3] = c11.y;
+                    __syncwarp();  // the block has been read: its inverse goes in its place, for the row blocks further down
+                    uint32_t hi[4], lo[4];
+                    split_frag(xd, hi, lo);
+                    const uint32_t ia = smem_u32(sA);
+                    stmatrix_x4(ia + blk_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+                    stmatrix_x4(ia + blk_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
                 }
                 team_sync(team);
-                // level 1 (16 -> 32): X_10 = -X_11 A_10 X_00, X_32 = -X_33 A_32 X_22; warp = (pair, 8-column half);
-                // the intermediate A_10 X_00 is parked in the unused block above the diagonal
+                // ---- the row block's other blocks, then T = X diag(beta) and dT = diag(d) T as bf16 swizzled tiles (row = token i,
+                //      64 columns j)
                 {
-                    const int pr = tw >> 1, n0 = 8 * (tw & 1);
-                    const int i0 = 16 * (2 * pr + 1), j0 = 16 * (2 * pr);
-                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+                    const uint32_t aa = smem_u32(tbase + L::kOffA), ia = smem_u32(tbase + L::kOffDiag);
+                    auto finish = [&](auto r_tag) {
+                        constexpr int R = decltype(r_tag)::value;
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_blk(d, sA, i0, j0 + 8 * ks, sA, j0 + 8 * ks, j0 + n0, LD, lane);
-                    store_block(d, 1.f, sA, LD, j0, i0 + n0, lane);
-                    __syncwarp();  // the 8 columns of the intermediate are this warp's alone
-                    float e[4] = {0.f, 0.f, 0.f, 0.f};
+                        for (int i = 0; i < 8; ++i) x[R][i >> 2][i & 3] = xd[i >> 2][i & 3];
+                        row_blocks<R>(x, aa, ia, lane);
+                        const int row = 16 * R + g;
+                        const float d0 = kNorm ? sD[row] * sRn[row] : sD[row], d1 = kNorm ? sD[row + 8] * sRn[row + 8] : sD[row + 8];
+                        const f2 dd[2] = {pk(d0, d0), pk(d1, d1)};
+                        const uint32_t tile = smem_u32(sT);
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_blk(e, sA, i0, i0 + 8 * ks, sA, j0 + 8 * ks, i0 + n0, LD, lane);
-                    pair_sync(2 * team + pr);  // both warps of the pair have read A_10
-                    store_block(e, -1.f, sA, LD, i0, j0 + n0, lane);
-                }
-                team_sync(team);
-                // level 2 (32 -> 64): X_[2:4,0:2] = -X_[2:4,2:4] A_[2:4,0:2] X_[0:2,0:2]; warp = 8 columns of the result, so
-                // that its part of the intermediate (parked in the unused upper-right quadrant) is its own as well
-                {
-                    const int n0 = 8 * tw;
-                    float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                        for (int c = 0; c < 4; ++c) {
+                            uint32_t tv[4] = {0u, 0u, 0u, 0u}, wv[4] = {0u, 0u, 0u, 0u};
+                            if (c <= R) {
 #pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {
-                        if (ks >= tw) {  // (blocks of X above the diagonal are zero)
-                            uint32_t af[4], bf[2];
-                            load_b(bf, sA, LD, 8 * ks, n0, lane);  // shared by the two row tiles
-#pragma unroll
-                            for (int mt = 0; mt < 2; ++mt) {
-                                load_a(af, sA, LD, 32 + 16 * mt, 8 * ks, lane);
-                                mma_tf32(d[mt], af, bf);
+                                for (int i = 0; i < 4; ++i) {  // [8 columns][row g, g + 8]
+                                    const f2 be = *reinterpret_cast<const f2*>(&sBeta[16 * c + 8 * (i >> 1) + 2 * tq]);
+                                    const f2 t = mul2(pk(x[c][i >> 1][2 * (i & 1)], x[c][i >> 1][2 * (i & 1) + 1]), be);
+                                    float a, b;
+                                    unpk(t, a, b);
+                                    tv[i] = pack_bf16(a, b);
+                                    unpk(mul2(t, dd[i & 1]), a, b);
+                                    wv[i] = pack_bf16(a, b);
+                                }
                             }
+                            const uint32_t off = sw128_offset(16 * R + (lane & 15), 16 * c + 8 * (lane >> 4));
+                            stmatrix_x4(tile + off, tv[0], tv[1], tv[2], tv[3]);
+                            stmatrix_x4(tile + 8192 + off, wv[0], wv[1], wv[2], wv[3]);
                         }
-                    }
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) store_block(d[mt], 1.f, sA, LD, 16 * mt, 32 + n0, lane);
-                    __syncwarp();
-                    float e[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {
-                        uint32_t af[4], bf[2];
-                        load_b(bf, sA, LD, 8 * ks, 32 + n0, lane);
-#pragma unroll
-                        for (int mt = 0; mt < 2; ++mt) {
-                            if (ks < 2 * (mt + 1)) {
-                                load_a(af, sA, LD, 32 + 16 * mt, 32 + 8 * ks, lane);
-                                mma_tf32(e[mt], af, bf);
-                            }
-                        }
-                    }
-                    team_sync(team);  // every warp has read A_[2:4,0:2]
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) store_block(e[mt], -1.f, sA, LD, 32 + 16 * mt, n0, lane);
-                }
-                team_sync(team);
-                // ---- T = X diag(beta) and dT = diag(d) T as bf16 swizzled tiles (row = token i, 64 columns j) over X;
-                //      every thread first pulls its 32 values of X into registers
-                {
-                    // (16 rows and both halves per warp: eight rows per phase of a 16-byte access, no bank conflicts)
-                    const int i = 16 * tw + (lane & 15), c0 = (lane >> 4) * 32;
-                    float xs[32];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float4 t = *reinterpret_cast<const float4*>(&sA[i * LD + c0 + 4 * q]);
-                        const bool valid = ((c0 + 4 * q) >> 4) <= (i >> 4);  // blocks above the diagonal hold scratch
-                        xs[4 * q] = valid ? t.x : 0.f; xs[4 * q + 1] = valid ? t.y : 0.f;
-                        xs[4 * q + 2] = valid ? t.z : 0.f; xs[4 * q + 3] = valid ? t.w : 0.f;
-                    }
-                    const float di = kNorm ? sD[i] * sRn[i] : sD[i];
-                    const f2 di2 = pk(di, di);
-                    team_sync(team);
-#pragma unroll
-                    for (int ch = 0; ch < 4; ++ch) {
-                        const float4 b0 = *reinterpret_cast<const float4*>(&sBeta[c0 + 8 * ch]);
-                        const float4 b1 = *reinterpret_cast<const float4*>(&sBeta[c0 + 8 * ch + 4]);
-                        const float* x = xs + 8 * ch;
-                        const f2 t0 = mul2(pk(x[0], x[1]), pk(b0.x, b0.y)), t1 = mul2(pk(x[2], x[3]), pk(b0.z, b0.w));
-                        const f2 t2 = mul2(pk(x[4], x[5]), pk(b1.x, b1.y)), t3 = mul2(pk(x[6], x[7]), pk(b1.z, b1.w));
-                        float v[8], w[8];
-                        unpk(t0, v[0], v[1]); unpk(t1, v[2], v[3]); unpk(t2, v[4], v[5]); unpk(t3, v[6], v[7]);
-                        unpk(mul2(t0, di2), w[0], w[1]); unpk(mul2(t1, di2), w[2], w[3]);
-                        unpk(mul2(t2, di2), w[4], w[5]); unpk(mul2(t3, di2), w[6], w[7]);
-                        const uint32_t off = sw128_offset(i, c0 + 8 * ch);
-                        const uint4 hv = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-                        const uint4 hw = make_uint4(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), pack_bf16(w[4], w[5]), pack_bf16(w[6], w[7]));
-                        *reinterpret_cast<uint4*>(sT + off) = hv;
-                        *reinterpret_cast<uint4*>(sTd + off) = hw;
-                    }
+                    };
+                    if (rblk == 0) finish(std::integral_constant<int, 0>{});
+                    else if (rblk == 1) finish(std::integral_constant<int, 1>{});
+                    else if (rblk == 2) finish(std::integral_constant<int, 2>{});
+                    else finish(std::integral_constant<int, 3>{});
                 }
                 fence_proxy_async_smem();
                 team_sync(team);
-                // ---- Z = (dT)^T K as two 64-column halves (lanes +0 / +16 of the team's columns), PT = P T
+                // ---- Z = (dT)^T K and PT = P T; team 0 in lanes +0, team 1 in lanes +16 of the same columns
                 if (tw == 0) {
                     tc_fence_after_sync();
                     constexpr uint32_t idesc = make_idesc_bf16(64, 64, false, true);   // PT: A K-major, B MN-major
-                    constexpr uint32_t idescz = make_idesc_bf16(64, 64, true, true);   // Z: A = (dT)^T read MN-major too
+                    constexpr uint32_t idescz = make_idesc_bf16(64, 128, true, true);  // Z: A = (dT)^T read MN-major too
                     const uint64_t dTd = make_smem_desc_sw128(smem_u32(sTd), 8192, 1024);       // A, read MN-major
                     const uint64_t dPa = make_smem_desc_sw128(smem_u32(sP), 0, 1024);           // A, K-major
                     const uint64_t dTb = make_smem_desc_sw128(smem_u32(sT), 8192, 1024);        // B, read MN-major
-                    const uint64_t dK = make_smem_desc_sw128(smem_u32(sKQ), 8192, 1024);        // B, K columns 0-63, MN-major
-                    const uint32_t tZ = tmem + kTmZ + 64u * team;
+                    const uint64_t dK = make_smem_desc_sw128(smem_u32(sKQ), 16384, 1024);       // B, K, MN-major: two 64-column atoms
+                    const uint32_t tZ = tmem + kTmZ + (team ? (16u << 16) : 0u);
                     const uint32_t tPT = tmem + kTmPT + (team ? (16u << 16) : 0u);
+                    mma_ss_w<false>(tZ, dTd, dK, idescz);
 #pragma unroll
-                    for (int a = 0; a < NA; ++a) {  // 64 columns of Z each
-                        const uint32_t tz = tZ + (a ? (16u << 16) : 0u);
-                        const uint64_t dk = desc_advance(dK, a * 16384);
-                        mma_ss_w<false>(tz, dTd, dk, idescz);
-#pragma unroll
-                        for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tz, desc_advance(dTd, ks * 2048), desc_advance(dk, ks * 2048), idescz);
-                    }
+                    for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tZ, desc_advance(dTd, ks * 2048), desc_advance(dK, ks * 2048), idescz);
                     mma_ss_w<false>(tPT, dPa, dTb, idesc);
 #pragma unroll
                     for (int ks = 1; ks < 4; ++ks) mma_ss_w<true>(tPT, desc_advance(dPa, ks * 32), desc_advance(dTb, ks * 2048), idesc);
                     mma_commit_w(&bar_mma[team]);
                 }
                 __syncwarp();
+                // the next round's scalars, requested in front of a long wait: anywhere else other loads that share their
+                // scoreboard wait for DRAM with them (the substitution took 700 cycles instead of 250 behind them)
+                if (rd + 1 < rounds) {
+                    fetch_scalars(cur, rd + 1, b_next, g_next);
+                } else {
+                    nxt = unit_at(table);
+                    fetch_scalars(nxt, 0, b_next, g_next);
+                }
                 mbar_wait(&bar_mma[team], mma_it & 1u, abort_flag);
                 ++mma_it;
                 tc_fence_after_sync();
@@ -602,54 +659,43 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 }
             }
             if (active) {
-                const int row = 16 * tw + (lane & 15), hi = lane >> 4;
-                const uint32_t tl = static_cast<uint32_t>(32 * tw) << 16;
-                // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> two bulk copies
-                uint8_t* stZ = tbase + L::kOffA;
+                const int row = 16 * tw + (lane & 15);
+                const uint32_t tl = static_cast<uint32_t>(32 * tw + 16 * team) << 16;
+                // ---- accumulators -> bf16 -> staged tiles (Z over T / dT, PT over P) -> one bulk copy.  As fragments: 16 lanes of
+                //      tensor memory are one team's.
 #pragma unroll
-                for (int cb = 0; cb < 2; ++cb) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem + kTmZ + 64u * team + tl + 32 * cb, r);
+                for (int cb = 0; cb < 6; cb += 2) {  // 32 columns each: four of Z, two of PT
+                    uint32_t r[2][16];
+                    const uint32_t col = cb < 4 ? kTmZ + 32 * cb : kTmPT;
+                    tmem_ld_frag32(tmem + col + tl, r[0]);
+                    tmem_ld_frag32(tmem + col + 32 + tl, r[1]);
                     tmem_wait_ld();
+                    const uint32_t tile = smem_u32(cb < 4 ? sT : sP);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        *reinterpret_cast<uint4*>(stZ + tile_off(row, 8 * hi + 4 * cb + q)) = make_uint4(
-                            pack_bf16(__uint_as_float(r[8 * q + 0]), __uint_as_float(r[8 * q + 1])),
-                            pack_bf16(__uint_as_float(r[8 * q + 2]), __uint_as_float(r[8 * q + 3])),
-                            pack_bf16(__uint_as_float(r[8 * q + 4]), __uint_as_float(r[8 * q + 5])),
-                            pack_bf16(__uint_as_float(r[8 * q + 6]), __uint_as_float(r[8 * q + 7])));
-                }
+                    for (int h = 0; h < 4; ++h) {  // 16 columns
+                        uint32_t w[4];
 #pragma unroll
-                for (int cb = 0; cb < 2; ++cb) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem + kTmPT + tl + 32 * cb, r);  // lanes +0: team 0's PT, lanes +16: team 1's
-                    tmem_wait_ld();
-                    if (hi == team) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            *reinterpret_cast<uint4*>(sP + tile_off(row, 4 * cb + q)) = make_uint4(
-                                pack_bf16(__uint_as_float(r[8 * q + 0]), __uint_as_float(r[8 * q + 1])),
-                                pack_bf16(__uint_as_float(r[8 * q + 2]), __uint_as_float(r[8 * q + 3])),
-                                pack_bf16(__uint_as_float(r[8 * q + 4]), __uint_as_float(r[8 * q + 5])),
-                                pack_bf16(__uint_as_float(r[8 * q + 6]), __uint_as_float(r[8 * q + 7])));
+                        for (int i = 0; i < 4; ++i) {  // [8 columns][row l/4, l/4 + 8]
+                            const uint32_t* const v = &r[h >> 1][8 * (h & 1) + 2 * i];
+                            w[i] = pack_bf16(__uint_as_float(v[0]), __uint_as_float(v[1]));
+                        }
+                        stmatrix_x4(tile + tile_off(row, 4 * (cb & 3) + 2 * h + (lane >> 4)), w[0], w[1], w[2], w[3]);
                     }
                 }
                 fence_proxy_async_smem();
                 tc_fence_before_sync();
                 team_sync(team);
-                if (tt == 0 && *abort_flag == 0) {  // nothing is written once a wait has given up
-                    uint8_t* dst = p.blocks + (static_cast<size_t>(chunk) * p.vh + head) * kZPBlockBytes;
+                if (tt == 64 && *abort_flag == 0) {  // nothing is written once a wait has given up
                     // the state kernel reads these blocks back soon: ask L2 to hold on to them
-                    const uint64_t keep = l2_policy_evict_last();
-                    bulk_store_hint(dst, stZ, 16384, keep);
-                    bulk_store_hint(dst + 16384, sP, 8192, keep);
+                    bulk_store_hint(p.blocks + (static_cast<size_t>(chunk) * p.vh + head) * kZPBlockBytes, sT, kZPBlockBytes,
+                                    l2_policy_evict_last());
                     bulk_commit();
                 }
                 stores_pending = true;
             }
         }  // head pairs
     }      // units
-    if (stores_pending && tt == 0) bulk_wait_read<0>();
+    if (stores_pending && tt == 64) bulk_wait_read<0>();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 256);

@@ -367,6 +367,11 @@ GDN_DEVICE void ldmatrix_x4_trans(uint32_t saddr, uint32_t* r) {
                  : "r"(saddr)
                  : "memory");
 }
+// (not transposed: register m of lane l holds columns 2(l%4), 2(l%4)+1 of row l/4)
+GDN_DEVICE void stmatrix_x4(uint32_t saddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(saddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+                 : "memory");
+}
 GDN_DEVICE void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(saddr), "r"(r0), "r"(r1), "r"(r2),
                  "r"(r3)
