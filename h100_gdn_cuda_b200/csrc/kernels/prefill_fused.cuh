@@ -145,8 +145,11 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     uint64_t* bar_o = bars + 8;
     uint64_t* bar_ofree = bars + 9;
     uint64_t* bar_full2 = bars + 10;  // [2]: Z, PT, Q of a stage (bar_full: K, V and the gate vectors)
-    uint64_t* bar_go = bars + 12;     // state warps are past their chunk-boundary work: the epilogue may run
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    // [2] state warps are past the chunk-boundary work of an even / odd chunk: the epilogue of the one before may run.  Two,
+    // because they can be a whole chunk ahead of the output warps, which would take the phase after next for the one before
+    // it on a single barrier and never see it (they cannot be two ahead: O2 of chunk c + 1 waits for the epilogue of chunk c).
+    uint64_t* bar_go = bars + 12;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
     int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
     volatile int* issued = abort_flag + 1;  // chunks whose loads the producer has issued (read by the L2 prefetcher)
 
@@ -201,7 +204,8 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         mbar_init(&bar_empty[1], 1);
         mbar_init(&bar_full2[0], 1);
         mbar_init(&bar_full2[1], 1);
-        mbar_init(bar_go, 8);
+        mbar_init(&bar_go[0], 8);
+        mbar_init(&bar_go[1], 8);
         mbar_init(bar_sbf, 8);
         mbar_init(bar_d1, 1);
         mbar_init(bar_un, 8);
@@ -294,7 +298,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             // The state warps now idle until D1 arrives: the window in which the output warps (which
             // share the schedulers) run the previous chunk's epilogue without slowing the chain down.
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_go);
+            if (lane == 0) mbar_arrive(&bar_go[c & 1]);
             mbar_wait(bar_d1, par, abort_flag);
             tc_fence_after_sync();
             {
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
                 if (lane == 0) mbar_arrive(bar_sbf);
             }
         }
-        if (lane == 0) mbar_arrive(bar_go);  // releases the last chunk's epilogue
+        if (lane == 0) mbar_arrive(&bar_go[nchunks & 1]);  // releases the last chunk's epilogue
         // nothing is written once a wait of this CTA has given up (the results would be garbage)
         const bool healthy = *abort_flag == 0;
         if (!healthy) {
@@ -405,9 +409,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             uint8_t* sO = smem + L::kOffO + (c & 1) * L::kTile;
             const uint32_t tO1 = tmem + ((c & 1) ? kTmO1b : kTmO1a) + tm_lane;
             const uint32_t tO2 = tmem + kTmO2 + tm_lane;
-            mbar_wait_relaxed<200>(&bar_full[c & 1], static_cast<uint32_t>((c >> 1) & 1), abort_flag);
+            // (not on bar_full, which may be two phases on by now: its stage is free once the MMAs have read it.  The gate factors
+            // are visible through bar_go: the state warps have waited for bar_full.)
             mbar_wait_relaxed<100>(bar_o, par, abort_flag);
-            mbar_wait_relaxed<50>(bar_go, static_cast<uint32_t>((c + 1) & 1), abort_flag);
+            mbar_wait_relaxed<50>(&bar_go[(c + 1) & 1], static_cast<uint32_t>(((c + 1) >> 1) & 1), abort_flag);
             tc_fence_after_sync();
             const uint32_t sOa = smem_u32(sO);
 #pragma unroll
