@@ -426,12 +426,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     const bool is_p = tw >= 2;
                     const int g = lane >> 2, tq = lane & 3;
                     const uint32_t pt = smem_u32(sP);
-                    auto row_block = [&](auto rb_tag, auto h_tag) {
+                    auto row_block = [&](auto rb_tag, auto h_tag, const uint32_t (*kq)[16]) {
                         constexpr int rb = decltype(rb_tag)::value, h = decltype(h_tag)::value, r = 2 * rb + h;
-                        const uint32_t ta = tmem + kTmKQ + (static_cast<uint32_t>(32 * tw + 16 * h) << 16);
-                        uint32_t kq[2][16];
-                        tmem_ld_frag32(ta, kq[0]);
-                        if (rb) tmem_ld_frag32(ta + 32, kq[1]);
                         float gi[2], f[2];  // rows g and g + 8 of the block
 #pragma unroll
                         for (int a = 0; a < 2; ++a) {
@@ -443,7 +439,6 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                         const float gr = sG[16 * r];
                         const float w0 = f[0] * ex2(gi[0] - gr), w1 = f[1] * ex2(gi[1] - gr);
                         const f2 fo[2] = {pk(w0, w0), pk(w1, w1)}, fd[2] = {pk(f[0], f[0]), pk(f[1], f[1])};
-                        tmem_wait_ld();
                         // one block; `v`: its products
                         auto block = [&](int c, const uint32_t* v, auto diag_tag) {
                             constexpr bool kDiagonal = decltype(diag_tag)::value;
@@ -508,12 +503,20 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     };
                     using I0 = std::integral_constant<int, 0>;
                     using I1 = std::integral_constant<int, 1>;
+                    const uint32_t ta = tmem + kTmKQ + (static_cast<uint32_t>(32 * tw) << 16), tb = ta + (16u << 16);
+                    uint32_t k0[2][16], k1[2][16];  // 32 columns each
+                    tmem_ld_frag32(ta, k0[0]);
+                    tmem_ld_frag32(tb, k1[0]);
                     if (tw & 1) {
-                        row_block(I1{}, I0{});
-                        row_block(I1{}, I1{});
+                        tmem_ld_frag32(ta + 32, k0[1]);
+                        tmem_ld_frag32(tb + 32, k1[1]);
+                        tmem_wait_ld();
+                        row_block(I1{}, I0{}, k0);
+                        row_block(I1{}, I1{}, k1);
                     } else {
-                        row_block(I0{}, I0{});
-                        row_block(I0{}, I1{});
+                        tmem_wait_ld();
+                        row_block(I0{}, I0{}, k0);
+                        row_block(I0{}, I1{}, k1);
                     }
                 }
                 tc_fence_before_sync();
@@ -524,28 +527,30 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 //      stays in registers).
                 const int rblk = team ? 3 - tw : tw;
                 const int g = lane >> 2, tq = lane & 3;
-                float x[4][2][4], xd[2][4];  // blocks X_r0 .. X_rr of the row block and its diagonal block, as accumulator fragments
+                float x[4][2][4], xd[2][4];  // blocks X_r0 .. X_rr of the row block (diagonal block first in all) and its diagonal block, as accumulator fragments
                 {
                     constexpr int LD = L::kLdD;
                     float* const sA = reinterpret_cast<float*>(tbase + L::kOffDiag + rblk * L::kDiag);
                     const int hb = (lane >> 3) & 1, j = lane & 7;
                     const int o = 8 * hb;  // first row / column of this lane's 8x8 block
-                    float xc[8];
+                    float xc[8], a[8][8];
+#pragma unroll
+                    for (int i = 1; i < 8; ++i) {
+#pragma unroll
+                        for (int q = 0; q < (i + 3) / 4; ++q) {
+                            const float4 t = *reinterpret_cast<const float4*>(&sA[(o + i) * LD + o + 4 * q]);
+                            a[i][4 * q] = t.x; a[i][4 * q + 1] = t.y; a[i][4 * q + 2] = t.z; a[i][4 * q + 3] = t.w;
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < 8; ++i) xc[i] = (i == j) ? 1.f : 0.f;
                     // x_j = 1, x_i = -sum_{m<i} A_im x_m
 #pragma unroll
                     for (int i = 1; i < 8; ++i) {
-                        float a[8];
-#pragma unroll
-                        for (int q = 0; q < (i + 3) / 4; ++q) {
-                            const float4 t = *reinterpret_cast<const float4*>(&sA[(o + i) * LD + o + 4 * q]);
-                            a[4 * q] = t.x; a[4 * q + 1] = t.y; a[4 * q + 2] = t.z; a[4 * q + 3] = t.w;
-                        }
                         float acc = 0.f;
 #pragma unroll
-                        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[m], xc[m], acc);
-                        if (i > j) xc[i] = -fmaf(a[i - 1], xc[i - 1], acc);
+                        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[i][m], xc[m], acc);
+                        if (i > j) xc[i] = -fmaf(a[i][i - 1], xc[i - 1], acc);
                     }
                     __syncwarp();  // the block is private to this warp: every lane has read it
                     if (lane < 16) {
@@ -581,39 +586,38 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 //      64 columns j)
                 {
                     const uint32_t aa = smem_u32(tbase + L::kOffA), ia = smem_u32(tbase + L::kOffDiag);
-                    auto finish = [&](auto r_tag) {
-                        constexpr int R = decltype(r_tag)::value;
+                    // (one copy of the code below for all row blocks: the kernel's loop does not fit the instruction cache as it is)
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) x[R][i >> 2][i & 3] = xd[i >> 2][i & 3];
-                        row_blocks<R>(x, aa, ia, lane);
-                        const int row = 16 * R + g;
-                        const float d0 = kNorm ? sD[row] * sRn[row] : sD[row], d1 = kNorm ? sD[row + 8] * sRn[row + 8] : sD[row + 8];
-                        const f2 dd[2] = {pk(d0, d0), pk(d1, d1)};
-                        const uint32_t tile = smem_u32(sT);
+                    for (int c = 0; c < 4; ++c) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            uint32_t tv[4] = {0u, 0u, 0u, 0u}, wv[4] = {0u, 0u, 0u, 0u};
-                            if (c <= R) {
+                        for (int i = 0; i < 8; ++i) x[c][i >> 2][i & 3] = xd[i >> 2][i & 3];
+                    }
+                    if (rblk == 1) row_blocks<1>(x, aa, ia, lane);
+                    else if (rblk == 2) row_blocks<2>(x, aa, ia, lane);
+                    else if (rblk == 3) row_blocks<3>(x, aa, ia, lane);
+                    const int row = 16 * rblk + g;
+                    const float d0 = kNorm ? sD[row] * sRn[row] : sD[row], d1 = kNorm ? sD[row + 8] * sRn[row + 8] : sD[row + 8];
+                    const f2 dd[2] = {pk(d0, d0), pk(d1, d1)};
+                    const uint32_t tile = smem_u32(sT);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {  // [8 columns][row g, g + 8]
-                                    const f2 be = *reinterpret_cast<const f2*>(&sBeta[16 * c + 8 * (i >> 1) + 2 * tq]);
-                                    const f2 t = mul2(pk(x[c][i >> 1][2 * (i & 1)], x[c][i >> 1][2 * (i & 1) + 1]), be);
-                                    float a, b;
-                                    unpk(t, a, b);
-                                    tv[i] = pack_bf16(a, b);
-                                    unpk(mul2(t, dd[i & 1]), a, b);
-                                    wv[i] = pack_bf16(a, b);
-                                }
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t tv[4] = {0u, 0u, 0u, 0u}, wv[4] = {0u, 0u, 0u, 0u};
+                        if (c <= rblk) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {  // [8 columns][row g, g + 8]
+                                const f2 be = *reinterpret_cast<const f2*>(&sBeta[16 * c + 8 * (i >> 1) + 2 * tq]);
+                                const f2 t = mul2(pk(x[c][i >> 1][2 * (i & 1)], x[c][i >> 1][2 * (i & 1) + 1]), be);
+                                float a, b;
+                                unpk(t, a, b);
+                                tv[i] = pack_bf16(a, b);
+                                unpk(mul2(t, dd[i & 1]), a, b);
+                                wv[i] = pack_bf16(a, b);
                             }
-                            const uint32_t off = sw128_offset(16 * R + (lane & 15), 16 * c + 8 * (lane >> 4));
-                            stmatrix_x4(tile + off, tv[0], tv[1], tv[2], tv[3]);
-                            stmatrix_x4(tile + 8192 + off, wv[0], wv[1], wv[2], wv[3]);
                         }
-                    };
-                    if (rblk == 0) finish(std::integral_constant<int, 0>{});
-                    else if (rblk == 1) finish(std::integral_constant<int, 1>{});
-                    else if (rblk == 2) finish(std::integral_constant<int, 2>{});
-                    else finish(std::integral_constant<int, 3>{});
+                        const uint32_t off = sw128_offset(16 * rblk + (lane & 15), 16 * c + 8 * (lane >> 4));
+                        stmatrix_x4(tile + off, tv[0], tv[1], tv[2], tv[3]);
+                        stmatrix_x4(tile + 8192 + off, wv[0], wv[1], wv[2], wv[3]);
+                    }
                 }
                 fence_proxy_async_smem();
                 team_sync(team);
