@@ -170,15 +170,16 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
 }
 
 // Long runs of tokens whose last state alone is wanted: blocks of tokens on warp matrix instructions (recurrent_block.cuh),
-// unless the runs are but one token longer than a block and the CTAs are many: a block with one token takes as long as one with
-// 16, and the token recurrence fills the GPU then.  Token recurrence against this, 32 v-heads: d=128, T=17 B=64 316 : 342 us, B=8
-// 48 : 45, B=1 (one wave of CTAs) 14.2 : 8.1; T=24 B=64 430 : 343; d=64, T=17 B=64 105 : 143, B=8 17.2 : 21.5, T=24 138 : 144, T=40
-// 222 : 187; d=256, 8 v-heads, T=17 B=16 59 : 60, T=32 102 : 61.
+// unless the runs are but little longer than a block and the CTAs are many: a second block with few tokens takes as long as a
+// full one, and the token recurrence fills the GPU then.  Token recurrence against this in us: 32 v-heads, d=128, T=20 / 22 / 24 B=64 365 / 401
+// / 431 : 395 / 400 / 403, B=20 121 / 132 / 142 : 125 / 126 / 127, B=8 55 / 60 / 64 : 51 / 52 / 52, T=17 B=1 (one wave of CTAs)
+// 14 : 8; d=64, T=28 / 32 / 40 B=64 159 / 179 / 223 : 175 / 173 / 210, B=16 48 / 53 / 66 : 46 / 45 / 55; 8 v-heads, d=256, T=20 / 24 / 32
+// B=64 236 / 276 / 360 : 259 / 261 / 261.
 static bool block_takes(const GdnShape& s, bool steps, int sms) {
     if (steps || (s.head_dim_k != 64 && s.head_dim_k != 128 && s.head_dim_k != 192 && s.head_dim_k != 256)) return false;
     const long long tokens = s.cu_seqlens ? s.total_tokens : static_cast<long long>(s.seq_len) * s.batch;
     const long long ctas = static_cast<long long>(s.batch) * s.num_v_heads * (s.head_dim_v / kBlkRows);
-    return ctas <= 2ll * sms || tokens >= (s.head_dim_k == 64 ? 26ll : 20ll) * s.batch;
+    return ctas <= 2ll * sms || tokens >= (s.head_dim_k == 64 ? 31ll : 23ll) * s.batch;
 }
 template <int DK, bool kF32 = false>
 static int launch_block_t(const RecurrentParams& p, cudaStream_t st) {

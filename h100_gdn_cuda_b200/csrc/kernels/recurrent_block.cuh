@@ -12,19 +12,21 @@
 //
 // Why: the token recurrence (recurrent.cuh, ring instance) is a chain of about 1 250 cycles per token, and a sequence of a
 // few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of products (1 000
-// cycles), sums and a triangular solve (850), the update (500) and the outputs (400): B=2, T=1500, 8 v-heads, d=256 996 -> 256 us,
-// T=700, 4 v-heads, d=192 401 -> 73, T=65 42 -> 12.5; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.75 ms.  With two CTAs per SM
-// the matrix instructions set the pace (16 cycles each, 84 per scheduler, block and CTA: 2 700 of 4 450 cycles), with one the
-// chain.  Against 64 bits an fp32 state is off by 2.6e-7 instead of 2.9e-7 after 1500 tokens of weak decay, 1.2e-7 instead of
-// 3.4e-7 without decay, 5.7e-8 instead of 5.8e-8 with a strong one (d=128, relative 2-norm).
+// cycles), sums and a triangular solve (850) and the update (500): B=2, T=1500, 8 v-heads, d=256 996 -> 233 us (253 with the
+// outputs written by the warps that hold the state, another 400 cycles of the chain), 4 v-heads B=1 994 -> 151, T=700, d=192
+// 401 -> 71, T=65 42 -> 12.7; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM the matrix instructions set the pace
+// (16 cycles each, 84 per scheduler, block and CTA: 2 700 of 4 000 cycles), with one the chain.  Against 64 bits an fp32 state
+// is off by 2.6e-7 instead of 2.9e-7 after 1500 tokens of weak decay, 1.2e-7 instead of 3.4e-7 without decay, 5.7e-8 instead of
+// 5.8e-8 with a strong one (d=128, relative 2-norm).
 //
 // A CTA owns 16 state rows (M of the products) of one (sequence, v-head) and walks its blocks:
 //   warps 0-3   a quarter of the columns each, kept as accumulator fragments, which are the A operands of the product
 //               S_0 [k; q]^T as they lie.  The four partial products meet in shared memory; then EVERY warp sums them and
 //               solves for c (lane r + 16 h: row r, tokens 8 h .. 8 h + 7), which costs less than a second barrier and a
-//               trip through shared memory, and updates its own columns.  Each warp writes a quarter of the tokens' outputs.
+//               trip through shared memory, and updates its own columns.
 //   warps 4-7   prepare blocks in turn (warp 4 + j: blocks j, j + 4, ..), up to four ahead: copies of k, q, v, the Gram matrices
-//               k k^T and q k^T on matrix instructions, decay products, norms, and from them the matrices A and P.
+//               k k^T and q k^T on matrix instructions, decay products, norms, and from them the matrices A and P; when a
+//               block is through they write its outputs.
 //               (Four of them, so that their work is spread over the four schedulers.)
 // Two CTAs per SM at dk = 256: one's chain fills the gaps of the other.
 #pragma once
@@ -45,6 +47,9 @@ struct BlockSmem {
     static constexpr int kOffQ = kBlkTok * kRow, kOffV = 2 * kBlkTok * kRow;
     static constexpr int kStage = kOffV + kBlkTok * kBlkRows * 2;
     static constexpr int kStages = 4;  // one per preparing warp
+    // over q once its products are there: what the outputs are made of, scale G_t (S_0 q_t) and c, 16 rows of 16 tokens each
+    static constexpr int kOffO = kOffQ, kOffC1 = kOffQ + kBlkRows * kBlkTok * 4;
+    static_assert(kOffC1 + kBlkRows * kBlkTok * 4 <= kOffV, "they fit over q");
     // what a block's solve needs, floats: A as [s][t], P as [t][s], beta v as [row][t] (before that: decay products), factors
     static constexpr int kA = 0, kP = 256, kR0 = 512, kLdR = 20, kCk = kR0 + 16 * kLdR, kCq = kCk + 16, kW = kCq + 16, kG = kW + 16;
     static constexpr int kPrepFloats = kG + 4;
@@ -89,6 +94,8 @@ __device__ __forceinline__ void mma16f(float* d, const uint32_t* a, uint32_t b0,
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes below 16: zeros for the rest
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
 }
+// 16-byte piece `c` of row `r` of such a 16 x 16 fp32 tile: eight rows of a piece lie in different banks
+__device__ __forceinline__ uint32_t piece_off(int r, int c) { return static_cast<uint32_t>(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 // this thread's arrival at `bar` once all its copies so far have landed
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -104,7 +111,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     constexpr int NK = DK / 64;  // K-steps of 16 columns per warp
     static_assert(DK % 64 == 0, "four warps with whole K-steps each");
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ uint64_t full[4], ready[4], done[4];  // k, q, v have landed / the block is prepared / its buffers have been read
+    __shared__ uint64_t full[4], ready[4], done[4];  // k, q, v have landed / the block is prepared / it is through
     __shared__ int abort_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -141,7 +148,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     auto prep_of = [&](int b) { return reinterpret_cast<float*>(smem + L::kOffPrep) + (b & 3) * L::kPrepFloats; };
 
     if (warp >= 4) {
-        // =============================================================== preparation
+        // =============================================================== preparation and outputs
         const int j = warp - 4;
         uint8_t* const st = smem + j * L::kStage;
         float* const pr = prep_of(j);
@@ -149,6 +156,8 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         const __nv_bfloat16* const kp = p.k + bidx * p.k_sb + tok0 * p.k_st + khead * p.k_sh;
         const __nv_bfloat16* const qp = p.q + bidx * p.q_sb + tok0 * p.q_st + khead * p.q_sh;
         const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * kBlkRows;
+        const int r = lane & 15, h = lane >> 4;  // for the outputs: row r, tokens 8 h .. 8 h + 7
+        __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
         float al = 0.f, db = 0.f;
         if (p.fused_gating) {
             al = __expf(from_bits(ld_bits(p.A_log, p.gating_param_f32, head), p.gating_param_f32));
@@ -164,11 +173,24 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             }
         };
         fetch(j);
-        for (int b = j; b < nblk; b += 4) {
+        for (int b = j; b < nblk + 4; b += 4) {
             const uint32_t it = static_cast<uint32_t>(b >> 2);
-            if (b >= 4 && !mbar_wait(&done[j], (it - 1) & 1u, &abort_flag)) break;
+            const bool next = b < nblk;
             const int n = min(kBlkTok, ntok - b * kBlkTok);
-            {
+            float o[8], c0[8], c1[8];
+            if (b >= 4) {  // block b - 4 is through: what its outputs are made of
+                if (!mbar_wait(&done[j], (it - 1) & 1u, &abort_flag)) break;
+                auto row8 = [&](int off, int c, float* x) {
+                    const float4 u = *reinterpret_cast<const float4*>(st + off + piece_off(r, c));
+                    const float4 w = *reinterpret_cast<const float4*>(st + off + piece_off(r, c + 1));
+                    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
+                };
+                row8(L::kOffO, 2 * h, o);
+                row8(L::kOffC1, 0, c0);
+                row8(L::kOffC1, 2, c1);
+                __syncwarp();
+            }
+            if (next) {
                 // rows past the end of the sequence are filled with zeros (their address is that of the last row)
                 constexpr int kPieces = DK / 8;
                 const uint32_t dst = smem_u32(st);
@@ -187,6 +209,32 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 }
                 cp_async_arrive(&full[j]);
             }
+            if (b >= 4) {
+                // ---- outputs of block b - 4.  Coefficients of later tokens are left out, not multiplied by zero: an infinite or
+                //      undefined value stays behind its token.
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float* const P = pr + L::kP + (8 * h + i) * 16;
+                    const float4 u = *reinterpret_cast<const float4*>(P), w = *reinterpret_cast<const float4*>(P + 4);
+                    const float pw[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int s = 0; s < 8; ++s)
+                        if (s <= i || h) o[i] = fmaf(pw[s], c0[s], o[i]);
+                    if (h) {
+                        const float4 y = *reinterpret_cast<const float4*>(P + 8), z = *reinterpret_cast<const float4*>(P + 12);
+                        const float pz[8] = {y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+#pragma unroll
+                        for (int s = 0; s <= i; ++s) o[i] = fmaf(pz[s], c1[s], o[i]);
+                    }
+                }
+                __syncwarp();
+                if (*static_cast<volatile int*>(&abort_flag)) break;  // nothing is stored once a wait has given up
+                const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
+            }
+            if (!next) break;
             // ---- scalars; tokens past the end: beta 0, decay 1
             float beta = from_bits(b_next, p.beta_f32), gate = from_bits(g_next, p.gate_f32);
             if (p.fused_gating) {
@@ -328,14 +376,16 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
 #pragma unroll
             for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
         }
-        __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
         uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
         bool ok = true;  // false once a wait has given up: nothing is stored from then on
+        bool ahead = false;  // this lane has seen the next block's preparation complete
         for (int b = 0; b < nblk; ++b) {
-            ok = mbar_wait(&ready[b & 3], static_cast<uint32_t>((b >> 2) & 1), &abort_flag) && ok;
+            ok = (ahead || mbar_wait(&ready[b & 3], static_cast<uint32_t>((b >> 2) & 1), &abort_flag)) && ok;
+            __syncwarp();
             const int n = min(kBlkTok, ntok - b * kBlkTok);
+            uint8_t* const st = smem + (b & 3) * L::kStage;
             const float* const pr = prep_of(b);
-            const uint32_t kaddr = smem_u32(smem + (b & 3) * L::kStage) + lm_row * L::kRow + (col0 + lm_col) * 2;
+            const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + (col0 + lm_col) * 2;
             float* const D = reinterpret_cast<float*>(smem + L::kOffD) + (b & 1) * (4 * kBlkRows * L::kLdD);
             // ---- this warp's columns of S_0 [k; q]^T: tokens 0 - 7 and 8 - 15 of k, then of q.  The first terms have sums of their own:
             //      they are the long ones, and the chains are shorter.
@@ -493,39 +543,21 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     }
                 }
             }
-            // ---- outputs of row r, tokens 4 warp + 2 h and the next.  Coefficients of later tokens are left out, not multiplied by
-            //      zero: an infinite or undefined value stays behind its token.
+            // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t), and c
             {
-                float c1[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) c1[i] = __shfl_sync(0xffffffffu, c[i], r + 16);
-                const int t0 = 4 * warp + 2 * h;
-                const float* const d = D + r * L::kLdD + 16 + t0;
+                const int i = 32 * warp + lane, row = i >> 3, t2 = 2 * (i & 7);
+                const float* const d = D + row * L::kLdD + 16 + t2;
                 float2 x[4];
 #pragma unroll
                 for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
-                const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t0);
-                float o0 = cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), o1 = cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y));
-                const float* const P = pr + L::kP + t0 * 16;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (q > warp) break;
-                    const float4 pa = *reinterpret_cast<const float4*>(P + 4 * q), pb = *reinterpret_cast<const float4*>(P + 16 + 4 * q);
-                    const float* const cc = (q < 2 ? c0 : c1) + 4 * (q & 1);
-                    o0 = fmaf(pa.x, cc[0], o0);
-                    o1 = fmaf(pb.x, cc[0], o1);
-                    o1 = fmaf(pb.y, cc[1], o1);
-                    if (q < warp || h) {  // q == warp: tokens 4 q + 2 h and + 1
-                        o0 = fmaf(pa.y, cc[1], o0);
-                        o0 = fmaf(pa.z, cc[2], o0);
-                        o1 = fmaf(pb.z, cc[2], o1);
-                        o1 = fmaf(pb.w, cc[3], o1);
-                    }
-                    if (q < warp) o0 = fmaf(pa.w, cc[3], o0);
+                const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
+                ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
+                *reinterpret_cast<float2*>(st + L::kOffO + piece_off(row, t2 >> 2) + 4 * (t2 & 2)) =
+                    make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
+                if (warp == (b & 3)) {
+                    *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
+                    *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
                 }
-                const long long i = static_cast<long long>(b) * kBlkTok + t0;
-                if (ok && t0 < n) out[i * p.o_st] = __float2bfloat16(o0);
-                if (ok && t0 + 1 < n) out[(i + 1) * p.o_st] = __float2bfloat16(o1);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[b & 3]);
