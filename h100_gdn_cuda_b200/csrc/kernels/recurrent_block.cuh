@@ -14,8 +14,9 @@
 // few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of products (1 000
 // cycles), sums and a triangular solve (850) and the update (500): B=2, T=1500, 8 v-heads, d=256 996 -> 233 us (253 with the
 // outputs written by the warps that hold the state, another 400 cycles of the chain), 4 v-heads B=1 994 -> 151, T=700, d=192
-// 401 -> 71, T=65 42 -> 12.7; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM the matrix instructions set the pace
-// (16 cycles each, 84 per scheduler, block and CTA: 2 700 of 4 000 cycles), with one the chain.  Against 64 bits an fp32 state
+// 401 -> 71, T=65 42 -> 12.7; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM issue
+// (5 100 warp instructions per block and CTA, 54 % of the slots), shared memory (1 270 wavefronts, as much) and the matrix
+// instructions (26 %) share the time without one of them filling it; with one CTA the chain does.  Against 64 bits an fp32 state
 // is off by 2.6e-7 instead of 2.9e-7 after 1500 tokens of weak decay, 1.2e-7 instead of 3.4e-7 without decay, 5.7e-8 instead of
 // 5.8e-8 with a strong one (d=128, relative 2-norm).
 //
