@@ -24,9 +24,10 @@
 // lie; A and the inverses are B operands in shared memory.  All of them enter the products as two bf16 terms (16
 // significand bits; a doubling scheme on TF32, 11 bits, was here before).
 // What bounds it: the latency of a unit's dependent phases (11 200 cycles with four teams per SM, 8 700 with two; before
-// 12 100).  The doubling scheme had ten barriers per unit (five now), 5 660 warp instructions and 1 808 wavefronts of
+// 12 100).  The doubling scheme had ten barriers per unit (five now), 5 660 warp instructions (4 990) and 1 808 wavefronts (1 220) of
 // shared-memory accesses, besides some 900 of MMA operands and copies, of the 3 000 cycles a unit took an SM.
-// B=4 T=4096, 32 v-heads, whole step 214.7 -> 204.0 us; 16 packed sequences of 32768 tokens 458 -> 423; B=2 T=131072, 4 v-heads 618 -> 578.
+// B=4 T=4096, 32 v-heads, whole step 200.1 -> 194.8 us; 16 packed sequences of 32768 tokens 427 -> 403; B=2 T=131072, 4 v-heads 592 ->
+// 572 (one GPU).
 // Persistent CTAs, two per SM (111 KB of shared memory, 256 tensor-memory columns each).
 #pragma once
 #include <cuda.h>
