@@ -95,6 +95,7 @@ __device__ __forceinline__ void mma16f(float* d, const uint32_t* a, uint32_t b0,
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes below 16: zeros for the rest
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // 16-byte piece `c` of row `r` of such a 16 x 16 fp32 tile: eight rows of a piece lie in different banks
 __device__ __forceinline__ uint32_t piece_off(int r, int c) { return static_cast<uint32_t>(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 // this thread's arrival at `bar` once all its copies so far have landed
@@ -174,13 +175,16 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             }
         };
         fetch(j);
+        // false once a wait has given up.  Every lane polls for itself and the answers of two lanes can differ, so the loop is walked to its end: a
+        // warp whose lanes parted here would hang in its next shuffle.
+        bool ok = true;
         for (int b = j; b < nblk + 4; b += 4) {
             const uint32_t it = static_cast<uint32_t>(b >> 2);
             const bool next = b < nblk;
             const int n = min(kBlkTok, ntok - b * kBlkTok);
             float o[8], c0[8], c1[8];
             if (b >= 4) {  // block b - 4 is through: what its outputs are made of
-                if (!mbar_wait(&done[j], (it - 1) & 1u, &abort_flag)) break;
+                ok = mbar_wait(&done[j], (it - 1) & 1u, &abort_flag) && ok;
                 auto row8 = [&](int off, int c, float* x) {
                     const float4 u = *reinterpret_cast<const float4*>(st + off + piece_off(r, c));
                     const float4 w = *reinterpret_cast<const float4*>(st + off + piece_off(r, c + 1));
@@ -229,11 +233,11 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     }
                 }
                 __syncwarp();
-                if (*static_cast<volatile int*>(&abort_flag)) break;  // nothing is stored once a wait has given up
+                const bool good = ok && *static_cast<volatile int*>(&abort_flag) == 0;  // nothing is stored once a wait has given up
                 const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    if (i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
+                    if (good && i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
             }
             if (!next) break;
             // ---- scalars; tokens past the end: beta 0, decay 1
@@ -255,7 +259,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 if (lane == 16 || lane < i) run *= ai;
                 if (lane <= 16) X[i * L::kLdR + lane] = run;  // (entries s > t are not used)
             }
-            if (!mbar_wait(&full[j], it & 1u, &abort_flag)) break;  // not handed on: the other warps' waits end with it
+            ok = mbar_wait(&full[j], it & 1u, &abort_flag) && ok;
             // ---- Gram matrices.  kk, qk: tokens 0 .. 15 against tokens 0 .. 7 of k; hh: tokens 8 .. 15 of k and of q against tokens
             //      8 .. 15 of k; qq: the diagonals of q q^T.  The matrix instructions cut their sums off, so only two follow one another.
             float kk[4] = {}, qk[4] = {}, hh[4] = {}, qq0[4] = {}, qq1[4] = {};
@@ -348,7 +352,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&ready[j]);
+            if (lane == 0 && ok) mbar_arrive(&ready[j]);  // not handed on once a wait has given up: the other warps' waits end with it
         }
     } else {
         // =============================================================== state
@@ -563,7 +567,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[b & 3]);
         }
-        if (ok) {
+        if (ok && *static_cast<volatile int*>(&abort_flag) == 0) {
             const long long base = static_cast<long long>(slot) * p.so_ss + head * p.so_sh + srow;
 #pragma unroll
             for (int i = 0; i < 2 * NK; ++i) {
@@ -578,7 +582,10 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         }
     }
     __syncthreads();
-    if (tid == 0 && abort_flag && p.status) atomicExch(p.status, 1);
+    if (abort_flag) {
+        cp_async_wait_all();  // the copies whose wait gave up
+        if (tid == 0 && p.status) atomicExch(p.status, 1);
+    }
 }
 
 template <int DK, bool kF32 = false>
