@@ -169,32 +169,56 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
     return GDN_OK;
 }
 
-// Long runs of tokens whose last state alone is wanted: blocks of tokens on warp matrix instructions (recurrent_block.cuh),
-// unless the runs are but little longer than a block and the CTAs are many: a second block with few tokens takes as long as a
-// full one, and the token recurrence fills the GPU then.  Token recurrence against this in us: 32 v-heads, d=128, T=20 / 22 / 24 B=64 365 / 401
-// / 431 : 395 / 400 / 403, B=20 121 / 132 / 142 : 125 / 126 / 127, B=8 55 / 60 / 64 : 51 / 52 / 52, T=17 B=1 (one wave of CTAs)
-// 14 : 8; d=64, T=28 / 32 / 40 B=64 159 / 179 / 223 : 175 / 173 / 210, B=16 48 / 53 / 66 : 46 / 45 / 55; 8 v-heads, d=256, T=20 / 24 / 32
-// B=64 236 / 276 / 360 : 259 / 261 / 261.
-static bool block_takes(const GdnShape& s, bool steps, int sms) {
-    if (steps || (s.head_dim_k != 64 && s.head_dim_k != 128 && s.head_dim_k != 192 && s.head_dim_k != 256)) return false;
-    const long long tokens = s.cu_seqlens ? s.total_tokens : static_cast<long long>(s.seq_len) * s.batch;
-    const long long ctas = static_cast<long long>(s.batch) * s.num_v_heads * (s.head_dim_v / kBlkRows);
-    return ctas <= 2ll * sms || tokens >= (s.head_dim_k == 64 ? 31ll : 23ll) * s.batch;
+// Long runs of tokens whose last state alone is wanted: blocks of tokens on warp matrix instructions (recurrent_block.cuh) from
+// this many tokens on.  The sums go in another order there, so the choice is made by what belongs to the sequence - its tokens
+// (before any cap), head dim, state type - and not by the batch, the heads or the other sequences: a sequence, or a shard's heads,
+// come out with the same bits alone and in company.  A second block with few tokens takes as long as a full one, and where the CTAs
+// fill the GPU the token recurrence is no slower up to here.  Token recurrence against blocks in us, B=64, L2 flushed: 32 v-heads
+// d=64 T=33 184 : 212, T=39 208 : 212, T=41 216 : 212 (fp32 states 185 : 213, 209 : 214, 217 : 212); d=128 T=23 385 : 397, T=25 414 : 395
+// (fp32 386 : 399, 414 : 398); 8 v-heads d=192 T=23 164 : 185, T=25 176 : 184, T=27 188 : 184 (B=8 the same at T=27); d=256 T=23 259 : 259.
+// With few CTAs the blocks would win earlier (B=1 d=128 T=17 14 us : 8).  Packed batches hold both kinds and take two launches, each
+// of which leaves the other's sequences out: 16 sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336, 8 of about 100 (32
+// v-heads, d=128) 113 -> 118; one of 1500 among 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31.
+static int block_min_tokens(int dk, bool f32, bool steps, int ring_min) {
+    if (steps || (f32 && dk != 64 && dk != 128)) return kRecNoLongRun;
+    const int from = dk == 64 ? 41 : dk == 128 ? 25 : dk == 192 ? 27 : dk == 256 ? 23 : kRecNoLongRun;
+    return std::max(from, ring_min < kRecNoLongRun ? ring_min + 1 : kRecNoLongRun);
 }
-template <int DK, bool kF32 = false>
-static int launch_block_t(const RecurrentParams& p, cudaStream_t st) {
+template <int DK, bool kF32, BlkUnits kUnits>
+static int launch_block_t(const RecurrentParams& p, long long grid, cudaStream_t st) {
     constexpr int smem = BlockSmem<DK>::kBytes;
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     GDN_CUDA(cudaGetDevice(&dev));
     if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kF32, kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev & 63].store(true, std::memory_order_release);
     }
-    const long long grid = static_cast<long long>(p.batch) * p.vh * (p.dv / kBlkRows);
     GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
-    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kF32>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
+    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kF32, kUnits>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
     return GDN_OK;
+}
+template <BlkUnits kUnits>
+static int launch_block_as(const RecurrentParams& p, int dk, bool f32, long long grid, cudaStream_t st) {
+    switch (f32 ? -dk : dk) {
+        case 64: return launch_block_t<64, false, kUnits>(p, grid, st);
+        case 128: return launch_block_t<128, false, kUnits>(p, grid, st);
+        case 192: return launch_block_t<192, false, kUnits>(p, grid, st);
+        case 256: return launch_block_t<256, false, kUnits>(p, grid, st);
+        case -64: return launch_block_t<64, true, kUnits>(p, grid, st);
+        case -128: return launch_block_t<128, true, kUnits>(p, grid, st);
+    }
+    return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: no token-block kernel for dk = %d", dk);
+}
+// Packed mode: no more than total_tokens / long_run sequences can be that long.  Where that is all of them, a CTA per unit, as for
+// padded batches; otherwise a wave of CTAs walks the units (100 sequences of one token and one of 1500, d=256: 69 times the CTAs
+// there is work for).  The walk itself costs registers (d=256: 260 bytes spilled, 20 % of the time).
+static int launch_block(const RecurrentParams& p, int dk, bool f32, long long total_tokens, int sms, cudaStream_t st) {
+    const long long per_seq = static_cast<long long>(p.vh) * (p.dv / kBlkRows);
+    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, f32, p.batch * per_seq, st);
+    const long long seqs = total_tokens / p.long_run;
+    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, f32, p.batch * per_seq, st);
+    return launch_block_as<BlkUnits::kWalk>(p, dk, f32, std::min(seqs * per_seq, 2ll * sms), st);
 }
 
 // Head dimensions without a prebuilt kernel (or every call when GDN_JIT_RECURRENT=1) go through
@@ -532,32 +556,33 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     const int slots_per_sm = s.head_dim_k > 128 ? 2 : (a->state_dtype == GDN_F32 && s.head_dim_k > 64 ? 3 : 4);
     if (!ring && !s.cu_seqlens && s.seq_len == 1) p.split_tiles = p.num_tiles <= static_cast<long long>(d->sms) * slots_per_sm;
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
-    if (force_jit && a->state_dtype != GDN_F32) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
-    if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
-    if (ring && block_takes(s, p.store_step != 0, d->sms)) {
-        switch (s.head_dim_k * (a->state_dtype == GDN_F32 ? -1 : 1)) {
-            case 64: return launch_block_t<64>(p, st);
-            case 128: return launch_block_t<128>(p, st);
-            case 192: return launch_block_t<192>(p, st);
-            case 256: return launch_block_t<256>(p, st);
-            case -64: return launch_block_t<64, true>(p, st);
-            case -128: return launch_block_t<128, true>(p, st);
+    const bool f32 = a->state_dtype == GDN_F32;
+    const bool jit = force_jit && !f32;
+    p.long_run = jit ? kRecNoLongRun : block_min_tokens(s.head_dim_k, f32, p.store_step != 0, ring_min);
+    // (packed: no more tokens than sequences is a batch of single tokens)
+    if (s.cu_seqlens ? s.total_tokens < p.long_run || s.total_tokens <= s.batch : s.seq_len < p.long_run) p.long_run = kRecNoLongRun;
+    if (p.long_run != kRecNoLongRun && !s.cu_seqlens) return launch_block(p, s.head_dim_k, f32, 0, d->sms, st);
+    auto token_recurrence = [&]() -> int {
+        if (jit) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
+        if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
+        if (f32) {
+            // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
+            if (s.head_dim_k == 128) return launch_recurrent_f32<128>(p, d->sms, st, ring);
+            if (s.head_dim_k == 64) return launch_recurrent_f32<64>(p, d->sms, st, ring);
+            return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: fp32 states are built for dk = 64 and 128 (got %d)", s.head_dim_k);
         }
-    }
-    if (a->state_dtype == GDN_F32) {
-        // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
-        if (s.head_dim_k == 128) return launch_recurrent_f32<128>(p, d->sms, st, ring);
-        if (s.head_dim_k == 64) return launch_recurrent_f32<64>(p, d->sms, st, ring);
-        return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: fp32 states are built for dk = 64 and 128 (got %d)", s.head_dim_k);
-    }
-    const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx && !p.split_tiles;
-    switch (s.head_dim_k) {
-        case 64: return launch_recurrent<64>(p, d->sms, st, ring, lean);
-        case 128: return launch_recurrent<128>(p, d->sms, st, ring, lean);
-        case 192: return launch_recurrent<192>(p, d->sms, st, ring, lean);
-        case 256: return launch_recurrent<256>(p, d->sms, st, ring, lean);
-    }
-    return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring);  // 320 .. 512: compiled on first use
+        const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx && !p.split_tiles;
+        switch (s.head_dim_k) {
+            case 64: return launch_recurrent<64>(p, d->sms, st, ring, lean);
+            case 128: return launch_recurrent<128>(p, d->sms, st, ring, lean);
+            case 192: return launch_recurrent<192>(p, d->sms, st, ring, lean);
+            case 256: return launch_recurrent<256>(p, d->sms, st, ring, lean);
+        }
+        return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring);  // 320 .. 512: compiled on first use
+    };
+    if (int rc = token_recurrence()) return rc;
+    // packed: the sequences that launch has left out
+    return p.long_run == kRecNoLongRun ? GDN_OK : launch_block(p, s.head_dim_k, f32, s.total_tokens, d->sms, st);
 }
 
 }  // extern "C"

@@ -18,9 +18,9 @@
 // The eight row sums are reduced over 16 lanes with a transposing butterfly (8 shuffles
 // instead of 32).  For single-token decode q/k normalisation and k.q are computed once per
 // unit, not per tile.  New states leave through coalesced 8-byte stores from registers.
-// Long runs of tokens take recurrent_block.cuh, or where that is no better, or a state per token is wanted, a second
-// instance of the kernel (kRing), chosen by the host when the sequences average more than
-// kRecTokRingMin tokens: every tile is a work unit of its own, so that a few long sequences
+// Runs of many tokens take recurrent_block.cuh (in packed batches those sequences are left out here, RecurrentParams::long_run).
+// Runs of more than kRecTokRingMin tokens (packed: on average) that are not that long, or want a state per token, take a second
+// instance of the kernel (kRing) with the same arithmetic: every tile is a work unit of its own, so that a few long sequences
 // still spread over all CTAs, and k, q, v arrive 8 tokens at a time by bulk copies: the first
 // block with the tile's stage, the others through a two-slot ring.  (With one token fetched ahead
 // of the one in work, as the decode instance does for its few tokens, every token paid the whole
@@ -59,6 +59,7 @@ struct RecurrentParams {
     const void* A_log;
     const void* dt_bias;
     int split_tiles;  // 1: every 32-row tile is a work unit (ring instance; small decode batches: the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
+    int long_run;  // packed mode: sequences of at least this many tokens are recurrent_block.cuh's, in a launch of their own; shorter ones this kernel's
     long long num_tiles;
     int* status;
 };
@@ -69,6 +70,7 @@ constexpr int kRecStagesRing = 2;  // in the multi-token instance a tile lasts f
 constexpr int kRecThreads = 128;
 constexpr int kRecTokBlock = 8;     // tokens per slot of the multi-token ring
 constexpr int kRecTokRingMin = 16;  // sequences longer than this use it
+constexpr int kRecNoLongRun = 0x7fffffff;  // RecurrentParams::long_run: every sequence of the batch is gdn_recurrent_kernel's
 
 // One ring stage: the 32 x DK state tile, then k and q (DK bf16 each) and the 32 entries of v that
 // belong to the tile's rows, for the unit's first token (decode instance) or its first
@@ -181,6 +183,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     using ST = typename StateElem<kF32>::type;
     const ST* const state_in = static_cast<const ST*>(p.state_in);
     ST* const state_out = static_cast<ST*>(p.state_out);
+    constexpr bool kSkips = !kLean && !kSplit;  // (those run padded batches)
     constexpr int NQ = DK / 32;  // packed pairs per row per lane (lane owns 4 columns of every 64)
     extern __shared__ __align__(128) uint8_t smem[];
     using TokSlot = RecTokSlot<DK>;
@@ -213,6 +216,9 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     // The kernel is launched as a programmatic dependent of the preceding work in the stream: its CTAs are placed
     // while that work drains and wait here, before the first access to global memory (a no-op for an ordinary launch).
     grid_dep_wait();
+    // Packed runs some of which are the token-block kernel's: it is launched behind this one, may start now (what precedes this launch
+    // is complete) and works on other sequences.
+    if (kSkips && p.long_run != kRecNoLongRun) grid_dep_launch();
     if (p.fused_gating) {
         for (int h = threadIdx.x; h < min(p.vh, kGateTable); h += blockDim.x) {
             s_alog[h] = p.gating_param_f32 ? __ldg(reinterpret_cast<const float*>(p.A_log) + h)
@@ -254,10 +260,12 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
             t.head = sh - t.seq * p.vh;
         }
         t.khead = rep_shift >= 0 ? (t.head >> rep_shift) : (t.head / rep);
+        bool other = false;  // packed: a sequence of another launch
         if (p.cu_seqlens) {
             t.tok0 = p.cu_seqlens[t.seq];
             t.ntok = p.cu_seqlens[t.seq + 1] - static_cast<int>(t.tok0);
             t.bidx = 0;
+            other = kSkips && t.ntok >= p.long_run;
         } else {
             t.tok0 = 0;
             t.ntok = p.seq_len;
@@ -269,6 +277,10 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
             t.slot = p.state_idx[t.seq];
             if (t.slot < 0) t.ntok = 0;
         }
+        if (other) {
+            t.slot = -1;
+            t.ntok = 0;
+        }
         return t;
     };
     // Producer (one thread): everything tile `rb` of `unit` needs for its first token.
@@ -278,7 +290,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     const __nv_bfloat16* prod_q = nullptr;
     const __nv_bfloat16* prod_v = nullptr;
     auto producer_bases = [&](const Unit& t) {
-        prod_s = has_in ? state_in + static_cast<long long>(max(t.slot, 0)) * p.si_ss + t.head * p.si_sh : nullptr;
+        prod_s = has_in && (!kSkips || t.slot >= 0) ? state_in + static_cast<long long>(max(t.slot, 0)) * p.si_ss + t.head * p.si_sh : nullptr;
         prod_k = p.k + t.bidx * p.k_sb + t.tok0 * p.k_st + t.khead * p.k_sh;
         prod_q = p.q + t.bidx * p.q_sb + t.tok0 * p.q_st + t.khead * p.q_sh;
         prod_v = p.v + t.bidx * p.v_sb + t.tok0 * p.v_st + t.head * p.v_sh;
@@ -286,9 +298,10 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     auto issue = [&](const Unit& t, int rb, int stage) {
         uint8_t* dst = smem + stage * Stage::kBytes;
         const int nt0 = min(t.ntok, Stage::kTok);  // tokens whose k, q, v travel with the tile
-        const uint32_t bytes = (has_in ? Stage::kTileBytes : 0) + static_cast<uint32_t>(nt0) * (4 * DK + kRecTileRows * 2);
+        const bool tile = kSkips ? prod_s != nullptr : has_in;
+        const uint32_t bytes = (tile ? Stage::kTileBytes : 0) + static_cast<uint32_t>(nt0) * (4 * DK + kRecTileRows * 2);
         mbar_arrive_expect_tx(&full[stage], bytes);
-        if (has_in) bulk_load(dst, prod_s + rb * (kRecTileRows * DK), Stage::kTileBytes, &full[stage]);
+        if (tile) bulk_load(dst, prod_s + rb * (kRecTileRows * DK), Stage::kTileBytes, &full[stage]);
         for (int i = 0; i < nt0; ++i) {
             bulk_load(dst + Stage::kOffK + i * DK * 2, prod_k + i * p.k_st, DK * 2, &full[stage]);
             bulk_load(dst + Stage::kOffQ + i * DK * 2, prod_q + i * p.q_st, DK * 2, &full[stage]);

@@ -102,10 +102,33 @@ __device__ __forceinline__ uint32_t piece_off(int r, int c) { return static_cast
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The `rank`-th packed sequence of at least `min_run` tokens, or -1.  All lanes of a warp.
+__device__ __forceinline__ int long_sequence(const int* cu_seqlens, int batch, int min_run, int rank) {
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < batch; s0 += 32) {
+        const int s = s0 + lane;
+        unsigned m = __ballot_sync(0xffffffffu, s < batch && cu_seqlens[s + 1] - cu_seqlens[s] >= min_run);
+        const int c = __popc(m);
+        if (rank < c) {
+            for (; rank > 0; --rank) m &= m - 1;
+            return s0 + __ffs(m) - 1;
+        }
+        rank -= c;
+    }
+    return -1;
+}
 }  // namespace blk
 
-template <int DK, bool kF32>
+// Packed sequences: this launch takes those of at least p.long_run tokens, the others are gdn_recurrent_kernel's (decided per sequence,
+// so that a sequence has the same bits whatever it is packed with).  How many there are is known here alone.
+enum class BlkUnits {
+    kPadded,  // a CTA per unit
+    kPacked,  // a CTA per unit of as many sequences as can be that long; those past the last one end at once
+    kWalk,    // packed, far fewer long sequences than could be: a wave of CTAs walks the units with a stride of the grid
+};
+template <int DK, bool kF32, BlkUnits kUnits = BlkUnits::kPadded>
 __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& p) {
+    constexpr bool kPacked = kUnits != BlkUnits::kPadded;
     using namespace ptx;
     using namespace step;
     using namespace blk;
@@ -117,470 +140,515 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     __shared__ int abort_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    if (tid == 0) {
-        abort_flag = 0;
+    auto init_barriers = [&]() {
         for (int i = 0; i < 4; ++i) {
             mbar_init(&full[i], 32);
             mbar_init(&ready[i], 1);
             mbar_init(&done[i], 4);
         }
         mbar_fence_init();
+    };
+    if (tid == 0) {
+        abort_flag = 0;
+        init_barriers();
     }
     __syncthreads();
-    // a programmatic dependent of the work before it; every kernel launched that way waits for the whole of its predecessor
-    grid_dep_wait();
-    grid_dep_launch();
+    // a programmatic dependent of the work before it; every kernel launched that way waits for the whole of its predecessor.  (Packed:
+    // what precedes this launch is gdn_recurrent_kernel on the batch's other sequences.  It lets this one start when everything
+    // before is complete, so only the end has to wait, for whoever waits for this grid; and that one is not let in early, its CTAs
+    // would settle unevenly around those that wait here: 64 sequences of 4 tokens 56.8 -> 61.0 us.)
+    if (!kPacked) {
+        grid_dep_wait();
+        grid_dep_launch();
+    }
 
     const int rblocks = p.dv / kBlkRows;
-    const int unit = static_cast<int>(blockIdx.x) / rblocks, rb = static_cast<int>(blockIdx.x) - unit * rblocks;
-    const int seq = unit / p.vh, head = unit - seq * p.vh, khead = head / (p.vh / p.kh);
-    long long tok0 = 0, bidx = seq;
-    int ntok = p.seq_len;
-    if (p.cu_seqlens) {
-        tok0 = p.cu_seqlens[seq];
-        ntok = p.cu_seqlens[seq + 1] - static_cast<int>(tok0);
-        bidx = 0;
-    }
-    if (p.num_accepted) ntok = min(ntok, p.num_accepted[seq]);
-    const int slot = p.state_idx ? p.state_idx[seq] : seq;
-    if (slot < 0) return;  // padding sequence: no tokens, no state
-    const int nblk = ntok > 0 ? (ntok + kBlkTok - 1) / kBlkTok : 0;
-    // ldmatrix: lane l addresses row l & 7 of 8x8 matrix l >> 3; matrices 1 and 3 are rows 8 .. 15, matrices 2 and 3 columns 8 .. 15
-    const int lm_row = lane & 15, lm_col = 8 * (lane >> 4);
-    auto prep_of = [&](int b) { return reinterpret_cast<float*>(smem + L::kOffPrep) + (b & 3) * L::kPrepFloats; };
+    auto run = [&](int seq, int head, int rb) {
+        const int khead = head / (p.vh / p.kh);
+        long long tok0 = 0, bidx = seq;
+        int ntok = p.seq_len;
+        if (kPacked) {
+            tok0 = p.cu_seqlens[seq];
+            ntok = p.cu_seqlens[seq + 1] - static_cast<int>(tok0);
+            bidx = 0;
+        }
+        if (p.num_accepted) ntok = min(ntok, p.num_accepted[seq]);
+        const int slot = p.state_idx ? p.state_idx[seq] : seq;
+        if (slot < 0) return;  // padding sequence: no tokens, no state
+        const int nblk = ntok > 0 ? (ntok + kBlkTok - 1) / kBlkTok : 0;
+        // ldmatrix: lane l addresses row l & 7 of 8x8 matrix l >> 3; matrices 1 and 3 are rows 8 .. 15, matrices 2 and 3 columns 8 .. 15
+        const int lm_row = lane & 15, lm_col = 8 * (lane >> 4);
+        auto prep_of = [&](int b) { return reinterpret_cast<float*>(smem + L::kOffPrep) + (b & 3) * L::kPrepFloats; };
 
-    if (warp >= 4) {
-        // =============================================================== preparation and outputs
-        const int j = warp - 4;
-        uint8_t* const st = smem + j * L::kStage;
-        float* const pr = prep_of(j);
-        float* const X = pr + L::kR0;  // [t][s] = Gamma_ts, [t][16] = G_t, [t][17], [t][18] = inverse norms of k_t, q_t
-        const __nv_bfloat16* const kp = p.k + bidx * p.k_sb + tok0 * p.k_st + khead * p.k_sh;
-        const __nv_bfloat16* const qp = p.q + bidx * p.q_sb + tok0 * p.q_st + khead * p.q_sh;
-        const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * kBlkRows;
-        const int r = lane & 15, h = lane >> 4;  // for the outputs: row r, tokens 8 h .. 8 h + 7
-        __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
-        float al = 0.f, db = 0.f;
-        if (p.fused_gating) {
-            al = __expf(from_bits(ld_bits(p.A_log, p.gating_param_f32, head), p.gating_param_f32));
-            db = from_bits(ld_bits(p.dt_bias, p.gating_param_f32, head), p.gating_param_f32);
-        }
-        uint32_t b_next = 0u, g_next = 0u;  // bits of beta and the gate (or of the raw projections) of token `lane` of the next block
-        auto fetch = [&](int b) {
-            b_next = g_next = 0u;
-            const long long i = static_cast<long long>(b) * kBlkTok + lane;
-            if (lane < kBlkTok && i < ntok) {
-                b_next = ld_bits(p.beta, p.beta_f32, bidx * p.beta_sb + (tok0 + i) * p.beta_st + head * p.beta_sh);
-                if (p.gate) g_next = ld_bits(p.gate, p.gate_f32, bidx * p.gate_sb + (tok0 + i) * p.gate_st + head * p.gate_sh);
-            }
-        };
-        fetch(j);
-        // false once a wait has given up.  Every lane polls for itself and the answers of two lanes can differ, so the loop is walked to its end: a
-        // warp whose lanes parted here would hang in its next shuffle.
-        bool ok = true;
-        for (int b = j; b < nblk + 4; b += 4) {
-            const uint32_t it = static_cast<uint32_t>(b >> 2);
-            const bool next = b < nblk;
-            const int n = min(kBlkTok, ntok - b * kBlkTok);
-            float o[8], c0[8], c1[8];
-            if (b >= 4) {  // block b - 4 is through: what its outputs are made of
-                ok = mbar_wait(&done[j], (it - 1) & 1u, &abort_flag) && ok;
-                auto row8 = [&](int off, int c, float* x) {
-                    const float4 u = *reinterpret_cast<const float4*>(st + off + piece_off(r, c));
-                    const float4 w = *reinterpret_cast<const float4*>(st + off + piece_off(r, c + 1));
-                    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
-                };
-                row8(L::kOffO, 2 * h, o);
-                row8(L::kOffC1, 0, c0);
-                row8(L::kOffC1, 2, c1);
-                __syncwarp();
-            }
-            if (next) {
-                // rows past the end of the sequence are filled with zeros (their address is that of the last row)
-                constexpr int kPieces = DK / 8;
-                const uint32_t dst = smem_u32(st);
-#pragma unroll 4
-                for (int i = lane; i < kBlkTok * kPieces; i += 32) {
-                    const int row = i / kPieces, c = i % kPieces;
-                    const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
-                    const uint32_t bytes = row < n ? 16u : 0u;
-                    cp_async16(dst + row * L::kRow + 16 * c, kp + at * p.k_st + 8 * c, bytes);
-                    cp_async16(dst + L::kOffQ + row * L::kRow + 16 * c, qp + at * p.q_st + 8 * c, bytes);
-                }
-                {
-                    const int row = lane >> 1;
-                    const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
-                    cp_async16(dst + L::kOffV + 16 * lane, vp + at * p.v_st + 8 * (lane & 1), row < n ? 16u : 0u);
-                }
-                cp_async_arrive(&full[j]);
-            }
-            if (b >= 4) {
-                // ---- outputs of block b - 4.  Coefficients of later tokens are left out, not multiplied by zero: an infinite or
-                //      undefined value stays behind its token.
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float* const P = pr + L::kP + (8 * h + i) * 16;
-                    const float4 u = *reinterpret_cast<const float4*>(P), w = *reinterpret_cast<const float4*>(P + 4);
-                    const float pw[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-#pragma unroll
-                    for (int s = 0; s < 8; ++s)
-                        if (s <= i || h) o[i] = fmaf(pw[s], c0[s], o[i]);
-                    if (h) {
-                        const float4 y = *reinterpret_cast<const float4*>(P + 8), z = *reinterpret_cast<const float4*>(P + 12);
-                        const float pz[8] = {y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
-#pragma unroll
-                        for (int s = 0; s <= i; ++s) o[i] = fmaf(pz[s], c1[s], o[i]);
-                    }
-                }
-                __syncwarp();
-                const bool good = ok && *static_cast<volatile int*>(&abort_flag) == 0;  // nothing is stored once a wait has given up
-                const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (good && i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
-            }
-            if (!next) break;
-            // ---- scalars; tokens past the end: beta 0, decay 1
-            float beta = from_bits(b_next, p.beta_f32), gate = from_bits(g_next, p.gate_f32);
+        if (warp >= 4) {
+            // =============================================================== preparation and outputs
+            const int j = warp - 4;
+            uint8_t* const st = smem + j * L::kStage;
+            float* const pr = prep_of(j);
+            float* const X = pr + L::kR0;  // [t][s] = Gamma_ts, [t][16] = G_t, [t][17], [t][18] = inverse norms of k_t, q_t
+            const __nv_bfloat16* const kp = p.k + bidx * p.k_sb + tok0 * p.k_st + khead * p.k_sh;
+            const __nv_bfloat16* const qp = p.q + bidx * p.q_sb + tok0 * p.q_st + khead * p.q_sh;
+            const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * kBlkRows;
+            const int r = lane & 15, h = lane >> 4;  // for the outputs: row r, tokens 8 h .. 8 h + 7
+            __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
+            float al = 0.f, db = 0.f;
             if (p.fused_gating) {
-                // softplus and sigmoid on the fast exponential, logarithm and reciprocal, as in recurrent.cuh
-                const float x = gate + db, e = __expf(x);
-                gate = -al * (x > 20.f ? x : (x < -15.f ? e : __logf(1.f + e)));
-                beta = __fdividef(1.f, 1.f + __expf(-beta));
+                al = __expf(from_bits(ld_bits(p.A_log, p.gating_param_f32, head), p.gating_param_f32));
+                db = from_bits(ld_bits(p.dt_bias, p.gating_param_f32, head), p.gating_param_f32);
             }
-            const bool real = lane < n;
-            const float a = real ? __expf(gate) : 1.f;
-            if (!real) beta = 0.f;
-            fetch(b + 4);
-            float run = 1.f;
-#pragma unroll
-            for (int i = 0; i < kBlkTok; ++i) {
-                const float ai = __shfl_sync(0xffffffffu, a, i);
-                if (lane == 16 || lane < i) run *= ai;
-                if (lane <= 16) X[i * L::kLdR + lane] = run;  // (entries s > t are not used)
-            }
-            ok = mbar_wait(&full[j], it & 1u, &abort_flag) && ok;
-            // ---- Gram matrices.  kk, qk: tokens 0 .. 15 against tokens 0 .. 7 of k; hh: tokens 8 .. 15 of k and of q against tokens
-            //      8 .. 15 of k; qq: the diagonals of q q^T.  The matrix instructions cut their sums off, so only two follow one another.
-            float kk[4] = {}, qk[4] = {}, hh[4] = {}, qq0[4] = {}, qq1[4] = {};
-            const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + lm_col * 2, qaddr = kaddr + L::kOffQ;
-#pragma unroll 2
-            for (int ks = 0; ks < DK / 16; ks += 2) {
-                uint32_t x[2][4], y[2][4];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    ldmatrix_x4(kaddr + 32 * (ks + e), x[e]);
-                    ldmatrix_x4(qaddr + 32 * (ks + e), y[e]);
+            uint32_t b_next = 0u, g_next = 0u;  // bits of beta and the gate (or of the raw projections) of token `lane` of the next block
+            auto fetch = [&](int b) {
+                b_next = g_next = 0u;
+                const long long i = static_cast<long long>(b) * kBlkTok + lane;
+                if (lane < kBlkTok && i < ntok) {
+                    b_next = ld_bits(p.beta, p.beta_f32, bidx * p.beta_sb + (tok0 + i) * p.beta_st + head * p.beta_sh);
+                    if (p.gate) g_next = ld_bits(p.gate, p.gate_f32, bidx * p.gate_sb + (tok0 + i) * p.gate_st + head * p.gate_sh);
                 }
-                float s0[4] = {}, s1[4] = {}, s2[4] = {};
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const uint32_t h[4] = {x[e][1], y[e][1], x[e][3], y[e][3]};
-                    mma16f(s0, x[e], x[e][0], x[e][2]);
-                    mma16f(s1, y[e], x[e][0], x[e][2]);
-                    mma16f(s2, h, x[e][1], x[e][3]);
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    kk[e] += s0[e];
-                    qk[e] += s1[e];
-                    hh[e] += s2[e];
-                }
-                if (p.is_qk_norm) {
-                    float s3[4] = {}, s4[4] = {};
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        mma16f(s3, y[e], y[e][0], y[e][2]);
-                        mma16f(s4, y[e], y[e][1], y[e][3]);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        qq0[e] += s3[e];
-                        qq1[e] += s4[e];
-                    }
-                }
-            }
-            if (t == (g >> 1)) {  // this lane holds the diagonal entries of tokens g and g + 8
-                float r0 = 1.f, r1 = 1.f, r2 = 1.f, r3 = 1.f;
-                if (p.is_qk_norm) {
-                    r0 = rsqrtf(((g & 1) ? kk[1] : kk[0]) + 1e-6f);
-                    r1 = rsqrtf(((g & 1) ? hh[1] : hh[0]) + 1e-6f);
-                    r2 = rsqrtf(((g & 1) ? qq0[1] : qq0[0]) + 1e-6f);
-                    r3 = rsqrtf(((g & 1) ? qq1[3] : qq1[2]) + 1e-6f);
-                }
-                X[g * L::kLdR + 17] = r0;
-                X[(g + 8) * L::kLdR + 17] = r1;
-                X[g * L::kLdR + 18] = r2;
-                X[(g + 8) * L::kLdR + 18] = r3;
-            }
-            __syncwarp();
-            const float beta_g = __shfl_sync(0xffffffffu, beta, g), beta_h = __shfl_sync(0xffffffffu, beta, g + 8);
-            const float rk_g = X[g * L::kLdR + 17], rk_h = X[(g + 8) * L::kLdR + 17];
-            const float rq_g = p.scale * X[g * L::kLdR + 18], rq_h = p.scale * X[(g + 8) * L::kLdR + 18];
-            // [s][t] = beta_t Gamma_ts k_s.k_t  and  [t][s] = scale Gamma_ts k_s.q_t (entries s >= t and s > t are not read)
-            auto put = [&](int ti, int si, float kkv, float qkv, float bt, float rq) {
-                const float w = X[ti * L::kLdR + si] * X[si * L::kLdR + 17];
-                pr[L::kA + si * 16 + ti] = bt * w * kkv;
-                pr[L::kP + ti * 16 + si] = rq * w * qkv;
             };
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int s0 = 2 * t + e;
-                put(g, s0, kk[e], qk[e], beta_g * rk_g, rq_g);
-                put(g + 8, s0, kk[2 + e], qk[2 + e], beta_h * rk_h, rq_h);
-                put(g + 8, s0 + 8, hh[e], hh[2 + e], beta_h * rk_h, rq_h);
-            }
-            if (lane < kBlkTok) {
-                const float G = X[lane * L::kLdR + 16], rk = X[lane * L::kLdR + 17], rq = X[lane * L::kLdR + 18];
-                pr[L::kCk + lane] = beta * G * rk;
-                pr[L::kCq + lane] = p.scale * G * rq;
-                pr[L::kW + lane] = real ? X[(n - 1) * L::kLdR + lane] * rk : 0.f;
-                if (lane == n - 1) pr[L::kG] = G;
-            }
-            __syncwarp();
-            // ---- beta v over the decay products
-            {
-                const int tk = lane & 15;
-                const uint4 v = *reinterpret_cast<const uint4*>(st + L::kOffV + tk * kBlkRows * 2 + 16 * (lane >> 4));
-                const float bt = __shfl_sync(0xffffffffu, beta, tk);
-                float* const R = X + 8 * (lane >> 4) * L::kLdR + tk;
-                const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
-                    R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
+            fetch(j);
+            // false once a wait has given up.  Every lane polls for itself and the answers of two lanes can differ, so the loop is walked to its end: a
+            // warp whose lanes parted here would hang in its next shuffle.
+            bool ok = true;
+            for (int b = j; b < nblk + 4; b += 4) {
+                const uint32_t it = static_cast<uint32_t>(b >> 2);
+                const bool next = b < nblk;
+                const int n = min(kBlkTok, ntok - b * kBlkTok);
+                float o[8], c0[8], c1[8];
+                if (b >= 4) {  // block b - 4 is through: what its outputs are made of
+                    ok = mbar_wait(&done[j], (it - 1) & 1u, &abort_flag) && ok;
+                    auto row8 = [&](int off, int c, float* x) {
+                        const float4 u = *reinterpret_cast<const float4*>(st + off + piece_off(r, c));
+                        const float4 w = *reinterpret_cast<const float4*>(st + off + piece_off(r, c + 1));
+                        x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
+                    };
+                    row8(L::kOffO, 2 * h, o);
+                    row8(L::kOffC1, 0, c0);
+                    row8(L::kOffC1, 2, c1);
+                    __syncwarp();
                 }
-            }
-            __syncwarp();
-            if (lane == 0 && ok) mbar_arrive(&ready[j]);  // not handed on once a wait has given up: the other warps' waits end with it
-        }
-    } else {
-        // =============================================================== state
-        const int col0 = warp * (DK / 4);
-        const int r = lane & 15, h = lane >> 4;  // in the solve: row r, tokens 8 h .. 8 h + 7
-        float S[2 * NK][4];  // 8 columns each: rows g (0, 1) and g + 8 (2, 3), columns 2t, 2t + 1
-        const long long srow = static_cast<long long>(rb * kBlkRows + g) * DK + col0 + 2 * t;
-        if (p.state_in) {
-            const long long base = static_cast<long long>(slot) * p.si_ss + head * p.si_sh + srow;
-#pragma unroll
-            for (int i = 0; i < 2 * NK; ++i) {
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (kF32) {
-                        const float2 w = *reinterpret_cast<const float2*>(static_cast<const float*>(p.state_in) + base + 8 * e * DK + 8 * i);
-                        S[i][2 * e] = w.x;
-                        S[i][2 * e + 1] = w.y;
-                    } else {
-                        const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.state_in) + base + 8 * e * DK + 8 * i);
-                        S[i][2 * e] = bf16_lo(w);
-                        S[i][2 * e + 1] = bf16_hi(w);
+                if (next) {
+                    // rows past the end of the sequence are filled with zeros (their address is that of the last row)
+                    constexpr int kPieces = DK / 8;
+                    const uint32_t dst = smem_u32(st);
+    #pragma unroll 4
+                    for (int i = lane; i < kBlkTok * kPieces; i += 32) {
+                        const int row = i / kPieces, c = i % kPieces;
+                        const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
+                        const uint32_t bytes = row < n ? 16u : 0u;
+                        cp_async16(dst + row * L::kRow + 16 * c, kp + at * p.k_st + 8 * c, bytes);
+                        cp_async16(dst + L::kOffQ + row * L::kRow + 16 * c, qp + at * p.q_st + 8 * c, bytes);
+                    }
+                    {
+                        const int row = lane >> 1;
+                        const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
+                        cp_async16(dst + L::kOffV + 16 * lane, vp + at * p.v_st + 8 * (lane & 1), row < n ? 16u : 0u);
+                    }
+                    cp_async_arrive(&full[j]);
+                }
+                if (b >= 4) {
+                    // ---- outputs of block b - 4.  Coefficients of later tokens are left out, not multiplied by zero: an infinite or
+                    //      undefined value stays behind its token.
+    #pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float* const P = pr + L::kP + (8 * h + i) * 16;
+                        const float4 u = *reinterpret_cast<const float4*>(P), w = *reinterpret_cast<const float4*>(P + 4);
+                        const float pw[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+    #pragma unroll
+                        for (int s = 0; s < 8; ++s)
+                            if (s <= i || h) o[i] = fmaf(pw[s], c0[s], o[i]);
+                        if (h) {
+                            const float4 y = *reinterpret_cast<const float4*>(P + 8), z = *reinterpret_cast<const float4*>(P + 12);
+                            const float pz[8] = {y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+    #pragma unroll
+                            for (int s = 0; s <= i; ++s) o[i] = fmaf(pz[s], c1[s], o[i]);
+                        }
+                    }
+                    __syncwarp();
+                    const bool good = ok && *static_cast<volatile int*>(&abort_flag) == 0;  // nothing is stored once a wait has given up
+                    const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
+    #pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (good && i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
+                }
+                if (!next) break;
+                // ---- scalars; tokens past the end: beta 0, decay 1
+                float beta = from_bits(b_next, p.beta_f32), gate = from_bits(g_next, p.gate_f32);
+                if (p.fused_gating) {
+                    // softplus and sigmoid on the fast exponential, logarithm and reciprocal, as in recurrent.cuh
+                    const float x = gate + db, e = __expf(x);
+                    gate = -al * (x > 20.f ? x : (x < -15.f ? e : __logf(1.f + e)));
+                    beta = __fdividef(1.f, 1.f + __expf(-beta));
+                }
+                const bool real = lane < n;
+                const float a = real ? __expf(gate) : 1.f;
+                if (!real) beta = 0.f;
+                fetch(b + 4);
+                float run = 1.f;
+    #pragma unroll
+                for (int i = 0; i < kBlkTok; ++i) {
+                    const float ai = __shfl_sync(0xffffffffu, a, i);
+                    if (lane == 16 || lane < i) run *= ai;
+                    if (lane <= 16) X[i * L::kLdR + lane] = run;  // (entries s > t are not used)
+                }
+                ok = mbar_wait(&full[j], it & 1u, &abort_flag) && ok;
+                // ---- Gram matrices.  kk, qk: tokens 0 .. 15 against tokens 0 .. 7 of k; hh: tokens 8 .. 15 of k and of q against tokens
+                //      8 .. 15 of k; qq: the diagonals of q q^T.  The matrix instructions cut their sums off, so only two follow one another.
+                float kk[4] = {}, qk[4] = {}, hh[4] = {}, qq0[4] = {}, qq1[4] = {};
+                const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + lm_col * 2, qaddr = kaddr + L::kOffQ;
+    #pragma unroll 2
+                for (int ks = 0; ks < DK / 16; ks += 2) {
+                    uint32_t x[2][4], y[2][4];
+    #pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        ldmatrix_x4(kaddr + 32 * (ks + e), x[e]);
+                        ldmatrix_x4(qaddr + 32 * (ks + e), y[e]);
+                    }
+                    float s0[4] = {}, s1[4] = {}, s2[4] = {};
+    #pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const uint32_t h[4] = {x[e][1], y[e][1], x[e][3], y[e][3]};
+                        mma16f(s0, x[e], x[e][0], x[e][2]);
+                        mma16f(s1, y[e], x[e][0], x[e][2]);
+                        mma16f(s2, h, x[e][1], x[e][3]);
+                    }
+    #pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        kk[e] += s0[e];
+                        qk[e] += s1[e];
+                        hh[e] += s2[e];
+                    }
+                    if (p.is_qk_norm) {
+                        float s3[4] = {}, s4[4] = {};
+    #pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            mma16f(s3, y[e], y[e][0], y[e][2]);
+                            mma16f(s4, y[e], y[e][1], y[e][3]);
+                        }
+    #pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            qq0[e] += s3[e];
+                            qq1[e] += s4[e];
+                        }
                     }
                 }
+                if (t == (g >> 1)) {  // this lane holds the diagonal entries of tokens g and g + 8
+                    float r0 = 1.f, r1 = 1.f, r2 = 1.f, r3 = 1.f;
+                    if (p.is_qk_norm) {
+                        r0 = rsqrtf(((g & 1) ? kk[1] : kk[0]) + 1e-6f);
+                        r1 = rsqrtf(((g & 1) ? hh[1] : hh[0]) + 1e-6f);
+                        r2 = rsqrtf(((g & 1) ? qq0[1] : qq0[0]) + 1e-6f);
+                        r3 = rsqrtf(((g & 1) ? qq1[3] : qq1[2]) + 1e-6f);
+                    }
+                    X[g * L::kLdR + 17] = r0;
+                    X[(g + 8) * L::kLdR + 17] = r1;
+                    X[g * L::kLdR + 18] = r2;
+                    X[(g + 8) * L::kLdR + 18] = r3;
+                }
+                __syncwarp();
+                const float beta_g = __shfl_sync(0xffffffffu, beta, g), beta_h = __shfl_sync(0xffffffffu, beta, g + 8);
+                const float rk_g = X[g * L::kLdR + 17], rk_h = X[(g + 8) * L::kLdR + 17];
+                const float rq_g = p.scale * X[g * L::kLdR + 18], rq_h = p.scale * X[(g + 8) * L::kLdR + 18];
+                // [s][t] = beta_t Gamma_ts k_s.k_t  and  [t][s] = scale Gamma_ts k_s.q_t (entries s >= t and s > t are not read)
+                auto put = [&](int ti, int si, float kkv, float qkv, float bt, float rq) {
+                    const float w = X[ti * L::kLdR + si] * X[si * L::kLdR + 17];
+                    pr[L::kA + si * 16 + ti] = bt * w * kkv;
+                    pr[L::kP + ti * 16 + si] = rq * w * qkv;
+                };
+    #pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int s0 = 2 * t + e;
+                    put(g, s0, kk[e], qk[e], beta_g * rk_g, rq_g);
+                    put(g + 8, s0, kk[2 + e], qk[2 + e], beta_h * rk_h, rq_h);
+                    put(g + 8, s0 + 8, hh[e], hh[2 + e], beta_h * rk_h, rq_h);
+                }
+                if (lane < kBlkTok) {
+                    const float G = X[lane * L::kLdR + 16], rk = X[lane * L::kLdR + 17], rq = X[lane * L::kLdR + 18];
+                    pr[L::kCk + lane] = beta * G * rk;
+                    pr[L::kCq + lane] = p.scale * G * rq;
+                    pr[L::kW + lane] = real ? X[(n - 1) * L::kLdR + lane] * rk : 0.f;
+                    if (lane == n - 1) pr[L::kG] = G;
+                }
+                __syncwarp();
+                // ---- beta v over the decay products
+                {
+                    const int tk = lane & 15;
+                    const uint4 v = *reinterpret_cast<const uint4*>(st + L::kOffV + tk * kBlkRows * 2 + 16 * (lane >> 4));
+                    const float bt = __shfl_sync(0xffffffffu, beta, tk);
+                    float* const R = X + 8 * (lane >> 4) * L::kLdR + tk;
+                    const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
+                        R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0 && ok) mbar_arrive(&ready[j]);  // not handed on once a wait has given up: the other warps' waits end with it
             }
         } else {
-#pragma unroll
-            for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
-        }
-        uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
-        bool ok = true;  // false once a wait has given up: nothing is stored from then on
-        bool ahead = false;  // this lane has seen the next block's preparation complete
-        for (int b = 0; b < nblk; ++b) {
-            ok = (ahead || mbar_wait(&ready[b & 3], static_cast<uint32_t>((b >> 2) & 1), &abort_flag)) && ok;
-            __syncwarp();
-            const int n = min(kBlkTok, ntok - b * kBlkTok);
-            uint8_t* const st = smem + (b & 3) * L::kStage;
-            const float* const pr = prep_of(b);
-            const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + (col0 + lm_col) * 2;
-            float* const D = reinterpret_cast<float*>(smem + L::kOffD) + (b & 1) * (4 * kBlkRows * L::kLdD);
-            // ---- this warp's columns of S_0 [k; q]^T: tokens 0 - 7 and 8 - 15 of k, then of q.  The first terms have sums of their own:
-            //      they are the long ones, and the chains are shorter.
-            {
-                float dh[4][4], dl[4][4];
-                auto products = [&](auto safe_tag) {
-                    constexpr bool kSafe = decltype(safe_tag)::value;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) dh[i][e] = dl[i][e] = 0.f;
-                    uint32_t x[2][4], y[2][4];
-                    ldmatrix_x4(kaddr, x[0]);
-                    ldmatrix_x4(kaddr + L::kOffQ, y[0]);
-#pragma unroll
-                    for (int kc = 0; kc < NK; ++kc) {
-                        if (kc + 1 < NK) {
-                            ldmatrix_x4(kaddr + 32 * (kc + 1), x[(kc + 1) & 1]);
-                            ldmatrix_x4(kaddr + L::kOffQ + 32 * (kc + 1), y[(kc + 1) & 1]);
+            // =============================================================== state
+            const int col0 = warp * (DK / 4);
+            const int r = lane & 15, h = lane >> 4;  // in the solve: row r, tokens 8 h .. 8 h + 7
+            float S[2 * NK][4];  // 8 columns each: rows g (0, 1) and g + 8 (2, 3), columns 2t, 2t + 1
+            const long long srow = static_cast<long long>(rb * kBlkRows + g) * DK + col0 + 2 * t;
+            if (p.state_in) {
+                const long long base = static_cast<long long>(slot) * p.si_ss + head * p.si_sh + srow;
+    #pragma unroll
+                for (int i = 0; i < 2 * NK; ++i) {
+    #pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (kF32) {
+                            const float2 w = *reinterpret_cast<const float2*>(static_cast<const float*>(p.state_in) + base + 8 * e * DK + 8 * i);
+                            S[i][2 * e] = w.x;
+                            S[i][2 * e + 1] = w.y;
+                        } else {
+                            const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.state_in) + base + 8 * e * DK + 8 * i);
+                            S[i][2 * e] = bf16_lo(w);
+                            S[i][2 * e + 1] = bf16_hi(w);
                         }
-                        const uint32_t* const xk = x[kc & 1];
-                        const uint32_t* const yk = y[kc & 1];
-                        uint32_t hi[4], mid[4], lo[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float* s = &S[2 * kc + (e >> 1)][2 * (e & 1)];
-                            split3<kSafe>(s[0], s[1], hi[e], mid[e], lo[e]);
+                    }
+                }
+            } else {
+    #pragma unroll
+                for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
+            }
+            uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
+            bool ok = true;  // false once a wait has given up: nothing is stored from then on
+            bool ahead = false;  // this lane has seen the next block's preparation complete
+            for (int b = 0; b < nblk; ++b) {
+                ok = (ahead || mbar_wait(&ready[b & 3], static_cast<uint32_t>((b >> 2) & 1), &abort_flag)) && ok;
+                __syncwarp();
+                const int n = min(kBlkTok, ntok - b * kBlkTok);
+                uint8_t* const st = smem + (b & 3) * L::kStage;
+                const float* const pr = prep_of(b);
+                const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + (col0 + lm_col) * 2;
+                float* const D = reinterpret_cast<float*>(smem + L::kOffD) + (b & 1) * (4 * kBlkRows * L::kLdD);
+                // ---- this warp's columns of S_0 [k; q]^T: tokens 0 - 7 and 8 - 15 of k, then of q.  The first terms have sums of their own:
+                //      they are the long ones, and the chains are shorter.
+                {
+                    float dh[4][4], dl[4][4];
+                    auto products = [&](auto safe_tag) {
+                        constexpr bool kSafe = decltype(safe_tag)::value;
+    #pragma unroll
+                        for (int i = 0; i < 4; ++i)
+    #pragma unroll
+                            for (int e = 0; e < 4; ++e) dh[i][e] = dl[i][e] = 0.f;
+                        uint32_t x[2][4], y[2][4];
+                        ldmatrix_x4(kaddr, x[0]);
+                        ldmatrix_x4(kaddr + L::kOffQ, y[0]);
+    #pragma unroll
+                        for (int kc = 0; kc < NK; ++kc) {
+                            if (kc + 1 < NK) {
+                                ldmatrix_x4(kaddr + 32 * (kc + 1), x[(kc + 1) & 1]);
+                                ldmatrix_x4(kaddr + L::kOffQ + 32 * (kc + 1), y[(kc + 1) & 1]);
+                            }
+                            const uint32_t* const xk = x[kc & 1];
+                            const uint32_t* const yk = y[kc & 1];
+                            uint32_t hi[4], mid[4], lo[4];
+    #pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float* s = &S[2 * kc + (e >> 1)][2 * (e & 1)];
+                                split3<kSafe>(s[0], s[1], hi[e], mid[e], lo[e]);
+                            }
+                            mma16f(dl[0], lo, xk[0], xk[2]);
+                            mma16f(dl[1], lo, xk[1], xk[3]);
+                            mma16f(dl[2], lo, yk[0], yk[2]);
+                            mma16f(dl[3], lo, yk[1], yk[3]);
+                            mma16f(dh[0], hi, xk[0], xk[2]);
+                            mma16f(dh[1], hi, xk[1], xk[3]);
+                            mma16f(dh[2], hi, yk[0], yk[2]);
+                            mma16f(dh[3], hi, yk[1], yk[3]);
+                            mma16f(dl[0], mid, xk[0], xk[2]);
+                            mma16f(dl[1], mid, xk[1], xk[3]);
+                            mma16f(dl[2], mid, yk[0], yk[2]);
+                            mma16f(dl[3], mid, yk[1], yk[3]);
                         }
-                        mma16f(dl[0], lo, xk[0], xk[2]);
-                        mma16f(dl[1], lo, xk[1], xk[3]);
-                        mma16f(dl[2], lo, yk[0], yk[2]);
-                        mma16f(dl[3], lo, yk[1], yk[3]);
-                        mma16f(dh[0], hi, xk[0], xk[2]);
-                        mma16f(dh[1], hi, xk[1], xk[3]);
-                        mma16f(dh[2], hi, yk[0], yk[2]);
-                        mma16f(dh[3], hi, yk[1], yk[3]);
-                        mma16f(dl[0], mid, xk[0], xk[2]);
-                        mma16f(dl[1], mid, xk[1], xk[3]);
-                        mma16f(dl[2], mid, yk[0], yk[2]);
-                        mma16f(dl[3], mid, yk[1], yk[3]);
+                    };
+                    products(std::false_type{});
+                    // a row of the state with an infinity has undefined low terms in every column: taken again with care
+                    const float chk = dl[0][0] + dl[0][2];
+                    if (__any_sync(0xffffffffu, chk != chk)) products(std::true_type{});
+                    float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
+    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        *reinterpret_cast<float2*>(d + 8 * i) = make_float2(dh[i][0] + dl[i][0], dh[i][1] + dl[i][1]);
+                        *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
+                    }
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                // ---- c of row r, tokens 8 h ..: right-hand sides, then forward substitution, first half of the tokens before the second
+                float c[8];
+                {
+                    const float* const d = D + r * L::kLdD + 8 * h;
+                    float sum[8];
+    #pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        float4 x[4];
+    #pragma unroll
+                        for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float4*>(d + w * (kBlkRows * L::kLdD) + 4 * q);
+                        sum[4 * q] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
+                        sum[4 * q + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+                        sum[4 * q + 2] = (x[0].z + x[1].z) + (x[2].z + x[3].z);
+                        sum[4 * q + 3] = (x[0].w + x[1].w) + (x[2].w + x[3].w);
+                    }
+    #pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + r * L::kLdR + 8 * h + 4 * q);
+                        const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
+                        c[4 * q] = fmaf(-ck.x, sum[4 * q], bv.x);
+                        c[4 * q + 1] = fmaf(-ck.y, sum[4 * q + 1], bv.y);
+                        c[4 * q + 2] = fmaf(-ck.z, sum[4 * q + 2], bv.z);
+                        c[4 * q + 3] = fmaf(-ck.w, sum[4 * q + 3], bv.w);
+                    }
+                }
+                // column s of A, tokens 8 th .. 8 th + 7
+                auto col_of = [&](int s, int th, float* x) {
+                    const float4 u = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th);
+                    const float4 v = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th + 4);
+                    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+                };
+                // (what a token gets from the tokens before it is summed apart from its own, larger, term)
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                auto substitute = [&](int half) {
+    #pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        c[s] -= acc[s];
+                        if (s == 7) break;
+                        float x[8];
+                        col_of(8 * half + s, half, x);
+    #pragma unroll
+                        for (int i = s + 1; i < 8; ++i) acc[i] = fmaf(x[i], c[s], acc[i]);
                     }
                 };
-                products(std::false_type{});
-                // a row of the state with an infinity has undefined low terms in every column: taken again with care
-                const float chk = dl[0][0] + dl[0][2];
-                if (__any_sync(0xffffffffu, chk != chk)) products(std::true_type{});
-                float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    *reinterpret_cast<float2*>(d + 8 * i) = make_float2(dh[i][0] + dl[i][0], dh[i][1] + dl[i][1]);
-                    *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
-                }
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            // ---- c of row r, tokens 8 h ..: right-hand sides, then forward substitution, first half of the tokens before the second
-            float c[8];
-            {
-                const float* const d = D + r * L::kLdD + 8 * h;
-                float sum[8];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    float4 x[4];
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float4*>(d + w * (kBlkRows * L::kLdD) + 4 * q);
-                    sum[4 * q] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
-                    sum[4 * q + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
-                    sum[4 * q + 2] = (x[0].z + x[1].z) + (x[2].z + x[3].z);
-                    sum[4 * q + 3] = (x[0].w + x[1].w) + (x[2].w + x[3].w);
-                }
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + r * L::kLdR + 8 * h + 4 * q);
-                    const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
-                    c[4 * q] = fmaf(-ck.x, sum[4 * q], bv.x);
-                    c[4 * q + 1] = fmaf(-ck.y, sum[4 * q + 1], bv.y);
-                    c[4 * q + 2] = fmaf(-ck.z, sum[4 * q + 2], bv.z);
-                    c[4 * q + 3] = fmaf(-ck.w, sum[4 * q + 3], bv.w);
-                }
-            }
-            // column s of A, tokens 8 th .. 8 th + 7
-            auto col_of = [&](int s, int th, float* x) {
-                const float4 u = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th);
-                const float4 v = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th + 4);
-                x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
-            };
-            // (what a token gets from the tokens before it is summed apart from its own, larger, term)
-            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            auto substitute = [&](int half) {
-#pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    c[s] -= acc[s];
-                    if (s == 7) break;
-                    float x[8];
-                    col_of(8 * half + s, half, x);
-#pragma unroll
-                    for (int i = s + 1; i < 8; ++i) acc[i] = fmaf(x[i], c[s], acc[i]);
-                }
-            };
-            if (h == 0) substitute(0);
-            __syncwarp();
-            float c0[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) c0[i] = __shfl_sync(0xffffffffu, c[i], r);
-            if (h == 1) {
-#pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    float x[8];
-                    col_of(s, 1, x);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = fmaf(x[i], c0[s], acc[i]);
-                }
-                substitute(1);
-            }
-            if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
-#pragma unroll
-                for (int i = 0; i < 8; ++i) c[i] = 8 * h + i < n ? c[i] : 0.f;
-            }
-            __syncwarp();
-            // ---- S <- G S + sum_s (Gamma_ns r_s c_s) k_s^T
-            {
-                uint32_t hi[4], mid[4], lo[4];
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const float4 w = *reinterpret_cast<const float4*>(pr + L::kW + 8 * h + 4 * q);
-                    split3<true>(w.x * c[4 * q], w.y * c[4 * q + 1], hi[2 * q], mid[2 * q], lo[2 * q]);
-                    split3<true>(w.z * c[4 * q + 2], w.w * c[4 * q + 3], hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1]);
-                }
-                uint8_t* const o = sc + r * L::kRowC + 16 * h;
-                *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(o + kBlkRows * L::kRowC) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-                *reinterpret_cast<uint4*>(o + 2 * kBlkRows * L::kRowC) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                if (h == 0) substitute(0);
                 __syncwarp();
-                const uint32_t caddr = smem_u32(sc) + lm_row * L::kRowC + lm_col * 2;
-                ldmatrix_x4(caddr, hi);
-                ldmatrix_x4(caddr + kBlkRows * L::kRowC, mid);
-                ldmatrix_x4(caddr + 2 * kBlkRows * L::kRowC, lo);
-                const float G = pr[L::kG];
-#pragma unroll
-                for (int kc = 0; kc < NK; ++kc) {
-                    uint32_t x[4];
-                    ldmatrix_x4_trans(kaddr + 32 * kc, x);  // tokens of k in pairs, columns 0 - 7 and 8 - 15
-                    // first terms and the others apart: the matrix instructions cut their sums off, which the short sums of first
-                    // terms lose next to nothing by, and an fp32 addition rounds
-                    float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f}, f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma16f(e0, lo, x[0], x[1]);
-                    mma16f(e1, lo, x[2], x[3]);
-                    mma16f(f0, hi, x[0], x[1]);
-                    mma16f(f1, hi, x[2], x[3]);
-                    mma16f(e0, mid, x[0], x[1]);
-                    mma16f(e1, mid, x[2], x[3]);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        S[2 * kc][e] = fmaf(G, S[2 * kc][e], f0[e] + e0[e]);
-                        S[2 * kc + 1][e] = fmaf(G, S[2 * kc + 1][e], f1[e] + e1[e]);
+                float c0[8];
+    #pragma unroll
+                for (int i = 0; i < 8; ++i) c0[i] = __shfl_sync(0xffffffffu, c[i], r);
+                if (h == 1) {
+    #pragma unroll
+                    for (int s = 0; s < 8; ++s) {
+                        float x[8];
+                        col_of(s, 1, x);
+    #pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[i] = fmaf(x[i], c0[s], acc[i]);
+                    }
+                    substitute(1);
+                }
+                if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
+    #pragma unroll
+                    for (int i = 0; i < 8; ++i) c[i] = 8 * h + i < n ? c[i] : 0.f;
+                }
+                __syncwarp();
+                // ---- S <- G S + sum_s (Gamma_ns r_s c_s) k_s^T
+                {
+                    uint32_t hi[4], mid[4], lo[4];
+    #pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float4 w = *reinterpret_cast<const float4*>(pr + L::kW + 8 * h + 4 * q);
+                        split3<true>(w.x * c[4 * q], w.y * c[4 * q + 1], hi[2 * q], mid[2 * q], lo[2 * q]);
+                        split3<true>(w.z * c[4 * q + 2], w.w * c[4 * q + 3], hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1]);
+                    }
+                    uint8_t* const o = sc + r * L::kRowC + 16 * h;
+                    *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    *reinterpret_cast<uint4*>(o + kBlkRows * L::kRowC) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+                    *reinterpret_cast<uint4*>(o + 2 * kBlkRows * L::kRowC) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    __syncwarp();
+                    const uint32_t caddr = smem_u32(sc) + lm_row * L::kRowC + lm_col * 2;
+                    ldmatrix_x4(caddr, hi);
+                    ldmatrix_x4(caddr + kBlkRows * L::kRowC, mid);
+                    ldmatrix_x4(caddr + 2 * kBlkRows * L::kRowC, lo);
+                    const float G = pr[L::kG];
+    #pragma unroll
+                    for (int kc = 0; kc < NK; ++kc) {
+                        uint32_t x[4];
+                        ldmatrix_x4_trans(kaddr + 32 * kc, x);  // tokens of k in pairs, columns 0 - 7 and 8 - 15
+                        // first terms and the others apart: the matrix instructions cut their sums off, which the short sums of first
+                        // terms lose next to nothing by, and an fp32 addition rounds
+                        float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f}, f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma16f(e0, lo, x[0], x[1]);
+                        mma16f(e1, lo, x[2], x[3]);
+                        mma16f(f0, hi, x[0], x[1]);
+                        mma16f(f1, hi, x[2], x[3]);
+                        mma16f(e0, mid, x[0], x[1]);
+                        mma16f(e1, mid, x[2], x[3]);
+    #pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            S[2 * kc][e] = fmaf(G, S[2 * kc][e], f0[e] + e0[e]);
+                            S[2 * kc + 1][e] = fmaf(G, S[2 * kc + 1][e], f1[e] + e1[e]);
+                        }
+                    }
+                }
+                // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t), and c
+                {
+                    const int i = 32 * warp + lane, row = i >> 3, t2 = 2 * (i & 7);
+                    const float* const d = D + row * L::kLdD + 16 + t2;
+                    float2 x[4];
+    #pragma unroll
+                    for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
+                    const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
+                    ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
+                    *reinterpret_cast<float2*>(st + L::kOffO + piece_off(row, t2 >> 2) + 4 * (t2 & 2)) =
+                        make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
+                    if (warp == (b & 3)) {
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&done[b & 3]);
+            }
+            if (ok && *static_cast<volatile int*>(&abort_flag) == 0) {
+                const long long base = static_cast<long long>(slot) * p.so_ss + head * p.so_sh + srow;
+    #pragma unroll
+                for (int i = 0; i < 2 * NK; ++i) {
+    #pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if (kF32)
+                            *reinterpret_cast<float2*>(static_cast<float*>(p.state_out) + base + 8 * e * DK + 8 * i) = make_float2(S[i][2 * e], S[i][2 * e + 1]);
+                        else
+                            *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.state_out) + base + 8 * e * DK + 8 * i) = pack_bf16(S[i][2 * e], S[i][2 * e + 1]);
                     }
                 }
             }
-            // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t), and c
-            {
-                const int i = 32 * warp + lane, row = i >> 3, t2 = 2 * (i & 7);
-                const float* const d = D + row * L::kLdD + 16 + t2;
-                float2 x[4];
-#pragma unroll
-                for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
-                const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
-                ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
-                *reinterpret_cast<float2*>(st + L::kOffO + piece_off(row, t2 >> 2) + 4 * (t2 & 2)) =
-                    make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
-                if (warp == (b & 3)) {
-                    *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
-                    *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&done[b & 3]);
         }
-        if (ok && *static_cast<volatile int*>(&abort_flag) == 0) {
-            const long long base = static_cast<long long>(slot) * p.so_ss + head * p.so_sh + srow;
-#pragma unroll
-            for (int i = 0; i < 2 * NK; ++i) {
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (kF32)
-                        *reinterpret_cast<float2*>(static_cast<float*>(p.state_out) + base + 8 * e * DK + 8 * i) = make_float2(S[i][2 * e], S[i][2 * e + 1]);
-                    else
-                        *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.state_out) + base + 8 * e * DK + 8 * i) = pack_bf16(S[i][2 * e], S[i][2 * e + 1]);
+    };  // run
+
+    if constexpr (kUnits == BlkUnits::kWalk) {
+        // (the walk's state is in shared memory: registers are all taken)
+        __shared__ long long s_unit;
+        __shared__ int s_seq;
+        if (tid == 0) s_unit = blockIdx.x;
+        while (true) {
+            __syncthreads();
+            if (tid < 32) {
+                const int seq = long_sequence(p.cu_seqlens, p.batch, p.long_run, static_cast<int>(s_unit / (p.vh * rblocks)));
+                if (tid == 0) s_seq = seq;
+            }
+            __syncthreads();
+            if (s_seq < 0) break;
+            const int rem = static_cast<int>(s_unit % (p.vh * rblocks));
+            run(s_seq, rem / rblocks, rem % rblocks);
+            __syncthreads();  // no warp waits on the unit's barriers any more
+            if (abort_flag) break;
+            if (tid == 0) {
+                for (int i = 0; i < 4; ++i) {
+                    mbar_inval(&full[i]);
+                    mbar_inval(&ready[i]);
+                    mbar_inval(&done[i]);
                 }
+                init_barriers();
+                s_unit += gridDim.x;
             }
         }
+    } else {
+        const int unit = static_cast<int>(blockIdx.x) / rblocks, rb = static_cast<int>(blockIdx.x) - unit * rblocks;
+        int seq = unit / p.vh;
+        const int head = unit - seq * p.vh;
+        if (kPacked) seq = long_sequence(p.cu_seqlens, p.batch, p.long_run, seq);
+        if (seq >= 0) run(seq, head, rb);
     }
+    if (kPacked) grid_dep_wait();
     __syncthreads();
     if (abort_flag) {
         cp_async_wait_all();  // the copies whose wait gave up
@@ -588,9 +656,9 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     }
 }
 
-template <int DK, bool kF32 = false>
+template <int DK, bool kF32 = false, BlkUnits kUnits = BlkUnits::kPadded>
 __global__ void __launch_bounds__(kBlkThreads, 2) gdn_recurrent_block_kernel(const RecurrentParams p) {
-    gdn_recurrent_block_body<DK, kF32>(p);
+    gdn_recurrent_block_body<DK, kF32, kUnits>(p);
 }
 
 }  // namespace gdn

@@ -106,3 +106,63 @@ def test_undefined_values_stay_behind_their_token(gdn, what, bad):
             assert not torch.isfinite(o1[0, at:, 0, 9]).any()
         else:
             assert not torch.isfinite(o1[:, at:]).any()
+
+
+def unit(x):
+    return torch.nn.functional.normalize(x, dim=-1).bfloat16()
+
+
+def flat_inputs(n, kh, vh, d, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    return unit(r(n, kh, d)), unit(r(n, kh, d)), r(n, vh, d).bfloat16(), torch.sigmoid(r(n, vh)).bfloat16(), -torch.nn.functional.softplus(r(n, vh))
+
+
+# on both sides of the line between the token recurrence and the blocks of every head dim and state type
+@pytest.mark.parametrize("d,f32,T", [(64, False, 31), (64, False, 40), (64, False, 41), (64, True, 40), (64, True, 41), (128, False, 17), (128, False, 24),
+                                     (128, False, 25), (128, True, 24), (128, True, 25), (192, False, 26), (192, False, 27), (256, False, 22), (256, False, 23)])
+def test_bits_do_not_depend_on_company(gdn, d, f32, T):
+    """a sequence alone, in a batch that fills the GPU and packed, and a shard of its heads: the same bits"""
+    B, kh, vh = 40, 4, 8
+    x = [t.view(B, T, *t.shape[1:]) for t in flat_inputs(B * T, kh, vh, d, d + T)]
+    s0 = (torch.randn(B, vh, d, d, device="cuda") * 0.02).to(torch.float32 if f32 else torch.bfloat16)
+    run = lambda x, s, **kw: gdn.recurrent_forward(*x[:3], s, *x[3:], inference_mode=gdn.Decode, **kw)
+    o, s = run(x, s0)
+    for i in (0, 39):
+        oi, si = run([t[i:i + 1] for t in x], s0[i:i + 1])
+        assert torch.equal(oi, o[i:i + 1]) and torch.equal(si, s[i:i + 1])
+    heads = [t[:, :, :1] for t in x[:2]] + [t[:, :, :2] for t in x[2:]]
+    oh, sh = run(heads, s0[:, :2].contiguous())
+    assert torch.equal(oh, o[:, :, :2]) and torch.equal(sh, s[:, :2])
+    cu = torch.arange(0, B * T + 1, T, dtype=torch.int32, device="cuda")
+    op, sp = run([t.flatten(0, 1) for t in x], s0, cu_seqlens=cu)
+    assert torch.equal(op.view_as(o), o) and torch.equal(sp, s)
+
+
+@pytest.mark.parametrize("chunked", [False, True])
+@pytest.mark.parametrize("d", [64, 128, 192, 256])
+@pytest.mark.parametrize("lens", [[300] + [1] * 99 + [22, 41, 0, 25, 27, 60, 17], [0] * 70 + [40, 0, 41, 26, 200], [23, 24, 45, 1000, 64, 41]])
+def test_packed_runs_of_unequal_length(gdn, lens, d, chunked):
+    """few long sequences among many short ones, among empty ones, and none but long ones: the bits each has alone"""
+    if chunked and d <= 128:
+        pytest.skip("head dims up to 128 have kernels of their own in chunked_forward")
+    kh, vh = 2, 4
+    x = flat_inputs(sum(lens), kh, vh, d, d)
+    s0 = (torch.randn(len(lens), vh, d, d, device="cuda") * 0.02).bfloat16()
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    if chunked:
+        run = lambda x, s, *meta: gdn.chunked_forward(*x, None, s, *meta)
+        o, s = run(x, s0, i32(cu), i32(synthetic.prepare_chunk_indices(cu)), i32(synthetic.prepare_cu_chunks(cu)))
+    else:
+        run = lambda x, s, **kw: gdn.recurrent_forward(*x[:3], s, *x[3:], inference_mode=gdn.Decode, **kw)
+        o, s = run(x, s0, cu_seqlens=i32(cu))
+    for i, n in enumerate(lens):
+        if not n:
+            assert torch.equal(s[i], s0[i])
+        elif n > 8 or i in (1, 50, 99):
+            sl = slice(cu[i], cu[i + 1])
+            oi, si = run([t[None, sl] for t in x], s0[i:i + 1])
+            assert torch.equal(oi[0], o[sl]) and torch.equal(si[0], s[i]), n
