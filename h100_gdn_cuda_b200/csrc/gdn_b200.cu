@@ -184,9 +184,31 @@ static int block_min_tokens(int dk, bool f32, bool steps, int ring_min) {
     const int from = dk == 64 ? 41 : dk == 128 ? 25 : dk == 192 ? 27 : dk == 256 ? 23 : kRecNoLongRun;
     return std::max(from, ring_min < kRecNoLongRun ? ring_min + 1 : kRecNoLongRun);
 }
+// The same kernel, compiled at run time (GDN_JIT_RECURRENT=1; bf16 states).
+static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, int smem, unsigned grid, cudaStream_t st) {
+    const char* const kind[3] = {"kPadded", "kPacked", "kWalk"};
+    char src[512];
+    snprintf(src, sizeof(src),
+             "#include \"kernels/recurrent_block.cuh\"\n"
+             "extern \"C\" __global__ void __launch_bounds__(%d, 2) gdn_recurrent_jit(const gdn::RecurrentParams p) {\n"
+             "    gdn::gdn_recurrent_block_body<%d, false, gdn::BlkUnits::%s>(p);\n}\n",
+             kBlkThreads, dk, kind[static_cast<int>(units)]);
+    jit::LoadedKernel k;
+    std::string err;
+    const char* const suffix[3] = {".block", ".block_packed", ".block_walk"};
+    if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + suffix[static_cast<int>(units)], src, "gdn_recurrent_jit", &k, &err))
+        return fail(rc, "%s", err.c_str());
+    GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    RecurrentParams pc = p;
+    void* args[] = {&pc};
+    GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(kBlkThreads), args, smem, st));
+    return GDN_OK;
+}
 template <int DK, bool kF32, BlkUnits kUnits>
-static int launch_block_t(const RecurrentParams& p, long long grid, cudaStream_t st) {
+static int launch_block_t(const RecurrentParams& p, bool jit, long long grid, cudaStream_t st) {
     constexpr int smem = BlockSmem<DK>::kBytes;
+    GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
+    if (jit) return launch_block_jit(p, DK, kUnits, smem, static_cast<unsigned>(grid), st);
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     GDN_CUDA(cudaGetDevice(&dev));
@@ -194,31 +216,30 @@ static int launch_block_t(const RecurrentParams& p, long long grid, cudaStream_t
         GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kF32, kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev & 63].store(true, std::memory_order_release);
     }
-    GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
     GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kF32, kUnits>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
     return GDN_OK;
 }
 template <BlkUnits kUnits>
-static int launch_block_as(const RecurrentParams& p, int dk, bool f32, long long grid, cudaStream_t st) {
+static int launch_block_as(const RecurrentParams& p, int dk, bool f32, bool jit, long long grid, cudaStream_t st) {
     switch (f32 ? -dk : dk) {
-        case 64: return launch_block_t<64, false, kUnits>(p, grid, st);
-        case 128: return launch_block_t<128, false, kUnits>(p, grid, st);
-        case 192: return launch_block_t<192, false, kUnits>(p, grid, st);
-        case 256: return launch_block_t<256, false, kUnits>(p, grid, st);
-        case -64: return launch_block_t<64, true, kUnits>(p, grid, st);
-        case -128: return launch_block_t<128, true, kUnits>(p, grid, st);
+        case 64: return launch_block_t<64, false, kUnits>(p, jit, grid, st);
+        case 128: return launch_block_t<128, false, kUnits>(p, jit, grid, st);
+        case 192: return launch_block_t<192, false, kUnits>(p, jit, grid, st);
+        case 256: return launch_block_t<256, false, kUnits>(p, jit, grid, st);
+        case -64: return launch_block_t<64, true, kUnits>(p, jit, grid, st);
+        case -128: return launch_block_t<128, true, kUnits>(p, jit, grid, st);
     }
     return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: no token-block kernel for dk = %d", dk);
 }
 // Packed mode: no more than total_tokens / long_run sequences can be that long.  Where that is all of them, a CTA per unit, as for
 // padded batches; otherwise a wave of CTAs walks the units (100 sequences of one token and one of 1500, d=256: 69 times the CTAs
 // there is work for).  The walk itself costs registers (d=256: 260 bytes spilled, 20 % of the time).
-static int launch_block(const RecurrentParams& p, int dk, bool f32, long long total_tokens, int sms, cudaStream_t st) {
+static int launch_block(const RecurrentParams& p, int dk, bool f32, bool jit, long long total_tokens, int sms, cudaStream_t st) {
     const long long per_seq = static_cast<long long>(p.vh) * (p.dv / kBlkRows);
-    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, f32, p.batch * per_seq, st);
+    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, f32, jit, p.batch * per_seq, st);
     const long long seqs = total_tokens / p.long_run;
-    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, f32, p.batch * per_seq, st);
-    return launch_block_as<BlkUnits::kWalk>(p, dk, f32, std::min(seqs * per_seq, 2ll * sms), st);
+    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, f32, jit, p.batch * per_seq, st);
+    return launch_block_as<BlkUnits::kWalk>(p, dk, f32, jit, std::min(seqs * per_seq, 2ll * sms), st);
 }
 
 // Head dimensions without a prebuilt kernel (or every call when GDN_JIT_RECURRENT=1) go through
@@ -558,10 +579,10 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
     const bool f32 = a->state_dtype == GDN_F32;
     const bool jit = force_jit && !f32;
-    p.long_run = jit ? kRecNoLongRun : block_min_tokens(s.head_dim_k, f32, p.store_step != 0, ring_min);
+    p.long_run = block_min_tokens(s.head_dim_k, f32, p.store_step != 0, ring_min);
     // (packed: no more tokens than sequences is a batch of single tokens)
     if (s.cu_seqlens ? s.total_tokens < p.long_run || s.total_tokens <= s.batch : s.seq_len < p.long_run) p.long_run = kRecNoLongRun;
-    if (p.long_run != kRecNoLongRun && !s.cu_seqlens) return launch_block(p, s.head_dim_k, f32, 0, d->sms, st);
+    if (p.long_run != kRecNoLongRun && !s.cu_seqlens) return launch_block(p, s.head_dim_k, f32, jit, 0, d->sms, st);
     auto token_recurrence = [&]() -> int {
         if (jit) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
         if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
@@ -582,7 +603,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     };
     if (int rc = token_recurrence()) return rc;
     // packed: the sequences that launch has left out
-    return p.long_run == kRecNoLongRun ? GDN_OK : launch_block(p, s.head_dim_k, f32, s.total_tokens, d->sms, st);
+    return p.long_run == kRecNoLongRun ? GDN_OK : launch_block(p, s.head_dim_k, f32, jit, s.total_tokens, d->sms, st);
 }
 
 }  // extern "C"

@@ -31,8 +31,6 @@
 //               (Four of them, so that their work is spread over the four schedulers.)
 // Two CTAs per SM at dk = 256: one's chain fills the gaps of the other.
 #pragma once
-#include <type_traits>
-
 #include "recurrent_step.cuh"
 
 namespace gdn {
@@ -65,6 +63,10 @@ struct BlockSmem {
 
 namespace blk {
 using ptx::smem_u32;
+template <bool kValue>
+struct Flag {  // (the run-time compiler has no standard library)
+    static constexpr bool value = kValue;
+};
 __device__ __forceinline__ void ldmatrix_x4(uint32_t saddr, uint32_t* r) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -464,10 +466,10 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                             mma16f(dl[3], mid, yk[1], yk[3]);
                         }
                     };
-                    products(std::false_type{});
+                    products(Flag<false>{});
                     // a row of the state with an infinity has undefined low terms in every column: taken again with care
                     const float chk = dl[0][0] + dl[0][2];
-                    if (__any_sync(0xffffffffu, chk != chk)) products(std::true_type{});
+                    if (__any_sync(0xffffffffu, chk != chk)) products(Flag<true>{});
                     float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
     #pragma unroll
                     for (int i = 0; i < 4; ++i) {

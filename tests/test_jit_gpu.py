@@ -50,6 +50,30 @@ def test_jit_recurrent_equals_prebuilt(gdn, monkeypatch, tmp_path, use_nvrtc):
         gdn.init(ROOT, cuda_home)
 
 
+@pytest.mark.parametrize("d,lens,suffix", [(128, None, "block"), (64, None, "block"), (192, [27, 40, 300], "block_packed"), (256, [1, 70, 0, 22, 23] + [2] * 20, "block_walk")])
+@pytest.mark.parametrize("use_nvrtc", ["1", "0"])
+def test_jit_token_blocks_equal_prebuilt(gdn, monkeypatch, tmp_path, d, lens, suffix, use_nvrtc):
+    """long runs: the same kernel, and the same bits, as an ahead-of-time launch of the call takes"""
+    if lens is None:
+        p = synthetic.prefill_inputs(2, 50, 1, 2, d, seed=7, mild_gate=True)
+    else:
+        p = synthetic.varlen_inputs(lens, 1, 2, d, seed=7, mild_gate=True)
+    pd = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+    run = lambda: gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], pd["state"], pd["beta"], pd["g"], pd.get("cu_seqlens"), inference_mode=1)
+    o_ref, s_ref = run()
+    monkeypatch.setenv("GDN_JIT_RECURRENT", "1")
+    monkeypatch.setenv("JIT_USE_NVRTC", use_nvrtc)
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    gdn.init(ROOT, cuda_home)
+    try:
+        o, s = run()
+        assert torch.equal(o, o_ref) and torch.equal(s, s_ref)
+        assert any(f.startswith("kernel.recurrent_dk%d.%s." % (d, suffix)) for f in os.listdir(tmp_path))
+    finally:
+        monkeypatch.delenv("GDN_JIT_RECURRENT")
+        gdn.init(ROOT, cuda_home)
+
+
 def test_head_dim_without_prebuilt_kernel(gdn):
     p = synthetic.decode_inputs(3, 2, 1, 2, 320, seed=6)
     beta, g = O.gating_ref(p["A_log"], p["dt_bias"], p["a"], p["b"])
