@@ -368,6 +368,14 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             // ---- K K^T (lanes 0-63) and Q K^T (lanes 64-127): once per unit, shared by its v-heads
             if (rd == 0) {
                 mbar_wait(bar_load, it & 1u, abort_flag);
+                if (n < kChunk) {
+                    // Keys past the end, in packed mode another sequence's, meet zero rows of dT in Z; cleared all the same, so that no
+                    // infinity or NaN of a neighbour can enter.
+                    for (int i = tid; i < (kChunk - n) * 8 * NA; i += kThreads)
+                        *reinterpret_cast<uint4*>(sKQ + (i & (NA - 1)) * 16384 + (n + i / (8 * NA)) * 128 + ((i / NA) & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                    fence_proxy_async_smem();
+                    __syncthreads();
+                }
                 if (kNorm) {
                     // inverse L2 norm of every row of the stacked K | Q tile: two threads per row, half the columns each
                     const int r = tid >> 1, hf = tid & 1;

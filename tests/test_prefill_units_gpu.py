@@ -67,3 +67,22 @@ def test_segmented_launches_without_a_second_segment():
     for _ in range(20):
         o, s = gdn.chunked_forward(*args, ci.flatten(), p["cu_chunks"])
         assert torch.equal(o, o_ref) and torch.equal(s, s_ref)
+
+
+@pytest.mark.parametrize("lens,kh,vh", [([70, 130, 40], 2, 4), ([1, 64, 1], 1, 3), ([2100, 1500, 900], 1, 2)])  # the last in segments
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_undefined_values_of_a_neighbour(lens, kh, vh, norm, what, bad):
+    """a packed sequence whose inputs are not finite: the sequences before and behind it keep their bits"""
+    import h100_gdn_cuda_b200 as gdn
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.varlen_inputs(lens, kh, vh, 128, seed=4, mild_gate=True).items()}
+    run = lambda: gdn.chunked_forward(p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], p["cu_seqlens"], p["chunk_indices"],
+                                      p["cu_chunks"], is_qk_norm=norm)
+    o0, s0 = run()
+    a, b = lens[0], lens[0] + lens[1]
+    p[what] = p[what].clone()
+    p[what][a:b] = bad
+    o1, s1 = run()
+    assert torch.equal(o0[:a], o1[:a]) and torch.equal(s0[0], s1[0])
+    assert torch.equal(o0[b:], o1[b:]) and torch.equal(s0[2], s1[2])
