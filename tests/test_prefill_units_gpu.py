@@ -1,6 +1,7 @@
-"""The chunk-parallel prefill kernel works out the coordinates of its work units 256 per CTA at a time.  More units than
-that (76 800 = 300 sequences x 8 chunks x 32 k-heads on 296 CTAs, 260 each): every sequence must come out with the bits it
-has in a call of its own.  Padded, and packed with ragged lengths."""
+"""The chunk-parallel prefill kernel works out the coordinates of its work units 64 per CTA at a time.  Exactly that
+many (74 sequences x 8 chunks x 32 k-heads on 296 CTAs), one more for most CTAs (75 sequences), and a table filled five times
+(300 sequences, 260 units each): every sequence must come out with the bits it has in a call of its own.  Padded, and packed with
+ragged lengths."""
 import pytest
 import torch
 
@@ -9,17 +10,18 @@ from h100_gdn_cuda_b200 import synthetic
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("B", [74, 75, 300])
 @pytest.mark.parametrize("packed", [False, True])
-def test_more_units_than_one_table(packed):
+def test_more_units_than_one_table(packed, B):
     import h100_gdn_cuda_b200 as gdn
-    B, T, H, d = 300, 512, 32, 16
+    T, H, d = 512, 32, 16
     g = torch.Generator(device="cuda").manual_seed(3)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)
     q, k = (torch.nn.functional.normalize(r(B * T, H, d), dim=-1).bfloat16() for _ in range(2))
     v, beta = r(B * T, H, d).bfloat16(), torch.sigmoid(r(B * T, H)).bfloat16()
     gate, s0 = -torch.nn.functional.softplus(r(B * T, H)), (r(B, H, d, d) * 0.02).bfloat16()
     if packed:
-        lens = [T - 1 if i % 2 else T + 1 for i in range(B)]  # 8 and 9 chunks
+        lens = [T - 1 if i % 2 else T + 1 for i in range(B - B % 2)] + [T] * (B % 2)  # 8 and 9 chunks
         cu = [0]
         for n in lens:
             cu.append(cu[-1] + n)
@@ -31,7 +33,7 @@ def test_more_units_than_one_table(packed):
         x4 = lambda x: x.view(B, T, *x.shape[1:])
         o, s = gdn.chunked_forward(x4(q), x4(k), x4(v), x4(beta), x4(gate), None, s0)
         o = o.view(B * T, H, d)
-    for i in (0, 1, 149, 290, 297, 299):
+    for i in (0, 1, B // 2, B - 10, B - 3, B - 1):
         sl = slice(cu[i], cu[i + 1])
         oi, si = gdn.chunked_forward(q[None, sl], k[None, sl], v[None, sl], beta[None, sl], gate[None, sl], None, s0[i:i + 1])
         assert torch.equal(oi[0], o[sl]) and torch.equal(si[0], s[i])
@@ -86,3 +88,24 @@ def test_undefined_values_of_a_neighbour(lens, kh, vh, norm, what, bad):
     o1, s1 = run()
     assert torch.equal(o0[:a], o1[:a]) and torch.equal(s0[0], s1[0])
     assert torch.equal(o0[b:], o1[b:]) and torch.equal(s0[2], s1[2])
+
+
+def test_packed_calls_back_to_back():
+    """Small packed batches whose calls follow one another without a pause: their blocks stay in L2, and the state kernel's warps can run
+    a whole chunk ahead of those that write the outputs.  No wait may run out (the status word), and every call has the bits of the first."""
+    import ctypes as C
+    import h100_gdn_cuda_b200 as gdn
+    from h100_gdn_cuda_b200 import _cabi
+    lens = [700, 70, 300, 64, 1, 900, 130, 33] * 4
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.varlen_inputs(lens, 4, 8, 128, seed=8, mild_gate=True).items()}
+    run = lambda: gdn.chunked_forward(p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], p["cu_seqlens"], p["chunk_indices"], p["cu_chunks"])
+    st = C.c_int(-1)
+    assert _cabi.load().gdn_device_status(0, C.byref(st)) == 0
+    o0, s0 = run()
+    differ = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(30):
+        outs = [run() for _ in range(10)]
+        for o, s in outs:
+            differ += (o != o0).sum() + (s != s0).sum()
+    assert differ.item() == 0
+    assert _cabi.load().gdn_device_status(0, C.byref(st)) == 0 and st.value == 0

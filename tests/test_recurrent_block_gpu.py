@@ -166,3 +166,66 @@ def test_packed_runs_of_unequal_length(gdn, lens, d, chunked):
             sl = slice(cu[i], cu[i + 1])
             oi, si = run([t[None, sl] for t in x], s0[i:i + 1])
             assert torch.equal(oi[0], o[sl]) and torch.equal(si[0], s[i]), n
+
+
+# The token recurrence for runs of more than 16 tokens and the blocks, each next to the line between them, on more CTAs than the GPU
+# holds at a time
+LINES = [(64, False, 17), (64, False, 40), (64, False, 41), (64, True, 40), (64, True, 41), (128, False, 17), (128, False, 24), (128, False, 25),
+         (128, True, 22), (128, True, 24), (128, True, 25), (192, False, 20), (192, False, 26), (192, False, 27), (256, False, 20), (256, False, 22), (256, False, 23)]
+
+
+@pytest.mark.parametrize("d,f32,T", LINES)
+def test_either_side_of_the_line(gdn, d, f32, T):
+    norm = T % 2 == 0
+    p, c = inputs(40, T, 4, 8, d, norm, d + T)
+    s0 = p["state"].float() + (1e-4 * torch.randn(p["state"].shape, generator=torch.Generator().manual_seed(1)) if f32 else 0.0)
+    o, s = gdn.recurrent_forward(c["q"], c["k"], c["v"], s0.cuda() if f32 else c["state"], c["beta"], c["g"], inference_mode=gdn.Decode,
+                                 is_qk_norm=norm)
+    o_ref, s_ref = O.recurrent_ref(p["q"].float(), p["k"].float(), p["v"].float(), p["beta"].float(), p["g"], s0, is_qk_norm=norm)
+    close(o, o_ref, REL, "O")
+    close(s, s_ref, REL32 if f32 else REL, "state")
+
+
+@pytest.mark.parametrize("d,f32,T", [l for l in LINES if l[2] > 17])
+def test_caps_pool_and_gating_either_side(gdn, d, f32, T):
+    """accepted-token caps, states in a pool with padding sequences, beta and the gate made inside"""
+    B, kh, vh = 24, 2, 4
+    gen = torch.Generator().manual_seed(d + T)
+    p, c = inputs(B, T, kh, vh, d, True, T)
+    A_log, dt_bias = torch.rand(vh, generator=gen).bfloat16(), torch.randn(vh, generator=gen).bfloat16()
+    a, b = torch.randn(B, T, vh, generator=gen).bfloat16(), torch.randn(B, T, vh, generator=gen).bfloat16()
+    nat = torch.randint(0, T + 1, (B,), generator=gen, dtype=torch.int32)
+    nat[0], nat[1], nat[2] = T, 0, 1
+    slots = torch.randperm(B + 6, generator=gen)[:B].int()
+    slots[5] = slots[17] = -1
+    pool = torch.randn(B + 6, vh, d, d, generator=gen) * 0.02
+    pool = pool if f32 else pool.bfloat16()
+    beta, g = O.gating_ref(A_log, dt_bias, a, b)
+    got = pool.cuda()
+    o, _ = gdn.recurrent_forward(c["q"], c["k"], c["v"], got, None, None, None, nat.cuda(), gdn.Decode, True,
+                                 gating=(A_log.cuda(), dt_bias.cuda(), a.cuda(), b.cuda()), state_indices=slots.cuda())
+    live = (slots >= 0).nonzero().flatten()
+    at = slots[live].long()
+    o_ref, s_ref = O.recurrent_ref(p["q"][live].float(), p["k"][live].float(), p["v"][live].float(), beta[live].float(), g[live], pool[at].float(),
+                                   is_qk_norm=True, num_accepted_tokens=nat[live])
+    rows = torch.arange(T)[None] < nat[live][:, None]
+    close(o.cpu()[live][rows], o_ref[rows], REL, "O")
+    # (the fast exponential and logarithm of the gating inside are a few units of 2^-22 off, which T tokens add up)
+    close(got[at], s_ref, REL32 + T * 2.0 ** -20 if f32 else REL, "pool")
+    rest = [i for i in range(B + 6) if i not in at.tolist()]
+    assert torch.equal(got[rest].cpu(), pool[rest])
+
+
+@pytest.mark.parametrize("d,f32", [(64, False), (64, True), (128, False), (128, True), (192, False), (256, False)])
+def test_packed_about_the_line(gdn, d, f32):
+    """packed runs of 0 to 44 tokens, 20 on average: sequences of either kernel, in every order"""
+    gen = torch.Generator().manual_seed(d)
+    lens = torch.randint(0, 45, (60,), generator=gen).tolist() + [16, 17, 22, 23, 24, 25, 26, 27, 40, 41] + [1] * 10
+    p = synthetic.varlen_inputs(lens, 2, 4, d, seed=d, mild_gate=True)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+    s0 = c["state"].float() if f32 else c["state"]
+    o, s = gdn.recurrent_forward(c["q"], c["k"], c["v"], s0, c["beta"], c["g"], cu_seqlens=c["cu_seqlens"], inference_mode=gdn.Decode)
+    o_ref, s_ref = O.recurrent_ref(p["q"].float(), p["k"].float(), p["v"].float(), p["beta"].float(), p["g"], p["state"].float(),
+                                   cu_seqlens=p["cu_seqlens"])
+    close(o, o_ref, REL, "O")
+    close(s, s_ref, REL32 if f32 else REL, "states")

@@ -149,7 +149,7 @@ def test_long_runs_step_states_and_accepted(gdn, d):
 
 
 def test_recurrent_varlen_short_and_long_sequences(gdn):
-    # one launch with sequences on both sides of the 16-token threshold (and an empty one)
+    # one call with sequences on both sides of 16 tokens and of the token-block kernel's 25 (and an empty one)
     lens = [40, 3, 0, 17, 100, 1, 16, 33]
     p = synthetic.varlen_inputs(lens, 2, 4, 128, seed=14, mild_gate=True)
     pd = dev(p)
