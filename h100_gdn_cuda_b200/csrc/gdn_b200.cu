@@ -169,29 +169,32 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
     return GDN_OK;
 }
 
-// Long runs of tokens whose last state alone is wanted: blocks of tokens on warp matrix instructions (recurrent_block.cuh) from
-// this many tokens on.  The sums go in another order there, so the choice is made by what belongs to the sequence - its tokens
+// Long runs of tokens whose last state alone is wanted, in bf16: blocks of tokens on warp matrix instructions (recurrent_block.cuh)
+// from this many tokens on.  The sums go in another order there, so the choice is made by what belongs to the sequence - its tokens
 // (before any cap), head dim, state type - and not by the batch, the heads or the other sequences: a sequence, or a shard's heads,
 // come out with the same bits alone and in company.  A second block with few tokens takes as long as a full one, and where the CTAs
 // fill the GPU the token recurrence is no slower up to here.  Token recurrence against blocks in us, B=64, L2 flushed: 32 v-heads
-// d=64 T=33 184 : 212, T=39 208 : 212, T=41 216 : 212 (fp32 states 185 : 213, 209 : 214, 217 : 212); d=128 T=23 385 : 397, T=25 414 : 395
-// (fp32 386 : 399, 414 : 398); 8 v-heads d=192 T=23 164 : 185, T=25 176 : 184, T=27 188 : 184 (B=8 the same at T=27); d=256 T=23 259 : 259.
-// With few CTAs the blocks would win earlier (B=1 d=128 T=17 14 us : 8).  Packed batches hold both kinds and take two launches, each
-// of which leaves the other's sequences out: 16 sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336, 8 of about 100 (32
-// v-heads, d=128) 113 -> 118; one of 1500 among 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31.
+// d=64 T=33 184 : 212, T=39 208 : 212, T=41 216 : 212; d=128 T=23 385 : 397, T=25 414 : 395; 8 v-heads d=192 T=23 164 : 185, T=25
+// 176 : 184, T=27 188 : 184 (B=8 the same at T=27); d=256 T=23 259 : 259.  With few CTAs the blocks would win earlier (B=1 d=128
+// T=17 14 us : 8).  Packed batches hold both kinds and take two launches, each of which leaves the other's sequences out: 16
+// sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336, 8 of about 100 (32 v-heads, d=128) 113 -> 118; one of 1500 among
+// 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31.
+// fp32 states stay with the token recurrence: in blocks (d=128, B=2 T=512 337 -> 136 us) the state, rounded once per block, was nearer to
+// 64 bits without decay (3.5e-7 of it -> 1.2e-7 after 1500 tokens) but further off with one, up to 40 % at a mean gate of -0.8
+// (6.1e-8 -> 8.5e-8): the matrix instructions cut their sums off.
 static int block_min_tokens(int dk, bool f32, bool steps, int ring_min) {
-    if (steps || (f32 && dk != 64 && dk != 128)) return kRecNoLongRun;
+    if (steps || f32) return kRecNoLongRun;
     const int from = dk == 64 ? 41 : dk == 128 ? 25 : dk == 192 ? 27 : dk == 256 ? 23 : kRecNoLongRun;
     return std::max(from, ring_min < kRecNoLongRun ? ring_min + 1 : kRecNoLongRun);
 }
-// The same kernel, compiled at run time (GDN_JIT_RECURRENT=1; bf16 states).
+// The same kernel, compiled at run time (GDN_JIT_RECURRENT=1).
 static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, int smem, unsigned grid, cudaStream_t st) {
     const char* const kind[3] = {"kPadded", "kPacked", "kWalk"};
     char src[512];
     snprintf(src, sizeof(src),
              "#include \"kernels/recurrent_block.cuh\"\n"
              "extern \"C\" __global__ void __launch_bounds__(%d, 2) gdn_recurrent_jit(const gdn::RecurrentParams p) {\n"
-             "    gdn::gdn_recurrent_block_body<%d, false, gdn::BlkUnits::%s>(p);\n}\n",
+             "    gdn::gdn_recurrent_block_body<%d, gdn::BlkUnits::%s>(p);\n}\n",
              kBlkThreads, dk, kind[static_cast<int>(units)]);
     jit::LoadedKernel k;
     std::string err;
@@ -204,7 +207,7 @@ static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, in
     GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(kBlkThreads), args, smem, st));
     return GDN_OK;
 }
-template <int DK, bool kF32, BlkUnits kUnits>
+template <int DK, BlkUnits kUnits>
 static int launch_block_t(const RecurrentParams& p, bool jit, long long grid, cudaStream_t st) {
     constexpr int smem = BlockSmem<DK>::kBytes;
     GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
@@ -213,33 +216,31 @@ static int launch_block_t(const RecurrentParams& p, bool jit, long long grid, cu
     int dev = 0;
     GDN_CUDA(cudaGetDevice(&dev));
     if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kF32, kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev & 63].store(true, std::memory_order_release);
     }
-    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kF32, kUnits>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
+    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kUnits>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
     return GDN_OK;
 }
 template <BlkUnits kUnits>
-static int launch_block_as(const RecurrentParams& p, int dk, bool f32, bool jit, long long grid, cudaStream_t st) {
-    switch (f32 ? -dk : dk) {
-        case 64: return launch_block_t<64, false, kUnits>(p, jit, grid, st);
-        case 128: return launch_block_t<128, false, kUnits>(p, jit, grid, st);
-        case 192: return launch_block_t<192, false, kUnits>(p, jit, grid, st);
-        case 256: return launch_block_t<256, false, kUnits>(p, jit, grid, st);
-        case -64: return launch_block_t<64, true, kUnits>(p, jit, grid, st);
-        case -128: return launch_block_t<128, true, kUnits>(p, jit, grid, st);
+static int launch_block_as(const RecurrentParams& p, int dk, bool jit, long long grid, cudaStream_t st) {
+    switch (dk) {
+        case 64: return launch_block_t<64, kUnits>(p, jit, grid, st);
+        case 128: return launch_block_t<128, kUnits>(p, jit, grid, st);
+        case 192: return launch_block_t<192, kUnits>(p, jit, grid, st);
+        case 256: return launch_block_t<256, kUnits>(p, jit, grid, st);
     }
     return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: no token-block kernel for dk = %d", dk);
 }
 // Packed mode: no more than total_tokens / long_run sequences can be that long.  Where that is all of them, a CTA per unit, as for
 // padded batches; otherwise a wave of CTAs walks the units (100 sequences of one token and one of 1500, d=256: 69 times the CTAs
 // there is work for).  The walk itself costs registers (d=256: 260 bytes spilled, 20 % of the time).
-static int launch_block(const RecurrentParams& p, int dk, bool f32, bool jit, long long total_tokens, int sms, cudaStream_t st) {
+static int launch_block(const RecurrentParams& p, int dk, bool jit, long long total_tokens, int sms, cudaStream_t st) {
     const long long per_seq = static_cast<long long>(p.vh) * (p.dv / kBlkRows);
-    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, f32, jit, p.batch * per_seq, st);
+    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, jit, p.batch * per_seq, st);
     const long long seqs = total_tokens / p.long_run;
-    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, f32, jit, p.batch * per_seq, st);
-    return launch_block_as<BlkUnits::kWalk>(p, dk, f32, jit, std::min(seqs * per_seq, 2ll * sms), st);
+    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, jit, p.batch * per_seq, st);
+    return launch_block_as<BlkUnits::kWalk>(p, dk, jit, std::min(seqs * per_seq, 2ll * sms), st);
 }
 
 // Head dimensions without a prebuilt kernel (or every call when GDN_JIT_RECURRENT=1) go through
@@ -582,7 +583,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     p.long_run = block_min_tokens(s.head_dim_k, f32, p.store_step != 0, ring_min);
     // (packed: no more tokens than sequences is a batch of single tokens)
     if (s.cu_seqlens ? s.total_tokens < p.long_run || s.total_tokens <= s.batch : s.seq_len < p.long_run) p.long_run = kRecNoLongRun;
-    if (p.long_run != kRecNoLongRun && !s.cu_seqlens) return launch_block(p, s.head_dim_k, f32, jit, 0, d->sms, st);
+    if (p.long_run != kRecNoLongRun && !s.cu_seqlens) return launch_block(p, s.head_dim_k, jit, 0, d->sms, st);
     auto token_recurrence = [&]() -> int {
         if (jit) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
         if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
@@ -603,7 +604,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     };
     if (int rc = token_recurrence()) return rc;
     // packed: the sequences that launch has left out
-    return p.long_run == kRecNoLongRun ? GDN_OK : launch_block(p, s.head_dim_k, f32, jit, s.total_tokens, d->sms, st);
+    return p.long_run == kRecNoLongRun ? GDN_OK : launch_block(p, s.head_dim_k, jit, s.total_tokens, d->sms, st);
 }
 
 }  // extern "C"

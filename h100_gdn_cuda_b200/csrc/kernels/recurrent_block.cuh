@@ -4,21 +4,22 @@
 //     c_t = beta_t v_t - beta_t G_t (S_0 k_t) - sum_{s<t} A_ts c_s,   A_ts = beta_t Gamma_ts (k_s.k_t)
 //     o_t = scale G_t (S_0 q_t) + sum_{s<=t} P_ts c_s,                P_ts = scale Gamma_ts (k_s.q_t)
 //     S  <- G_n S_0 + sum_s (Gamma_ns c_s) k_s^T
-// Precision is that of fp32 arithmetic.  The state stays in fp32 registers from the first token to the last; it enters
-// S_0 [k; q] as three bf16 terms, which is all 24 bits of it, and so do the coefficients of the update; k and q are the bf16
-// values they are (their norms are fp32 factors of the results).  Products of bf16 values are exact, their sums are fp32; the
-// solve and the outputs are fp32 FMAs; the update is added to the decayed state by one fp32 FMA per element and BLOCK, where
-// the token recurrence rounds the state at every token.
+// The state stays in fp32 registers from the first token to the last; it enters S_0 [k; q] as three bf16 terms, which is all 24 bits
+// of it, and so do the coefficients of the update; k and q are the bf16 values they are (their norms are fp32 factors of the
+// results).  Products of bf16 values are exact; sums inside a matrix instruction are cut off at about 24 bits, sums of their results
+// are rounded; the solve and the outputs are fp32 FMAs; the update is added to the decayed state by one fp32 FMA per element and BLOCK, where
+// the token recurrence rounds the state at every token.  Share of the bf16 outputs after 1000 tokens that are not the 64-bit value
+// rounded to bf16, token recurrence : here, d=256: no decay 4.1e-4 : 1.7e-4, mean gate -0.016 8.0e-4 : 7.8e-4, -0.16 1.8e-4 : 1.6e-4,
+// -0.8 9.0e-5 : 8.9e-5, -5 6.5e-5 : 5.4e-5.  (A state kept in fp32 outside would show the sums that are cut off: with a decay it was up to
+// 40 % further off than token by token, so those take the token recurrence.)
 //
 // Why: the token recurrence (recurrent.cuh, ring instance) is a chain of about 1 250 cycles per token, and a sequence of a
-// few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of products (1 000
-// cycles), sums and a triangular solve (850) and the update (500): B=2, T=1500, 8 v-heads, d=256 996 -> 233 us (253 with the
-// outputs written by the warps that hold the state, another 400 cycles of the chain), 4 v-heads B=1 994 -> 151, T=700, d=192
-// 401 -> 71, T=65 42 -> 12.7; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM issue
+// few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of some 3 000 cycles: products (1 000),
+// sums and a triangular solve (850), the update (500), and the barrier, the hand-over to the writing warps and the waits between them:
+// B=2, T=1500, 8 v-heads, d=256 996 -> 236 us (another 400 cycles a block with the outputs written by the warps that hold the state), 4 v-heads
+// B=1 994 -> 150, T=700, d=192 401 -> 66; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM issue
 // (5 100 warp instructions per block and CTA, 54 % of the slots), shared memory (1 270 wavefronts, as much) and the matrix
-// instructions (26 %) share the time without one of them filling it; with one CTA the chain does.  Against 64 bits an fp32 state
-// is off by 2.6e-7 instead of 2.9e-7 after 1500 tokens of weak decay, 1.2e-7 instead of 3.4e-7 without decay, 5.7e-8 instead of
-// 5.8e-8 with a strong one (d=128, relative 2-norm).
+// instructions (26 %) share the time without one of them filling it; with one CTA the chain does.
 //
 // A CTA owns 16 state rows (M of the products) of one (sequence, v-head) and walks its blocks:
 //   warps 0-3   a quarter of the columns each, kept as accumulator fragments, which are the A operands of the product
@@ -128,7 +129,7 @@ enum class BlkUnits {
     kPacked,  // a CTA per unit of as many sequences as can be that long; those past the last one end at once
     kWalk,    // packed, far fewer long sequences than could be: a wave of CTAs walks the units with a stride of the grid
 };
-template <int DK, bool kF32, BlkUnits kUnits = BlkUnits::kPadded>
+template <int DK, BlkUnits kUnits = BlkUnits::kPadded>
 __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& p) {
     constexpr bool kPacked = kUnits != BlkUnits::kPadded;
     using namespace ptx;
@@ -232,7 +233,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     // rows past the end of the sequence are filled with zeros (their address is that of the last row)
                     constexpr int kPieces = DK / 8;
                     const uint32_t dst = smem_u32(st);
-    #pragma unroll 4
+#pragma unroll 4
                     for (int i = lane; i < kBlkTok * kPieces; i += 32) {
                         const int row = i / kPieces, c = i % kPieces;
                         const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
@@ -250,25 +251,25 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 if (b >= 4) {
                     // ---- outputs of block b - 4.  Coefficients of later tokens are left out, not multiplied by zero: an infinite or
                     //      undefined value stays behind its token.
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const float* const P = pr + L::kP + (8 * h + i) * 16;
                         const float4 u = *reinterpret_cast<const float4*>(P), w = *reinterpret_cast<const float4*>(P + 4);
                         const float pw[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-    #pragma unroll
+#pragma unroll
                         for (int s = 0; s < 8; ++s)
                             if (s <= i || h) o[i] = fmaf(pw[s], c0[s], o[i]);
                         if (h) {
                             const float4 y = *reinterpret_cast<const float4*>(P + 8), z = *reinterpret_cast<const float4*>(P + 12);
                             const float pz[8] = {y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
-    #pragma unroll
+#pragma unroll
                             for (int s = 0; s <= i; ++s) o[i] = fmaf(pz[s], c1[s], o[i]);
                         }
                     }
                     __syncwarp();
                     const bool good = ok && *static_cast<volatile int*>(&abort_flag) == 0;  // nothing is stored once a wait has given up
                     const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 8; ++i)
                         if (good && i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
                 }
@@ -286,7 +287,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 if (!real) beta = 0.f;
                 fetch(b + 4);
                 float run = 1.f;
-    #pragma unroll
+#pragma unroll
                 for (int i = 0; i < kBlkTok; ++i) {
                     const float ai = __shfl_sync(0xffffffffu, a, i);
                     if (lane == 16 || lane < i) run *= ai;
@@ -297,23 +298,23 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 //      8 .. 15 of k; qq: the diagonals of q q^T.  The matrix instructions cut their sums off, so only two follow one another.
                 float kk[4] = {}, qk[4] = {}, hh[4] = {}, qq0[4] = {}, qq1[4] = {};
                 const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + lm_col * 2, qaddr = kaddr + L::kOffQ;
-    #pragma unroll 2
+#pragma unroll 2
                 for (int ks = 0; ks < DK / 16; ks += 2) {
                     uint32_t x[2][4], y[2][4];
-    #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         ldmatrix_x4(kaddr + 32 * (ks + e), x[e]);
                         ldmatrix_x4(qaddr + 32 * (ks + e), y[e]);
                     }
                     float s0[4] = {}, s1[4] = {}, s2[4] = {};
-    #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const uint32_t h[4] = {x[e][1], y[e][1], x[e][3], y[e][3]};
                         mma16f(s0, x[e], x[e][0], x[e][2]);
                         mma16f(s1, y[e], x[e][0], x[e][2]);
                         mma16f(s2, h, x[e][1], x[e][3]);
                     }
-    #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         kk[e] += s0[e];
                         qk[e] += s1[e];
@@ -321,12 +322,12 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     }
                     if (p.is_qk_norm) {
                         float s3[4] = {}, s4[4] = {};
-    #pragma unroll
+#pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             mma16f(s3, y[e], y[e][0], y[e][2]);
                             mma16f(s4, y[e], y[e][1], y[e][3]);
                         }
-    #pragma unroll
+#pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             qq0[e] += s3[e];
                             qq1[e] += s4[e];
@@ -356,7 +357,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     pr[L::kA + si * 16 + ti] = bt * w * kkv;
                     pr[L::kP + ti * 16 + si] = rq * w * qkv;
                 };
-    #pragma unroll
+#pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int s0 = 2 * t + e;
                     put(g, s0, kk[e], qk[e], beta_g * rk_g, rq_g);
@@ -378,7 +379,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     const float bt = __shfl_sync(0xffffffffu, beta, tk);
                     float* const R = X + 8 * (lane >> 4) * L::kLdR + tk;
                     const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
                         R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
@@ -395,23 +396,17 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             const long long srow = static_cast<long long>(rb * kBlkRows + g) * DK + col0 + 2 * t;
             if (p.state_in) {
                 const long long base = static_cast<long long>(slot) * p.si_ss + head * p.si_sh + srow;
-    #pragma unroll
+#pragma unroll
                 for (int i = 0; i < 2 * NK; ++i) {
-    #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        if (kF32) {
-                            const float2 w = *reinterpret_cast<const float2*>(static_cast<const float*>(p.state_in) + base + 8 * e * DK + 8 * i);
-                            S[i][2 * e] = w.x;
-                            S[i][2 * e + 1] = w.y;
-                        } else {
-                            const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.state_in) + base + 8 * e * DK + 8 * i);
-                            S[i][2 * e] = bf16_lo(w);
-                            S[i][2 * e + 1] = bf16_hi(w);
-                        }
+                        const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const __nv_bfloat16*>(p.state_in) + base + 8 * e * DK + 8 * i);
+                        S[i][2 * e] = bf16_lo(w);
+                        S[i][2 * e + 1] = bf16_hi(w);
                     }
                 }
             } else {
-    #pragma unroll
+#pragma unroll
                 for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
             }
             uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
@@ -431,14 +426,14 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     float dh[4][4], dl[4][4];
                     auto products = [&](auto safe_tag) {
                         constexpr bool kSafe = decltype(safe_tag)::value;
-    #pragma unroll
+#pragma unroll
                         for (int i = 0; i < 4; ++i)
-    #pragma unroll
+#pragma unroll
                             for (int e = 0; e < 4; ++e) dh[i][e] = dl[i][e] = 0.f;
                         uint32_t x[2][4], y[2][4];
                         ldmatrix_x4(kaddr, x[0]);
                         ldmatrix_x4(kaddr + L::kOffQ, y[0]);
-    #pragma unroll
+#pragma unroll
                         for (int kc = 0; kc < NK; ++kc) {
                             if (kc + 1 < NK) {
                                 ldmatrix_x4(kaddr + 32 * (kc + 1), x[(kc + 1) & 1]);
@@ -447,7 +442,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                             const uint32_t* const xk = x[kc & 1];
                             const uint32_t* const yk = y[kc & 1];
                             uint32_t hi[4], mid[4], lo[4];
-    #pragma unroll
+#pragma unroll
                             for (int e = 0; e < 4; ++e) {
                                 const float* s = &S[2 * kc + (e >> 1)][2 * (e & 1)];
                                 split3<kSafe>(s[0], s[1], hi[e], mid[e], lo[e]);
@@ -471,7 +466,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     const float chk = dl[0][0] + dl[0][2];
                     if (__any_sync(0xffffffffu, chk != chk)) products(Flag<true>{});
                     float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         *reinterpret_cast<float2*>(d + 8 * i) = make_float2(dh[i][0] + dl[i][0], dh[i][1] + dl[i][1]);
                         *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
@@ -483,17 +478,17 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 {
                     const float* const d = D + r * L::kLdD + 8 * h;
                     float sum[8];
-    #pragma unroll
+#pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         float4 x[4];
-    #pragma unroll
+#pragma unroll
                         for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float4*>(d + w * (kBlkRows * L::kLdD) + 4 * q);
                         sum[4 * q] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
                         sum[4 * q + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
                         sum[4 * q + 2] = (x[0].z + x[1].z) + (x[2].z + x[3].z);
                         sum[4 * q + 3] = (x[0].w + x[1].w) + (x[2].w + x[3].w);
                     }
-    #pragma unroll
+#pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + r * L::kLdR + 8 * h + 4 * q);
                         const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
@@ -512,40 +507,40 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 // (what a token gets from the tokens before it is summed apart from its own, larger, term)
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 auto substitute = [&](int half) {
-    #pragma unroll
+#pragma unroll
                     for (int s = 0; s < 8; ++s) {
                         c[s] -= acc[s];
                         if (s == 7) break;
                         float x[8];
                         col_of(8 * half + s, half, x);
-    #pragma unroll
+#pragma unroll
                         for (int i = s + 1; i < 8; ++i) acc[i] = fmaf(x[i], c[s], acc[i]);
                     }
                 };
                 if (h == 0) substitute(0);
                 __syncwarp();
                 float c0[8];
-    #pragma unroll
+#pragma unroll
                 for (int i = 0; i < 8; ++i) c0[i] = __shfl_sync(0xffffffffu, c[i], r);
                 if (h == 1) {
-    #pragma unroll
+#pragma unroll
                     for (int s = 0; s < 8; ++s) {
                         float x[8];
                         col_of(s, 1, x);
-    #pragma unroll
+#pragma unroll
                         for (int i = 0; i < 8; ++i) acc[i] = fmaf(x[i], c0[s], acc[i]);
                     }
                     substitute(1);
                 }
                 if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 8; ++i) c[i] = 8 * h + i < n ? c[i] : 0.f;
                 }
                 __syncwarp();
                 // ---- S <- G S + sum_s (Gamma_ns r_s c_s) k_s^T
                 {
                     uint32_t hi[4], mid[4], lo[4];
-    #pragma unroll
+#pragma unroll
                     for (int q = 0; q < 2; ++q) {
                         const float4 w = *reinterpret_cast<const float4*>(pr + L::kW + 8 * h + 4 * q);
                         split3<true>(w.x * c[4 * q], w.y * c[4 * q + 1], hi[2 * q], mid[2 * q], lo[2 * q]);
@@ -561,7 +556,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     ldmatrix_x4(caddr + kBlkRows * L::kRowC, mid);
                     ldmatrix_x4(caddr + 2 * kBlkRows * L::kRowC, lo);
                     const float G = pr[L::kG];
-    #pragma unroll
+#pragma unroll
                     for (int kc = 0; kc < NK; ++kc) {
                         uint32_t x[4];
                         ldmatrix_x4_trans(kaddr + 32 * kc, x);  // tokens of k in pairs, columns 0 - 7 and 8 - 15
@@ -574,7 +569,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         mma16f(f1, hi, x[2], x[3]);
                         mma16f(e0, mid, x[0], x[1]);
                         mma16f(e1, mid, x[2], x[3]);
-    #pragma unroll
+#pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             S[2 * kc][e] = fmaf(G, S[2 * kc][e], f0[e] + e0[e]);
                             S[2 * kc + 1][e] = fmaf(G, S[2 * kc + 1][e], f1[e] + e1[e]);
@@ -586,7 +581,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     const int i = 32 * warp + lane, row = i >> 3, t2 = 2 * (i & 7);
                     const float* const d = D + row * L::kLdD + 16 + t2;
                     float2 x[4];
-    #pragma unroll
+#pragma unroll
                     for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
                     const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
                     ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
@@ -602,14 +597,11 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             }
             if (ok && *static_cast<volatile int*>(&abort_flag) == 0) {
                 const long long base = static_cast<long long>(slot) * p.so_ss + head * p.so_sh + srow;
-    #pragma unroll
+#pragma unroll
                 for (int i = 0; i < 2 * NK; ++i) {
-    #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        if (kF32)
-                            *reinterpret_cast<float2*>(static_cast<float*>(p.state_out) + base + 8 * e * DK + 8 * i) = make_float2(S[i][2 * e], S[i][2 * e + 1]);
-                        else
-                            *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.state_out) + base + 8 * e * DK + 8 * i) = pack_bf16(S[i][2 * e], S[i][2 * e + 1]);
+                        *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.state_out) + base + 8 * e * DK + 8 * i) = pack_bf16(S[i][2 * e], S[i][2 * e + 1]);
                     }
                 }
             }
@@ -658,9 +650,9 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     }
 }
 
-template <int DK, bool kF32 = false, BlkUnits kUnits = BlkUnits::kPadded>
+template <int DK, BlkUnits kUnits = BlkUnits::kPadded>
 __global__ void __launch_bounds__(kBlkThreads, 2) gdn_recurrent_block_kernel(const RecurrentParams p) {
-    gdn_recurrent_block_body<DK, kF32, kUnits>(p);
+    gdn_recurrent_block_body<DK, kUnits>(p);
 }
 
 }  // namespace gdn

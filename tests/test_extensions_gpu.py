@@ -220,7 +220,7 @@ def test_indexed_state_pool(gdn, T):
 @pytest.mark.parametrize("B,T,kh,vh,d", [(6, 1, 2, 4, 128), (3, 4, 2, 4, 64), (2, 40, 1, 2, 128)])
 def test_fp32_state(gdn, B, T, kh, vh, d):
     """A state kept in fp32: read, updated and returned as fp32 (decode, a few tokens, and a run long enough for
-    the token-block kernel).  The state is compared with a tighter gate than bf16 states allow."""
+    the multi-token instance).  The state is compared with a tighter gate than bf16 states allow."""
     p = synthetic.decode_inputs(B, T, kh, vh, d, seed=51 + T)
     beta, g = O.gating_ref(p["A_log"], p["dt_bias"], p["a"], p["b"])
     s0 = p["state"].float() + 1e-4 * torch.randn(p["state"].shape, generator=torch.Generator().manual_seed(1))  # not bf16-exact

@@ -1,6 +1,6 @@
 """Long runs of tokens through recurrent_forward (blocks of 16 tokens, the state in fp32 from the first token to the last)
 against the fp32 oracle.  bf16 results are off by their rounding, 2^-9 relative per element at most; the rest are sums of at
-most 256 products in fp32, 64 terms of 2^-17 in the worst direction: 2^-9 + 2^-11.  An fp32 state has no rounding to bf16:
+most 256 products in fp32, 64 terms of 2^-17 in the worst direction: 2^-9 + 2^-11.  An fp32 state (token by token) has no rounding to bf16:
 sums of 256 products rounded to 2^-24 each, added up over the tokens a state remembers, 2^-24 * 256 = 2^-16.
 """
 import pytest
@@ -229,3 +229,15 @@ def test_packed_about_the_line(gdn, d, f32):
                                    cu_seqlens=p["cu_seqlens"])
     close(o, o_ref, REL, "O")
     close(s, s_ref, REL32 if f32 else REL, "states")
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_fp32_state_is_the_token_recurrences(gdn, d):
+    """The matrix instructions cut their sums off, which an fp32 state would show: it is advanced token by token whatever the run's
+    length, with the bits of the last one where a state per token is kept."""
+    B, T, kh, vh = 2, 100, 2, 4
+    x = [t.view(B, T, *t.shape[1:]) for t in flat_inputs(B * T, kh, vh, d, d)]
+    s0 = torch.randn(B, vh, d, d, device="cuda") * 0.02
+    o, s = gdn.recurrent_forward(*x[:3], s0, *x[3:], inference_mode=gdn.Decode)
+    o1, steps = gdn.recurrent_forward(*x[:3], s0, *x[3:], inference_mode=gdn.SpecVerify)
+    assert torch.equal(o, o1) and torch.equal(s, steps[:, -1])
