@@ -59,7 +59,7 @@ struct ZPSmem {
     static constexpr int kTeam = kAtoms * 16384;         // per-team area starts here, two of them
     static constexpr int kOffT = 0, kOffTd = 8192;       // T and dT (8 KB each), later the staged Z
     static constexpr int kOffP = 16384;                  // P tile (8 KB), later the staged PT
-    // 16x16 blocks of A below the diagonal, block (r, c) at r (r - 1) / 2 + c, as two bf16 terms: see blk_off
+    // 16x16 blocks of A below the diagonal, block (r, c) at r (r - 1) / 2 + c, as two bf16 terms
     static constexpr int kOffA = kOffP + 8192;
     // diagonal blocks of A in fp32, 20 floats per row; each makes way for its inverse as two bf16 terms
     static constexpr int kLdD = 20, kDiag = 16 * kLdD * 4;
@@ -83,27 +83,19 @@ constexpr uint32_t kTmPT = 64;   // PT of team 0 (lanes +0) and team 1 (lanes +1
 constexpr uint32_t kTmZ = 128;   // Z, 128 columns (lanes +0: team 0, +16: team 1)
 // the two warps of a team that write P
 __device__ __forceinline__ void pair_sync(int team) { asm volatile("bar.sync %0, 64;" ::"r"(3 + team) : "memory"); }
-// TF32 operands of the inverse's block products: 16x8 fragment of `m` at [r0][k0] as the A operand (kRows 8: the lower
-// half is zero), 8x8 at [k0][n0] as the B operand
-template <int kRows = 16>
-__device__ __forceinline__ void load_a(uint32_t* a, const float* m, int ld, int r0, int k0, int lane) {
+// TF32 operands of the 8 -> 16 step of the inverse: 8x8 block of `m` at [r0][k0] as the upper half of the A operand (the lower is
+// zero), at [k0][n0] as the B operand
+__device__ __forceinline__ void load_a8(uint32_t* a, const float* m, int ld, int r0, int k0, int lane) {
     const int g = lane >> 2, t = lane & 3;
     a[0] = uw::to_tf32(m[(r0 + g) * ld + k0 + t]);
-    a[1] = kRows == 16 ? uw::to_tf32(m[(r0 + g + 8) * ld + k0 + t]) : 0u;
+    a[1] = 0u;
     a[2] = uw::to_tf32(m[(r0 + g) * ld + k0 + t + 4]);
-    a[3] = kRows == 16 ? uw::to_tf32(m[(r0 + g + 8) * ld + k0 + t + 4]) : 0u;
+    a[3] = 0u;
 }
-__device__ __forceinline__ void load_b(uint32_t* b, const float* m, int ld, int k0, int n0, int lane) {
+__device__ __forceinline__ void load_b8(uint32_t* b, const float* m, int ld, int k0, int n0, int lane) {
     const int g = lane >> 2, t = lane & 3;
     b[0] = uw::to_tf32(m[(k0 + t) * ld + n0 + g]);
     b[1] = uw::to_tf32(m[(k0 + t + 4) * ld + n0 + g]);
-}
-template <int kRows = 16>
-__device__ __forceinline__ void mma_blk(float* d, const float* am, int r0, int k0, const float* bm, int k0b, int n0, int ld, int lane) {
-    uint32_t a[4], b[2];
-    load_a<kRows>(a, am, ld, r0, k0, lane);
-    load_b(b, bm, ld, k0b, n0, lane);
-    uw::mma_tf32(d, a, b);
 }
 __device__ __forceinline__ void team_sync(int team) {
     if (team)
@@ -111,9 +103,8 @@ __device__ __forceinline__ void team_sync(int team) {
     else
         asm volatile("bar.sync 1, 128;" ::: "memory");
 }
-// A 16x16 block as two bf16 terms: 16 rows of 64 bytes, 16-byte pieces { first terms of columns 0-7, 8-15, second terms of
-// the same }, swizzled so that one piece of eight rows covers all banks.
-__device__ __forceinline__ uint32_t blk_off(int row, int piece) { return static_cast<uint32_t>(row * 64 + ((piece ^ ((row >> 1) & 3)) << 4)); }
+// A 16x16 block as two bf16 terms: 16 rows of 64 bytes (row64_off), 16-byte pieces { first terms of columns 0-7, 8-15, second terms
+// of the same }.
 // two fp32 values as two bf16 terms each
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
     hi = pack_bf16(x0, x1);
@@ -124,23 +115,18 @@ __device__ __forceinline__ void split_frag(const float (*x)[4], uint32_t* hi, ui
 #pragma unroll
     for (int i = 0; i < 4; ++i) split2(x[i >> 1][2 * (i & 1)], x[i >> 1][2 * (i & 1) + 1], hi[i], lo[i]);
 }
-__device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// acc += X B for 16x16 blocks: X as fragments of two terms, B in shared memory (blk_off); the product of the second terms is
+// acc += X B for 16x16 blocks: X as fragments of two terms, B in shared memory (row64_off); the product of the second terms is
 // below 2^-16 of the result
 __device__ __forceinline__ void mma_blk16(float (*acc)[4], const uint32_t* xh, const uint32_t* xl, uint32_t b_saddr, int lane) {
     uint32_t bh[4], bl[4];  // { columns 0-7: rows 0-7, 8-15; columns 8-15: the same }
-    ldmatrix_x4_trans(b_saddr + blk_off(lane & 15, lane >> 4), bh);
-    ldmatrix_x4_trans(b_saddr + blk_off(lane & 15, 2 + (lane >> 4)), bl);
-    mma_bf16(acc[0], xl, bh[0], bh[1]);
-    mma_bf16(acc[1], xl, bh[2], bh[3]);
-    mma_bf16(acc[0], xh, bl[0], bl[1]);
-    mma_bf16(acc[1], xh, bl[2], bl[3]);
-    mma_bf16(acc[0], xh, bh[0], bh[1]);
-    mma_bf16(acc[1], xh, bh[2], bh[3]);
+    ldmatrix_x4_trans(b_saddr + row64_off(lane & 15, lane >> 4), bh);
+    ldmatrix_x4_trans(b_saddr + row64_off(lane & 15, 2 + (lane >> 4)), bl);
+    mma_16816(acc[0], xl, bh[0], bh[1]);
+    mma_16816(acc[1], xl, bh[2], bh[3]);
+    mma_16816(acc[0], xh, bl[0], bl[1]);
+    mma_16816(acc[1], xh, bl[2], bl[3]);
+    mma_16816(acc[0], xh, bh[0], bh[1]);
+    mma_16816(acc[1], xh, bh[2], bh[3]);
 }
 // Row block R of X = (I + A)^-1 from its diagonal block on, right to left.  x: fragments of the blocks X_R0 .. X_RR.
 template <int R>
@@ -429,8 +415,9 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 // ---- A = tril(beta_i (k_i.k_j) e^{g_i-g_j}, -1) (warps 0, 1 of the team) and P = scale tril((q_i.k_j) e^{g_i-g_j})
                 //      as a bf16 tile (warps 2, 3), 16x16 block by block as accumulator fragments: a warp has two rows of blocks and
                 //      nothing of what lies above the diagonal is touched.  A: the diagonal blocks in fp32, the others as two bf16 terms.
-                //      In a block below the diagonal e^{g_i-g_j} = e^{g_i-g_r} e^{g_r-g_j} with r the first of its rows, both factors
-                //      <= 1 (the cumulative gate only falls): the column factors come from a table, no ex2 is left per element.
+                //      In a block below the diagonal e^{g_i-g_j} = e^{g_i-g_r} e^{g_r-g_j} with r the first of its rows: the column factors
+                //      come from a table, no ex2 is left per element.  Both factors are <= 1 while the cumulative gate falls.  Where it rises
+                //      they are entries of the same matrices (tokens i and r, r and j): neither is infinite unless the exact result is.
                 {
                     const bool is_p = tw >= 2;
                     const int g = lane >> 2, tq = lane & 3;
@@ -490,8 +477,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                                 uint32_t hi[4], lo[4];
                                 split_frag(o, hi, lo);
                                 const uint32_t ob = smem_u32(tbase + L::kOffA + (r * (r - 1) / 2 + c) * 1024);
-                                stmatrix_x4(ob + blk_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
-                                stmatrix_x4(ob + blk_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
+                                stmatrix_x4(ob + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+                                stmatrix_x4(ob + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
                             }
                         };
                         constexpr std::false_type below{};
@@ -569,14 +556,18 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     __syncwarp();
                     // 8 -> 16
                     float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_blk<8>(d, sA, 8, 0, sA, 0, 0, LD, lane);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
+                    uint32_t bfrag[2], afrag[4];
+                    load_a8(afrag, sA, LD, 8, 0, lane);
+                    load_b8(bfrag, sA, LD, 0, 0, lane);
+                    mma_tf32(d, afrag, bfrag);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
                     // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
                     const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
                     const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
                     const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
                     const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
-                    uint32_t bfrag[2] = {to_tf32((g & 1) ? v01 : v00), to_tf32((g & 1) ? v11 : v10)}, afrag[4];
-                    load_a<8>(afrag, sA, LD, 8, 8, lane);
+                    bfrag[0] = to_tf32((g & 1) ? v01 : v00);
+                    bfrag[1] = to_tf32((g & 1) ? v11 : v10);
+                    load_a8(afrag, sA, LD, 8, 8, lane);
                     const float2 c00 = *reinterpret_cast<const float2*>(&sA[g * LD + 2 * tq]);
                     const float2 c11 = *reinterpret_cast<const float2*>(&sA[(8 + g) * LD + 8 + 2 * tq]);
                     float e[4] = {0.f, 0.f, 0.f, 0.f};
@@ -587,8 +578,8 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     uint32_t hi[4], lo[4];
                     split_frag(xd, hi, lo);
                     const uint32_t ia = smem_u32(sA);
-                    stmatrix_x4(ia + blk_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
-                    stmatrix_x4(ia + blk_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
+                    stmatrix_x4(ia + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+                    stmatrix_x4(ia + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
                 }
                 team_sync(team);
                 // ---- the row block's other blocks, then T = X diag(beta) and dT = diag(d) T as bf16 swizzled tiles (row = token i,

@@ -89,18 +89,10 @@ __device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_
     mid = __byte_perm(w0, w1, 0x7632);
     lo = __byte_perm(__float_as_uint(r0 - __uint_as_float(w0 & 0xFFFF0000u)), __float_as_uint(r1 - __uint_as_float(w1 & 0xFFFF0000u)), 0x7632);
 }
-// (not volatile: results of their operands alone, to be scheduled freely)
-__device__ __forceinline__ void mma16f(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes below 16: zeros for the rest
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// 16-byte piece `c` of row `r` of such a 16 x 16 fp32 tile: eight rows of a piece lie in different banks
-__device__ __forceinline__ uint32_t piece_off(int r, int c) { return static_cast<uint32_t>(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 // this thread's arrival at `bar` once all its copies so far have landed
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -220,8 +212,8 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 if (b >= 4) {  // block b - 4 is through: what its outputs are made of
                     ok = mbar_wait(&done[j], (it - 1) & 1u, &abort_flag) && ok;
                     auto row8 = [&](int off, int c, float* x) {
-                        const float4 u = *reinterpret_cast<const float4*>(st + off + piece_off(r, c));
-                        const float4 w = *reinterpret_cast<const float4*>(st + off + piece_off(r, c + 1));
+                        const float4 u = *reinterpret_cast<const float4*>(st + off + row64_off(r, c));
+                        const float4 w = *reinterpret_cast<const float4*>(st + off + row64_off(r, c + 1));
                         x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
                     };
                     row8(L::kOffO, 2 * h, o);
@@ -310,9 +302,9 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const uint32_t h[4] = {x[e][1], y[e][1], x[e][3], y[e][3]};
-                        mma16f(s0, x[e], x[e][0], x[e][2]);
-                        mma16f(s1, y[e], x[e][0], x[e][2]);
-                        mma16f(s2, h, x[e][1], x[e][3]);
+                        mma_16816(s0, x[e], x[e][0], x[e][2]);
+                        mma_16816(s1, y[e], x[e][0], x[e][2]);
+                        mma_16816(s2, h, x[e][1], x[e][3]);
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -324,8 +316,8 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         float s3[4] = {}, s4[4] = {};
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            mma16f(s3, y[e], y[e][0], y[e][2]);
-                            mma16f(s4, y[e], y[e][1], y[e][3]);
+                            mma_16816(s3, y[e], y[e][0], y[e][2]);
+                            mma_16816(s4, y[e], y[e][1], y[e][3]);
                         }
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
@@ -447,18 +439,18 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                                 const float* s = &S[2 * kc + (e >> 1)][2 * (e & 1)];
                                 split3<kSafe>(s[0], s[1], hi[e], mid[e], lo[e]);
                             }
-                            mma16f(dl[0], lo, xk[0], xk[2]);
-                            mma16f(dl[1], lo, xk[1], xk[3]);
-                            mma16f(dl[2], lo, yk[0], yk[2]);
-                            mma16f(dl[3], lo, yk[1], yk[3]);
-                            mma16f(dh[0], hi, xk[0], xk[2]);
-                            mma16f(dh[1], hi, xk[1], xk[3]);
-                            mma16f(dh[2], hi, yk[0], yk[2]);
-                            mma16f(dh[3], hi, yk[1], yk[3]);
-                            mma16f(dl[0], mid, xk[0], xk[2]);
-                            mma16f(dl[1], mid, xk[1], xk[3]);
-                            mma16f(dl[2], mid, yk[0], yk[2]);
-                            mma16f(dl[3], mid, yk[1], yk[3]);
+                            mma_16816(dl[0], lo, xk[0], xk[2]);
+                            mma_16816(dl[1], lo, xk[1], xk[3]);
+                            mma_16816(dl[2], lo, yk[0], yk[2]);
+                            mma_16816(dl[3], lo, yk[1], yk[3]);
+                            mma_16816(dh[0], hi, xk[0], xk[2]);
+                            mma_16816(dh[1], hi, xk[1], xk[3]);
+                            mma_16816(dh[2], hi, yk[0], yk[2]);
+                            mma_16816(dh[3], hi, yk[1], yk[3]);
+                            mma_16816(dl[0], mid, xk[0], xk[2]);
+                            mma_16816(dl[1], mid, xk[1], xk[3]);
+                            mma_16816(dl[2], mid, yk[0], yk[2]);
+                            mma_16816(dl[3], mid, yk[1], yk[3]);
                         }
                     };
                     products(Flag<false>{});
@@ -563,12 +555,12 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         // first terms and the others apart: the matrix instructions cut their sums off, which the short sums of first
                         // terms lose next to nothing by, and an fp32 addition rounds
                         float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f}, f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f};
-                        mma16f(e0, lo, x[0], x[1]);
-                        mma16f(e1, lo, x[2], x[3]);
-                        mma16f(f0, hi, x[0], x[1]);
-                        mma16f(f1, hi, x[2], x[3]);
-                        mma16f(e0, mid, x[0], x[1]);
-                        mma16f(e1, mid, x[2], x[3]);
+                        mma_16816(e0, lo, x[0], x[1]);
+                        mma_16816(e1, lo, x[2], x[3]);
+                        mma_16816(f0, hi, x[0], x[1]);
+                        mma_16816(f1, hi, x[2], x[3]);
+                        mma_16816(e0, mid, x[0], x[1]);
+                        mma_16816(e1, mid, x[2], x[3]);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             S[2 * kc][e] = fmaf(G, S[2 * kc][e], f0[e] + e0[e]);
@@ -585,11 +577,11 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
                     const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
                     ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
-                    *reinterpret_cast<float2*>(st + L::kOffO + piece_off(row, t2 >> 2) + 4 * (t2 & 2)) =
+                    *reinterpret_cast<float2*>(st + L::kOffO + row64_off(row, t2 >> 2) + 4 * (t2 & 2)) =
                         make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
                     if (warp == (b & 3)) {
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + piece_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + row64_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + row64_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
                     }
                 }
                 __syncwarp();

@@ -360,6 +360,14 @@ GDN_DEVICE void tmem_st_frag16(uint32_t taddr, const uint32_t* r) {
                  "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
+// d += a b: 16 x 16 bf16 fragments of a, 16 x 8 of b (not volatile: the result of its operands alone, to be scheduled freely)
+GDN_DEVICE void mma_16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// 16-byte piece `c` (0 .. 3) of row `r` of a tile with 64-byte rows: eight rows of one piece lie in different banks
+GDN_DEVICE uint32_t row64_off(int r, int c) { return static_cast<uint32_t>(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
 // Four 8x8 bf16 blocks between shared memory and fragments, transposed: lane 8m + r gives the address of row r of block m,
 // register m of lane l holds rows 2(l%4), 2(l%4)+1 of column l/4.
 GDN_DEVICE void ldmatrix_x4_trans(uint32_t saddr, uint32_t* r) {
