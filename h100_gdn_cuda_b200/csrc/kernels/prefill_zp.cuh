@@ -26,8 +26,8 @@
 // What bounds it: the latency of a unit's dependent phases (11 200 cycles with four teams per SM, 8 700 with two; before
 // 12 100).  The doubling scheme had ten barriers per unit (five now), 5 660 warp instructions (4 990) and 1 808 wavefronts (1 220) of
 // shared-memory accesses, besides some 900 of MMA operands and copies, of the 3 000 cycles a unit took an SM.
-// B=4 T=4096, 32 v-heads, whole step 200.1 -> 194.8 us; 16 packed sequences of 32768 tokens 427 -> 403; B=2 T=131072, 4 v-heads 592 ->
-// 572 (one GPU).
+// Whole calls with the doubling scheme and now, in turn on one GPU: B=4 T=4096, 32 v-heads 215.4 -> 210.3 us; 16 packed sequences of 32768
+// tokens 457.6 -> 437.9; B=2 T=131072, 4 v-heads 621.7 -> 599.9.
 // Persistent CTAs, two per SM (111 KB of shared memory, 256 tensor-memory columns each).
 #pragma once
 #include <cuda.h>
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
             // ---- K K^T (lanes 0-63) and Q K^T (lanes 64-127): once per unit, shared by its v-heads
             if (rd == 0) {
                 mbar_wait(bar_load, it & 1u, abort_flag);
-                if (n < kChunk) {
-                    // Keys past the end, in packed mode another sequence's, meet zero rows of dT in Z; cleared all the same, so that no
-                    // infinity or NaN of a neighbour can enter.
+                if (p.map.cu_seqlens && n < kChunk) {
+                    // Keys past the end are another sequence's (in padded mode the copies deliver zeros).  They meet zero rows of dT in Z, and are
+                    // cleared all the same, so that no infinity or NaN of a neighbour can enter.
                     for (int i = tid; i < (kChunk - n) * 8 * NA; i += kThreads)
                         *reinterpret_cast<uint4*>(sKQ + (i & (NA - 1)) * 16384 + (n + i / (8 * NA)) * 128 + ((i / NA) & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
                     fence_proxy_async_smem();
