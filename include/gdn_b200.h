@@ -174,7 +174,11 @@ int gdn_transpose_mn_major(const void* input, void* output, int32_t elem_size, i
  *                           state_in and writes the new one to the same slot of state_out (addressed
  *                           slot*stride_seq; the two may be the same pool).  A negative slot marks a padding
  *                           sequence: nothing is read, computed or written for it.  Not combined with
- *                           store_step_state. */
+ *                           store_step_state.
+ * Runs of many tokens without store_step_state, on bf16 states of dk 64, 128, 192 or 256, go through another
+ * kernel that sums in another order.  Which one a sequence takes depends on its own number of tokens (before
+ * any cap) alone: for 9 tokens and more the bits of its results are the same in any batch, padded or packed,
+ * and for any subset of the heads. */
 typedef struct {
     GdnShape shape;
     GdnTokenTensor q, k, v, out;
@@ -253,7 +257,10 @@ int gdn_compute_o(const GdnComputeOArgs* args, gdn_stream_t stream);
  * 128 is taken as it is (the tensor maps deliver zero columns past it, states are d x d; no padded copies),
  * callers zero-pad other head dims below 128;
  * dk = dv = 192 or 256 are accepted as well and run on the kernel of gdn_recurrent_forward
- * (no workspace: gdn_chunked_forward_workspace_bytes returns 0; final_state.ptr must be given). */
+ * (no workspace: gdn_chunked_forward_workspace_bytes returns 0; final_state.ptr must be given).
+ * Gates may have either sign, but e^(sum of the gates) from any token of a 64-token chunk to any later one
+ * is formed in fp32: where such a sum exceeds 88 the results of the sequence are not finite (a layer's own
+ * gates are never positive). */
 typedef struct {
     GdnShape shape;
     GdnTokenTensor q, k, v, out;
