@@ -136,6 +136,15 @@ __device__ __forceinline__ uint32_t tile_off(int row, int c16) {
     return static_cast<uint32_t>((c16 >> 3) * 8192 + row * 128 + (((c16 & 7) ^ (row & 7)) << 4));
 }
 
+// Rows [n, 64) of such a tile, in packed mode the tokens of the next sequence, set to zero by all threads of the CTA.  They meet zero
+// rows or columns of the other operand, but zero times an infinity or a NaN of a neighbour is a NaN.  (The caller fences and
+// synchronises before the tile is read.)
+template <int THREADS>
+__device__ __forceinline__ void clear_tile_rows(uint8_t* tile, int n, int tid) {
+    for (int i = max(n, 0) * 16 + tid; i < kChunk * 16; i += THREADS)
+        *reinterpret_cast<uint4*>(tile + (i & 1) * 8192 + (i >> 1) * 16) = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Row-predicated copy of rows [0, n) of such a tile to global memory (used where a TMA store
 // would write past the end of a packed sequence).
 // `pieces`: 16-byte pieces of a row that exist in the destination (head dim / 8).

@@ -103,6 +103,11 @@ __global__ void __launch_bounds__(128, 2) gdn_o_kernel(const __grid_constant__ C
     __syncthreads();
 
     mbar_wait(bar_load, 0, abort_flag);
+    if (p.map.cu_seqlens && n < kChunk) {
+        clear_tile_rows<128>(sU, n, tid);
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
     const uint32_t tLo = tmem, tHi = tmem + (16u << 16);
     if (warp == 0) {
         tc_fence_after_sync();

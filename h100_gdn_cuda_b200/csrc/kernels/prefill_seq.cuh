@@ -249,6 +249,12 @@ __global__ void __launch_bounds__(256, 1) gdn_seq_kernel(const __grid_constant__
 
         // ---- first wave of MMAs
         mbar_wait(&bar_full[stage], static_cast<uint32_t>((c >> 1) & 1), &abort_flag);
+        if (p.map.cu_seqlens && n < kChunk) {
+            clear_tile_rows<256>(st + L::kOffK, n, tid);
+            clear_tile_rows<256>(st + L::kOffU, n, tid);
+            fence_proxy_async_smem();
+            __syncthreads();
+        }
         if (tid == 0) {
             tc_fence_after_sync();
             if (kComputeO) {

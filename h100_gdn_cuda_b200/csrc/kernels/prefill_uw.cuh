@@ -214,6 +214,12 @@ __global__ void __launch_bounds__(128, 4) gdn_uw_kernel(const __grid_constant__ 
 
     // ---- A_raw = K K^T, columns 0-31 into lanes +0 and columns 32-63 into lanes +16
     mbar_wait(bar_load, load_par0, abort_flag);
+    if (p.map.cu_seqlens && n < kChunk) {
+        clear_tile_rows<128>(sK, n, tid);
+        clear_tile_rows<128>(sV, n, tid);
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
     // Every accumulator has its own issuing warp (warp-uniform issue, one elected lane): the issue
     // rate of one warp, not the tensor pipe, is what bounds these small MMAs.
     //   warp 0: K K^T columns 0-31 (lanes +0)    warp 1: K K^T columns 32-63 (lanes +16)

@@ -90,6 +90,34 @@ def test_undefined_values_of_a_neighbour(lens, kh, vh, norm, what, bad):
     assert torch.equal(o0[b:], o1[b:]) and torch.equal(s0[2], s1[2])
 
 
+@pytest.mark.parametrize("what", ["k", "v"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_undefined_values_of_a_neighbour_stage_by_stage(what, bad):
+    """the same for the stage kernels of the low-level functions"""
+    import h100_gdn_cuda_b200 as gdn
+    from h100_gdn_cuda_b200 import api
+    lens, vh, d = [70, 130, 40], 4, 128
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.varlen_inputs(lens, 2, vh, d, seed=4, mild_gate=True).items()}
+    n, nc, cu, ci, cc = sum(lens), p["total_chunks"], p["cu_seqlens"], p["chunk_indices"], p["cu_chunks"]
+    gate = api._chunk_local_cumsum_f32(p["g"], 1, n, vh, cu, ci)
+
+    def run():
+        new = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+        u, w, h, fin, o = new(n, vh, d), new(n, vh, d), new(nc, vh, d, d), new(3, vh, d, d), new(n, vh, d)
+        gdn.bf16_gdn_compute_u_w(p["k"], p["v"], u, w, p["beta"], gate, cu_seqlens=cu, chunk_indices=ci)
+        u_new = u.clone()
+        gdn.bf16_chunked_seq_state_update(p["k"], u_new, w, p["state"], h, fin, gate, cu_seqlens=cu, cu_chunks=cc, total_chunks=nc)
+        gdn.bf16_gdn_chunked_compute_O(p["q"], h, p["k"], u_new, o, gate, cu_seqlens=cu, chunk_indices=ci, cu_chunks=cc)
+        own = lambda x, a, b: torch.cat([x[:a], x[b:]])
+        a, b = cc[1].item(), cc[2].item()
+        return [own(x, lens[0], lens[0] + lens[1]) for x in (u, w, u_new, o)] + [own(h, a, b), own(fin, 1, 2)]
+
+    ref = run()
+    p[what] = p[what].clone()
+    p[what][lens[0]:lens[0] + lens[1]] = bad
+    assert all(torch.equal(x, y) for x, y in zip(run(), ref))
+
+
 def test_packed_calls_back_to_back():
     """Small packed batches whose calls follow one another without a pause: their blocks stay in L2, and the state kernel's warps can run
     a whole chunk ahead of those that write the outputs.  No wait may run out (the status word), and every call has the bits of the first."""
