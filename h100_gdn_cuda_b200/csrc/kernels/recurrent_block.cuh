@@ -615,8 +615,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             if (s_seq < 0) break;
             const int rem = static_cast<int>(s_unit % (p.vh * rblocks));
             run(s_seq, rem / rblocks, rem % rblocks);
-            __syncthreads();  // no warp waits on the unit's barriers any more
-            if (abort_flag) break;
+            if (__syncthreads_or(abort_flag)) break;  // no warp waits on the unit's barriers any more
             if (tid == 0) {
                 for (int i = 0; i < 4; ++i) {
                     mbar_inval(&full[i]);

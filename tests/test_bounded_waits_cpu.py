@@ -8,7 +8,7 @@ import pytest
 
 KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "h100_gdn_cuda_b200", "csrc", "kernels")
 LEAVES = re.compile(r"if \((?P<cond>.*(mbar_\w*wait\w*|abort_flag).*)\)\s*(\{\s*)?(break|return|continue)\b")
-VOTE = re.compile(r"__(all|any)_sync\(")
+VOTE = re.compile(r"__(all|any)_sync\(|__syncthreads_or\(")
 
 
 def lone_exits(text):
