@@ -178,7 +178,8 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
 // 176 : 184, T=27 188 : 184 (B=8 the same at T=27); d=256 T=23 259 : 259.  With few CTAs the blocks would win earlier (B=1 d=128
 // T=17 14 us : 8).  Packed batches hold both kinds and take two launches, each of which leaves the other's sequences out: 16
 // sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336, 8 of about 100 (32 v-heads, d=128) 113 -> 118; one of 1500 among
-// 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31.
+// 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31; 2 v-heads, 2000 of 30 tokens 766 us -> 817, 200 of 60
+// among 3800 of one 878 -> 231.
 // fp32 states stay with the token recurrence: in blocks (d=128, B=2 T=512 337 -> 136 us) the state, rounded once per block, was nearer to
 // 64 bits without decay (3.5e-7 of it -> 1.2e-7 after 1500 tokens) but further off with one, up to 40 % at a mean gate of -0.8
 // (6.1e-8 -> 8.5e-8): the matrix instructions cut their sums off.

@@ -97,18 +97,19 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// The `rank`-th packed sequence of at least `min_run` tokens, or -1.  All lanes of a warp.
-__device__ __forceinline__ int long_sequence(const int* cu_seqlens, int batch, int min_run, int rank) {
+// The `rank`-th packed sequence of at least `min_run` tokens, or -1.  The search starts at sequence `from` with `before` such sequences in
+// front of it and leaves both where the one found can be found again.  All lanes of a warp.
+__device__ __forceinline__ int long_sequence(const int* cu_seqlens, int batch, int min_run, int rank, int& from, int& before) {
     const int lane = threadIdx.x & 31;
-    for (int s0 = 0; s0 < batch; s0 += 32) {
-        const int s = s0 + lane;
+    for (; from < batch; from += 32) {
+        const int s = from + lane;
         unsigned m = __ballot_sync(0xffffffffu, s < batch && cu_seqlens[s + 1] - cu_seqlens[s] >= min_run);
         const int c = __popc(m);
-        if (rank < c) {
-            for (; rank > 0; --rank) m &= m - 1;
-            return s0 + __ffs(m) - 1;
+        if (rank < before + c) {
+            for (int i = before; i < rank; ++i) m &= m - 1;
+            return from + __ffs(m) - 1;
         }
-        rank -= c;
+        before += c;
     }
     return -1;
 }
@@ -118,8 +119,8 @@ __device__ __forceinline__ int long_sequence(const int* cu_seqlens, int batch, i
 // so that a sequence has the same bits whatever it is packed with).  How many there are is known here alone.
 enum class BlkUnits {
     kPadded,  // a CTA per unit
-    kPacked,  // a CTA per unit of as many sequences as can be that long; those past the last one end at once
-    kWalk,    // packed, far fewer long sequences than could be: a wave of CTAs walks the units with a stride of the grid
+    kPacked,  // a CTA per unit of every sequence; those of shorter ones end at once
+    kWalk,    // packed, most sequences are shorter: a wave of CTAs walks the long ones' units with a stride of the grid
 };
 template <int DK, BlkUnits kUnits = BlkUnits::kPadded>
 __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& p) {
@@ -603,13 +604,22 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     if constexpr (kUnits == BlkUnits::kWalk) {
         // (the walk's state is in shared memory: registers are all taken)
         __shared__ long long s_unit;
-        __shared__ int s_seq;
-        if (tid == 0) s_unit = blockIdx.x;
+        __shared__ int s_seq, s_from, s_before;
+        if (tid == 0) {
+            s_unit = blockIdx.x;
+            s_from = s_before = 0;
+        }
         while (true) {
             __syncthreads();
             if (tid < 32) {
-                const int seq = long_sequence(p.cu_seqlens, p.batch, p.long_run, static_cast<int>(s_unit / (p.vh * rblocks)));
-                if (tid == 0) s_seq = seq;
+                int from = s_from, before = s_before;
+                const int seq = long_sequence(p.cu_seqlens, p.batch, p.long_run, static_cast<int>(s_unit / (p.vh * rblocks)), from, before);
+                __syncwarp();
+                if (tid == 0) {
+                    s_seq = seq;
+                    s_from = from;
+                    s_before = before;
+                }
             }
             __syncthreads();
             if (s_seq < 0) break;
@@ -628,10 +638,8 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         }
     } else {
         const int unit = static_cast<int>(blockIdx.x) / rblocks, rb = static_cast<int>(blockIdx.x) - unit * rblocks;
-        int seq = unit / p.vh;
-        const int head = unit - seq * p.vh;
-        if (kPacked) seq = long_sequence(p.cu_seqlens, p.batch, p.long_run, seq);
-        if (seq >= 0) run(seq, head, rb);
+        const int seq = unit / p.vh, head = unit - seq * p.vh;
+        if (!kPacked || p.cu_seqlens[seq + 1] - p.cu_seqlens[seq] >= p.long_run) run(seq, head, rb);
     }
     if (kPacked) grid_dep_wait();
     __syncthreads();

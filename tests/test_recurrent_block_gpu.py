@@ -141,9 +141,10 @@ def test_bits_do_not_depend_on_company(gdn, d, f32, T):
 
 @pytest.mark.parametrize("chunked", [False, True])
 @pytest.mark.parametrize("d", [64, 128, 192, 256])
-@pytest.mark.parametrize("lens", [[300] + [1] * 99 + [22, 41, 0, 25, 27, 60, 17], [0] * 70 + [40, 0, 41, 26, 200], [23, 24, 45, 1000, 64, 41]])
+@pytest.mark.parametrize("lens", [[300] + [1] * 99 + [22, 41, 0, 25, 27, 60, 17], [0] * 70 + [40, 0, 41, 26, 200], [23, 24, 45, 1000, 64, 41],
+                                  [45 + i % 4 if i % 5 == 0 or i > 190 else 1 for i in range(200)], [70 + i % 3 for i in range(50)]])
 def test_packed_runs_of_unequal_length(gdn, lens, d, chunked):
-    """few long sequences among many short ones, among empty ones, and none but long ones: the bits each has alone"""
+    """few long sequences among many short ones, among empty ones, none but long ones, more of either than CTAs: the bits each has alone"""
     if chunked and d <= 128:
         pytest.skip("head dims up to 128 have kernels of their own in chunked_forward")
     kh, vh = 2, 4
