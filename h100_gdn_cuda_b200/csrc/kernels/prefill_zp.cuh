@@ -28,6 +28,8 @@
 // shared-memory accesses, besides some 900 of MMA operands and copies, of the 3 000 cycles a unit took an SM.
 // Whole calls with the doubling scheme and now, in turn on one GPU: B=4 T=4096, 32 v-heads 215.4 -> 210.3 us; 16 packed sequences of 32768
 // tokens 457.6 -> 437.9; B=2 T=131072, 4 v-heads 621.7 -> 599.9.
+// Not kept: two of A's seven blocks of warp 1 made by warp 0 from their mirror images and both diagonal blocks of a warp inverted in its 32
+// lanes, with a barrier less (the critical path 700 cycles shorter on paper): 206.8 -> 208.3 us.
 // Persistent CTAs, two per SM (111 KB of shared memory, 256 tensor-memory columns each).
 #pragma once
 #include <cuda.h>
@@ -115,12 +117,12 @@ __device__ __forceinline__ void split_frag(const float (*x)[4], uint32_t* hi, ui
 #pragma unroll
     for (int i = 0; i < 4; ++i) split2(x[i >> 1][2 * (i & 1)], x[i >> 1][2 * (i & 1) + 1], hi[i], lo[i]);
 }
-// acc += X B for 16x16 blocks: X as fragments of two terms, B in shared memory (row64_off); the product of the second terms is
-// below 2^-16 of the result
-__device__ __forceinline__ void mma_blk16(float (*acc)[4], const uint32_t* xh, const uint32_t* xl, uint32_t b_saddr, int lane) {
+// acc += X B for 16x16 blocks: X as fragments of two terms, B in shared memory (`b_lane`: its address plus row64_off(lane & 15,
+// lane >> 4)); the product of the second terms is below 2^-16 of the result
+__device__ __forceinline__ void mma_blk16(float (*acc)[4], const uint32_t* xh, const uint32_t* xl, uint32_t b_lane) {
     uint32_t bh[4], bl[4];  // { columns 0-7: rows 0-7, 8-15; columns 8-15: the same }
-    ldmatrix_x4_trans(b_saddr + row64_off(lane & 15, lane >> 4), bh);
-    ldmatrix_x4_trans(b_saddr + row64_off(lane & 15, 2 + (lane >> 4)), bl);
+    ldmatrix_x4_trans(b_lane, bh);
+    ldmatrix_x4_trans(b_lane ^ 32u, bl);  // (pieces 2, 3 of a row)
     mma_16816(acc[0], xl, bh[0], bh[1]);
     mma_16816(acc[1], xl, bh[2], bh[3]);
     mma_16816(acc[0], xh, bl[0], bl[1]);
@@ -128,24 +130,261 @@ __device__ __forceinline__ void mma_blk16(float (*acc)[4], const uint32_t* xh, c
     mma_16816(acc[0], xh, bh[0], bh[1]);
     mma_16816(acc[1], xh, bh[2], bh[3]);
 }
-// Row block R of X = (I + A)^-1 from its diagonal block on, right to left.  x: fragments of the blocks X_R0 .. X_RR.
-template <int R>
-__device__ __forceinline__ void row_blocks(float (*x)[2][4], uint32_t a_saddr, uint32_t inv_saddr, int lane) {
-    uint32_t xh[4][4], xl[4][4];
-    if (R > 0) split_frag(x[R], xh[R], xl[R]);
+// Row block R of X = (I + A)^-1 from its diagonal block `x` on, right to left: emit(d, fragment of X_R,R-d).  (Counted by the distance from
+// the diagonal, so that one copy of the code serves every R.)
+template <class Emit>
+__device__ __forceinline__ void row_blocks(int R, const float (*x)[4], uint32_t a_saddr, uint32_t inv_saddr, int lane, Emit emit) {
+    const uint32_t lo = row64_off(lane & 15, lane >> 4);
+    uint32_t xh[3][4], xl[3][4];
+    uint32_t row[3];  // blocks (R - e, 0) of A, then of the present column
 #pragma unroll
-    for (int c = R - 1; c >= 0; --c) {
+    for (int e = 0; e < 3; ++e) row[e] = a_saddr + lo + static_cast<uint32_t>((R - e) * (R - e - 1) / 2 + R) * 1024u;
+    uint32_t inv = inv_saddr + lo + static_cast<uint32_t>(R * ZPSmem::kDiag);
+    split_frag(x, xh[0], xl[0]);
+    emit(std::integral_constant<int, 0>{}, x);
+    auto step = [&](auto d_tag) {
+        constexpr int d = decltype(d_tag)::value;
         float s[2][4] = {};
 #pragma unroll
-        for (int m = R; m > c; --m) mma_blk16(s, xh[m], xl[m], a_saddr + (m * (m - 1) / 2 + c) * 1024, lane);
+        for (int e = 0; e < d; ++e) {
+            row[e] -= e + 1 < d ? 1024u : static_cast<uint32_t>(d) * 1024u;
+            mma_blk16(s, xh[e], xl[e], row[e]);
+        }
         uint32_t sh[4], sl[4];
         split_frag(s, sh, sl);
         float y[2][4] = {};
-        mma_blk16(y, sh, sl, inv_saddr + c * ZPSmem::kDiag, lane);
+        inv -= ZPSmem::kDiag;
+        mma_blk16(y, sh, sl, inv);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[c][i >> 2][i & 3] = -y[i >> 2][i & 3];
-        if (c > 0) split_frag(x[c], xh[c], xl[c]);
+        for (int i = 0; i < 8; ++i) y[i >> 2][i & 3] = -y[i >> 2][i & 3];
+        if (d < 3) split_frag(y, xh[d < 3 ? d : 0], xl[d < 3 ? d : 0]);
+        emit(d_tag, y);
+    };
+    if (R >= 1) step(std::integral_constant<int, 1>{});
+    if (R >= 2) step(std::integral_constant<int, 2>{});
+    if (R >= 3) step(std::integral_constant<int, 3>{});
+}
+// Raw gates of the tokens `lane` and `lane + 32` -> the chunk's cumulative gate times log2(e) (decay factors are ex2 of differences).
+__device__ __forceinline__ void scan_gate(float& g0, float& g1, int lane) {
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const float y0 = __shfl_up_sync(0xffffffffu, g0, m), y1 = __shfl_up_sync(0xffffffffu, g1, m);
+        if (lane >= m) {
+            g0 += y0;
+            g1 += y1;
+        }
     }
+    g1 += __shfl_sync(0xffffffffu, g0, 31);
+    g0 *= 1.4426950408889634f;
+    g1 *= 1.4426950408889634f;
+}
+// This warp's tables: g [64], and the decay to the first token of its two row blocks (`upper`: blocks 2 and 3):
+// e^{g_32 - g_j} [32], e^{g_48 - g_j} [48], or e^{g_16 - g_j} [16].
+__device__ __forceinline__ void decay_tables(float g0, float g1, float* sG, float* sC, bool upper, int lane) {
+    using uw::ex2;
+    sG[lane] = g0;
+    sG[lane + 32] = g1;
+    if (upper) {
+        const float r2 = __shfl_sync(0xffffffffu, g1, 0), r3 = __shfl_sync(0xffffffffu, g1, 16);
+        sC[lane] = ex2(r2 - g0);
+        sC[32 + lane] = ex2(r3 - g0);
+        if (lane < 16) sC[64 + lane] = ex2(r3 - g1);
+    } else {
+        const float r1 = __shfl_sync(0xffffffffu, g0, 16);
+        if (lane < 16) sC[lane] = ex2(r1 - g0);
+    }
+}
+// Tiles and tables of a team of four warps that works on one (chunk, v-head).
+struct TeamTiles {
+    uint8_t* p;      // P, bf16, 128-byte rows, swizzled
+    uint8_t* a;      // 16x16 blocks of A below the diagonal, block (r, c) at r (r - 1) / 2 + c, as two bf16 terms
+    uint8_t* diag;   // its diagonal blocks in fp32, kDiag bytes apart; the inverses go in their place as two bf16 terms
+    const float* g;  // this warp's g log2e [64]
+    const float* c;  // its column factors
+    const float* rn; // kNorm: inverse row norms of K [64] and Q [64]
+};
+// A = tril(beta_i (k_i.k_j) e^{g_i-g_j}, -1) (warps 0, 1 of the team) and P = scale tril((q_i.k_j) e^{g_i-g_j}) as a bf16 tile
+// (warps 2, 3), 16x16 block by block as accumulator fragments: a warp has two rows of blocks and nothing of what lies above the
+// diagonal is touched.  A: the diagonal blocks in fp32, the others as two bf16 terms.
+// In a block below the diagonal e^{g_i-g_j} = e^{g_i-g_r} e^{g_r-g_j} with r the first of its rows: the column factors come from a
+// table, no ex2 is left per element.  Both factors are <= 1 while the cumulative gate falls.  Where it rises they are entries of the
+// same matrices (tokens i and r, r and j): neither is infinite unless the exact result is.
+// `tm_kq`: column of K K^T (lanes 0-63) and Q K^T (64-127).
+// A loop, block by block.  Written out (ten copies of a block, and three of row_blocks) the kernel was 67 KB of code, now 55, and waited for
+// instructions in 0.60 of 9.3 warp cycles per issue, now 0.31: B=4 T=4096, 32 v-heads 208.4 -> 206.8 us a call, 16 packed sequences of
+// 32768 tokens 443.7 -> 438.3.
+template <bool kNorm>
+__device__ __forceinline__ void ap_pass(uint32_t tm_kq, const TeamTiles& t, int tw, int lane, int n, float g_mine, const float* b_mine,
+                                        float p_scale) {
+    using namespace uw;
+    const bool is_p = tw >= 2;
+    const int g = lane >> 2, tq = lane & 3, rb = tw & 1;
+    const float bm = rb ? b_mine[1] : b_mine[0];
+    const uint32_t pt = smem_u32(t.p) + 128u * (lane & 15);
+    // `v`: products of a block, 16 rows; o: its entries [8 columns][row g: two columns, row g + 8: two]
+    auto finish = [&](int r, float (*o)[4]) {
+        if (n < kChunk) {  // rows past the end: nothing, whatever lies there
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (16 * r + g + 8 * ((i >> 1) & 1) >= n) o[i >> 2][i & 3] = 0.f;
+        }
+    };
+    auto store_p = [&](int r, int c, const float (*o)[4]) {
+        stmatrix_x4(pt + 2048u * r + (((2 * c + (lane >> 4)) ^ (lane & 7)) << 4), pack_bf16(o[0][0], o[0][1]), pack_bf16(o[0][2], o[0][3]),
+                    pack_bf16(o[1][0], o[1][1]), pack_bf16(o[1][2], o[1][3]));
+    };
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const int r = 2 * rb + h;
+        const uint32_t ta = tm_kq + (static_cast<uint32_t>(32 * tw + 16 * h) << 16);
+        float gi[2], f[2];  // rows g and g + 8 of the block
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            gi[a] = __shfl_sync(0xffffffffu, g_mine, 16 * h + g + 8 * a);
+            f[a] = __shfl_sync(0xffffffffu, bm, 16 * h + g + 8 * a);
+            if (is_p) f[a] = p_scale;
+            if (kNorm) f[a] *= t.rn[(is_p ? 64 : 0) + 16 * r + g + 8 * a];
+        }
+        {
+            const float gr = t.g[16 * r];
+            const float w0 = f[0] * ex2(gi[0] - gr), w1 = f[1] * ex2(gi[1] - gr);
+            const f2 fo[2] = {pk(w0, w0), pk(w1, w1)};
+            const float* const col = t.c + (rb ? 32 * h : 0) + 2 * tq;
+#pragma unroll 1
+            for (int c = 0; c < r; ++c) {
+                uint32_t v[8];
+                tmem_ld_frag16(ta + 16 * c, v);
+                f2 cf[2], rn[2];
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    cf[nt] = *reinterpret_cast<const f2*>(col + 16 * c + 8 * nt);
+                    if (kNorm) rn[nt] = *reinterpret_cast<const f2*>(t.rn + 16 * c + 8 * nt + 2 * tq);  // the key's norm
+                }
+                float o[2][4];
+                tmem_wait_ld();
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        f2 x = pk(__uint_as_float(v[4 * nt + 2 * a]), __uint_as_float(v[4 * nt + 2 * a + 1]));
+                        if (kNorm) x = mul2(x, rn[nt]);
+                        unpk(mul2(mul2(x, fo[a]), cf[nt]), o[nt][2 * a], o[nt][2 * a + 1]);
+                    }
+                }
+                finish(r, o);
+                if (is_p) {
+                    store_p(r, c, o);
+                } else {
+                    uint32_t hi[4], lo[4];
+                    split_frag(o, hi, lo);
+                    const uint32_t ob = smem_u32(t.a) + static_cast<uint32_t>(r * (r - 1) / 2 + c) * 1024u;
+                    stmatrix_x4(ob + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+                    stmatrix_x4(ob + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
+                }
+            }
+        }
+        // the diagonal block: one ex2 per element, selected
+        uint32_t v[8];
+        tmem_ld_frag16(ta + 16 * r, v);
+        float o[2][4], e[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            const float2 cg = *reinterpret_cast<const float2*>(t.g + 16 * r + 8 * nt + 2 * tq);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                e[nt][2 * a] = ex2(gi[a] - cg.x);
+                e[nt][2 * a + 1] = ex2(gi[a] - cg.y);
+            }
+        }
+        tmem_wait_ld();
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            const int cl = 8 * nt + 2 * tq;  // column within the block
+            f2 rn = pk(1.f, 1.f);
+            if (kNorm) rn = *reinterpret_cast<const f2*>(t.rn + 16 * r + cl);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                f2 x = pk(__uint_as_float(v[4 * nt + 2 * a]), __uint_as_float(v[4 * nt + 2 * a + 1]));
+                if (kNorm) x = mul2(x, rn);
+                const int lim = g + 8 * a - (is_p ? 0 : 1);  // columns kept: cl <= lim
+                unpk(mul2(mul2(x, pk(f[a], f[a])), pk(e[nt][2 * a], e[nt][2 * a + 1])), o[nt][2 * a], o[nt][2 * a + 1]);
+                if (cl > lim) o[nt][2 * a] = 0.f;
+                if (cl + 1 > lim) o[nt][2 * a + 1] = 0.f;
+            }
+        }
+        finish(r, o);
+        if (is_p) {
+            store_p(r, r, o);
+#pragma unroll 1
+            for (int c = r + 1; c < 4; ++c) stmatrix_x4(pt + 2048u * r + (((2 * c + (lane >> 4)) ^ (lane & 7)) << 4), 0u, 0u, 0u, 0u);
+        } else {
+            float* const o2 = reinterpret_cast<float*>(t.diag + r * ZPSmem::kDiag) + g * ZPSmem::kLdD + 2 * tq;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                *reinterpret_cast<float2*>(o2 + (i & 1) * 8 * ZPSmem::kLdD + 8 * (i >> 1)) = make_float2(o[i >> 1][2 * (i & 1)], o[i >> 1][2 * (i & 1) + 1]);
+        }
+    }
+}
+// A diagonal block of A (fp32 at `sA`) -> its block of X = (I + A)^-1 as accumulator fragments, and in place of the block as two bf16
+// terms.  The two 8x8 diagonal blocks by forward substitution in fp32 (one column per lane, 16 lanes), then X_10 = -X_11 A_10 X_00
+// with two TF32 warp MMAs (the intermediate stays in registers).
+__device__ __forceinline__ void invert_diagonal(float* const sA, int lane, float (*xd)[4]) {
+    using namespace uw;
+    const int g = lane >> 2, tq = lane & 3;
+    constexpr int LD = ZPSmem::kLdD;
+    const int hb = (lane >> 3) & 1, j = lane & 7;
+    const int o = 8 * hb;  // first row / column of this lane's 8x8 block
+    float xc[8], a[8][8];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+#pragma unroll
+        for (int q = 0; q < (i + 3) / 4; ++q) {
+            const float4 t = *reinterpret_cast<const float4*>(&sA[(o + i) * LD + o + 4 * q]);
+            a[i][4 * q] = t.x; a[i][4 * q + 1] = t.y; a[i][4 * q + 2] = t.z; a[i][4 * q + 3] = t.w;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xc[i] = (i == j) ? 1.f : 0.f;
+    // x_j = 1, x_i = -sum_{m<i} A_im x_m
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        float acc = 0.f;
+#pragma unroll
+        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[i][m], xc[m], acc);
+        if (i > j) xc[i] = -fmaf(a[i][i - 1], xc[i - 1], acc);
+    }
+    __syncwarp();  // the block is private to this warp: every lane has read it
+    if (lane < 16) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sA[(o + i) * LD + o + j] = xc[i];
+    }
+    __syncwarp();
+    // 8 -> 16
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    uint32_t bfrag[2], afrag[4];
+    load_a8(afrag, sA, LD, 8, 0, lane);
+    load_b8(bfrag, sA, LD, 0, 0, lane);
+    mma_tf32(d, afrag, bfrag);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
+    // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
+    const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
+    const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
+    const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
+    const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
+    bfrag[0] = to_tf32((g & 1) ? v01 : v00);
+    bfrag[1] = to_tf32((g & 1) ? v11 : v10);
+    load_a8(afrag, sA, LD, 8, 8, lane);
+    const float2 c00 = *reinterpret_cast<const float2*>(&sA[g * LD + 2 * tq]);
+    const float2 c11 = *reinterpret_cast<const float2*>(&sA[(8 + g) * LD + 8 + 2 * tq]);
+    float e[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_tf32(e, afrag, bfrag);  // X_11 t
+    xd[0][0] = c00.x; xd[0][1] = c00.y; xd[0][2] = -e[0]; xd[0][3] = -e[1];
+    xd[1][0] = 0.f; xd[1][1] = 0.f; xd[1][2] = c11.x; xd[1][3] = c11.y;
+    __syncwarp();  // the block has been read: its inverse goes in its place, for the row blocks further down
+    uint32_t hi[4], lo[4];
+    split_frag(xd, hi, lo);
+    const uint32_t ia = smem_u32(sA);
+    stmatrix_x4(ia + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
+    stmatrix_x4(ia + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
 }
 }  // namespace zp
 
@@ -174,8 +413,9 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
     float* sBeta = reinterpret_cast<float*>(tbase + L::kOffVec);
     float* sD = sBeta + 64;
     float* sG = sD + 64 + 144 * tw;  // this warp's own copy
-    float* sC = sG + 64;  // decay to the first token of this warp's two row blocks: e^{g_32 - g_j} [32], e^{g_48 - g_j} [48] (tw & 1), or e^{g_16 - g_j} [16]
+    float* sC = sG + 64;
     float* sRn = reinterpret_cast<float*>(smem + L::kOffNorm);  // [128] inverse norms (K rows, then Q rows)
+    const TeamTiles tiles{sP, tbase + L::kOffA, tbase + L::kOffDiag, sG, sC, sRn};
     uint64_t* bar_load = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
     uint64_t* bar_kq = bar_load + 1;
     uint64_t* bar_mma = bar_load + 2;  // [2], one per team
@@ -317,29 +557,9 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 b_mine[0] = p.beta.value(b_next[0]);
                 b_mine[1] = p.beta.value(b_next[1]);
                 float g0 = p.gate.value(g_next[0]), g1 = p.gate.value(g_next[1]);
-#pragma unroll
-                for (int m = 1; m < 32; m <<= 1) {
-                    const float y0 = __shfl_up_sync(0xffffffffu, g0, m), y1 = __shfl_up_sync(0xffffffffu, g1, m);
-                    if (lane >= m) {
-                        g0 += y0;
-                        g1 += y1;
-                    }
-                }
-                g1 += __shfl_sync(0xffffffffu, g0, 31);
-                g0 *= 1.4426950408889634f;  // times log2(e): decay factors are ex2 of differences
-                g1 *= 1.4426950408889634f;
+                scan_gate(g0, g1, lane);
                 g_mine = (tw & 1) ? g1 : g0;
-                sG[lane] = g0;
-                sG[lane + 32] = g1;
-                if (tw & 1) {
-                    const float r2 = __shfl_sync(0xffffffffu, g1, 0), r3 = __shfl_sync(0xffffffffu, g1, 16);
-                    sC[lane] = ex2(r2 - g0);
-                    sC[32 + lane] = ex2(r3 - g0);
-                    if (lane < 16) sC[64 + lane] = ex2(r3 - g1);
-                } else {
-                    const float r1 = __shfl_sync(0xffffffffu, g0, 16);
-                    if (lane < 16) sC[lane] = ex2(r1 - g0);
-                }
+                decay_tables(g0, g1, sG, sC, tw & 1, lane);
                 if (tw == 0) {
                     sBeta[lane] = b_mine[0];
                     sBeta[lane + 32] = b_mine[1];
@@ -412,211 +632,47 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                     if (tt == 64) bulk_wait_read<0>();
                     pair_sync(team);
                 }
-                // ---- A = tril(beta_i (k_i.k_j) e^{g_i-g_j}, -1) (warps 0, 1 of the team) and P = scale tril((q_i.k_j) e^{g_i-g_j})
-                //      as a bf16 tile (warps 2, 3), 16x16 block by block as accumulator fragments: a warp has two rows of blocks and
-                //      nothing of what lies above the diagonal is touched.  A: the diagonal blocks in fp32, the others as two bf16 terms.
-                //      In a block below the diagonal e^{g_i-g_j} = e^{g_i-g_r} e^{g_r-g_j} with r the first of its rows: the column factors
-                //      come from a table, no ex2 is left per element.  Both factors are <= 1 while the cumulative gate falls.  Where it rises
-                //      they are entries of the same matrices (tokens i and r, r and j): neither is infinite unless the exact result is.
-                {
-                    const bool is_p = tw >= 2;
-                    const int g = lane >> 2, tq = lane & 3;
-                    const uint32_t pt = smem_u32(sP);
-                    auto row_block = [&](auto rb_tag, auto h_tag, const uint32_t (*kq)[16]) {
-                        constexpr int rb = decltype(rb_tag)::value, h = decltype(h_tag)::value, r = 2 * rb + h;
-                        float gi[2], f[2];  // rows g and g + 8 of the block
-#pragma unroll
-                        for (int a = 0; a < 2; ++a) {
-                            gi[a] = __shfl_sync(0xffffffffu, g_mine, 16 * h + g + 8 * a);
-                            f[a] = __shfl_sync(0xffffffffu, rb ? b_mine[1] : b_mine[0], 16 * h + g + 8 * a);
-                            if (is_p) f[a] = p.p_scale;
-                            if (kNorm) f[a] *= sRn[(is_p ? 64 : 0) + 16 * r + g + 8 * a];
-                        }
-                        const float gr = sG[16 * r];
-                        const float w0 = f[0] * ex2(gi[0] - gr), w1 = f[1] * ex2(gi[1] - gr);
-                        const f2 fo[2] = {pk(w0, w0), pk(w1, w1)}, fd[2] = {pk(f[0], f[0]), pk(f[1], f[1])};
-                        // one block; `v`: its products
-                        auto block = [&](int c, const uint32_t* v, auto diag_tag) {
-                            constexpr bool kDiagonal = decltype(diag_tag)::value;
-                            float o[2][4];  // [8 columns][row g: two columns, row g + 8: two]
-#pragma unroll
-                            for (int nt = 0; nt < 2; ++nt) {
-                                const int cl = 8 * nt + 2 * tq;  // column within the block
-                                float2 rn = make_float2(1.f, 1.f);
-                                if (kNorm) rn = *reinterpret_cast<const float2*>(sRn + 16 * c + cl);  // the key's norm
-                                const float2 cf = *reinterpret_cast<const float2*>(kDiagonal ? sG + 16 * c + cl : sC + (rb ? 32 * h : 0) + 16 * c + cl);
-#pragma unroll
-                                for (int a = 0; a < 2; ++a) {
-                                    f2 x = pk(__uint_as_float(v[4 * nt + 2 * a]), __uint_as_float(v[4 * nt + 2 * a + 1]));
-                                    if (kNorm) x = mul2(x, pk(rn.x, rn.y));
-                                    if (kDiagonal) {
-                                        const int lim = g + 8 * a - (is_p ? 0 : 1);  // columns kept: cl <= lim
-                                        const float e0 = ex2(gi[a] - cf.x), e1 = ex2(gi[a] - cf.y);
-                                        unpk(mul2(mul2(x, fd[a]), pk(e0, e1)), o[nt][2 * a], o[nt][2 * a + 1]);
-                                        if (cl > lim) o[nt][2 * a] = 0.f;
-                                        if (cl + 1 > lim) o[nt][2 * a + 1] = 0.f;
-                                    } else {
-                                        unpk(mul2(mul2(x, fo[a]), pk(cf.x, cf.y)), o[nt][2 * a], o[nt][2 * a + 1]);
-                                    }
-                                }
-                            }
-                            if (n < kChunk) {  // rows past the end: nothing, whatever lies there
-#pragma unroll
-                                for (int i = 0; i < 8; ++i)
-                                    if (16 * r + g + 8 * ((i >> 1) & 1) >= n) o[i >> 2][i & 3] = 0.f;
-                            }
-                            if (is_p) {
-                                stmatrix_x4(pt + tile_off(16 * r + (lane & 15), 2 * c + (lane >> 4)), pack_bf16(o[0][0], o[0][1]),
-                                            pack_bf16(o[0][2], o[0][3]), pack_bf16(o[1][0], o[1][1]), pack_bf16(o[1][2], o[1][3]));
-                            } else if (kDiagonal) {
-                                float* const o2 = reinterpret_cast<float*>(tbase + L::kOffDiag + r * L::kDiag) + g * L::kLdD + 2 * tq;
-#pragma unroll
-                                for (int i = 0; i < 4; ++i)
-                                    *reinterpret_cast<float2*>(o2 + (i & 1) * 8 * L::kLdD + 8 * (i >> 1)) = make_float2(o[i >> 1][2 * (i & 1)], o[i >> 1][2 * (i & 1) + 1]);
-                            } else {
-                                uint32_t hi[4], lo[4];
-                                split_frag(o, hi, lo);
-                                const uint32_t ob = smem_u32(tbase + L::kOffA + (r * (r - 1) / 2 + c) * 1024);
-                                stmatrix_x4(ob + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
-                                stmatrix_x4(ob + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
-                            }
-                        };
-                        constexpr std::false_type below{};
-                        constexpr std::true_type diagonal{};
-                        if (rb) {
-                            block(0, kq[0], below);
-                            block(1, kq[0] + 8, below);
-                            if (h) block(2, kq[1], below);
-                        } else if (h) {
-                            block(0, kq[0], below);
-                        }
-                        block(r, h == 0 ? (rb ? kq[1] : kq[0]) : (rb ? kq[1] + 8 : kq[0] + 8), diagonal);
-                        if (is_p) {  // the blocks above the diagonal: zeros
-#pragma unroll
-                            for (int c = 1; c < 4; ++c)
-                                if (c > r) stmatrix_x4(pt + tile_off(16 * r + (lane & 15), 2 * c + (lane >> 4)), 0u, 0u, 0u, 0u);
-                        }
-                    };
-                    using I0 = std::integral_constant<int, 0>;
-                    using I1 = std::integral_constant<int, 1>;
-                    const uint32_t ta = tmem + kTmKQ + (static_cast<uint32_t>(32 * tw) << 16), tb = ta + (16u << 16);
-                    uint32_t k0[2][16], k1[2][16];  // 32 columns each
-                    tmem_ld_frag32(ta, k0[0]);
-                    tmem_ld_frag32(tb, k1[0]);
-                    if (tw & 1) {
-                        tmem_ld_frag32(ta + 32, k0[1]);
-                        tmem_ld_frag32(tb + 32, k1[1]);
-                        tmem_wait_ld();
-                        row_block(I1{}, I0{}, k0);
-                        row_block(I1{}, I1{}, k1);
-                    } else {
-                        tmem_wait_ld();
-                        row_block(I0{}, I0{}, k0);
-                        row_block(I0{}, I1{}, k1);
-                    }
-                }
+                // ---- A and P, then X = (I + A)^-1
+                ap_pass<kNorm>(tmem + kTmKQ, tiles, tw, lane, n, g_mine, b_mine, p.p_scale);
                 tc_fence_before_sync();
                 team_sync(team);
-                // ---- X = (I + A)^-1.  Every warp owns a 16-row block (team 1 in reverse order: the last one is the longest, and warps w of
-                //      both teams share a scheduler).  Its diagonal block first: the two 8x8 diagonal blocks by forward substitution in
-                //      fp32 (one column per lane, 16 lanes), then X_10 = -X_11 A_10 X_00 with two TF32 warp MMAs (the intermediate
-                //      stays in registers).
+                // Every warp owns a 16-row block of X (team 1 in reverse order: the last one is the longest, and warps w of both teams
+                // share a scheduler).
                 const int rblk = team ? 3 - tw : tw;
                 const int g = lane >> 2, tq = lane & 3;
-                float x[4][2][4], xd[2][4];  // blocks X_r0 .. X_rr of the row block (diagonal block first in all) and its diagonal block, as accumulator fragments
-                {
-                    constexpr int LD = L::kLdD;
-                    float* const sA = reinterpret_cast<float*>(tbase + L::kOffDiag + rblk * L::kDiag);
-                    const int hb = (lane >> 3) & 1, j = lane & 7;
-                    const int o = 8 * hb;  // first row / column of this lane's 8x8 block
-                    float xc[8], a[8][8];
-#pragma unroll
-                    for (int i = 1; i < 8; ++i) {
-#pragma unroll
-                        for (int q = 0; q < (i + 3) / 4; ++q) {
-                            const float4 t = *reinterpret_cast<const float4*>(&sA[(o + i) * LD + o + 4 * q]);
-                            a[i][4 * q] = t.x; a[i][4 * q + 1] = t.y; a[i][4 * q + 2] = t.z; a[i][4 * q + 3] = t.w;
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) xc[i] = (i == j) ? 1.f : 0.f;
-                    // x_j = 1, x_i = -sum_{m<i} A_im x_m
-#pragma unroll
-                    for (int i = 1; i < 8; ++i) {
-                        float acc = 0.f;
-#pragma unroll
-                        for (int m = 0; m + 1 < i; ++m) acc = fmaf(a[i][m], xc[m], acc);
-                        if (i > j) xc[i] = -fmaf(a[i][i - 1], xc[i - 1], acc);
-                    }
-                    __syncwarp();  // the block is private to this warp: every lane has read it
-                    if (lane < 16) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) sA[(o + i) * LD + o + j] = xc[i];
-                    }
-                    __syncwarp();
-                    // 8 -> 16
-                    float d[4] = {0.f, 0.f, 0.f, 0.f};
-                    uint32_t bfrag[2], afrag[4];
-                    load_a8(afrag, sA, LD, 8, 0, lane);
-                    load_b8(bfrag, sA, LD, 0, 0, lane);
-                    mma_tf32(d, afrag, bfrag);  // t = A_10 X_00; lane (g, t) holds t[g][2t], t[g][2t+1]
-                    // t as the B operand of the next product: lane (g, t) needs t[t][g] and t[t + 4][g]
-                    const float v00 = __shfl_sync(0xffffffffu, d[0], 4 * tq + (g >> 1));
-                    const float v01 = __shfl_sync(0xffffffffu, d[1], 4 * tq + (g >> 1));
-                    const float v10 = __shfl_sync(0xffffffffu, d[0], 4 * (tq + 4) + (g >> 1));
-                    const float v11 = __shfl_sync(0xffffffffu, d[1], 4 * (tq + 4) + (g >> 1));
-                    bfrag[0] = to_tf32((g & 1) ? v01 : v00);
-                    bfrag[1] = to_tf32((g & 1) ? v11 : v10);
-                    load_a8(afrag, sA, LD, 8, 8, lane);
-                    const float2 c00 = *reinterpret_cast<const float2*>(&sA[g * LD + 2 * tq]);
-                    const float2 c11 = *reinterpret_cast<const float2*>(&sA[(8 + g) * LD + 8 + 2 * tq]);
-                    float e[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_tf32(e, afrag, bfrag);  // X_11 t
-                    xd[0][0] = c00.x; xd[0][1] = c00.y; xd[0][2] = -e[0]; xd[0][3] = -e[1];
-                    xd[1][0] = 0.f; xd[1][1] = 0.f; xd[1][2] = c11.x; xd[1][3] = c11.y;
-                    __syncwarp();  // the block has been read: its inverse goes in its place, for the row blocks further down
-                    uint32_t hi[4], lo[4];
-                    split_frag(xd, hi, lo);
-                    const uint32_t ia = smem_u32(sA);
-                    stmatrix_x4(ia + row64_off(lane & 15, lane >> 4), hi[0], hi[1], hi[2], hi[3]);
-                    stmatrix_x4(ia + row64_off(lane & 15, 2 + (lane >> 4)), lo[0], lo[1], lo[2], lo[3]);
-                }
+                float xd[2][4];  // its diagonal block as an accumulator fragment
+                invert_diagonal(reinterpret_cast<float*>(tiles.diag + rblk * L::kDiag), lane, xd);
                 team_sync(team);
                 // ---- the row block's other blocks, then T = X diag(beta) and dT = diag(d) T as bf16 swizzled tiles (row = token i,
                 //      64 columns j)
                 {
-                    const uint32_t aa = smem_u32(tbase + L::kOffA), ia = smem_u32(tbase + L::kOffDiag);
-                    // (one copy of the code below for all row blocks: the kernel's loop does not fit the instruction cache as it is)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) x[c][i >> 2][i & 3] = xd[i >> 2][i & 3];
-                    }
-                    if (rblk == 1) row_blocks<1>(x, aa, ia, lane);
-                    else if (rblk == 2) row_blocks<2>(x, aa, ia, lane);
-                    else if (rblk == 3) row_blocks<3>(x, aa, ia, lane);
-                    const int row = 16 * rblk + g;
+                    const uint32_t aa = smem_u32(tiles.a), ia = smem_u32(tiles.diag);
+const int row = 16 * rblk + g;
                     const float d0 = kNorm ? sD[row] * sRn[row] : sD[row], d1 = kNorm ? sD[row + 8] * sRn[row + 8] : sD[row + 8];
                     const f2 dd[2] = {pk(d0, d0), pk(d1, d1)};
                     const uint32_t tile = smem_u32(sT);
+                    row_blocks(rblk, xd, aa, ia, lane, [&](auto d_tag, const float (*x)[4]) {
+                        const int c = rblk - decltype(d_tag)::value;
+                        uint32_t tv[4], wv[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t tv[4] = {0u, 0u, 0u, 0u}, wv[4] = {0u, 0u, 0u, 0u};
-                        if (c <= rblk) {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {  // [8 columns][row g, g + 8]
-                                const f2 be = *reinterpret_cast<const f2*>(&sBeta[16 * c + 8 * (i >> 1) + 2 * tq]);
-                                const f2 t = mul2(pk(x[c][i >> 1][2 * (i & 1)], x[c][i >> 1][2 * (i & 1) + 1]), be);
-                                float a, b;
-                                unpk(t, a, b);
-                                tv[i] = pack_bf16(a, b);
-                                unpk(mul2(t, dd[i & 1]), a, b);
-                                wv[i] = pack_bf16(a, b);
-                            }
+                        for (int i = 0; i < 4; ++i) {  // [8 columns][row g, g + 8]
+                            const f2 be = *reinterpret_cast<const f2*>(&sBeta[16 * c + 8 * (i >> 1) + 2 * tq]);
+                            const f2 t = mul2(pk(x[i >> 1][2 * (i & 1)], x[i >> 1][2 * (i & 1) + 1]), be);
+                            float a, b;
+                            unpk(t, a, b);
+                            tv[i] = pack_bf16(a, b);
+                            unpk(mul2(t, dd[i & 1]), a, b);
+                            wv[i] = pack_bf16(a, b);
                         }
-                        const uint32_t off = sw128_offset(16 * rblk + (lane & 15), 16 * c + 8 * (lane >> 4));
+                        const uint32_t off = tile_off(16 * rblk + (lane & 15), 2 * c + (lane >> 4));
                         stmatrix_x4(tile + off, tv[0], tv[1], tv[2], tv[3]);
                         stmatrix_x4(tile + 8192 + off, wv[0], wv[1], wv[2], wv[3]);
+                    });
+#pragma unroll 1
+                    for (int c = rblk + 1; c < 4; ++c) {  // above the diagonal
+                        const uint32_t off = tile_off(16 * rblk + (lane & 15), 2 * c + (lane >> 4));
+                        stmatrix_x4(tile + off, 0u, 0u, 0u, 0u);
+                        stmatrix_x4(tile + 8192 + off, 0u, 0u, 0u, 0u);
                     }
                 }
                 fence_proxy_async_smem();

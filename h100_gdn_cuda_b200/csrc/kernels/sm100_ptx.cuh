@@ -354,6 +354,13 @@ GDN_DEVICE void tmem_ld_frag32(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+// (16 lanes x 16 columns the same way)
+GDN_DEVICE void tmem_ld_frag16(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 // The matching store of 16 lanes x 16 words: r[2i] is row l/4, word 4i + l%4, r[2i+1] the same word of row l/4 + 8.
 GDN_DEVICE void tmem_st_frag16(uint32_t taddr, const uint32_t* r) {
     asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
