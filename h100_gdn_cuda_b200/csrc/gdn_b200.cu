@@ -189,14 +189,14 @@ static int block_min_tokens(int dk, bool f32, bool steps, int ring_min) {
     return std::max(from, ring_min < kRecNoLongRun ? ring_min + 1 : kRecNoLongRun);
 }
 // The same kernel, compiled at run time (GDN_JIT_RECURRENT=1).
-static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, int smem, unsigned grid, cudaStream_t st) {
+static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, int groups, int smem, unsigned grid, cudaStream_t st) {
     const char* const kind[3] = {"kPadded", "kPacked", "kWalk"};
     char src[512];
     snprintf(src, sizeof(src),
              "#include \"kernels/recurrent_block.cuh\"\n"
-             "extern \"C\" __global__ void __launch_bounds__(%d, 2) gdn_recurrent_jit(const gdn::RecurrentParams p) {\n"
-             "    gdn::gdn_recurrent_block_body<%d, gdn::BlkUnits::%s>(p);\n}\n",
-             kBlkThreads, dk, kind[static_cast<int>(units)]);
+             "extern \"C\" __global__ void __launch_bounds__(%d, %d) gdn_recurrent_jit(const gdn::RecurrentParams p) {\n"
+             "    gdn::gdn_recurrent_block_body<%d, gdn::BlkUnits::%s, %d>(p);\n}\n",
+             blk_threads(groups), groups == 1 ? 2 : 1, dk, kind[static_cast<int>(units)], groups);
     jit::LoadedKernel k;
     std::string err;
     const char* const suffix[3] = {".block", ".block_packed", ".block_walk"};
@@ -205,43 +205,53 @@ static int launch_block_jit(const RecurrentParams& p, int dk, BlkUnits units, in
     GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     RecurrentParams pc = p;
     void* args[] = {&pc};
-    GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(kBlkThreads), args, smem, st));
+    GDN_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(k.kernel), dim3(grid), dim3(blk_threads(groups)), args, smem, st));
     return GDN_OK;
 }
-template <int DK, BlkUnits kUnits>
-static int launch_block_t(const RecurrentParams& p, bool jit, long long grid, cudaStream_t st) {
-    constexpr int smem = BlockSmem<DK>::kBytes;
-    GDN_REQUIRE(grid < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
-    if (jit) return launch_block_jit(p, DK, kUnits, smem, static_cast<unsigned>(grid), st);
+template <int DK, BlkUnits kUnits, int kGroups>
+static int launch_block_g(const RecurrentParams& p, bool jit, long long grid, cudaStream_t st) {
+    constexpr int smem = BlockSmem<DK, kGroups>::kBytes;
+    constexpr auto kernel = gdn_recurrent_block_kernel<DK, kUnits, kGroups>;
+    if (jit) return launch_block_jit(p, DK, kUnits, kGroups, smem, static_cast<unsigned>(grid), st);
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     GDN_CUDA(cudaGetDevice(&dev));
     if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_block_kernel<DK, kUnits>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GDN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev & 63].store(true, std::memory_order_release);
     }
-    GDN_CUDA(launch_dependent(gdn_recurrent_block_kernel<DK, kUnits>, dim3(static_cast<unsigned>(grid)), kBlkThreads, smem, st, p));
+    GDN_CUDA(launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), blk_threads(kGroups), smem, st, p));
     return GDN_OK;
 }
+// `tiles`: tiles of 16 state rows (kWalk: of as many long sequences as there can be).
+template <int DK, BlkUnits kUnits>
+static int launch_block_t(const RecurrentParams& p, bool jit, long long tiles, int sms, cudaStream_t st) {
+    GDN_REQUIRE(kUnits == BlkUnits::kWalk || tiles < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
+    if constexpr (DK >= 192) {
+        if (block_groups(tiles, sms) == 2)
+            return launch_block_g<DK, kUnits, 2>(p, jit, kUnits == BlkUnits::kWalk ? std::min<long long>(tiles / 2, sms) : tiles / 2, st);
+    }
+    return launch_block_g<DK, kUnits, 1>(p, jit, kUnits == BlkUnits::kWalk ? std::min(tiles, 2ll * sms) : tiles, st);
+}
 template <BlkUnits kUnits>
-static int launch_block_as(const RecurrentParams& p, int dk, bool jit, long long grid, cudaStream_t st) {
+static int launch_block_as(const RecurrentParams& p, int dk, bool jit, long long tiles, int sms, cudaStream_t st) {
     switch (dk) {
-        case 64: return launch_block_t<64, kUnits>(p, jit, grid, st);
-        case 128: return launch_block_t<128, kUnits>(p, jit, grid, st);
-        case 192: return launch_block_t<192, kUnits>(p, jit, grid, st);
-        case 256: return launch_block_t<256, kUnits>(p, jit, grid, st);
+        case 64: return launch_block_t<64, kUnits>(p, jit, tiles, sms, st);
+        case 128: return launch_block_t<128, kUnits>(p, jit, tiles, sms, st);
+        case 192: return launch_block_t<192, kUnits>(p, jit, tiles, sms, st);
+        case 256: return launch_block_t<256, kUnits>(p, jit, tiles, sms, st);
     }
     return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: no token-block kernel for dk = %d", dk);
 }
 // Packed mode: no more than total_tokens / long_run sequences can be that long.  Where that is all of them, a CTA per unit, as for
 // padded batches; otherwise a wave of CTAs walks the units (100 sequences of one token and one of 1500, d=256: 69 times the CTAs
-// there is work for).  The walk itself costs registers (d=256: 260 bytes spilled, 20 % of the time).
+// there is work for).  The walk itself costs registers (d=256: 260 bytes spilled, 20 % of the time; 124 with two groups of rows).
 static int launch_block(const RecurrentParams& p, int dk, bool jit, long long total_tokens, int sms, cudaStream_t st) {
     const long long per_seq = static_cast<long long>(p.vh) * (p.dv / kBlkRows);
-    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, jit, p.batch * per_seq, st);
+    if (!p.cu_seqlens) return launch_block_as<BlkUnits::kPadded>(p, dk, jit, p.batch * per_seq, sms, st);
     const long long seqs = total_tokens / p.long_run;
-    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, jit, p.batch * per_seq, st);
-    return launch_block_as<BlkUnits::kWalk>(p, dk, jit, std::min(seqs * per_seq, 2ll * sms), st);
+    if (seqs >= p.batch) return launch_block_as<BlkUnits::kPacked>(p, dk, jit, p.batch * per_seq, sms, st);
+    return launch_block_as<BlkUnits::kWalk>(p, dk, jit, seqs * per_seq, sms, st);
 }
 
 // Head dimensions without a prebuilt kernel (or every call when GDN_JIT_RECURRENT=1) go through

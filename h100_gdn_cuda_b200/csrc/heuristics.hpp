@@ -30,6 +30,18 @@ inline RecurrentConfig recurrent_config(int dk, long long num_tiles, int sms, bo
     return c;
 }
 
+// Token-block kernel, head dims 192 and 256: groups of 16 state rows per CTA, 1 (two CTAs fit an SM) or 2 (one does; they share the
+// preparation of the blocks).  A row's sums are the same in either.  A block of 16 tokens takes about 3.0 thousand cycles where a CTA
+// with one group has the SM to itself, 4.7 where two share it, and 4.3 with two groups.  In us, one group : two: d=256, 8 v-heads, T=1500
+// B=2 236 : 217, T=1000 B=4 315 : 292, T=500 B=8 (a last wave of half the tiles) 291 : 305; d=192 B=2 T=700 101 : 96; 16 packed sequences of
+// 500 573 : 541.  (At d=128 one group is as fast or faster: B=8 T=512, 8 v-heads 120 : 121, B=4, 32 v-heads 213 : 239.)
+inline int block_groups(long long tiles, int sms) {
+    const long long pairs = 2ll * sms, rest = tiles % pairs;
+    const double one = 4.7 * static_cast<double>(tiles / pairs) + (rest == 0 ? 0.0 : rest <= sms ? 3.0 : 4.7);
+    const double two = 4.3 * static_cast<double>((tiles + pairs - 1) / pairs);
+    return two < one ? 2 : 1;
+}
+
 struct PrefillConfig {
     int uw_ctas_per_sm;     // WY/UT kernel: 4 (52 KB shared memory, 128 tensor-memory columns, 128 registers)
     int fused_threads;      // state/output kernel: 16 warps, one CTA per SM (all 512 tensor-memory columns)

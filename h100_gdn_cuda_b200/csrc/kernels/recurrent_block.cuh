@@ -30,35 +30,39 @@
 //               k k^T and q k^T on matrix instructions, decay products, norms, and from them the matrices A and P; when a
 //               block is through they write its outputs.
 //               (Four of them, so that their work is spread over the four schedulers.)
-// Two CTAs per SM at dk = 256: one's chain fills the gaps of the other.
+// Two CTAs per SM at dk = 256: one's chain fills the gaps of the other (4 700 cycles a block for the pair).  kGroups = 2: one CTA of two such
+// groups of four warps, 32 rows, with one preparation for both (4 300 cycles; B=2, T=1500, 8 v-heads, d=256 236 -> 217 us).  Four warps
+// with 32 rows each share k and q in registers too, and the substitution, but a warp is a chain of its own: 359 us.
 #pragma once
 #include "recurrent_step.cuh"
 
 namespace gdn {
 
 constexpr int kBlkTok = 16;   // tokens per block
-constexpr int kBlkRows = 16;  // state rows per CTA
-constexpr int kBlkThreads = 256;
+constexpr int kBlkRows = 16;  // state rows of a group of four warps
+__host__ __device__ constexpr int blk_threads(int groups) { return 128 * (groups + 1); }
 
-template <int DK>
+template <int DK, int kGroups>
 struct BlockSmem {
+    static constexpr int kRows = kGroups * kBlkRows;  // of the CTA
     // rows of k and q are 16 bytes longer than the data: eight rows at one column lie in different banks
     static constexpr int kRow = DK * 2 + 16;
     static constexpr int kOffQ = kBlkTok * kRow, kOffV = 2 * kBlkTok * kRow;
-    static constexpr int kStage = kOffV + kBlkTok * kBlkRows * 2;
+    static constexpr int kStage = kOffV + kBlkTok * kRows * 2;
     static constexpr int kStages = 4;  // one per preparing warp
-    // over q once its products are there: what the outputs are made of, scale G_t (S_0 q_t) and c, 16 rows of 16 tokens each
-    static constexpr int kOffO = kOffQ, kOffC1 = kOffQ + kBlkRows * kBlkTok * 4;
-    static_assert(kOffC1 + kBlkRows * kBlkTok * 4 <= kOffV, "they fit over q");
+    // over q once its products are there: what the outputs are made of, per group scale G_t (S_0 q_t) and c, 16 rows of 16 tokens each
+    static constexpr int kOffO = kOffQ, kOffC1 = kOffQ + kBlkRows * kBlkTok * 4, kOut = 2 * kBlkRows * kBlkTok * 4;
+    static_assert(kOffO + kGroups * kOut <= kOffV, "they fit over q");
     // what a block's solve needs, floats: A as [s][t], P as [t][s], beta v as [row][t] (before that: decay products), factors
-    static constexpr int kA = 0, kP = 256, kR0 = 512, kLdR = 20, kCk = kR0 + 16 * kLdR, kCq = kCk + 16, kW = kCq + 16, kG = kW + 16;
+    static constexpr int kA = 0, kP = 256, kR0 = 512, kLdR = 20, kCk = kR0 + kRows * kLdR, kCq = kCk + 16, kW = kCq + 16, kG = kW + 16;
     static constexpr int kPrepFloats = kG + 4;
     static constexpr int kOffPrep = kStages * kStage;
     static constexpr int kLdD = 36;  // partial products of a warp: 16 rows x (16 k tokens, 16 q tokens)
     static constexpr int kOffD = kOffPrep + kStages * kPrepFloats * 4;
-    static constexpr int kOffC = kOffD + 2 * 4 * kBlkRows * kLdD * 4;  // coefficients as operands: [warp][term][row], 48-byte rows
+    static constexpr int kDGroup = 2 * 4 * kBlkRows * kLdD * 4;
+    static constexpr int kOffC = kOffD + kGroups * kDGroup;  // coefficients as operands: [warp][term][row], 48-byte rows
     static constexpr int kRowC = 48;
-    static constexpr int kBytes = kOffC + 4 * 3 * kBlkRows * kRowC;
+    static constexpr int kBytes = kOffC + kGroups * 4 * 3 * kBlkRows * kRowC;
     static_assert(kStage % 16 == 0 && kOffPrep % 16 == 0 && (kPrepFloats * 4) % 16 == 0 && kOffD % 16 == 0 && kOffC % 16 == 0, "alignment");
 };
 
@@ -122,13 +126,13 @@ enum class BlkUnits {
     kPacked,  // a CTA per unit of every sequence; those of shorter ones end at once
     kWalk,    // packed, most sequences are shorter: a wave of CTAs walks the long ones' units with a stride of the grid
 };
-template <int DK, BlkUnits kUnits = BlkUnits::kPadded>
+template <int DK, BlkUnits kUnits = BlkUnits::kPadded, int kGroups = 1>
 __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& p) {
     constexpr bool kPacked = kUnits != BlkUnits::kPadded;
     using namespace ptx;
     using namespace step;
     using namespace blk;
-    using L = BlockSmem<DK>;
+    using L = BlockSmem<DK, kGroups>;
     constexpr int NK = DK / 64;  // K-steps of 16 columns per warp
     static_assert(DK % 64 == 0, "four warps with whole K-steps each");
     extern __shared__ __align__(128) uint8_t smem[];
@@ -140,7 +144,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         for (int i = 0; i < 4; ++i) {
             mbar_init(&full[i], 32);
             mbar_init(&ready[i], 1);
-            mbar_init(&done[i], 4);
+            mbar_init(&done[i], 4 * kGroups);
         }
         mbar_fence_init();
     };
@@ -158,7 +162,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         grid_dep_launch();
     }
 
-    const int rblocks = p.dv / kBlkRows;
+    const int rblocks = p.dv / L::kRows;
     auto run = [&](int seq, int head, int rb) {
         const int khead = head / (p.vh / p.kh);
         long long tok0 = 0, bidx = seq;
@@ -176,17 +180,17 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
         const int lm_row = lane & 15, lm_col = 8 * (lane >> 4);
         auto prep_of = [&](int b) { return reinterpret_cast<float*>(smem + L::kOffPrep) + (b & 3) * L::kPrepFloats; };
 
-        if (warp >= 4) {
+        if (warp >= 4 * kGroups) {
             // =============================================================== preparation and outputs
-            const int j = warp - 4;
+            const int j = warp - 4 * kGroups;
             uint8_t* const st = smem + j * L::kStage;
             float* const pr = prep_of(j);
             float* const X = pr + L::kR0;  // [t][s] = Gamma_ts, [t][16] = G_t, [t][17], [t][18] = inverse norms of k_t, q_t
             const __nv_bfloat16* const kp = p.k + bidx * p.k_sb + tok0 * p.k_st + khead * p.k_sh;
             const __nv_bfloat16* const qp = p.q + bidx * p.q_sb + tok0 * p.q_st + khead * p.q_sh;
-            const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * kBlkRows;
+            const __nv_bfloat16* const vp = p.v + bidx * p.v_sb + tok0 * p.v_st + head * p.v_sh + rb * L::kRows;
             const int r = lane & 15, h = lane >> 4;  // for the outputs: row r, tokens 8 h .. 8 h + 7
-            __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * kBlkRows + r;
+            __nv_bfloat16* const out = p.out + bidx * p.o_sb + tok0 * p.o_st + head * p.o_sh + rb * L::kRows + r;
             float al = 0.f, db = 0.f;
             if (p.fused_gating) {
                 al = __expf(from_bits(ld_bits(p.A_log, p.gating_param_f32, head), p.gating_param_f32));
@@ -209,7 +213,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 const uint32_t it = static_cast<uint32_t>(b >> 2);
                 const bool next = b < nblk;
                 const int n = min(kBlkTok, ntok - b * kBlkTok);
-                float o[8], c0[8], c1[8];
+                float o[kGroups][8], c0[kGroups][8], c1[kGroups][8];
                 if (b >= 4) {  // block b - 4 is through: what its outputs are made of
                     ok = mbar_wait(&done[j], (it - 1) & 1u, &abort_flag) && ok;
                     auto row8 = [&](int off, int c, float* x) {
@@ -217,9 +221,12 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         const float4 w = *reinterpret_cast<const float4*>(st + off + row64_off(r, c + 1));
                         x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
                     };
-                    row8(L::kOffO, 2 * h, o);
-                    row8(L::kOffC1, 0, c0);
-                    row8(L::kOffC1, 2, c1);
+#pragma unroll
+                    for (int q = 0; q < kGroups; ++q) {
+                        row8(L::kOffO + q * L::kOut, 2 * h, o[q]);
+                        row8(L::kOffC1 + q * L::kOut, 0, c0[q]);
+                        row8(L::kOffC1 + q * L::kOut, 2, c1[q]);
+                    }
                     __syncwarp();
                 }
                 if (next) {
@@ -234,10 +241,11 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         cp_async16(dst + row * L::kRow + 16 * c, kp + at * p.k_st + 8 * c, bytes);
                         cp_async16(dst + L::kOffQ + row * L::kRow + 16 * c, qp + at * p.q_st + 8 * c, bytes);
                     }
-                    {
-                        const int row = lane >> 1;
+#pragma unroll
+                    for (int i = lane; i < 32 * kGroups; i += 32) {
+                        const int row = i / (2 * kGroups);
                         const long long at = static_cast<long long>(b) * kBlkTok + min(row, n - 1);
-                        cp_async16(dst + L::kOffV + 16 * lane, vp + at * p.v_st + 8 * (lane & 1), row < n ? 16u : 0u);
+                        cp_async16(dst + L::kOffV + 16 * i, vp + at * p.v_st + 8 * (i % (2 * kGroups)), row < n ? 16u : 0u);
                     }
                     cp_async_arrive(&full[j]);
                 }
@@ -250,21 +258,30 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         const float4 u = *reinterpret_cast<const float4*>(P), w = *reinterpret_cast<const float4*>(P + 4);
                         const float pw[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
 #pragma unroll
-                        for (int s = 0; s < 8; ++s)
-                            if (s <= i || h) o[i] = fmaf(pw[s], c0[s], o[i]);
+                        for (int q = 0; q < kGroups; ++q) {
+#pragma unroll
+                            for (int s = 0; s < 8; ++s)
+                                if (s <= i || h) o[q][i] = fmaf(pw[s], c0[q][s], o[q][i]);
+                        }
                         if (h) {
                             const float4 y = *reinterpret_cast<const float4*>(P + 8), z = *reinterpret_cast<const float4*>(P + 12);
                             const float pz[8] = {y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
 #pragma unroll
-                            for (int s = 0; s <= i; ++s) o[i] = fmaf(pz[s], c1[s], o[i]);
+                            for (int q = 0; q < kGroups; ++q) {
+#pragma unroll
+                                for (int s = 0; s <= i; ++s) o[q][i] = fmaf(pz[s], c1[q][s], o[q][i]);
+                            }
                         }
                     }
                     __syncwarp();
                     const bool good = ok && *static_cast<volatile int*>(&abort_flag) == 0;  // nothing is stored once a wait has given up
                     const long long i0 = static_cast<long long>(b - 4) * kBlkTok + 8 * h;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (good && i0 + i < ntok) out[(i0 + i) * p.o_st] = __float2bfloat16(o[i]);
+                    for (int q = 0; q < kGroups; ++q) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (good && i0 + i < ntok) out[(i0 + i) * p.o_st + q * kBlkRows] = __float2bfloat16(o[q][i]);
+                    }
                 }
                 if (!next) break;
                 // ---- scalars; tokens past the end: beta 0, decay 1
@@ -368,14 +385,17 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 // ---- beta v over the decay products
                 {
                     const int tk = lane & 15;
-                    const uint4 v = *reinterpret_cast<const uint4*>(st + L::kOffV + tk * kBlkRows * 2 + 16 * (lane >> 4));
                     const float bt = __shfl_sync(0xffffffffu, beta, tk);
-                    float* const R = X + 8 * (lane >> 4) * L::kLdR + tk;
-                    const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
-                        R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
+                    for (int q = 0; q < kGroups; ++q) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(st + L::kOffV + tk * L::kRows * 2 + 32 * q + 16 * (lane >> 4));
+                        float* const R = X + (kBlkRows * q + 8 * (lane >> 4)) * L::kLdR + tk;
+                        const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            R[(2 * i) * L::kLdR] = bt * bf16_lo(vw[i]);
+                            R[(2 * i + 1) * L::kLdR] = bt * bf16_hi(vw[i]);
+                        }
                     }
                 }
                 __syncwarp();
@@ -383,10 +403,11 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             }
         } else {
             // =============================================================== state
-            const int col0 = warp * (DK / 4);
+            const int rg = kGroups > 1 ? warp >> 2 : 0, qw = kGroups > 1 ? warp & 3 : warp;  // group of rows, quarter of the columns
+            const int col0 = qw * (DK / 4);
             const int r = lane & 15, h = lane >> 4;  // in the solve: row r, tokens 8 h .. 8 h + 7
             float S[2 * NK][4];  // 8 columns each: rows g (0, 1) and g + 8 (2, 3), columns 2t, 2t + 1
-            const long long srow = static_cast<long long>(rb * kBlkRows + g) * DK + col0 + 2 * t;
+            const long long srow = static_cast<long long>(rb * L::kRows + rg * kBlkRows + g) * DK + col0 + 2 * t;
             if (p.state_in) {
                 const long long base = static_cast<long long>(slot) * p.si_ss + head * p.si_sh + srow;
 #pragma unroll
@@ -412,7 +433,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 uint8_t* const st = smem + (b & 3) * L::kStage;
                 const float* const pr = prep_of(b);
                 const uint32_t kaddr = smem_u32(st) + lm_row * L::kRow + (col0 + lm_col) * 2;
-                float* const D = reinterpret_cast<float*>(smem + L::kOffD) + (b & 1) * (4 * kBlkRows * L::kLdD);
+                float* const D = reinterpret_cast<float*>(smem + L::kOffD + rg * L::kDGroup) + (b & 1) * (4 * kBlkRows * L::kLdD);
                 // ---- this warp's columns of S_0 [k; q]^T: tokens 0 - 7 and 8 - 15 of k, then of q.  The first terms have sums of their own:
                 //      they are the long ones, and the chains are shorter.
                 {
@@ -458,14 +479,17 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     // a row of the state with an infinity has undefined low terms in every column: taken again with care
                     const float chk = dl[0][0] + dl[0][2];
                     if (__any_sync(0xffffffffu, chk != chk)) products(Flag<true>{});
-                    float* const d = D + (warp * kBlkRows + g) * L::kLdD + 2 * t;
+                    float* const d = D + (qw * kBlkRows + g) * L::kLdD + 2 * t;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         *reinterpret_cast<float2*>(d + 8 * i) = make_float2(dh[i][0] + dl[i][0], dh[i][1] + dl[i][1]);
                         *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
                     }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (kGroups == 1 || rg == 0)
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                else
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
                 // ---- c of row r, tokens 8 h ..: right-hand sides, then forward substitution, first half of the tokens before the second
                 float c[8];
                 {
@@ -483,7 +507,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                     }
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + r * L::kLdR + 8 * h + 4 * q);
+                        const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + (rg * kBlkRows + r) * L::kLdR + 8 * h + 4 * q);
                         const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
                         c[4 * q] = fmaf(-ck.x, sum[4 * q], bv.x);
                         c[4 * q + 1] = fmaf(-ck.y, sum[4 * q + 1], bv.y);
@@ -571,18 +595,18 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                 }
                 // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t), and c
                 {
-                    const int i = 32 * warp + lane, row = i >> 3, t2 = 2 * (i & 7);
+                    const int i = 32 * qw + lane, row = i >> 3, t2 = 2 * (i & 7);
                     const float* const d = D + row * L::kLdD + 16 + t2;
                     float2 x[4];
 #pragma unroll
                     for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
                     const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
                     ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
-                    *reinterpret_cast<float2*>(st + L::kOffO + row64_off(row, t2 >> 2) + 4 * (t2 & 2)) =
+                    *reinterpret_cast<float2*>(st + L::kOffO + rg * L::kOut + row64_off(row, t2 >> 2) + 4 * (t2 & 2)) =
                         make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
-                    if (warp == (b & 3)) {
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + row64_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + row64_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
+                    if (qw == (b & 3)) {
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + rg * L::kOut + row64_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
+                        *reinterpret_cast<float4*>(st + L::kOffC1 + rg * L::kOut + row64_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
                     }
                 }
                 __syncwarp();
@@ -649,9 +673,9 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
     }
 }
 
-template <int DK, BlkUnits kUnits = BlkUnits::kPadded>
-__global__ void __launch_bounds__(kBlkThreads, 2) gdn_recurrent_block_kernel(const RecurrentParams p) {
-    gdn_recurrent_block_body<DK, kUnits>(p);
+template <int DK, BlkUnits kUnits = BlkUnits::kPadded, int kGroups = 1>
+__global__ void __launch_bounds__(blk_threads(kGroups), kGroups == 1 ? 2 : 1) gdn_recurrent_block_kernel(const RecurrentParams p) {
+    gdn_recurrent_block_body<DK, kUnits, kGroups>(p);
 }
 
 }  // namespace gdn

@@ -175,6 +175,31 @@ LINES = [(64, False, 17), (64, False, 40), (64, False, 41), (64, True, 40), (64,
          (128, True, 22), (128, True, 24), (128, True, 25), (192, False, 20), (192, False, 26), (192, False, 27), (256, False, 20), (256, False, 22), (256, False, 23)]
 
 
+@pytest.mark.parametrize("d,vh", [(192, 7), (256, 6)])
+@pytest.mark.parametrize("lens", [[27, 27], [33, 33], [95, 95], [28, 96], [1200] + [1] * 30 + [27]])
+def test_two_groups_of_rows(gdn, d, vh, lens):
+    """Batches with more tiles of 16 rows than SMs whose CTAs own 32 rows (padded, packed, and walked): the bits of every sequence
+    alone, where they own 16."""
+    B, N = len(lens), sum(lens)
+    p = synthetic.varlen_inputs(lens, 1, vh, d, seed=d + N, mild_gate=True)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+    run = lambda sl, state, cu: gdn.recurrent_forward(c["q"][sl], c["k"][sl], c["v"][sl], state, c["beta"][sl], c["g"][sl], cu,
+                                                      inference_mode=gdn.Decode, is_qk_norm=True)
+    if lens == [lens[0]] * B:
+        x = lambda k: c[k].view(B, lens[0], *c[k].shape[1:])
+        o, s = gdn.recurrent_forward(x("q"), x("k"), x("v"), c["state"], x("beta"), x("g"), inference_mode=gdn.Decode, is_qk_norm=True)
+        o = o.view(N, vh, d)
+    else:
+        o, s = run(slice(None), c["state"], c["cu_seqlens"])
+    at = 0
+    for i, n in enumerate(lens):
+        if n > 1:
+            sl = slice(at, at + n)
+            oi, si = run(sl, c["state"][i:i + 1], torch.tensor([0, n], dtype=torch.int32, device="cuda"))
+            assert torch.equal(o[sl], oi) and torch.equal(s[i], si[0])
+        at += n
+
+
 @pytest.mark.parametrize("d,f32,T", LINES)
 def test_either_side_of_the_line(gdn, d, f32, T):
     norm = T % 2 == 0
