@@ -94,38 +94,35 @@ static cudaError_t launch_dependent(void (*kernel)(P), dim3 grid, int threads, s
     return cudaLaunchKernelEx(&cfg, kernel, params);
 }
 
-template <int DK, bool kRing, bool kLean = false, bool kF32 = false, bool kSplit = false>
+template <int DK, bool kRing, bool kLean = false, bool kF32 = false, bool kSplit = false, bool kPool = false>
 static int launch_recurrent_t(const RecurrentParams& p, int sms, cudaStream_t st) {
     constexpr int smem = recurrent_smem_bytes<DK, kRing, kF32>();
+    constexpr auto kernel = gdn_recurrent_kernel<DK, kRing, kLean, kF32, kSplit, kPool>;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev]) {
-        GDN_CUDA(cudaFuncSetAttribute(gdn_recurrent_kernel<DK, kRing, kLean, kF32, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GDN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr_set[dev] = true;
     }
     const int per_sm = recurrent_ctas_per_sm<DK, kRing, kF32>();
     const long long grid = std::min<long long>(p.num_tiles, static_cast<long long>(sms) * per_sm);
-    GDN_CUDA(launch_dependent(gdn_recurrent_kernel<DK, kRing, kLean, kF32, kSplit>, dim3(static_cast<unsigned>(grid)), kRecThreads, smem, st, p));
+    GDN_CUDA(launch_dependent(kernel, dim3(static_cast<unsigned>(grid)), kRecThreads, smem, st, p));
     return GDN_OK;
 }
 
 // `ring`: long runs of tokens (more than kRecTokRingMin per sequence on average) take the instance
 // with the multi-token ring; speculative verify keeps the decode instance; plain single-token decode
-// from a given state (`lean`) takes the decode instance with its run-time tests compiled away.
-template <int DK>
+// from a given state (`lean`), in place, from a pool or into other states, takes decode instances with the run-time tests compiled away.
+// States in a pool had taken the general one: d=128, 32 v-heads, B=24 15.1 -> 13.1 us, B=64 29.9 -> 26.0.
+template <int DK, bool kF32>
 static int launch_recurrent(const RecurrentParams& p, int sms, cudaStream_t st, bool ring, bool lean) {
-    if (ring) return launch_recurrent_t<DK, true>(p, sms, st);
-    if (lean) return launch_recurrent_t<DK, false, true>(p, sms, st);
-    if (p.split_tiles) return launch_recurrent_t<DK, false, false, false, true>(p, sms, st);
-    return launch_recurrent_t<DK, false>(p, sms, st);
-}
-
-template <int DK>
-static int launch_recurrent_f32(const RecurrentParams& p, int sms, cudaStream_t st, bool ring) {
-    if (ring) return launch_recurrent_t<DK, true, false, true>(p, sms, st);
-    if (p.split_tiles) return launch_recurrent_t<DK, false, false, true, true>(p, sms, st);
-    return launch_recurrent_t<DK, false, false, true>(p, sms, st);
+    if (ring) return launch_recurrent_t<DK, true, false, kF32>(p, sms, st);
+    if (lean && p.state_idx)
+        return p.split_tiles ? launch_recurrent_t<DK, false, true, kF32, true, true>(p, sms, st) : launch_recurrent_t<DK, false, true, kF32, false, true>(p, sms, st);
+    if (lean) return p.split_tiles ? launch_recurrent_t<DK, false, true, kF32, true>(p, sms, st) : launch_recurrent_t<DK, false, true, kF32>(p, sms, st);
+    if (p.split_tiles) return launch_recurrent_t<DK, false, false, kF32, true>(p, sms, st);
+    return launch_recurrent_t<DK, false, false, kF32>(p, sms, st);
 }
 
 // Short padded runs (2 .. kStepTok tokens) on bf16 states of the head dims serving configurations use take
@@ -582,12 +579,18 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
                                    : (s.seq_len > ring_min);
     // Work units: the ring instance (long token runs) makes every 32-row tile a unit of its own; the decode
     // instance keeps the tiles of a (sequence, v-head) together, which shares the q/k normalisation and the
-    // prepared tokens among them.  One-token batches with a CTA slot for every tile are split as well (B=1 with 32 v-heads
-    // of 128 rows: 5.3 -> 3.8 us, B=4 6.0 -> 4.8); with two tiles or more per slot a tile's own copies and norms cost more
-    // than the finer grain gives (B=8 6.9 -> 7.6 us, B=24 13.2 -> 17.4).
+    // prepared tokens among them, but for the last round of one-token batches (decode_split).
     p.split_tiles = ring ? 1 : 0;
     const int slots_per_sm = s.head_dim_k > 128 ? 2 : (a->state_dtype == GDN_F32 && s.head_dim_k > 64 ? 3 : 4);
-    if (!ring && !s.cu_seqlens && s.seq_len == 1) p.split_tiles = p.num_tiles <= static_cast<long long>(d->sms) * slots_per_sm;
+    if (!ring && !s.cu_seqlens && s.seq_len == 1) {
+        const DecodeSplit cut = decode_split(p.num_tiles, s.head_dim_v / kRecTileRows, static_cast<long long>(d->sms) * slots_per_sm,
+                                             a->state_dtype == GDN_F32 || a->state_indices != nullptr);
+        p.split_tiles = cut.parts > 1;
+        p.split_whole = static_cast<int>(cut.whole);
+        p.split_parts = cut.parts;
+    }
+    const long long pairs = static_cast<long long>(s.batch) * s.num_v_heads;
+    p.num_units = static_cast<int>(ring ? p.num_tiles : p.split_tiles ? p.split_whole + (pairs - p.split_whole) * p.split_parts : pairs);
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
     const bool f32 = a->state_dtype == GDN_F32;
     const bool jit = force_jit && !f32;
@@ -598,18 +601,18 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     auto token_recurrence = [&]() -> int {
         if (jit) return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring, step);
         if (step) return s.head_dim_k == 64 ? launch_step_t<64>(p, d->sms, st) : launch_step_t<128>(p, d->sms, st);
+        const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step;
         if (f32) {
             // fp32 states: the two head dims serving configurations use, on the decode and the multi-token instance
-            if (s.head_dim_k == 128) return launch_recurrent_f32<128>(p, d->sms, st, ring);
-            if (s.head_dim_k == 64) return launch_recurrent_f32<64>(p, d->sms, st, ring);
+            if (s.head_dim_k == 128) return launch_recurrent<128, true>(p, d->sms, st, ring, lean);
+            if (s.head_dim_k == 64) return launch_recurrent<64, true>(p, d->sms, st, ring, lean);
             return fail(GDN_ERR_UNSUPPORTED, "gdn_recurrent_forward: fp32 states are built for dk = 64 and 128 (got %d)", s.head_dim_k);
         }
-        const bool lean = !s.cu_seqlens && s.seq_len == 1 && p.state_in != nullptr && !p.store_step && !p.state_idx && !p.split_tiles;
         switch (s.head_dim_k) {
-            case 64: return launch_recurrent<64>(p, d->sms, st, ring, lean);
-            case 128: return launch_recurrent<128>(p, d->sms, st, ring, lean);
-            case 192: return launch_recurrent<192>(p, d->sms, st, ring, lean);
-            case 256: return launch_recurrent<256>(p, d->sms, st, ring, lean);
+            case 64: return launch_recurrent<64, false>(p, d->sms, st, ring, lean);
+            case 128: return launch_recurrent<128, false>(p, d->sms, st, ring, lean);
+            case 192: return launch_recurrent<192, false>(p, d->sms, st, ring, lean);
+            case 256: return launch_recurrent<256, false>(p, d->sms, st, ring, lean);
         }
         return launch_recurrent_jit(p, s.head_dim_k, d->sms, st, ring);  // 320 .. 512: compiled on first use
     };

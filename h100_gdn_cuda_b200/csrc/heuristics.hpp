@@ -42,6 +42,27 @@ inline int block_groups(long long tiles, int sms) {
     return two < one ? 2 : 1;
 }
 
+// One-token batches: the (sequence, v-head) units of `unit_tiles` tiles go round the `slots` CTAs; those of the last round, where it is not
+// full, are cut into as many parts as leave no CTA with two of them.  (Cut finer than that, a part's own copies and norms cost more than
+// the finer grain gives: every tile by itself, d=128, 32 v-heads, B=8 6.9 -> 7.6 us, B=24 13.2 -> 17.4.)  Whole : cut, us, 32 v-heads,
+// d=128, the states in place B=1 5.3 : 3.5, B=5 6.0 : 5.0, B=8 7.0 : 5.5, B=19 11.9 : 10.7, B=24 12.6 : 12.3, B=27 14.0 : 13.8; in a pool B=24 13.2 : 12.6,
+// B=40 18.3 : 17.8, B=56 22.9 : 22.2; fp32 B=5 7.6 : 6.3, B=14 14.7 : 12.8, B=28 23.7 : 22.5, B=46 35.5 : 34.9.  The instance that cuts is itself a
+// little slower: bf16 in place it gains nothing from the third round on (B=64 25.1 : 25.6), the others from the fifth on (B=80 30.4 :
+// 31.1); with two tiles per unit not from the second (d=64, B=24 6.43 : 6.46, B=46 10.3 : 10.5).
+struct DecodeSplit {
+    long long whole;  // units that stay whole
+    int parts;        // 1: nothing is cut
+};
+// `later`: states in a pool or in fp32
+inline DecodeSplit decode_split(long long num_tiles, int unit_tiles, long long slots, bool later) {
+    const long long units = num_tiles / unit_tiles, rest = units % slots;
+    DecodeSplit d{units - rest, 1};
+    if (units / slots > (unit_tiles < 4 ? 0 : later ? 3 : 1)) return d;
+    for (int f = 2; f <= unit_tiles && rest > 0 && rest * f <= slots; ++f)
+        if (unit_tiles % f == 0) d.parts = f;
+    return d;
+}
+
 struct PrefillConfig {
     int uw_ctas_per_sm;     // WY/UT kernel: 4 (52 KB shared memory, 128 tensor-memory columns, 128 registers)
     int fused_threads;      // state/output kernel: 16 warps, one CTA per SM (all 512 tensor-memory columns)

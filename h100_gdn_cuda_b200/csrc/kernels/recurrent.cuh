@@ -58,7 +58,11 @@ struct RecurrentParams {
     int fused_gating, gating_param_f32;
     const void* A_log;
     const void* dt_bias;
-    int split_tiles;  // 1: every 32-row tile is a work unit (ring instance; small decode batches: the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
+    int split_tiles;  // 1: every 32-row tile is a work unit (ring instance), or the units are cut as below (the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
+    // kSplit: the first split_whole (sequence, v-head) units, a multiple of the grid, are work units as they are, the others are cut into
+    // split_parts parts of equally many tiles, no more of them than the grid has CTAs.
+    int split_whole, split_parts;
+    int num_units;  // work units of the launch
     int long_run;  // packed mode: sequences of at least this many tokens are recurrent_block.cuh's, in a launch of their own; shorter ones this kernel's
     long long num_tiles;
     int* status;
@@ -161,8 +165,13 @@ __device__ __forceinline__ float hsum(f2 v) {
 // promises that, and the corresponding run-time tests compile away.
 // kF32: the state is kept in fp32 in memory (read, updated and written as such; serving engines that run
 // many decode steps on one state use it to avoid a bf16 rounding per step).
-// kSplit (decode instance only): every tile is a work unit of its own.  An instance, because with the tiles per unit decided at
-// run time the others took 3 to 7 % longer (states in a pool, d=64, B=64: 12.8 -> 13.5 us; fp32, d=128, B=16: 11.9 -> 12.85).
+// kSplit (decode instance only, one token per sequence): the units of the last round are cut into parts, see split_whole.  An instance,
+// because with the tiles per unit decided at run time the others take longer (d=128, 32 v-heads, B=64 25.1 -> 25.6 us).
+// kPool (lean instances only): the states lie in an indexed pool.  Lean ones for pools and for fp32 states, d=128, 32 v-heads, general instance : lean:
+// pool B=10 8.6 : 7.5 us, B=28 16.3 : 14.5, B=64 29.7 : 25.8, B=93 38.9 : 34.4; fp32 B=18 16.4 : 16.1, B=93 66.7 : 66.4.
+// The barriers are set up in front of the wait for the work before (B=1 3.42 -> 3.41 us, d=64 B=16 4.85 -> 4.70).  (Requesting the first tiles in front
+// of the loads of the gating table costs batches of 28 and more 0.5 to 0.8 us, letting the next launch in early helps where every CTA
+// has the same work and leaves the others with uneven SMs, B=10 6.9 -> 8.0 us.)
 namespace rec {
 template <bool kF32>
 struct StateElem {
@@ -173,17 +182,18 @@ struct StateElem<true> {
     typedef float type;
 };
 }  // namespace rec
-template <int DK, bool kRing = true, bool kLean = false, bool kF32 = false, bool kSplit = false>
+template <int DK, bool kRing = true, bool kLean = false, bool kF32 = false, bool kSplit = false, bool kPool = false>
 __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     static_assert(!(kRing && kLean), "the lean instance is a decode instance");
-    static_assert(!(kRing && kSplit) && !(kLean && kSplit), "the split instance is a decode instance, and not the lean one");
+    static_assert(!(kRing && kSplit), "the split instance is a decode instance");
+    static_assert(kLean || !kPool, "the other instances look at state_idx themselves");
     using namespace ptx;
     using namespace rec;
     using Stage = RecStage<DK, kRing, kF32>;
     using ST = typename StateElem<kF32>::type;
     const ST* const state_in = static_cast<const ST*>(p.state_in);
     ST* const state_out = static_cast<ST*>(p.state_out);
-    constexpr bool kSkips = !kLean && !kSplit;  // (those run padded batches)
+    constexpr bool kSkips = !kLean && !kSplit;  // packed batches, some of whose sequences can be another launch's
     constexpr int NQ = DK / 32;  // packed pairs per row per lane (lane owns 4 columns of every 64)
     extern __shared__ __align__(128) uint8_t smem[];
     using TokSlot = RecTokSlot<DK>;
@@ -197,8 +207,12 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     // dt_bias staged here once per CTA (heads beyond the table are read from global memory).
     constexpr int kGateTable = 128;
     __shared__ float s_alog[kGateTable], s_dtb[kGateTable];
-    constexpr bool kPrep = !kRing && !kLean;
+    constexpr bool kPrep = !kRing && !kLean && !kSplit;  // (kSplit: one token per sequence)
     __shared__ __align__(16) RecPrepBuf<DK, kPrep> prep;
+    // kPool: slots of this CTA's work units, kSlots of them ahead: a look at state_idx where a tile is requested would put a global
+    // latency in front of the request
+    constexpr int kSlots = 64;
+    __shared__ int s_slot[kPool ? 2 * kSlots : 1];
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
@@ -207,18 +221,47 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     const bool has_in = kLean || p.state_in != nullptr;
     const bool store_step = !kLean && p.store_step != 0;
     const int rep = p.vh / p.kh;
-    const int tpu = kSplit || (kRing && p.split_tiles) ? 1 : rblocks;  // tiles per work unit
+    const int tpu = kRing && p.split_tiles ? 1 : rblocks;  // tiles per work unit (kSplit: of a whole one)
     const int upg = rblocks / tpu;                // work units per (sequence, v-head)
     const int upg_shift = (upg & (upg - 1)) == 0 ? __ffs(upg) - 1 : -1;
-    const int num_units = static_cast<int>(p.num_tiles / tpu);
+    const int parts = kSplit ? p.split_parts : 1, parts_shift = kSplit && (parts & (parts - 1)) == 0 ? __ffs(parts) - 1 : -1;
+    const int part_tiles = kSplit ? (parts_shift >= 0 ? rblocks >> parts_shift : rblocks / parts) : tpu;
+    const int num_units = p.num_units;
     const int stride = static_cast<int>(gridDim.x);
 
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
+        mbar_init(&tokfull[0], 1);
+        mbar_init(&tokfull[1], 1);
+        mbar_fence_init();
+    }
     // The kernel is launched as a programmatic dependent of the preceding work in the stream: its CTAs are placed
     // while that work drains and wait here, before the first access to global memory (a no-op for an ordinary launch).
     grid_dep_wait();
     // Packed runs some of which are the token-block kernel's: it is launched behind this one, may start now (what precedes this launch
     // is complete) and works on other sequences.
     if (kSkips && p.long_run != kRecNoLongRun) grid_dep_launch();
+    // head counts are almost always powers of two: shifts instead of integer divisions then
+    const int vh_shift = (p.vh & (p.vh - 1)) == 0 ? __ffs(p.vh) - 1 : -1;
+    const int rep_shift = (rep & (rep - 1)) == 0 ? __ffs(rep) - 1 : -1;
+    // (sequence, v-head) of a work unit of the instance kSplit
+    auto split_pair = [&](int unit) {
+        if (unit < p.split_whole) return unit;
+        const int i = unit - p.split_whole;
+        return p.split_whole + (parts_shift >= 0 ? i >> parts_shift : i / parts);
+    };
+    auto load_slot = [&](int ord0) {  // of this CTA's unit ord0 + tid
+        const long long unit = static_cast<long long>(ord0 + tid) * stride + blockIdx.x;
+        if (!kPool || tid >= kSlots || unit >= num_units) return 0;
+        const int sh = kSplit ? split_pair(static_cast<int>(unit)) : static_cast<int>(unit);
+        return __ldg(p.state_idx + (vh_shift >= 0 ? sh >> vh_shift : sh / p.vh));
+    };
+    auto keep_slot = [&](int ord0, int slot) {  // (visible behind the next barrier)
+        if (kPool && tid < kSlots) s_slot[(ord0 + tid) & (2 * kSlots - 1)] = slot;
+    };
+    static_assert(kSlots <= kRecThreads, "one thread per entry");
+    const int slot0 = load_slot(0);  // (kept behind the loads that follow: they need not wait for it)
     if (p.fused_gating) {
         for (int h = threadIdx.x; h < min(p.vh, kGateTable); h += blockDim.x) {
             s_alog[h] = p.gating_param_f32 ? __ldg(reinterpret_cast<const float*>(p.A_log) + h)
@@ -227,28 +270,27 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
                                           : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.dt_bias)[h]);
         }
     }
-    if (tid == 0) {
-        abort_flag = 0;
-        for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
-        mbar_init(&tokfull[0], 1);
-        mbar_init(&tokfull[1], 1);
-        mbar_fence_init();
-    }
+    keep_slot(0, slot0);
     __syncthreads();
 
     struct Unit {
         int seq, head, khead, ntok, rb0;
+        int tiles;  // kSplit: tiles of the work unit
         int slot;  // where the sequence's state lives (its index, or its slot of an indexed pool; negative: skip)
         long long tok0, bidx;
     };
-    // head counts are almost always powers of two: shifts instead of integer divisions then
-    const int vh_shift = (p.vh & (p.vh - 1)) == 0 ? __ffs(p.vh) - 1 : -1;
-    const int rep_shift = (rep & (rep - 1)) == 0 ? __ffs(rep) - 1 : -1;
-    auto decode = [&](int unit) {
+    auto decode = [&](int unit, int ord) {  // ord: the how manieth of this CTA
         Unit t;
         int sh = unit;
         t.rb0 = 0;
-        if (upg != 1) {
+        t.tiles = tpu;
+        if (kSplit) {
+            sh = split_pair(unit);
+            if (unit >= p.split_whole) {
+                t.rb0 = (unit - p.split_whole - (sh - p.split_whole) * parts) * part_tiles;
+                t.tiles = part_tiles;
+            }
+        } else if (upg != 1) {
             sh = upg_shift >= 0 ? unit >> upg_shift : unit / upg;
             t.rb0 = (unit - sh * upg) * tpu;
         }
@@ -273,7 +315,10 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
         }
         if (p.num_accepted) t.ntok = min(t.ntok, p.num_accepted[t.seq]);
         t.slot = t.seq;
-        if (!kLean && p.state_idx) {
+        if (kPool) {
+            t.slot = s_slot[ord & (2 * kSlots - 1)];
+            if (t.slot < 0) t.ntok = 0;
+        } else if (!kLean && p.state_idx) {
             t.slot = p.state_idx[t.seq];
             if (t.slot < 0) t.ntok = 0;
         }
@@ -347,21 +392,22 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     };
 
     // The producer walks (unit, rb) pairs kStages-1 iterations ahead of the consumers.
-    int prod_unit = blockIdx.x, prod_rb = 0, prod_it = 0;
+    int prod_unit = blockIdx.x, prod_rb = 0, prod_it = 0, prod_ord = 0;
     Unit prod_u{};
     if (tid == 0 && prod_unit < num_units) {
-        prod_u = decode(prod_unit);
+        prod_u = decode(prod_unit, 0);
         producer_bases(prod_u);
     }
     auto produce_one = [&]() {
         if (prod_unit >= num_units) return;
         issue(prod_u, prod_u.rb0 + prod_rb, prod_it % kStages);
         ++prod_it;
-        if (++prod_rb == tpu) {
+        if (++prod_rb == (kSplit ? prod_u.tiles : tpu)) {
             prod_rb = 0;
             prod_unit += stride;
+            ++prod_ord;
             if (prod_unit < num_units) {
-                prod_u = decode(prod_unit);
+                prod_u = decode(prod_unit, prod_ord);
                 producer_bases(prod_u);
             }
         }
@@ -372,7 +418,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
 
     uint32_t beta_bits = 0u, g_bits = 0u;  // scalars of the first token of the current unit
     if (static_cast<int>(blockIdx.x) < num_units) {
-        const Unit t0 = decode(blockIdx.x);
+        const Unit t0 = decode(blockIdx.x, 0);
         const int tk = kRing ? lane : 0;  // multi-token instance: lane l holds the scalars of token l
         if (tk < t0.ntok) load_scalars(t0, tk, beta_bits, g_bits);
     }
@@ -380,13 +426,15 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     int it = 0;
     int tb_it = 0;  // blocks that have gone through the multi-token ring (slot and parity bookkeeping)
     Unit T_carry{};
-    if (static_cast<int>(blockIdx.x) < num_units) T_carry = decode(blockIdx.x);
-    for (int unit = blockIdx.x; unit < num_units; unit += stride) {
+    if (static_cast<int>(blockIdx.x) < num_units) T_carry = decode(blockIdx.x, 0);
+    int ord = 0;  // units done
+    for (int unit = blockIdx.x; unit < num_units; unit += stride, ++ord) {
+        if (kPool && num_units > kSlots * stride && (ord & (kSlots - 1)) == 0) keep_slot(ord + kSlots, load_slot(ord + kSlots));  // (the units before `ord` are done)
         const Unit T = T_carry;
         float beta_first = beta_of(beta_bits), g_first = gate_of(g_bits);
         uint32_t beta_next = 0u, g_next = 0u;
         if (unit + stride < num_units) {
-            T_carry = decode(unit + stride);
+            T_carry = decode(unit + stride, ord + 1);
             const int tk = kRing ? lane : 0;
             if (tk < T_carry.ntok) load_scalars(T_carry, tk, beta_next, g_next);
         }
@@ -476,7 +524,7 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
             }
         }
 
-        for (int r = 0; r < tpu; ++r, ++it) {
+        for (int r = 0; r < (kSplit ? T.tiles : tpu); ++r, ++it) {
             const int rb = T.rb0 + r;
             const int stage = it % kStages;
             const uint32_t parity = static_cast<uint32_t>((it / kStages) & 1);
@@ -794,9 +842,9 @@ constexpr int recurrent_ctas_per_sm() {
     return kRing ? (DK <= 64 ? 4 : 3) : (DK <= 128 ? ((kF32 && DK > 64) ? 3 : 4) : 2);
 }
 
-template <int DK, bool kRing = false, bool kLean = false, bool kF32 = false, bool kSplit = false>
+template <int DK, bool kRing = false, bool kLean = false, bool kF32 = false, bool kSplit = false, bool kPool = false>
 __global__ void __launch_bounds__(kRecThreads, recurrent_ctas_per_sm<DK, kRing, kF32>()) gdn_recurrent_kernel(const RecurrentParams p) {
-    gdn_recurrent_body<DK, kRing, kLean, kF32, kSplit>(p);
+    gdn_recurrent_body<DK, kRing, kLean, kF32, kSplit, kPool>(p);
 }
 
 }  // namespace gdn
