@@ -362,8 +362,12 @@ static size_t ws_base_bytes(const GdnShape& s) {
 
 // The segment plan of a problem (heuristics.hpp); num_segments == 1: not segmented.
 static SegmentPlan segment_plan_of(const GdnShape& s, long long max_units = plan_detail::kNoLimit) {
-    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, s.total_chunks > 0 ? s.total_chunks : 0, max_units);
-    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, (s.seq_len + kChunk - 1) / kChunk, false, max_units);
+    const long long total = s.total_chunks > 0 ? s.total_chunks : 0;
+    const long long chunks = s.cu_seqlens ? (total + s.batch - 1) / std::max(s.batch, 1) : (s.seq_len + kChunk - 1) / kChunk;
+    if (chunks <= kShortChunks && (!s.cu_seqlens || s.batch <= kMaxSegmentedSeqs))
+        return prefill_segments_short(s.batch, s.num_v_heads, chunks, s.cu_seqlens ? total : chunks * s.batch, s.cu_seqlens != nullptr, max_units);
+    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, total, max_units);
+    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, static_cast<int>(chunks), false, max_units);
     plan.slots = s.batch * plan.num_segments;
     return plan;
 }
@@ -475,20 +479,22 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             if (int rc = run_zp()) return rc;
             if (int rc = run_seq(dim3(s.batch, s.num_v_heads))) return rc;
         } else {
-            // composite transitions of all segments, their start states, then all segments at once
+            // the composite transitions of the segments and, beside them, the first segment of every sequence outright; the others' start
+            // states; then all of the others at once (long sequences: transitions of the first segments too, and all of them at once)
             float* seg_mn = reinterpret_cast<float*>(ws_extra);
             const size_t seg_units = static_cast<size_t>(plan.slots) * s.num_v_heads;
             float* seg_start = seg_mn + seg_units * 2 * kD * kD;
             p.seg_chunks = plan.seg_chunks;
             p.num_segments = plan.num_segments;
             p.num_seqs = s.batch;
+            p.first_apart = plan.first_apart;
             p.seg_mn = seg_mn;
             p.seg_start = seg_start;
             if (int rc = set_smem<gdn_seg_transition_kernel>(TransitionSmem::kBytes)) return rc;
             if (int rc = set_smem<gdn_seg_combine_kernel>(SegCombineSmem::kBytes)) return rc;
             if (int rc = run_zp()) return rc;
             // the launches of the segmented path, each a programmatic dependent of the one before it (every one of them waits
-            // before its first access to what that one wrote)
+            // before its first access to what that one wrote; the first segments run beside the transitions)
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -500,6 +506,10 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             cfg.blockDim = dim3(transition::kThreads);
             cfg.dynamicSmemBytes = TransitionSmem::kBytes;
             GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_transition_kernel, tmK, tmV, p));
+            if (plan.first_apart) {
+                p.mode = 1;
+                if (int rc = run_seq(dim3(s.batch, s.num_v_heads))) return rc;
+            }
             SegCombineParams cp{};
             cp.seg_mn = seg_mn;
             cp.seg_start = seg_start;
@@ -507,6 +517,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             cp.si_ss = p.si_ss;
             cp.si_sh = p.si_sh;
             cp.d = hd;
+            cp.first_apart = plan.first_apart;
             cp.vh = s.num_v_heads;
             cp.num_segments = plan.num_segments;
             cp.map = p.map;

@@ -84,6 +84,7 @@ struct SegmentPlan {
     int seg_chunks;    // chunks per segment
     int slots;         // (sequence, segment) pairs the launches cover: batch x num_segments in padded mode,
                        // an upper bound in packed mode (the lengths are only known on the device)
+    int first_apart = 0;  // 1: the first segments are walked outright beside the transitions of the others (FusedParams::mode 1)
 };
 namespace plan_detail {
 constexpr long long kSms = 148;
@@ -153,6 +154,44 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
             plan.num_segments = P;
             plan.seg_chunks = len;
             plan.slots = static_cast<int>(slots);
+        }
+    }
+    return plan;
+}
+
+// Plan of sequences of up to kShortChunks chunks, of `chunks` chunks each (packed: on average, with `total` in all).  The first segments are walked
+// outright beside the transitions of the others (FusedParams::mode 1), so P segments of c chains take c (P - 1) CTAs in either launch.
+// In chunks of the state kernel, fitted to 60 shapes of 2 to 48 chains and 16 to 500 chunks with 3 to 36 segments (its choices are within 3 %
+// of the best measured): both launches a chunk and more (what they read grows with the chains), one step of the start states for
+// every segment from the third on, longer where many chains share their kernel, and 10.5 for four launches instead of one.  d=128, whole : so,
+// us: 4 chains of 32 chunks 44.8 : 41.4, of 64 76.8 : 53.1, of 100 115 : 62.6, of 256 277 : 89.1; 16 of 64 88 : 75, of 256 322 : 170; 32 of 100 155 : 140,
+// of 256 384 : 289; 48 of 256 433 : 376.  Against the plan above, whose segments have 25 chunks and more and whose first ones are found like the
+// others: 1 sequence of 7919 tokens on 32 v-heads 177 : 161, 2 of 7344 on 8 125 : 101, 1 of 22109 on 4 121 : 103, packed 4 of 4000 on 4 165 : 82.
+// Longer sequences are bound by what the launches move, and a launch more costs them 1 % (4 chains of 1024 chunks in 32 segments 195 : 198): they
+// keep the plans above.
+constexpr int kShortChunks = 640, kManyChains = 48;
+inline SegmentPlan prefill_segments_short(long long seqs, int num_v_heads, long long chunks, long long total, bool packed,
+                                          long long max_units = plan_detail::kNoLimit) {
+    using namespace plan_detail;
+    SegmentPlan plan{1, static_cast<int>(chunks), packed ? 0 : static_cast<int>(seqs)};
+    const long long chains = seqs * num_v_heads;
+    if (chains <= 0 || chains > kManyChains) return plan;
+    const double c = static_cast<double>(chains);
+    double best = 0.985 * static_cast<double>(chunks + kFixed);
+    for (int P = 3; P <= 64 && chunks / P >= 5; ++P) {
+        const long long len = (chunks + P - 1) / P;
+        // packed: every sequence end but the last may add a short segment; slots for any split of the chunks over the sequences are
+        // launched and given scratch
+        const long long work = packed ? (total + len - 1) / len + seqs - 1 : seqs * P, slots = packed ? total / len + seqs : seqs * P;
+        if ((work - seqs) * num_v_heads > kSms) break;
+        if (slots * num_v_heads > max_units) continue;
+        const double cost = (2.0 + 0.01 * c) * static_cast<double>(len + kFixed) + (1.1 + 0.009 * c * c) * (P - 2) + 10.5;
+        if (cost < best) {
+            best = cost;
+            plan.num_segments = P;
+            plan.seg_chunks = static_cast<int>(len);
+            plan.slots = static_cast<int>(slots);
+            plan.first_apart = 1;
         }
     }
     return plan;

@@ -50,11 +50,17 @@ struct FusedParams {
     // S' = S M_c + N_c per chunk, so a segment of chunks has a composite (M, N) as well; gdn_seg_transition_kernel
     // leaves them in fp32 in seg_mn[(slot * vh + head) * 2 + {N, M}], slot = a (sequence, segment) pair (locate_segment).
     //   mode 0: one CTA walks the whole sequence (grid = sequences x heads, or heads x ranks with seq_order).
-    //   mode 2: grid = (slots, heads); starts from seg_start[slot * vh + head] (fp32), writes the
-    //           output of its chunks; the last segment of a sequence writes the final state.
-    int mode, seg_chunks, num_segments, num_seqs;
+    //   mode 1: the first segment of every sequence (grid = sequences x heads), beside the transitions of the segments behind it.  It
+    //           needs none itself: it starts from the initial state, writes its output, and leaves the start state of the second
+    //           segment (fp32), or the final state where there is no other.  A programmatic dependent of the transitions' launch, which
+    //           lets it start when the chunk-parallel kernel in front of both is complete; it waits for that launch at its end, so that who
+    //           waits for this one waits for both.  (The other way round the transitions, the longer of the two, start later: 4 v-heads of
+    //           2500 tokens 45.5 -> 47.5 us.)
+    //   mode 2: grid = (slots, heads), the other segments (first_apart 0: all of them, mode 1 is not launched); starts from
+    //           seg_start[slot * vh + head] (fp32), writes the output of its chunks; the last segment of a sequence writes the final state.
+    int mode, seg_chunks, num_segments, num_seqs, first_apart;
     float* seg_mn;
-    const float* seg_start;
+    float* seg_start;
     // Packed mode with more CTAs than SMs: sequences sorted by length, longest first (written by
     // gdn_seq_order_kernel).  Then blockIdx.x = head and blockIdx.y = rank of the sequence, so the
     // longest chains are dispatched first and the short ones fill the tail.  NULL: blockIdx.x =
@@ -155,9 +161,15 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     SegPos sp{0, 0, 1, 0};
-    if (p.mode != 0) {
+    if (p.mode == 1) {
+        sp = sequence_segments(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments);
+    } else if (p.mode == 2) {
         sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
-        if (sp.seq < 0) return;  // packed mode launches an upper bound of slots
+        if (sp.seq < 0 || (sp.segment == 0 && p.first_apart)) {  // packed mode launches an upper bound of slots; first segments are done
+            // Whoever waits for this grid waits for all of the call: the grid must not complete before the launches in front of it.
+            if (blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
+            return;
+        }
     }
     const int seq = p.mode != 0 ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
     const int head = p.mode == 0 && p.seq_order ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
@@ -378,7 +390,14 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // nothing is written once a wait of this CTA has given up (the results would be garbage)
         const bool healthy = *abort_flag == 0;
         if (!healthy) {
-        } else if (p.state_out && (p.mode == 0 || segment == seq_nseg - 1)) {
+        } else if (p.mode != 0 && segment != seq_nseg - 1) {
+            if (p.mode == 1) {
+                float4* d4 = reinterpret_cast<float4*>(p.seg_start + (static_cast<long long>(sp.first_slot + 1) * p.vh + head) * (D * D) +
+                                                       static_cast<long long>(row) * D + 64 * hf);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) d4[q] = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
+            }
+        } else if (p.state_out) {
             uint4* d4 = reinterpret_cast<uint4*>(p.state_out + seq * p.so_ss + head * p.so_sh +
                                                  static_cast<long long>(row) * p.d + 64 * hf);
 #pragma unroll
@@ -486,7 +505,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         load_raw(1, rb0, rb1);
         // Everything up to here (and the state warps' load of the initial state) touches only the caller's
         // inputs and may run while the chunk-parallel kernel drains; its blocks and norm factors are read below.
-        grid_dep_wait();
+        if (p.mode != 1)
+            grid_dep_wait();
+        else if (lane == 0)
+            grid_dep_launch();  // the start states' kernel sets itself up on the SMs that are left and waits there
         for (int c = 0; c < nchunks; ++c) {
             const int s = c & 1;
             const int n = chunk_n(c);
@@ -552,7 +574,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // kLead positions after the one the producer has just requested into L2, so that the producer's own
         // loads find them there.  A hint only: when its bounded wait runs out it simply stops.
         constexpr int kLead = 3;
-        grid_dep_wait();
+        if (p.mode != 1) grid_dep_wait();
         if (lane == 0) {
             for (int c = kLead; c < nchunks; ++c) {
                 int spins = 0;
@@ -620,6 +642,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         }
     }
 
+    if (p.mode == 1 && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);

@@ -1,5 +1,5 @@
 // Start states of the segments of a segmented prefill run (see FusedParams in prefill_fused.cuh):
-//     S_start[0] = initial state,   S_start[p + 1] = S_start[p] M_p + N_p
+//     S_start[0] = initial state (or S_start[1] as the first segment's run has left it),   S_start[p + 1] = S_start[p] M_p + N_p
 // with M_p, N_p the composite transition of segment p (fp32, dv x dk and dk x dk with dv = dk = 128)
 // produced by gdn_seg_transition_kernel.  Segment p of a sequence sits in launch
 // slot first_slot + p (locate_segment in prefill_common.cuh); in packed mode the sequences have
@@ -20,12 +20,12 @@ namespace gdn {
 
 struct SegCombineParams {
     const float* seg_mn;   // [slot][head][2][128][128]: N then M
-    float* seg_start;      // [slot][head][128][128]
-    ChunkMap map;
-    int seg_chunks;
+    float* seg_start;      // [slot][head][128][128]; first_apart: those of the second segments are given, and none is made for the first
     const __nv_bfloat16* state_in;  // or NULL; d x d per (sequence, head), zero outside when d < 128
     long long si_ss, si_sh;
-    int d;
+    int d, first_apart;
+    ChunkMap map;
+    int seg_chunks;
     int vh, num_segments;
     int* status;
 };
@@ -53,14 +53,17 @@ __global__ void __launch_bounds__(SegCombineSmem::kThreads) gdn_seg_combine_kern
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
     int* abort_flag = reinterpret_cast<int*>(bar + 2);
 
-    ptx::grid_dep_wait();  // launched as a programmatic dependent of the composite-transition launch
+    // launched as a programmatic dependent of the first segments' launch, or of the transitions'; the output launch may be placed as soon as all CTAs here are
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     const long long chain = blockIdx.x;
     const int warp = threadIdx.x >> 5, col = 4 * (threadIdx.x & 31);
     const int row = blockIdx.y * R + warp;  // this thread's piece of the running state: row `row`, columns col .. col + 3
     const int seq = static_cast<int>(chain / p.vh), head = static_cast<int>(chain % p.vh);
     const SegPos sp = sequence_segments(p.map, seq, p.seg_chunks, p.num_segments);
-    const int nseg = sp.nseg;
-    auto idx = [&](int s) { return static_cast<long long>(sp.first_slot + s) * p.vh + head; };
+    const int steps = sp.nseg - 1 - p.first_apart;  // products: S_start[first_apart + 1] and on
+    if (p.first_apart && steps <= 0) return;
+    auto idx = [&](int s) { return static_cast<long long>(sp.first_slot + p.first_apart + s) * p.vh + head; };
     auto request_m = [&](int s) {  // one thread
         mbar_arrive_expect_tx(&bar[s & 1], D * D * 4);
         bulk_load(sM + (s & 1) * D * D, p.seg_mn + (idx(s) * 2 + 1) * (D * D), D * D * 4, &bar[s & 1]);
@@ -70,22 +73,25 @@ __global__ void __launch_bounds__(SegCombineSmem::kThreads) gdn_seg_combine_kern
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         mbar_fence_init();
-        for (int s = 0; s < 2 && s + 1 < nseg; ++s) request_m(s);  // (the last segment's transition is not needed)
+        for (int s = 0; s < 2 && s < steps; ++s) request_m(s);
     }
     float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.state_in && row < p.d && col < p.d) {  // (d is a multiple of 8)
-        const uint2 w = *reinterpret_cast<const uint2*>(p.state_in + seq * p.si_ss + head * p.si_sh + static_cast<long long>(row) * p.d + col);
-        cur = make_float4(bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y));
+    if (p.first_apart) {
+        cur = *reinterpret_cast<const float4*>(p.seg_start + idx(0) * (D * D) + row * D + col);
+    } else {
+        if (p.state_in && row < p.d && col < p.d) {  // (d is a multiple of 8)
+            const uint2 w = *reinterpret_cast<const uint2*>(p.state_in + seq * p.si_ss + head * p.si_sh + static_cast<long long>(row) * p.d + col);
+            cur = make_float4(bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y));
+        }
+        *reinterpret_cast<float4*>(p.seg_start + idx(0) * (D * D) + row * D + col) = cur;
     }
     auto load_n = [&](int s) {
-        return s + 1 < nseg ? *reinterpret_cast<const float4*>(p.seg_mn + idx(s) * 2 * (D * D) + row * D + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return s < steps ? *reinterpret_cast<const float4*>(p.seg_mn + idx(s) * 2 * (D * D) + row * D + col) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     float4 nxt = load_n(0);  // N of the coming segment, fetched one iteration ahead
     *reinterpret_cast<float4*>(&sS[warp][col]) = cur;
     __syncthreads();
-    for (int s = 0; s < nseg; ++s) {
-        *reinterpret_cast<float4*>(p.seg_start + idx(s) * (D * D) + row * D + col) = cur;
-        if (s + 1 == nseg) break;
+    for (int s = 0; s < steps; ++s) {
         const float4 n = nxt;
         nxt = load_n(s + 1);
         mbar_wait(&bar[s & 1], static_cast<uint32_t>((s >> 1) & 1), abort_flag);
@@ -118,13 +124,14 @@ __global__ void __launch_bounds__(SegCombineSmem::kThreads) gdn_seg_combine_kern
 #pragma unroll
         for (int r = 0; r < R; ++r) *reinterpret_cast<ulonglong2*>(&sRed[warp][r][col]) = make_ulonglong2(acc[r][0], acc[r][1]);
         __syncthreads();  // the partial sums are there, sS and this M buffer free
-        if (threadIdx.x == 0 && s + 3 < nseg) request_m(s + 2);
+        if (threadIdx.x == 0 && s + 2 < steps) request_m(s + 2);
         cur = n;
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
             const float4 v = *reinterpret_cast<const float4*>(&sRed[w][warp][col]);
             cur.x += v.x; cur.y += v.y; cur.z += v.z; cur.w += v.w;
         }
+        *reinterpret_cast<float4*>(p.seg_start + idx(s + 1) * (D * D) + row * D + col) = cur;
         *reinterpret_cast<float4*>(&sS[warp][col]) = cur;
         __syncthreads();  // sS complete, the partial sums read
     }

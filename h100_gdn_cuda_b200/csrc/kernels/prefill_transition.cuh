@@ -6,7 +6,7 @@
 // A run is a chain of dependent steps that leaves the tensor pipe idle 80 % of the time and the schedulers 60 %; two runs
 // on the same tiles fill each other's gaps and read K, Z and the gates once.  Each run has 8 state warps of its own, the
 // first MMA's accumulator shares the columns of the second's (it is dead once R is published), so both fit tensor memory.
-// B=2, T=131072, 4 v-heads (136 CTAs of 114 chunks): replaces two waves of one run per CTA, see gdn_chunked_forward.
+// B=2, T=131072, 4 v-heads (128 CTAs of 114 chunks): replaces two waves of one run per CTA, see gdn_chunked_forward.
 #pragma once
 #include <cuda.h>
 
@@ -54,10 +54,11 @@ __global__ void __launch_bounds__(transition::kThreads, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const SegPos sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
-    if (sp.seq < 0 || sp.segment == sp.nseg - 1) {  // surplus slot; nothing follows a sequence's last segment
-        // The launches behind this one wait for this grid alone, so it must not complete before the chunk-parallel kernel
-        // has: every CTA waits for that, the ones without work too (all of them, where no sequence has a second segment).
-        grid_dep_wait();
+    // surplus slot; nothing follows a sequence's last segment; a first one is walked outright
+    if (sp.seq < 0 || sp.segment == sp.nseg - 1 || (sp.segment == 0 && p.first_apart)) {
+        // The launch behind this one starts when all CTAs here have let it or are gone, or waits for this grid, and takes it that the
+        // chunk-parallel kernel is complete then.  So the first CTA, whose segment is a first one, waits for that in any case.
+        if (blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
         return;
     }
     const int head = static_cast<int>(blockIdx.y), khead = head / (p.vh / p.kh);
@@ -215,6 +216,9 @@ __global__ void __launch_bounds__(transition::kThreads, 1)
         load_raw(0, ra0, ra1);
         load_raw(1, rb0, rb1);
         grid_dep_wait();
+        // what is launched next, the first segments, reads what this launch does, complete now, and runs beside it (or it is the start
+        // states' kernel, which sets itself up and waits)
+        if (lane == 0) grid_dep_launch();
         int s = 0;
         uint32_t ephase = 1;
         for (int c = 0; c < nchunks; ++c) {

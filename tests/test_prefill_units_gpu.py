@@ -137,3 +137,38 @@ def test_packed_calls_back_to_back():
             differ += (o != o0).sum() + (s != s0).sum()
     assert differ.item() == 0
     assert _cabi.load().gdn_device_status(0, C.byref(st)) == 0 and st.value == 0
+
+
+# segments of 5 chunks and more, first ones walked outright: sequences of one segment (empty, at the front), of two, of many, ragged ends;
+# and long ones, whose first segments are found like the others
+@pytest.mark.parametrize("lens,kh,vh,norm", [([3000], 1, 2, False), ([100, 3840, 2883, 1920], 1, 1, True), ([0, 6400, 5000, 0], 1, 1, False),
+                                             ([64 * 36], 2, 4, False), ([64 * 40, 64 * 41 + 1], 1, 3, True), ([700, 9000, 700], 1, 2, False),
+                                             ([42000], 1, 1, False)])
+@pytest.mark.parametrize("state", [False, True])
+def test_short_segments_back_to_back(lens, kh, vh, norm, state):
+    """against the oracle, and calls that follow one another without a pause, each from the states of the one before: what a launch
+    leaves for the next must be complete, whichever of them run side by side"""
+    import h100_gdn_cuda_b200 as gdn
+    from oracle import gdn_oracle as O
+    p = synthetic.varlen_inputs(lens, kh, vh, 128, seed=sum(lens), mild_gate=True, normalize=not norm)
+    s0 = p["state"] if state else None
+    o_ref, s_ref = O.recurrent_ref(*(p[k].float() for k in ("q", "k", "v", "beta")), p["g"], s0.float() if state else None,
+                                   cu_seqlens=p["cu_seqlens"], is_qk_norm=norm)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+    run = lambda s: gdn.chunked_forward(c["q"], c["k"], c["v"], c["beta"], c["g"], None, s, c["cu_seqlens"], c["chunk_indices"], c["cu_chunks"],
+                                        c["total_chunks"], is_qk_norm=norm)
+    o, s = run(c["state"] if state else None)
+    for x, ref in ((o, o_ref), (s, s_ref)):
+        assert O.rel_fro(x.float().cpu(), ref) <= 1e-2 and O.max_abs_over_max(x.float().cpu(), ref) <= 5e-2
+
+    def chain(sync):
+        x, outs = s, []
+        for _ in range(12):
+            y, x = run(x)
+            outs.append(y)
+            if sync:
+                torch.cuda.synchronize()
+        return outs, x
+
+    a, b = chain(True), chain(False)
+    assert torch.equal(a[1], b[1]) and all(torch.equal(x, y) for x, y in zip(a[0], b[0]))
