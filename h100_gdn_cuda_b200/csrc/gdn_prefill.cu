@@ -469,10 +469,14 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
         };
         if (plan.num_segments <= 1 && packed && s.batch > 1 && s.batch <= kMaxOrderedSeqs && chains > d->sms) {
             // more chains than SMs and unequal lengths: dispatch the longest sequences first
-            int* order = reinterpret_cast<int*>(ws_extra);
-            gdn_seq_order_kernel<<<(s.batch + 127) / 128, 128, 0, st>>>(s.cu_seqlens, s.batch, order);
-            GDN_CUDA(cudaGetLastError());
-            p.seq_order = order;
+            p.num_seqs = s.batch;
+            p.by_length = s.batch <= kMaxRankedSeqs;
+            if (!p.by_length) {
+                int* order = reinterpret_cast<int*>(ws_extra);
+                gdn_seq_order_kernel<<<(s.batch + 127) / 128, 128, 0, st>>>(s.cu_seqlens, s.batch, order);
+                GDN_CUDA(cudaGetLastError());
+                p.seq_order = order;
+            }
             if (int rc = run_zp()) return rc;
             if (int rc = run_seq(dim3(s.num_v_heads, s.batch))) return rc;
         } else if (plan.num_segments <= 1) {

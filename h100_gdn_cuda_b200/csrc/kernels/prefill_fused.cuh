@@ -61,10 +61,11 @@ struct FusedParams {
     int mode, seg_chunks, num_segments, num_seqs, first_apart;
     float* seg_mn;
     float* seg_start;
-    // Packed mode with more CTAs than SMs: sequences sorted by length, longest first (written by
-    // gdn_seq_order_kernel).  Then blockIdx.x = head and blockIdx.y = rank of the sequence, so the
-    // longest chains are dispatched first and the short ones fill the tail.  NULL: blockIdx.x =
-    // sequence, blockIdx.y = head.
+    // Packed mode with more CTAs than SMs: the longest sequences first.  Then blockIdx.x = head and blockIdx.y = rank of the sequence, so the
+    // longest chains are dispatched first and the short ones fill the tail.  by_length: every CTA finds the sequence of its rank itself
+    // (num_seqs of them, kMaxRankedSeqs at most); otherwise seq_order, if not NULL, has them (written by gdn_seq_order_kernel).  Neither:
+    // blockIdx.x = sequence, blockIdx.y = head.
+    int by_length;
     const int* seq_order;
 };
 
@@ -80,6 +81,10 @@ struct FusedSmem {
     static constexpr int kOffBar = kOffGate + 3 * kGateStride;
     static constexpr int kBytes = kOffBar + 128 + 1024;
 };
+
+// Sequences that a CTA ranks by itself, a lane each.  A launch for it costs more: 12 sequences of 3000 tokens on 16 v-heads 39.3 -> 38.3 us, 6 of 9000
+// on 32 137 -> 133; ranking 100 in every CTA costs more than the launch (4 v-heads, 6400 tokens 42.7 -> 43.3).
+constexpr int kMaxRankedSeqs = 32;
 
 namespace fused {
 constexpr int kThreads = 512;  // 16 warps = 4 warpgroups (the last holds the producer, the issuer and 2 idle warps)
@@ -171,8 +176,19 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             return;
         }
     }
-    const int seq = p.mode != 0 ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
-    const int head = p.mode == 0 && p.seq_order ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
+    if (p.by_length) {
+        // order of the sequences: more tokens first, of equally many the one in front first (every warp for itself)
+        const int mine = lane < p.num_seqs ? p.map.cu_seqlens[lane + 1] - p.map.cu_seqlens[lane] : -1;
+        int rank = 0;
+        for (int j = 0; j < p.num_seqs; ++j) {
+            const int other = __shfl_sync(0xffffffffu, mine, j);
+            rank += other > mine || (other == mine && j < lane);
+        }
+        sp.seq = __ffs(__ballot_sync(0xffffffffu, lane < p.num_seqs && rank == static_cast<int>(blockIdx.y))) - 1;
+    }
+    const bool ranked = p.by_length || p.seq_order;
+    const int seq = p.mode != 0 || p.by_length ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
+    const int head = ranked ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
     const int segment = sp.segment, seq_nseg = sp.nseg;
     const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;  // mode 2
     const int khead = head / (p.vh / p.kh);
