@@ -48,11 +48,13 @@ struct BlockSmem {
     // rows of k and q are 16 bytes longer than the data: eight rows at one column lie in different banks
     static constexpr int kRow = DK * 2 + 16;
     static constexpr int kOffQ = kBlkTok * kRow, kOffV = 2 * kBlkTok * kRow;
-    static constexpr int kStage = kOffV + kBlkTok * kRows * 2;
+    // What the outputs are made of, per group scale G_t (S_0 q_t) and c, 16 rows of 16 tokens each: over q once the group has its
+    // products, behind v where there is another group that may still be at its own.
+    static constexpr int kOut = 2 * kBlkRows * kBlkTok * 4, kOffO = kGroups == 1 ? kOffQ : kOffV + kBlkTok * kRows * 2;
+    static constexpr int kOffC1 = kOffO + kBlkRows * kBlkTok * 4;
+    static constexpr int kStage = kOffV + kBlkTok * kRows * 2 + (kGroups == 1 ? 0 : kGroups * kOut);
     static constexpr int kStages = 4;  // one per preparing warp
-    // over q once its products are there: what the outputs are made of, per group scale G_t (S_0 q_t) and c, 16 rows of 16 tokens each
-    static constexpr int kOffO = kOffQ, kOffC1 = kOffQ + kBlkRows * kBlkTok * 4, kOut = 2 * kBlkRows * kBlkTok * 4;
-    static_assert(kOffO + kGroups * kOut <= kOffV, "they fit over q");
+    static_assert(kGroups > 1 || kOffO + kOut <= kOffV, "they fit over q");
     // what a block's solve needs, floats: A as [s][t], P as [t][s], beta v as [row][t] (before that: decay products), factors
     static constexpr int kA = 0, kP = 256, kR0 = 512, kLdR = 20, kCk = kR0 + kRows * kLdR, kCq = kCk + 16, kW = kCq + 16, kG = kW + 16;
     static constexpr int kPrepFloats = kG + 4;

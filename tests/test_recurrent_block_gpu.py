@@ -200,6 +200,18 @@ def test_two_groups_of_rows(gdn, d, vh, lens):
         at += n
 
 
+@pytest.mark.parametrize("d,vh", [(192, 12), (256, 9)])
+def test_two_groups_repeat_bit_for_bit(gdn, d, vh):
+    """The groups of a CTA run apart by up to a block, differently each time: what one of them writes may not lie where the other still
+    reads."""
+    p, c = inputs(2, 600, vh, vh, d, False, d)
+    run = lambda: gdn.recurrent_forward(c["q"], c["k"], c["v"], c["state"], c["beta"], c["g"], inference_mode=gdn.Decode, is_qk_norm=False)
+    o, s = run()
+    for _ in range(40):
+        oi, si = run()
+        assert torch.equal(o, oi) and torch.equal(s, si)
+
+
 @pytest.mark.parametrize("d,f32,T", LINES)
 def test_either_side_of_the_line(gdn, d, f32, T):
     norm = T % 2 == 0
