@@ -312,7 +312,7 @@ int gdn_compute_o(const GdnComputeOArgs* a, gdn_stream_t stream) {
 // Head dims above the 128 the tensor-core kernels are built for (192 and 256, which the
 // reference's chunked kernels accept: sm90_bf16_gdn_compute_u_w.cuh:169) take the recurrent path: the same layer
 // semantics with the state and all intermediates in fp32 from the first token to the last, no scratch, one launch
-// (recurrent_block.cuh, sequences of many tokens in blocks of 16: B=2 T=1500 8 v-heads d=256 217 us, 997 token by token).  (A chunked form on 256
+// (recurrent_block.cuh, sequences of many tokens in blocks of 16: B=2 T=1500 8 v-heads d=256 200 us, 997 token by token).  (A chunked form on 256
 // columns whose operands were sums of two bf16 terms, 16 significand bits, took 121 us there but stood further from the
 // 64-bit result: 0.1 to 0.55 % of the bf16 outputs rounded the other way against 0.003 to 0.16 %.)
 static bool wide_heads(const GdnShape& s) { return s.head_dim_k > kD || s.head_dim_v > kD; }

@@ -31,14 +31,15 @@ inline RecurrentConfig recurrent_config(int dk, long long num_tiles, int sms, bo
 }
 
 // Token-block kernel, head dims 192 and 256: groups of 16 state rows per CTA, 1 (two CTAs fit an SM) or 2 (one does; they share the
-// preparation of the blocks).  A row's sums are the same in either.  A block of 16 tokens takes about 3.0 thousand cycles where a CTA
-// with one group has the SM to itself, 4.7 where two share it, and 4.3 with two groups.  In us, one group : two: d=256, 8 v-heads, T=1500
-// B=2 236 : 217, T=1000 B=4 315 : 292, T=500 B=8 (a last wave of half the tiles) 291 : 305; d=192 B=2 T=700 101 : 96; 16 packed sequences of
-// 500 573 : 541.  (At d=128 one group is as fast or faster: B=8 T=512, 8 v-heads 120 : 121, B=4, 32 v-heads 213 : 239.)
+// preparation of the blocks).  A row's sums are the same in either.  A block of 16 tokens takes about 2.8 thousand cycles where a CTA
+// with one group has the SM to itself, 4.3 where two share it, and 4.1 with two groups.  In us, one group : two: d=256, 8 v-heads, T=1500
+// B=2 211 : 200, T=1000 B=4 283 : 270, B=3 (a last wave of few tiles) 229 : 270, T=500 B=8 (a last wave of half the tiles) 261 : 283; d=192
+// T=700 B=2 91 : 84, B=4 144 : 163, B=6 178 : 164; 16 packed sequences of 500 510 : 501.  (At d=128, where two groups share less, one is as
+// fast or faster: B=8 T=512, 8 v-heads 120 : 121, B=4, 32 v-heads 213 : 239, measured with a solve that took 350 cycles more.)
 inline int block_groups(long long tiles, int sms) {
     const long long pairs = 2ll * sms, rest = tiles % pairs;
-    const double one = 4.7 * static_cast<double>(tiles / pairs) + (rest == 0 ? 0.0 : rest <= sms ? 3.0 : 4.7);
-    const double two = 4.3 * static_cast<double>((tiles + pairs - 1) / pairs);
+    const double one = 4.3 * static_cast<double>(tiles / pairs) + (rest == 0 ? 0.0 : rest <= sms ? 2.8 : 4.3);
+    const double two = 4.1 * static_cast<double>((tiles + pairs - 1) / pairs);
     return two < one ? 2 : 1;
 }
 

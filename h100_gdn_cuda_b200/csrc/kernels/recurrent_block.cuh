@@ -14,25 +14,27 @@
 // 40 % further off than token by token, so those take the token recurrence.)
 //
 // Why: the token recurrence (recurrent.cuh, ring instance) is a chain of about 1 250 cycles per token, and a sequence of a
-// few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of some 3 000 cycles: products (1 000),
-// sums and a triangular solve (850), the update (500), and the barrier, the hand-over to the writing warps and the waits between them:
-// B=2, T=1500, 8 v-heads, d=256 996 -> 236 us (another 400 cycles a block with the outputs written by the warps that hold the state), 4 v-heads
-// B=1 994 -> 150, T=700, d=192 401 -> 66; B=4, T=4096, 32 v-heads, d=128 5.54 -> 1.65 ms.  With two CTAs per SM issue
-// (5 100 warp instructions per block and CTA, 54 % of the slots), shared memory (1 270 wavefronts, as much) and the matrix
-// instructions (26 %) share the time without one of them filling it; with one CTA the chain does.
+// few v-heads gives it only some tiles to work on side by side.  Here a block of 16 tokens is one chain of some 2 800 cycles: products (1 000),
+// sums and a triangular solve (500), the update (500), two barriers, the hand-over to the writing warps and the waits between them:
+// B=2, T=1500, 8 v-heads, d=256 996 -> 200 us, 4 v-heads B=1 994 -> 138, T=700, d=192 401 -> 84; B=4, T=512, 32 v-heads, d=128 188 us.
+// With two CTAs per SM issue, shared memory (each about half of its time) and the matrix instructions (a quarter) share the time without one
+// of them filling it; with one CTA the chain does.
 //
 // A CTA owns 16 state rows (M of the products) of one (sequence, v-head) and walks its blocks:
 //   warps 0-3   a quarter of the columns each, kept as accumulator fragments, which are the A operands of the product
-//               S_0 [k; q]^T as they lie.  The four partial products meet in shared memory; then EVERY warp sums them and
-//               solves for c (lane r + 16 h: row r, tokens 8 h .. 8 h + 7), which costs less than a second barrier and a
-//               trip through shared memory, and updates its own columns.
+//               S_0 [k; q]^T as they lie.  The four partial products meet in shared memory; then each warp solves for c of four rows,
+//               eight lanes to a row with two tokens each, and hands them over as an operand of the update, which every warp makes
+//               of its own columns.  The substitution is seven exchanges between lanes of about 45 cycles: a lane takes its two
+//               tokens in one step.  (Every warp all 16 rows, a row in two lanes, needs no second barrier but four times the
+//               loads, and the solve takes 850 cycles: d=256 B=2 T=1500 217 us, B=1 152, T=700 d=192 95; one token per exchange 201, 141, 86.)
 //   warps 4-7   prepare blocks in turn (warp 4 + j: blocks j, j + 4, ..), up to four ahead: copies of k, q, v, the Gram matrices
 //               k k^T and q k^T on matrix instructions, decay products, norms, and from them the matrices A and P; when a
-//               block is through they write its outputs.
+//               block is through they write its outputs.  (Written by the warps that hold the state they cost 400 cycles a block.)
 //               (Four of them, so that their work is spread over the four schedulers.)
-// Two CTAs per SM at dk = 256: one's chain fills the gaps of the other (4 700 cycles a block for the pair).  kGroups = 2: one CTA of two such
-// groups of four warps, 32 rows, with one preparation for both (4 300 cycles; B=2, T=1500, 8 v-heads, d=256 236 -> 217 us).  Four warps
-// with 32 rows each share k and q in registers too, and the substitution, but a warp is a chain of its own: 359 us.
+// Two CTAs per SM at dk = 256: one's chain fills the gaps of the other (4 300 cycles a block for the pair).  kGroups = 2: one CTA of two such
+// groups of four warps, 32 rows, with one preparation for both (4 100 cycles; B=2, T=1500, 8 v-heads, d=256 211 -> 200 us).  Four warps
+// with 32 rows each share k and q in registers too, and the substitution, but a warp is a chain of its own: 359 us.  Additions and FMAs of the
+// state in pairs (f32x2) spill: 217 us.
 #pragma once
 #include "recurrent_step.cuh"
 
@@ -62,9 +64,9 @@ struct BlockSmem {
     static constexpr int kLdD = 36;  // partial products of a warp: 16 rows x (16 k tokens, 16 q tokens)
     static constexpr int kOffD = kOffPrep + kStages * kPrepFloats * 4;
     static constexpr int kDGroup = 2 * 4 * kBlkRows * kLdD * 4;
-    static constexpr int kOffC = kOffD + kGroups * kDGroup;  // coefficients as operands: [warp][term][row], 48-byte rows
+    static constexpr int kOffC = kOffD + kGroups * kDGroup;  // coefficients as operands: [group][term][row], 48-byte rows
     static constexpr int kRowC = 48;
-    static constexpr int kBytes = kOffC + kGroups * 4 * 3 * kBlkRows * kRowC;
+    static constexpr int kBytes = kOffC + kGroups * 3 * kBlkRows * kRowC;
     static_assert(kStage % 16 == 0 && kOffPrep % 16 == 0 && (kPrepFloats * 4) % 16 == 0 && kOffD % 16 == 0 && kOffC % 16 == 0, "alignment");
 };
 
@@ -407,7 +409,7 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
             // =============================================================== state
             const int rg = kGroups > 1 ? warp >> 2 : 0, qw = kGroups > 1 ? warp & 3 : warp;  // group of rows, quarter of the columns
             const int col0 = qw * (DK / 4);
-            const int r = lane & 15, h = lane >> 4;  // in the solve: row r, tokens 8 h .. 8 h + 7
+            const int r = 4 * qw + (lane >> 3), j2 = 2 * (lane & 7);  // in the solve: row r of the group, tokens j2 and j2 + 1
             float S[2 * NK][4];  // 8 columns each: rows g (0, 1) and g + 8 (2, 3), columns 2t, 2t + 1
             const long long srow = static_cast<long long>(rb * L::kRows + rg * kBlkRows + g) * DK + col0 + 2 * t;
             if (p.state_in) {
@@ -425,7 +427,13 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
 #pragma unroll
                 for (int i = 0; i < 2 * NK; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
             }
-            uint8_t* const sc = smem + L::kOffC + warp * (3 * kBlkRows * L::kRowC);
+            uint8_t* const sc = smem + L::kOffC + rg * (3 * kBlkRows * L::kRowC);
+            auto group_sync = [&]() {
+                if (kGroups == 1 || rg == 0)
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                else
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
+            };
             bool ok = true;  // false once a wait has given up: nothing is stored from then on
             bool ahead = false;  // this lane has seen the next block's preparation complete
             for (int b = 0; b < nblk; ++b) {
@@ -488,88 +496,54 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         *reinterpret_cast<float2*>(d + 8 * L::kLdD + 8 * i) = make_float2(dh[i][2] + dl[i][2], dh[i][3] + dl[i][3]);
                     }
                 }
-                if (kGroups == 1 || rg == 0)
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                else
-                    asm volatile("bar.sync 2, 128;" ::: "memory");
-                // ---- c of row r, tokens 8 h ..: right-hand sides, then forward substitution, first half of the tokens before the second
-                float c[8];
+                group_sync();
+                // ---- c of row r, tokens j2 and j2 + 1: right-hand sides, then forward substitution token by token, a row in eight lanes
+                float2 cc;
                 {
-                    const float* const d = D + r * L::kLdD + 8 * h;
-                    float sum[8];
+                    const float* const d = D + r * L::kLdD + j2;
+                    float2 x[4];
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        float4 x[4];
+                    for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
+                    const float2 bv = *reinterpret_cast<const float2*>(pr + L::kR0 + (rg * kBlkRows + r) * L::kLdR + j2);
+                    const float2 ck = *reinterpret_cast<const float2*>(pr + L::kCk + j2);
+                    cc.x = fmaf(-ck.x, (x[0].x + x[1].x) + (x[2].x + x[3].x), bv.x);
+                    cc.y = fmaf(-ck.y, (x[0].y + x[1].y) + (x[2].y + x[3].y), bv.y);
+                    // (what a token gets from the tokens before it is summed apart from its own, larger, term; those behind it are left out, not
+                    // multiplied by zero)
+                    float2 acc = make_float2(0.f, 0.f);
+                    const float own = pr[L::kA + j2 * 16 + j2 + 1];
 #pragma unroll
-                        for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float4*>(d + w * (kBlkRows * L::kLdD) + 4 * q);
-                        sum[4 * q] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
-                        sum[4 * q + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
-                        sum[4 * q + 2] = (x[0].z + x[1].z) + (x[2].z + x[3].z);
-                        sum[4 * q + 3] = (x[0].w + x[1].w) + (x[2].w + x[3].w);
+                    for (int i = 0; i < kBlkTok / 2 - 1; ++i) {
+                        const float2 a0 = *reinterpret_cast<const float2*>(pr + L::kA + (2 * i) * 16 + j2);  // columns 2 i, 2 i + 1 of A
+                        const float2 a1 = *reinterpret_cast<const float2*>(pr + L::kA + (2 * i + 1) * 16 + j2);
+                        const float x0 = cc.x - acc.x, x1 = cc.y - fmaf(own, x0, acc.y);  // c of two tokens, in the lane whose turn it is
+                        const float c0 = __shfl_sync(0xffffffffu, x0, (lane & 24) | i), c1 = __shfl_sync(0xffffffffu, x1, (lane & 24) | i);
+                        if (j2 > 2 * i) {
+                            acc.x = fmaf(a1.x, c1, fmaf(a0.x, c0, acc.x));
+                            acc.y = fmaf(a1.y, c1, fmaf(a0.y, c0, acc.y));
+                        }
                     }
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const float4 bv = *reinterpret_cast<const float4*>(pr + L::kR0 + (rg * kBlkRows + r) * L::kLdR + 8 * h + 4 * q);
-                        const float4 ck = *reinterpret_cast<const float4*>(pr + L::kCk + 8 * h + 4 * q);
-                        c[4 * q] = fmaf(-ck.x, sum[4 * q], bv.x);
-                        c[4 * q + 1] = fmaf(-ck.y, sum[4 * q + 1], bv.y);
-                        c[4 * q + 2] = fmaf(-ck.z, sum[4 * q + 2], bv.z);
-                        c[4 * q + 3] = fmaf(-ck.w, sum[4 * q + 3], bv.w);
+                    cc.x -= acc.x;
+                    cc.y -= fmaf(own, cc.x, acc.y);
+                    if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
+                        if (j2 >= n) cc.x = 0.f;
+                        if (j2 + 1 >= n) cc.y = 0.f;
                     }
                 }
-                // column s of A, tokens 8 th .. 8 th + 7
-                auto col_of = [&](int s, int th, float* x) {
-                    const float4 u = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th);
-                    const float4 v = *reinterpret_cast<const float4*>(pr + L::kA + s * 16 + 8 * th + 4);
-                    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
-                };
-                // (what a token gets from the tokens before it is summed apart from its own, larger, term)
-                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                auto substitute = [&](int half) {
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) {
-                        c[s] -= acc[s];
-                        if (s == 7) break;
-                        float x[8];
-                        col_of(8 * half + s, half, x);
-#pragma unroll
-                        for (int i = s + 1; i < 8; ++i) acc[i] = fmaf(x[i], c[s], acc[i]);
-                    }
-                };
-                if (h == 0) substitute(0);
-                __syncwarp();
-                float c0[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) c0[i] = __shfl_sync(0xffffffffu, c[i], r);
-                if (h == 1) {
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) {
-                        float x[8];
-                        col_of(s, 1, x);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[i] = fmaf(x[i], c0[s], acc[i]);
-                    }
-                    substitute(1);
-                }
-                if (n < kBlkTok) {  // tokens past the end: nothing, whatever the state holds
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) c[i] = 8 * h + i < n ? c[i] : 0.f;
-                }
-                __syncwarp();
                 // ---- S <- G S + sum_s (Gamma_ns r_s c_s) k_s^T
                 {
-                    uint32_t hi[4], mid[4], lo[4];
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const float4 w = *reinterpret_cast<const float4*>(pr + L::kW + 8 * h + 4 * q);
-                        split3<true>(w.x * c[4 * q], w.y * c[4 * q + 1], hi[2 * q], mid[2 * q], lo[2 * q]);
-                        split3<true>(w.z * c[4 * q + 2], w.w * c[4 * q + 3], hi[2 * q + 1], mid[2 * q + 1], lo[2 * q + 1]);
+                    {
+                        const float2 w = *reinterpret_cast<const float2*>(pr + L::kW + j2);
+                        uint32_t h, m, l;
+                        split3<true>(w.x * cc.x, w.y * cc.y, h, m, l);
+                        uint8_t* const o = sc + r * L::kRowC + 2 * j2;
+                        *reinterpret_cast<uint32_t*>(o) = h;
+                        *reinterpret_cast<uint32_t*>(o + kBlkRows * L::kRowC) = m;
+                        *reinterpret_cast<uint32_t*>(o + 2 * kBlkRows * L::kRowC) = l;
+                        *reinterpret_cast<float2*>(st + L::kOffC1 + rg * L::kOut + row64_off(r, j2 >> 2) + 4 * (j2 & 2)) = cc;  // for the outputs
                     }
-                    uint8_t* const o = sc + r * L::kRowC + 16 * h;
-                    *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                    *reinterpret_cast<uint4*>(o + kBlkRows * L::kRowC) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-                    *reinterpret_cast<uint4*>(o + 2 * kBlkRows * L::kRowC) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                    __syncwarp();
+                    group_sync();
+                    uint32_t hi[4], mid[4], lo[4];
                     const uint32_t caddr = smem_u32(sc) + lm_row * L::kRowC + lm_col * 2;
                     ldmatrix_x4(caddr, hi);
                     ldmatrix_x4(caddr + kBlkRows * L::kRowC, mid);
@@ -595,21 +569,16 @@ __device__ __forceinline__ void gdn_recurrent_block_body(const RecurrentParams& 
                         }
                     }
                 }
-                // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t), and c
+                // ---- for the outputs: this warp's quarter of scale G_t (S_0 q_t)
                 {
-                    const int i = 32 * qw + lane, row = i >> 3, t2 = 2 * (i & 7);
-                    const float* const d = D + row * L::kLdD + 16 + t2;
+                    const float* const d = D + r * L::kLdD + 16 + j2;
                     float2 x[4];
 #pragma unroll
                     for (int w = 0; w < 4; ++w) x[w] = *reinterpret_cast<const float2*>(d + w * (kBlkRows * L::kLdD));
-                    const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + t2);
+                    const float2 cq = *reinterpret_cast<const float2*>(pr + L::kCq + j2);
                     ahead = b + 1 < nblk && mbar_try_wait(&ready[(b + 1) & 3], static_cast<uint32_t>(((b + 1) >> 2) & 1));
-                    *reinterpret_cast<float2*>(st + L::kOffO + rg * L::kOut + row64_off(row, t2 >> 2) + 4 * (t2 & 2)) =
+                    *reinterpret_cast<float2*>(st + L::kOffO + rg * L::kOut + row64_off(r, j2 >> 2) + 4 * (j2 & 2)) =
                         make_float2(cq.x * ((x[0].x + x[1].x) + (x[2].x + x[3].x)), cq.y * ((x[0].y + x[1].y) + (x[2].y + x[3].y)));
-                    if (qw == (b & 3)) {
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + rg * L::kOut + row64_off(r, 2 * h)) = make_float4(c[0], c[1], c[2], c[3]);
-                        *reinterpret_cast<float4*>(st + L::kOffC1 + rg * L::kOut + row64_off(r, 2 * h + 1)) = make_float4(c[4], c[5], c[6], c[7]);
-                    }
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&done[b & 3]);
