@@ -146,7 +146,6 @@ static StepParams step_plan(const RecurrentParams& r, int sms, unsigned* grid) {
     p.r = r;
     p.num_tiles = static_cast<long long>(r.batch) * r.vh * (r.dv / kStepRows);
     const long long ctas = std::min<long long>(static_cast<long long>(sms) * kStepCtasPerSm, p.num_tiles);
-    p.stages = r.seq_len <= 6 ? 3 : 2;  // shared memory of a CTA: at most 100 KB
     *grid = static_cast<unsigned>(ctas);
     return p;
 }
@@ -162,7 +161,7 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
         attr_set[dev & 63].store(true, std::memory_order_release);
     }
     GDN_CUDA(launch_dependent(gdn_recurrent_step_kernel<DK>, dim3(grid), kRecThreads,
-                              static_cast<size_t>(kStepWarps) * step_warp_bytes(DK, r.seq_len, p.stages), st, p));
+                              static_cast<size_t>(kStepWarps) * step_warp_bytes(DK, r.seq_len), st, p));
     return GDN_OK;
 }
 
@@ -171,12 +170,13 @@ static int launch_step_t(const RecurrentParams& r, int sms, cudaStream_t st) {
 // (before any cap), head dim, state type - and not by the batch, the heads or the other sequences: a sequence, or a shard's heads,
 // come out with the same bits alone and in company.  A second block with few tokens takes as long as a full one, and where the CTAs
 // fill the GPU the token recurrence is no slower up to here.  Token recurrence against blocks in us, B=64, L2 flushed: 32 v-heads
-// d=64 T=33 184 : 212, T=39 208 : 212, T=41 216 : 212; d=128 T=23 385 : 397, T=25 414 : 395; 8 v-heads d=192 T=23 164 : 185, T=25
-// 176 : 184, T=27 188 : 184 (B=8 the same at T=27); d=256 T=23 259 : 259.  With few CTAs the blocks would win earlier (B=1 d=128
+// d=64 T=33 184 : 190, T=39 208 : 190, T=41 216 : 190; d=128 T=23 385 : 364, T=25 414 : 364; 8 v-heads d=192 T=23 164 : 174, T=25
+// 176 : 174, T=27 188 : 174; d=256 T=23 259 : 264.  (The line stays where an earlier, slower form of the blocks had put it: the results on
+// either side of it differ in their last bits.)  With few CTAs the blocks would win earlier (B=1 d=128
 // T=17 14 us : 8).  Packed batches hold both kinds and take two launches, each of which leaves the other's sequences out: 16
-// sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336, 8 of about 100 (32 v-heads, d=128) 113 -> 118; one of 1500 among
-// 100 of one token, which had gone token by token, 7.8 ms -> 0.21, d=256 11.0 -> 0.31; 2 v-heads, 2000 of 30 tokens 766 us -> 817, 200 of 60
-// among 3800 of one 878 -> 231.
+// sequences of 4 tokens 17.0 -> 18.2 us, 64 of 20 tokens 333 -> 336; 8 of about 100 (32 v-heads, d=128) 113 -> 107; one of 1500 among
+// 100 of one token, which had gone token by token, 7.8 ms -> 0.11, d=256 11.0 -> 0.22; 2 v-heads, 2000 of 30 tokens 766 us -> 763, 200 of 60
+// among 3800 of one 878 -> 239.
 // fp32 states stay with the token recurrence: in blocks (d=128, B=2 T=512 337 -> 136 us) the state, rounded once per block, was nearer to
 // 64 bits without decay (3.5e-7 of it -> 1.2e-7 after 1500 tokens) but further off with one, up to 40 % at a mean gate of -0.8
 // (6.1e-8 -> 8.5e-8): the matrix instructions cut their sums off.
@@ -273,7 +273,7 @@ static int launch_recurrent_jit(const RecurrentParams& p, int dk, int sms, cudaS
         if (int rc = jit::get_kernel("recurrent_dk" + std::to_string(dk) + ".step", src, "gdn_recurrent_jit", &k, &err)) return fail(rc, "%s", err.c_str());
         unsigned grid = 0;
         StepParams sp = step_plan(p, sms, &grid);
-        const size_t smem = static_cast<size_t>(kStepWarps) * step_warp_bytes(dk, p.seq_len, sp.stages);
+        const size_t smem = static_cast<size_t>(kStepWarps) * step_warp_bytes(dk, p.seq_len);
         GDN_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(k.kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(smem)));
         void* args[] = {&sp};
@@ -566,7 +566,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     p.state_idx = a->state_indices;
     p.batch = s.batch; p.seq_len = s.seq_len; p.kh = s.num_k_heads; p.vh = s.num_v_heads; p.dv = s.head_dim_v;
     p.scale = a->scale;
-    p.is_qk_norm = a->is_qk_norm; p.store_step = a->store_step_state;
+    p.is_qk_norm = a->is_qk_norm != 0; p.store_step = a->store_step_state != 0;
     p.num_tiles = static_cast<long long>(s.batch) * s.num_v_heads * (s.head_dim_v / kRecTileRows);
     GDN_REQUIRE(p.num_tiles < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
     p.status = d->status;
@@ -587,7 +587,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
                                              a->state_dtype == GDN_F32 || a->state_indices != nullptr);
         p.split_tiles = cut.parts > 1;
         p.split_whole = static_cast<int>(cut.whole);
-        p.split_parts = cut.parts;
+        p.split_parts = static_cast<uint8_t>(cut.parts);
     }
     const long long pairs = static_cast<long long>(s.batch) * s.num_v_heads;
     p.num_units = static_cast<int>(ring ? p.num_tiles : p.split_tiles ? p.split_whole + (pairs - p.split_whole) * p.split_parts : pairs);

@@ -41,7 +41,6 @@ struct RecurrentParams {
     int64_t o_sb, o_st, o_sh;
     const void* beta;
     const void* gate;
-    int beta_f32, gate_f32;
     int64_t beta_sb, beta_st, beta_sh;
     int64_t gate_sb, gate_st, gate_sh;
     const void* state_in;   // bf16, or fp32 in the kF32 instances; strides in elements of that type
@@ -52,21 +51,25 @@ struct RecurrentParams {
     const int* state_idx;  // indexed state pool: slot of every sequence (negative: padding sequence), or NULL
     int batch, seq_len, kh, vh, dv;
     float scale;
-    int is_qk_norm, store_step;
+    uint8_t is_qk_norm, store_step, beta_f32, gate_f32;
     // Fused gating: `beta` / `gate` then hold the layer's raw projections b / a and the kernel computes
     // beta = sigmoid(b), g = -exp(A_log[h]) softplus(a + dt_bias[h]) itself (fp32, nothing rounded to bf16).
-    int fused_gating, gating_param_f32;
-    const void* A_log;
-    const void* dt_bias;
-    int split_tiles;  // 1: every 32-row tile is a work unit (ring instance), or the units are cut as below (the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
+    uint8_t fused_gating, gating_param_f32;
+    uint8_t split_tiles;  // 1: every 32-row tile is a work unit (ring instance), or the units are cut as below (the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
     // kSplit: the first split_whole (sequence, v-head) units, a multiple of the grid, are work units as they are, the others are cut into
     // split_parts parts of equally many tiles, no more of them than the grid has CTAs.
-    int split_whole, split_parts;
+    uint8_t split_parts;
+    int split_whole;
     int num_units;  // work units of the launch
     int long_run;  // packed mode: sequences of at least this many tokens are recurrent_block.cuh's, in a launch of their own; shorter ones this kernel's
+    const void* A_log;
+    const void* dt_bias;
     long long num_tiles;
     int* status;
 };
+// A launch with more costs the host another 0.35 us, which is what bounds the smallest calls made one after another (one token, B=4, 8
+// v-heads: 368 bytes 4.65 us a call, 344 bytes 4.25).
+static_assert(sizeof(RecurrentParams) <= 352, "parameter bytes");
 
 constexpr int kRecTileRows = 32;
 constexpr int kRecStages = 4;      // state tiles in flight per CTA (decode)

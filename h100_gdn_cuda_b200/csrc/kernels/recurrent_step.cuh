@@ -46,15 +46,18 @@ static_assert(step_applies(2 * kStepRows) && !step_applies(kStepRows), "one tile
 
 // shared memory of one warp: the stages, the present item's k, q as MMA operands (16 rows), then for each stage room for the
 // k and q of an item's tokens
-__host__ __device__ constexpr int step_warp_bytes(int dk, int tokens, int stages) {
-    return ((stages + 1) * kStepRows + stages * 2 * tokens) * dk * 2;
+__host__ __device__ constexpr int step_stages(int tokens) { return tokens <= 6 ? 3 : 2; }  // shared memory of a CTA: at most 100 KB
+__host__ __device__ constexpr int step_warp_bytes(int dk, int tokens) {
+    return ((step_stages(tokens) + 1) * kStepRows + step_stages(tokens) * 2 * tokens) * dk * 2;
 }
 
 struct StepParams {
     RecurrentParams r;
     long long num_tiles;  // 16-row tiles of all (sequence, v-head) units
-    int stages;
 };
+// (As for RecurrentParams.  368 bytes, with the number of stages among them, : 352: B=1, T=3, 4 v-heads 5.5 : 5.2 us a call, on the device alone
+// B=1, T=4, 32 v-heads 5.41 : 5.25.)
+static_assert(sizeof(StepParams) <= 352, "parameter bytes");
 
 namespace step {
 __device__ __forceinline__ void mma16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -89,6 +92,7 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
     constexpr int NJ = DK / 32;  // 16-byte pieces per lane and row; two K-steps of 16 each
     constexpr int kTileBytes = kStepRows * DK * 2;
     const RecurrentParams& p = sp.r;
+    const int stages = step_stages(p.seq_len);
     extern __shared__ __align__(128) uint8_t smem_all[];
     __shared__ uint64_t full_all[kStepWarps][kStepMaxStages];
     __shared__ int abort_flag;
@@ -97,9 +101,9 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
     __shared__ float s_w[kStepWarps][kStepTok][kStepTok];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    uint8_t* const smem = smem_all + warp * step_warp_bytes(DK, p.seq_len, sp.stages);
-    uint4* const smem_kq = reinterpret_cast<uint4*>(smem + sp.stages * kTileBytes) + lane;  // [K-step][lane]
-    uint8_t* const smem_tok = smem + (sp.stages + 1) * kTileBytes;
+    uint8_t* const smem = smem_all + warp * step_warp_bytes(DK, p.seq_len);
+    uint4* const smem_kq = reinterpret_cast<uint4*>(smem + stages * kTileBytes) + lane;  // [K-step][lane]
+    uint8_t* const smem_tok = smem + (stages + 1) * kTileBytes;
     const int tok_bytes = p.seq_len * DK * 4;
     uint64_t* const full = full_all[warp];
     const int rblocks = p.dv / kStepRows;
@@ -180,7 +184,7 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
                     const int kh = rep_shift >= 0 ? u.head >> rep_shift : u.head / rep;
                     const __nv_bfloat16* kp = p.k + u.seq * p.k_sb + kh * p.k_sh;
                     const __nv_bfloat16* qp = p.q + u.seq * p.q_sb + kh * p.q_sh;
-                    uint8_t* dst = smem_tok + (req_item % sp.stages) * tok_bytes;
+                    uint8_t* dst = smem_tok + (req_item % stages) * tok_bytes;
                     mbar_arrive_expect_tx(&full[stage], (has_in ? kTileBytes : 0) + nt * DK * 4);
                     for (int i = 0; i < nt; ++i) {
                         bulk_load(dst + i * DK * 4, kp + i * p.k_st, DK * 2, &full[stage]);
@@ -199,7 +203,7 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
             req_r = req_item == rounds ? rb_first : 0;
         }
     };
-    for (int i = 0; i < sp.stages; ++i) request(i);
+    for (int i = 0; i < stages; ++i) request(i);
 
     // raw scalars of an item's tokens: lane i < 8 holds those of token i
     struct Scalars {
@@ -288,7 +292,7 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
             }
             __syncwarp();  // the stage has been read
             request(stage);
-            if (++stage == sp.stages) {
+            if (++stage == stages) {
                 stage = 0;
                 parity ^= 1u;
             }
@@ -304,7 +308,7 @@ __device__ __forceinline__ void gdn_recurrent_step_body(const StepParams& sp) {
             if (r == 0) {
                 // ---- products of the tokens and the coefficients made of them
                 float d[4] = {0.f, 0.f, 0.f, 0.f}, dq[4] = {0.f, 0.f, 0.f, 0.f};
-                const uint8_t* tk = smem_tok + (item % sp.stages) * tok_bytes + g * DK * 4 + 16 * t;
+                const uint8_t* tk = smem_tok + (item % stages) * tok_bytes + g * DK * 4 + 16 * t;
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
                     uint4 x = make_uint4(0u, 0u, 0u, 0u), y = x;
