@@ -364,15 +364,18 @@ static size_t ws_base_bytes(const GdnShape& s) {
 }
 
 // The segment plan of a problem (heuristics.hpp); num_segments == 1: not segmented.
+static SegmentPlan long_plan_of(const GdnShape& s, long long max_units = plan_detail::kNoLimit) {
+    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, s.total_chunks > 0 ? s.total_chunks : 0, max_units);
+    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, static_cast<int>((s.seq_len + kChunk - 1) / kChunk), false, max_units);
+    plan.slots = s.batch * plan.num_segments;
+    return plan;
+}
 static SegmentPlan segment_plan_of(const GdnShape& s, long long max_units = plan_detail::kNoLimit) {
     const long long total = s.total_chunks > 0 ? s.total_chunks : 0;
     const long long chunks = s.cu_seqlens ? (total + s.batch - 1) / std::max(s.batch, 1) : (s.seq_len + kChunk - 1) / kChunk;
     if (chunks <= kShortChunks && (!s.cu_seqlens || s.batch <= kMaxSegmentedSeqs))
         return prefill_segments_short(s.batch, s.num_v_heads, chunks, s.cu_seqlens ? total : chunks * s.batch, s.cu_seqlens != nullptr, max_units);
-    if (s.cu_seqlens) return prefill_segments_packed(s.batch, s.num_v_heads, total, max_units);
-    SegmentPlan plan = prefill_segments(static_cast<long long>(s.batch) * s.num_v_heads, static_cast<int>(chunks), false, max_units);
-    plan.slots = s.batch * plan.num_segments;
-    return plan;
+    return long_plan_of(s, max_units);
 }
 
 // Scratch of a run on `plan`: for a segmented one (few long sequences) three fp32 states per v-head and segment slot.
@@ -383,6 +386,20 @@ static size_t ws_bytes(const GdnShape& s, const SegmentPlan& plan) {
     else if (s.cu_seqlens && s.batch > 1 && s.batch <= kMaxOrderedSeqs)
         bytes += (static_cast<size_t>(s.batch) * sizeof(int) + 255) / 256 * 256;  // sequences by length
     return bytes;
+}
+
+// (slot, v-head) pairs whose segment states fit `bytes` of scratch
+static long long seg_units_in(const GdnShape& s, size_t bytes) {
+    const size_t base = ws_base_bytes(s) + 256;
+    return base < bytes ? static_cast<long long>((bytes - base) / kSegUnitBytes) : 0;
+}
+
+// The plan for a caller's scratch.  Short segments ask for more of it than the long ones that a sequence had otherwise; scratch laid out for
+// those still does, with as many segments as it holds.
+static SegmentPlan segment_plan_in(const GdnShape& s, size_t bytes) {
+    const SegmentPlan plan = segment_plan_of(s);
+    if (ws_bytes(s, plan) <= bytes || bytes < ws_bytes(s, long_plan_of(s))) return plan;
+    return segment_plan_of(s, seg_units_in(s, bytes));
 }
 
 size_t gdn_chunked_forward_workspace_bytes(const GdnShape* s) {
@@ -540,7 +557,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
 int gdn_chunked_forward(const GdnChunkedArgs* a, gdn_stream_t stream) {
     GDN_REQUIRE(a != nullptr, "gdn_chunked_forward: args is NULL");
     if (int rc = check_shape(a->shape, true)) return rc;
-    return chunked_forward_on(a, segment_plan_of(a->shape), stream);
+    return chunked_forward_on(a, segment_plan_in(a->shape, a->workspace_bytes), stream);
 }
 
 // ------------------------------------------------------------------ prefill on built-in scratch
@@ -555,9 +572,7 @@ int gdn_chunked_forward_static_scratch(const GdnChunkedArgs* a, gdn_stream_t str
     GDN_REQUIRE(a != nullptr, "gdn_chunked_forward_static_scratch: args is NULL");
     if (int rc = check_shape(a->shape, true)) return rc;
     // The plan that is the fastest with all the scratch it wants may not fit where fewer segments, or none, do.
-    const size_t base = ws_base_bytes(a->shape) + 256;
-    const SegmentPlan plan = segment_plan_of(
-        a->shape, base < GDN_STATIC_SCRATCH_BYTES ? static_cast<long long>((GDN_STATIC_SCRATCH_BYTES - base) / kSegUnitBytes) : 0);
+    const SegmentPlan plan = segment_plan_of(a->shape, seg_units_in(a->shape, GDN_STATIC_SCRATCH_BYTES));
     const size_t need = wide_heads(a->shape) ? 0 : ws_bytes(a->shape, plan);
     if (need > GDN_STATIC_SCRATCH_BYTES)
         return fail(GDN_ERR_WORKSPACE,

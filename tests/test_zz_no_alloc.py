@@ -117,3 +117,32 @@ def test_static_scratch_wide_heads_need_none():
         outs.append((out, final))
     assert torch.isfinite(outs[1][0].float()).all() and torch.isfinite(outs[1][1].float()).all()
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("B,T,kh,vh", [(1, 2500, 2, 4), (1, 5000, 8, 16), (2, 3000, 1, 2)])
+def test_scratch_of_a_longer_plan_is_enough(B, T, kh, vh):
+    """Scratch that has no room for all the segments a few short sequences would be cut into, down to none of them: fewer segments, the
+    same results but for the rounding; below that the call is refused."""
+    from h100_gdn_cuda_b200 import _cabi as cabi, api, build
+    build.build()
+    lib = cabi.load()
+    p = {k: (v.cuda() if torch.is_tensor(v) else v)
+         for k, v in synthetic.prefill_inputs(B, T, kh, vh, 128, seed=T, mild_gate=True).items()}
+    full = lib.gdn_chunked_forward_workspace_bytes(C.byref(api._shape(B, T, B * T, kh, vh, 128, 128)))
+    chunks, segment = B * ((T + 63) // 64), B * vh * 3 * 128 * 128 * 4
+    base = (chunks * vh * 24576 + 255) // 256 * 256 + (chunks * kh * 512 + 255) // 256 * 256 + 256
+    assert full >= base + 3 * segment
+    ref = None
+    for n in (full, full - segment, base + 2 * segment, base, base - 1):
+        ws = torch.full((n,), 255, dtype=torch.uint8, device="cuda")
+        out, final = torch.full_like(p["v"], float("nan")), torch.full_like(p["state"], float("nan"))
+        rc = lib.gdn_chunked_forward(C.byref(_args(api, cabi, p, out, final, ws.data_ptr(), n)), torch.cuda.current_stream().cuda_stream)
+        if n < base:
+            assert rc == -4
+            continue
+        assert rc == 0, lib.gdn_last_error()
+        torch.cuda.synchronize()
+        got = (out.float(), final.float())
+        ref = ref or got
+        for x, y in zip(ref, got):
+            assert torch.isfinite(y).all() and ((x - y).norm() / x.norm()).item() <= 1e-2
