@@ -588,9 +588,8 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
         p.split_tiles = cut.parts > 1;
         p.split_whole = static_cast<int>(cut.whole);
         p.split_parts = static_cast<uint8_t>(cut.parts);
+        p.num_units = static_cast<int>(cut.whole + (static_cast<long long>(s.batch) * s.num_v_heads - cut.whole) * cut.parts);
     }
-    const long long pairs = static_cast<long long>(s.batch) * s.num_v_heads;
-    p.num_units = static_cast<int>(ring ? p.num_tiles : p.split_tiles ? p.split_whole + (pairs - p.split_whole) * p.split_parts : pairs);
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);
     const bool f32 = a->state_dtype == GDN_F32;
     const bool jit = force_jit && !f32;

@@ -60,7 +60,7 @@ struct RecurrentParams {
     // split_parts parts of equally many tiles, no more of them than the grid has CTAs.
     uint8_t split_parts;
     int split_whole;
-    int num_units;  // work units of the launch
+    int num_units;  // kSplit: work units of the launch
     int long_run;  // packed mode: sequences of at least this many tokens are recurrent_block.cuh's, in a launch of their own; shorter ones this kernel's
     const void* A_log;
     const void* dt_bias;
@@ -229,7 +229,8 @@ __device__ __forceinline__ void gdn_recurrent_body(const RecurrentParams& p) {
     const int upg_shift = (upg & (upg - 1)) == 0 ? __ffs(upg) - 1 : -1;
     const int parts = kSplit ? p.split_parts : 1, parts_shift = kSplit && (parts & (parts - 1)) == 0 ? __ffs(parts) - 1 : -1;
     const int part_tiles = kSplit ? (parts_shift >= 0 ? rblocks >> parts_shift : rblocks / parts) : tpu;
-    const int num_units = p.num_units;
+    // (Read from the parameters by every instance, the scheduling of the loop comes out differently: B=256 in place 90.0 -> 91.8 us.)
+    const int num_units = kSplit ? p.num_units : static_cast<int>(p.num_tiles / tpu);
     const int stride = static_cast<int>(gridDim.x);
 
     if (tid == 0) {
