@@ -188,10 +188,8 @@ int launch_seq_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorM
 // Launch of the state kernel right after the chunk-parallel kernel in the same stream, with
 // programmatic stream serialization: its CTAs may be placed (each takes a whole SM) and set up while
 // that kernel drains; the kernel waits (grid_dep_wait) before it reads that kernel's results.
-template <SeqUnits kUnits>
-int launch_fused_after_zp(dim3 grid, cudaStream_t st, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
-                          const CUtensorMap& tmO, const FusedParams& p) {
-    if (int rc = set_smem<gdn_fused_seq_kernel<kUnits>>(FusedSmem::kBytes)) return rc;
+cudaError_t launch_fused_after_zp(dim3 grid, cudaStream_t st, const CUtensorMap& tmQ, const CUtensorMap& tmK,
+                                  const CUtensorMap& tmV, const CUtensorMap& tmO, const FusedParams& p) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(fused::kThreads);
@@ -202,8 +200,7 @@ int launch_fused_after_zp(dim3 grid, cudaStream_t st, const CUtensorMap& tmQ, co
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_fused_seq_kernel<kUnits>, tmQ, tmK, tmV, tmO, p));
-    return GDN_OK;
+    return cudaLaunchKernelEx(&cfg, gdn_fused_seq_kernel, tmQ, tmK, tmV, tmO, p);
 }
 
 }  // namespace
@@ -481,7 +478,12 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
         p.status = d->status;
         p.blocks = static_cast<const uint8_t*>(a->workspace);
         p.norms = norms;
+        if (int rc = set_smem<gdn_fused_seq_kernel>(FusedSmem::kBytes)) return rc;
         const long long chains = static_cast<long long>(s.batch) * s.num_v_heads;
+        auto run_seq = [&](dim3 grid) -> int {
+            GDN_CUDA(launch_fused_after_zp(grid, st, tmQ, tmK, tmV, tmO, p));
+            return GDN_OK;
+        };
         if (plan.num_segments <= 1 && packed && s.batch > 1 && s.batch <= kMaxOrderedSeqs && chains > d->sms) {
             // more chains than SMs and unequal lengths: dispatch the longest sequences first
             p.num_seqs = s.batch;
@@ -493,10 +495,10 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
                 p.seq_order = order;
             }
             if (int rc = run_zp()) return rc;
-            if (int rc = launch_fused_after_zp<SeqUnits::kRanked>(dim3(s.num_v_heads, s.batch), st, tmQ, tmK, tmV, tmO, p)) return rc;
+            if (int rc = run_seq(dim3(s.num_v_heads, s.batch))) return rc;
         } else if (plan.num_segments <= 1) {
             if (int rc = run_zp()) return rc;
-            if (int rc = launch_fused_after_zp<SeqUnits::kWhole>(dim3(s.batch, s.num_v_heads), st, tmQ, tmK, tmV, tmO, p)) return rc;
+            if (int rc = run_seq(dim3(s.batch, s.num_v_heads))) return rc;
         } else {
             // the composite transitions of the segments and, beside them, the first segment of every sequence outright; the others' start
             // states; then all of the others at once (long sequences: transitions of the first segments too, and all of them at once)
@@ -527,7 +529,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_transition_kernel, tmK, tmV, p));
             if (plan.first_apart) {
                 p.mode = 1;
-                if (int rc = launch_fused_after_zp<SeqUnits::kSegments>(dim3(s.batch, s.num_v_heads), st, tmQ, tmK, tmV, tmO, p)) return rc;
+                if (int rc = run_seq(dim3(s.batch, s.num_v_heads))) return rc;
             }
             SegCombineParams cp{};
             cp.seg_mn = seg_mn;
@@ -547,7 +549,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             cfg.dynamicSmemBytes = SegCombineSmem::kBytes;
             GDN_CUDA(cudaLaunchKernelEx(&cfg, gdn_seg_combine_kernel, cp));
             p.mode = 2;
-            if (int rc = launch_fused_after_zp<SeqUnits::kSegments>(dim3(plan.slots, s.num_v_heads), st, tmQ, tmK, tmV, tmO, p)) return rc;
+            if (int rc = run_seq(dim3(plan.slots, s.num_v_heads))) return rc;
         }
     }
     if (ev) GDN_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(ev[2]), st));

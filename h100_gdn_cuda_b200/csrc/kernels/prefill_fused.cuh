@@ -135,15 +135,6 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 }
 }  // namespace fused
 
-// What a CTA walks, an instance each: what only segments or ranked sequences need in front of their first load is not fetched by the
-// others (one instance for all : three, in graphs: one sequence of 256 tokens on 4 v-heads, d=64, 15.07 : 14.95 us, 200 on 32, d=128, 16.91 : 16.70;
-// 3 of 51, d=96, 12.93 : 12.70).
-enum class SeqUnits {
-    kWhole,     // sequence blockIdx.x, v-head blockIdx.y
-    kRanked,    // mode 0 with by_length or seq_order
-    kSegments,  // modes 1 and 2
-};
-template <SeqUnits kUnits>
 __global__ void __launch_bounds__(fused::kThreads, 1)
     gdn_fused_seq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -174,11 +165,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     volatile int* issued = abort_flag + 1;  // chunks whose loads the producer has issued (read by the L2 prefetcher)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mode = kUnits == SeqUnits::kSegments ? p.mode : 0;
     SegPos sp{0, 0, 1, 0};
-    if (mode == 1) {
+    if (p.mode == 1) {
         sp = sequence_segments(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments);
-    } else if (mode == 2) {
+    } else if (p.mode == 2) {
         sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
         if (sp.seq < 0 || (sp.segment == 0 && p.first_apart)) {  // packed mode launches an upper bound of slots; first segments are done
             // Whoever waits for this grid waits for all of the call: the grid must not complete before the launches in front of it.
@@ -186,7 +176,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             return;
         }
     }
-    if (kUnits == SeqUnits::kRanked && p.by_length) {
+    if (p.by_length) {
         // order of the sequences: more tokens first, of equally many the one in front first (every warp for itself)
         const int mine = lane < p.num_seqs ? p.map.cu_seqlens[lane + 1] - p.map.cu_seqlens[lane] : -1;
         int rank = 0;
@@ -196,12 +186,9 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         }
         sp.seq = __ffs(__ballot_sync(0xffffffffu, lane < p.num_seqs && rank == static_cast<int>(blockIdx.y))) - 1;
     }
-    int seq = sp.seq, head = static_cast<int>(blockIdx.y);
-    if (kUnits == SeqUnits::kWhole) seq = static_cast<int>(blockIdx.x);
-    if (kUnits == SeqUnits::kRanked) {
-        if (!p.by_length) seq = p.seq_order[blockIdx.y];
-        head = static_cast<int>(blockIdx.x);
-    }
+    const bool ranked = p.by_length || p.seq_order;
+    const int seq = p.mode != 0 || p.by_length ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
+    const int head = ranked ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
     const int segment = sp.segment, seq_nseg = sp.nseg;
     const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;  // mode 2
     const int khead = head / (p.vh / p.kh);
@@ -222,7 +209,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     }
     int nchunks = static_cast<int>((seq_tokens + kChunk - 1) / kChunk);
     // A segment is handled as a sequence of its own: shift the token and chunk origins.
-    if (mode != 0) {
+    if (p.mode != 0) {
         const int c0 = min(segment * p.seg_chunks, nchunks);
         const int c1 = min(c0 + p.seg_chunks, nchunks);
         seq_tok0 += static_cast<long long>(c0) * kChunk;
@@ -280,7 +267,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         const uint32_t vsw0 = vlane + ((vchunk ^ (lane & 7)) << 4), vsw1 = vlane + (((vchunk + 2) ^ (lane & 7)) << 4);
         const int t0 = 32 * hf + 2 * (lane & 3);  // first token of this lane's first pair; the others are 8 further on each
         float S[64];
-        if (mode == 2) {
+        if (p.mode == 2) {
             grid_dep_wait();  // the start states come from the kernel launched just before this one
             const float4* src = reinterpret_cast<const float4*>(p.seg_start + seg_idx * (D * D) +
                                                                 static_cast<long long>(row) * D + 64 * hf);
@@ -419,8 +406,8 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // nothing is written once a wait of this CTA has given up (the results would be garbage)
         const bool healthy = *abort_flag == 0;
         if (!healthy) {
-        } else if (mode != 0 && segment != seq_nseg - 1) {
-            if (mode == 1) {
+        } else if (p.mode != 0 && segment != seq_nseg - 1) {
+            if (p.mode == 1) {
                 float4* d4 = reinterpret_cast<float4*>(p.seg_start + (static_cast<long long>(sp.first_slot + 1) * p.vh + head) * (D * D) +
                                                        static_cast<long long>(row) * D + 64 * hf);
 #pragma unroll
@@ -534,7 +521,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         load_raw(1, rb0, rb1);
         // Everything up to here (and the state warps' load of the initial state) touches only the caller's
         // inputs and may run while the chunk-parallel kernel drains; its blocks and norm factors are read below.
-        if (mode != 1)
+        if (p.mode != 1)
             grid_dep_wait();
         else if (lane == 0)
             grid_dep_launch();  // the start states' kernel sets itself up on the SMs that are left and waits there
@@ -603,7 +590,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // kLead positions after the one the producer has just requested into L2, so that the producer's own
         // loads find them there.  A hint only: when its bounded wait runs out it simply stops.
         constexpr int kLead = 3;
-        if (mode != 1) grid_dep_wait();
+        if (p.mode != 1) grid_dep_wait();
         if (lane == 0) {
             for (int c = kLead; c < nchunks; ++c) {
                 int spins = 0;
@@ -671,7 +658,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         }
     }
 
-    if (mode == 1 && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
+    if (p.mode == 1 && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
