@@ -587,7 +587,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
                                              a->state_dtype == GDN_F32 || a->state_indices != nullptr);
         p.split_tiles = cut.parts > 1;
         p.split_whole = static_cast<int>(cut.whole);
-        p.split_parts = static_cast<uint8_t>(cut.parts);
+        p.split_parts = static_cast<uint16_t>(cut.parts);
         p.num_units = static_cast<int>(cut.whole + (static_cast<long long>(s.batch) * s.num_v_heads - cut.whole) * cut.parts);
     }
     const bool step = !ring && step_takes(s, a->state_dtype, p.store_step != 0, d->sms);

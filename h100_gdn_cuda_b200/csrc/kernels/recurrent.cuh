@@ -57,8 +57,9 @@ struct RecurrentParams {
     uint8_t fused_gating, gating_param_f32;
     uint8_t split_tiles;  // 1: every 32-row tile is a work unit (ring instance), or the units are cut as below (the instance kSplit); 0: a unit = all tiles of a (sequence, v-head)
     // kSplit: the first split_whole (sequence, v-head) units, a multiple of the grid, are work units as they are, the others are cut into
-    // split_parts parts of equally many tiles, no more of them than the grid has CTAs.
-    uint8_t split_parts;
+    // split_parts parts of equally many tiles, no more of them than the grid has CTAs (four per SM: more than a byte holds; dv, and with it
+    // the tiles of a unit, has no upper limit).
+    uint16_t split_parts;
     int split_whole;
     int num_units;  // kSplit: work units of the launch
     int long_run;  // packed mode: sequences of at least this many tokens are recurrent_block.cuh's, in a launch of their own; shorter ones this kernel's

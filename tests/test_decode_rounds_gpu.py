@@ -62,3 +62,40 @@ def test_more_units_than_one_table(B):
     o, s1 = step(gdn, q, k, v, par, a, b, s.clone(), idx, inplace=True)
     o_ref, s_ref = step(gdn, q, k, v, par, a, b, s[idx.long()].contiguous())
     assert torch.equal(o, o_ref) and torch.equal(s1[idx.long()], s_ref)
+
+
+@pytest.mark.parametrize("dv,vh,f32", [(8192, 1, False), (8224, 1, False), (8224, 2, True), (4096, 2, False)])
+def test_more_parts_than_a_byte_counts(dv, vh, f32):
+    """One sequence whose v-heads have more than 255 tiles of state rows (the C entry point has no upper limit on dv): every tile by itself, as
+    many parts as tiles.  A row of the state needs nothing of the others, so the same rows as heads of 32 each are the reference."""
+    import ctypes as C
+    import h100_gdn_cuda_b200 as gdn
+    from h100_gdn_cuda_b200 import _cabi as cabi, api
+    d = 128
+    q, k, _, par, a, b, _ = inputs(1, 1, vh, d, f32, 1, dv)
+    g = torch.Generator(device="cuda").manual_seed(dv + 1)
+    v = torch.randn(1, 1, vh, dv, device="cuda", generator=g).bfloat16()
+    s = (0.02 * torch.randn(1, vh, dv, d, device="cuda", generator=g)).bfloat16()
+    s = s.float() if f32 else s
+    out, s_out = torch.full_like(v, float("nan")), torch.full_like(s, float("nan"))
+    r = cabi.RecurrentArgs()
+    r.shape = api._shape(1, 1, 1, 1, vh, d, dv)
+    r.q, r.k, r.v, r.out = (api._token_tensor(t, False) for t in (q, k, v, out))
+    r.gating_a, r.gating_b = api._token_scalar(a, False), api._token_scalar(b, False)
+    r.A_log, r.dt_bias = par[0].data_ptr(), par[1].data_ptr()
+    r.state_in, r.state_out = api._state_desc(s), api._state_desc(s_out)
+    r.state_dtype = cabi.GDN_F32 if f32 else cabi.GDN_BF16
+    r.scale, r.is_qk_norm = d ** -0.5, 1
+    assert cabi.load().gdn_recurrent_forward(C.byref(r), torch.cuda.current_stream().cuda_stream) == 0, cabi.load().gdn_last_error()
+    heads = dv // 32
+    rep = lambda t: t.reshape(-1).repeat_interleave(heads)
+    o_ref, s_ref = torch.empty(1, 1, vh * heads, 32, device="cuda", dtype=torch.bfloat16), torch.empty(1, vh * heads, 32, d, device="cuda", dtype=s.dtype)
+    par2, a2, b2 = [rep(t) for t in par], rep(a).view(1, 1, -1), rep(b).view(1, 1, -1)
+    r.shape = api._shape(1, 1, 1, 1, vh * heads, d, 32)
+    r.v, r.out = api._token_tensor(v.view(1, 1, vh * heads, 32), False), api._token_tensor(o_ref, False)
+    r.gating_a, r.gating_b = api._token_scalar(a2, False), api._token_scalar(b2, False)
+    r.A_log, r.dt_bias = par2[0].data_ptr(), par2[1].data_ptr()
+    r.state_in, r.state_out = api._state_desc(s.view(1, vh * heads, 32, d)), api._state_desc(s_ref)
+    assert cabi.load().gdn_recurrent_forward(C.byref(r), torch.cuda.current_stream().cuda_stream) == 0, cabi.load().gdn_last_error()
+    assert torch.isfinite(o_ref.float()).all()
+    assert torch.equal(out.view(-1), o_ref.view(-1)) and torch.equal(s_out.view(-1), s_ref.view(-1))
