@@ -53,8 +53,8 @@ struct FusedParams {
     //   mode 1: the first segment of every sequence (grid = sequences x heads), beside the transitions of the segments behind it.  It
     //           needs none itself: it starts from the initial state, writes its output, and leaves the start state of the second
     //           segment (fp32), or the final state where there is no other.  A programmatic dependent of the transitions' launch, which
-    //           lets it start when the chunk-parallel kernel in front of both is complete; it waits for that launch at its end, so that who
-    //           waits for this one waits for both.  (The other way round the transitions, the longer of the two, start later: 4 v-heads of
+    //           lets it start when the chunk-parallel kernel in front of both is complete and hands on what that has written
+    //           (grid_dep_handover, grid_dep_takeover); it waits for that launch at its end, so that who waits for this one waits for both.  (The other way round the transitions, the longer of the two, start later: 4 v-heads of
     //           2500 tokens 45.5 -> 47.5 us.)
     //   mode 2: grid = (slots, heads), the other segments (first_apart 0: all of them, mode 1 is not launched); starts from
     //           seg_start[slot * vh + head] (fp32), writes the output of its chunks; the last segment of a sequence writes the final state.
@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // the Z, PT blocks and the V tiles are read exactly once: first in line for eviction from L2
         const uint64_t once = l2_policy_evict_first();
         uint32_t ra0, ra1, rb0, rb1;  // raw gates of chunks c and c + 1, as bits
+        if (p.mode == 1) grid_dep_takeover();  // (the blocks are complete, see FusedParams::mode; in front of this warp's loads, which the fence would wait for)
         load_raw(0, ra0, ra1);
         load_raw(1, rb0, rb1);
         // Everything up to here (and the state warps' load of the initial state) touches only the caller's
@@ -535,10 +536,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
             float rk0 = 1.f, rk1 = 1.f, rq0 = 1.f, rq1 = 1.f;
             if (p.norms) {  // requested here, used after the wait for a free stage
                 const float* nr = p.norms + (static_cast<size_t>(gchunk0 + c) * p.kh + khead) * 128;
-                rk0 = __ldg(nr + lane);
-                rk1 = __ldg(nr + 32 + lane);
-                rq0 = __ldg(nr + 64 + lane);
-                rq1 = __ldg(nr + 96 + lane);
+                rk0 = __ldcg(nr + lane);
+                rk1 = __ldcg(nr + 32 + lane);
+                rq0 = __ldcg(nr + 64 + lane);
+                rq1 = __ldcg(nr + 96 + lane);
             }
             // chunk-local cumulative gate
 #pragma unroll
@@ -590,7 +591,10 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         // kLead positions after the one the producer has just requested into L2, so that the producer's own
         // loads find them there.  A hint only: when its bounded wait runs out it simply stops.
         constexpr int kLead = 3;
-        if (p.mode != 1) grid_dep_wait();
+        if (p.mode != 1)
+            grid_dep_wait();
+        else
+            grid_dep_takeover();
         if (lane == 0) {
             for (int c = kLead; c < nchunks; ++c) {
                 int spins = 0;

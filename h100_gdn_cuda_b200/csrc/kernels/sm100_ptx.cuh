@@ -208,6 +208,16 @@ GDN_DEVICE void bulk_prefetch_l2(const void* src, uint32_t bytes) {
 // `grid_dep_launch` in the earlier kernel lets the later one be scheduled as SMs free up.
 GDN_DEVICE void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 GDN_DEVICE void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A dependent that needs what the launches in FRONT of its predecessor have written, and runs beside the predecessor, does not wait itself.
+// `grid_dep_wait` makes those writes visible to the grid that waits, so they are handed on: the predecessor releases them
+// (`grid_dep_handover`, by a thread behind its wait, in front of `grid_dep_launch` or the CTA's end), the dependent acquires them
+// (`grid_dep_takeover`, every thread that reads or copies them), for its loads and, with the proxy fence, for its copies.  Loads of such
+// data do not take the non-coherent path (__ldg).
+GDN_DEVICE void grid_dep_handover() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+GDN_DEVICE void grid_dep_takeover() {
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+}
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, bytes % 16 == 0.
 GDN_DEVICE void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile(
