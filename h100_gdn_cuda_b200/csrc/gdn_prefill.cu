@@ -486,6 +486,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
         };
         if (plan.num_segments <= 1 && packed && s.batch > 1 && s.batch <= kMaxOrderedSeqs && chains > d->sms) {
             // more chains than SMs and unequal lengths: dispatch the longest sequences first
+            p.special = 1;
             p.num_seqs = s.batch;
             p.by_length = s.batch <= kMaxRankedSeqs;
             if (!p.by_length) {
@@ -507,6 +508,7 @@ static int chunked_forward_on(const GdnChunkedArgs* a, const SegmentPlan& plan, 
             float* seg_start = seg_mn + seg_units * 2 * kD * kD;
             p.seg_chunks = plan.seg_chunks;
             p.num_segments = plan.num_segments;
+            p.special = 1;
             p.num_seqs = s.batch;
             p.first_apart = plan.first_apart;
             p.seg_mn = seg_mn;

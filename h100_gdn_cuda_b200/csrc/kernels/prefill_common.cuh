@@ -90,6 +90,7 @@ __device__ __forceinline__ int packed_seq_segments(const int* cu_seqlens, int s,
 __device__ __forceinline__ SegPos locate_segment(const ChunkMap& m, int slot, int seg_chunks, int num_segments, int num_seqs) {
     if (!m.cu_seqlens) return SegPos{slot / num_segments, slot % num_segments, num_segments, slot - slot % num_segments};
     int first = 0;
+#pragma unroll 1
     for (int s = 0; s < num_seqs; ++s) {
         const int n = packed_seq_segments(m.cu_seqlens, s, seg_chunks);
         if (slot < first + n) return SegPos{s, slot - first, n, first};
@@ -101,6 +102,7 @@ __device__ __forceinline__ SegPos locate_segment(const ChunkMap& m, int slot, in
 __device__ __forceinline__ SegPos sequence_segments(const ChunkMap& m, int seq, int seg_chunks, int num_segments) {
     if (!m.cu_seqlens) return SegPos{seq, 0, num_segments, seq * num_segments};
     int first = 0;
+#pragma unroll 1
     for (int s = 0; s < seq; ++s) first += packed_seq_segments(m.cu_seqlens, s, seg_chunks);
     return SegPos{seq, 0, packed_seq_segments(m.cu_seqlens, seq, seg_chunks), first};
 }

@@ -58,7 +58,8 @@ struct FusedParams {
     //           2500 tokens 45.5 -> 47.5 us.)
     //   mode 2: grid = (slots, heads), the other segments (first_apart 0: all of them, mode 1 is not launched); starts from
     //           seg_start[slot * vh + head] (fp32), writes the output of its chunks; the last segment of a sequence writes the final state.
-    uint8_t mode, first_apart, by_length;  // (as bytes: 16 bytes of parameters less, one sequence of 707 tokens, d=64, 24.56 -> 24.46 us)
+    // special: anything but a CTA per sequence and head in that order (mode 1 or 2, by_length or seq_order)
+    uint8_t mode, first_apart, by_length, special;  // (as bytes: 16 bytes of parameters less, one sequence of 707 tokens, d=64, 24.56 -> 24.46 us)
     int seg_chunks, num_segments, num_seqs;
     float* seg_mn;
     float* seg_start;
@@ -165,30 +166,39 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
     volatile int* issued = abort_flag + 1;  // chunks whose loads the producer has issued (read by the L2 prefetcher)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    SegPos sp{0, 0, 1, 0};
-    if (p.mode == 1) {
-        sp = sequence_segments(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments);
-    } else if (p.mode == 2) {
-        sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
-        if (sp.seq < 0 || (sp.segment == 0 && p.first_apart)) {  // packed mode launches an upper bound of slots; first segments are done
-            // Whoever waits for this grid waits for all of the call: the grid must not complete before the launches in front of it.
-            if (blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
-            return;
+    SegPos sp{static_cast<int>(blockIdx.x), 0, 1, 0};
+    int head = static_cast<int>(blockIdx.y);
+    // (One branch around all of it, its loops not unrolled, and the first segments' store at the end behind the final state's: a run of a few
+    // chunks pays for every line of instructions that it has to fetch or jump over.  128 chains of 2 chunks 17.75 -> 17.55 us, 56 of 4 18.15 -> 17.8.
+    // An instance without it is as fast for those and 2 % slower a chunk.)
+    if (p.special) {
+        if (p.mode == 1) {
+            sp = sequence_segments(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments);
+        } else if (p.mode == 2) {
+            sp = locate_segment(p.map, static_cast<int>(blockIdx.x), p.seg_chunks, p.num_segments, p.num_seqs);
+            if (sp.seq < 0 || (sp.segment == 0 && p.first_apart)) {  // packed mode launches an upper bound of slots; first segments are done
+                // Whoever waits for this grid waits for all of the call: the grid must not complete before the launches in front of it.
+                if (blockIdx.x == 0 && blockIdx.y == 0) grid_dep_wait();
+                return;
+            }
+        } else {
+            head = static_cast<int>(blockIdx.x);
+            if (p.by_length) {
+                // order of the sequences: more tokens first, of equally many the one in front first (every warp for itself)
+                const int mine = lane < p.num_seqs ? p.map.cu_seqlens[lane + 1] - p.map.cu_seqlens[lane] : -1;
+                int rank = 0;
+#pragma unroll 1
+                for (int j = 0; j < p.num_seqs; ++j) {
+                    const int other = __shfl_sync(0xffffffffu, mine, j);
+                    rank += other > mine || (other == mine && j < lane);
+                }
+                sp.seq = __ffs(__ballot_sync(0xffffffffu, lane < p.num_seqs && rank == static_cast<int>(blockIdx.y))) - 1;
+            } else {
+                sp.seq = p.seq_order[blockIdx.y];
+            }
         }
     }
-    if (p.by_length) {
-        // order of the sequences: more tokens first, of equally many the one in front first (every warp for itself)
-        const int mine = lane < p.num_seqs ? p.map.cu_seqlens[lane + 1] - p.map.cu_seqlens[lane] : -1;
-        int rank = 0;
-        for (int j = 0; j < p.num_seqs; ++j) {
-            const int other = __shfl_sync(0xffffffffu, mine, j);
-            rank += other > mine || (other == mine && j < lane);
-        }
-        sp.seq = __ffs(__ballot_sync(0xffffffffu, lane < p.num_seqs && rank == static_cast<int>(blockIdx.y))) - 1;
-    }
-    const bool ranked = p.by_length || p.seq_order;
-    const int seq = p.mode != 0 || p.by_length ? sp.seq : (p.seq_order ? p.seq_order[blockIdx.y] : static_cast<int>(blockIdx.x));
-    const int head = ranked ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.y);
+    const int seq = sp.seq;
     const int segment = sp.segment, seq_nseg = sp.nseg;
     const long long seg_idx = static_cast<long long>(blockIdx.x) * p.vh + head;  // mode 2
     const int khead = head / (p.vh / p.kh);
@@ -405,26 +415,25 @@ __global__ void __launch_bounds__(fused::kThreads, 1)
         if (lane == 0) mbar_arrive(&bar_go[nchunks & 1]);  // releases the last chunk's epilogue
         // nothing is written once a wait of this CTA has given up (the results would be garbage)
         const bool healthy = *abort_flag == 0;
-        if (!healthy) {
-        } else if (p.mode != 0 && segment != seq_nseg - 1) {
-            if (p.mode == 1) {
-                float4* d4 = reinterpret_cast<float4*>(p.seg_start + (static_cast<long long>(sp.first_slot + 1) * p.vh + head) * (D * D) +
-                                                       static_cast<long long>(row) * D + 64 * hf);
+        if (healthy && segment == seq_nseg - 1) {
+            if (p.state_out) {
+                uint4* d4 = reinterpret_cast<uint4*>(p.state_out + seq * p.so_ss + head * p.so_sh +
+                                                     static_cast<long long>(row) * p.d + 64 * hf);
 #pragma unroll
-                for (int q = 0; q < 16; ++q) d4[q] = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
+                for (int q = 0; q < 8; ++q) {
+                    uint4 v;
+                    v.x = pack_bf16(S[q * 8 + 0], S[q * 8 + 1]);
+                    v.y = pack_bf16(S[q * 8 + 2], S[q * 8 + 3]);
+                    v.z = pack_bf16(S[q * 8 + 4], S[q * 8 + 5]);
+                    v.w = pack_bf16(S[q * 8 + 6], S[q * 8 + 7]);
+                    if (row < p.d && 64 * hf + 8 * q < p.d) d4[q] = v;
+                }
             }
-        } else if (p.state_out) {
-            uint4* d4 = reinterpret_cast<uint4*>(p.state_out + seq * p.so_ss + head * p.so_sh +
-                                                 static_cast<long long>(row) * p.d + 64 * hf);
+        } else if (healthy && p.mode == 1) {
+            float4* d4 = reinterpret_cast<float4*>(p.seg_start + (static_cast<long long>(sp.first_slot + 1) * p.vh + head) * (D * D) +
+                                                   static_cast<long long>(row) * D + 64 * hf);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                uint4 v;
-                v.x = pack_bf16(S[q * 8 + 0], S[q * 8 + 1]);
-                v.y = pack_bf16(S[q * 8 + 2], S[q * 8 + 3]);
-                v.z = pack_bf16(S[q * 8 + 4], S[q * 8 + 5]);
-                v.w = pack_bf16(S[q * 8 + 6], S[q * 8 + 7]);
-                if (row < p.d && 64 * hf + 8 * q < p.d) d4[q] = v;
-            }
+            for (int q = 0; q < 16; ++q) d4[q] = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
         }
     } else if (warp < 12) {
         // =============================================================== output warps
