@@ -12,6 +12,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libgdn_b200.so")
 
 GDN_BF16, GDN_F32 = 0, 1
+GDN_ERR_WORKSPACE = -4
 
 
 class TokenTensor(C.Structure):

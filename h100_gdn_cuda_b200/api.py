@@ -391,16 +391,25 @@ def chunked_forward(query, key, value, beta, gate, scale: Optional[float] = None
     shape = _shape(batch, seq_len, total, kh, vh, D, D, cu_seqlens, chunk_indices, cu_chunks, tc)
     lib = cabi.load()
     ws_bytes = lib.gdn_chunked_forward_workspace_bytes(C.byref(shape))
-    ws = _workspace if _workspace is not None and _workspace.numel() >= ws_bytes else \
-        torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
     ev = None
     if _stage_events is not None:  # three torch.cuda.Event(enable_timing=True), already recorded once
         ev = (C.c_void_p * 3)(*[e.cuda_event for e in _stage_events])
-    args = cabi.ChunkedArgs(shape, _token_tensor(q, varlen), _token_tensor(k, varlen), _token_tensor(v, varlen),
-                            _token_tensor(out, varlen), _token_scalar(beta, varlen), _token_scalar(gate, varlen),
-                            _state_desc(s_in), _state_desc(final), float(scale), ws.data_ptr(), ws_bytes,
-                            ev, int(bool(is_qk_norm)))
-    cabi.check(lib.gdn_chunked_forward(C.byref(args), _stream()), "chunked_forward")
+
+    def run(ws, nbytes):
+        args = cabi.ChunkedArgs(shape, _token_tensor(q, varlen), _token_tensor(k, varlen), _token_tensor(v, varlen),
+                                _token_tensor(out, varlen), _token_scalar(beta, varlen), _token_scalar(gate, varlen),
+                                _state_desc(s_in), _state_desc(final), float(scale), ws.data_ptr(), nbytes,
+                                ev, int(bool(is_qk_norm)))
+        return lib.gdn_chunked_forward(C.byref(args), _stream())
+
+    # a given buffer below the fastest plan's size may hold a plan of fewer segments: the library says
+    given = _workspace if _workspace is not None and _workspace.numel() >= ws_bytes else None
+    rc = cabi.GDN_ERR_WORKSPACE
+    if given is None and _workspace is not None and _workspace.device == q.device and _workspace.dtype == torch.uint8 and _workspace.is_contiguous():
+        rc = run(_workspace, _workspace.numel())
+    if rc == cabi.GDN_ERR_WORKSPACE:
+        rc = run(torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if given is None else given, ws_bytes)
+    cabi.check(rc, "chunked_forward")
     if d != D:
         out, final = out[..., :d], final[..., :d, :d]
     return out, final

@@ -174,14 +174,25 @@ std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, c
     a.final_state = st(fin);
     a.scale = scale.value_or(default_scale(d));
     const size_t ws_bytes = gdn_chunked_forward_workspace_bytes(&a.shape);
-    const bool given = workspace.has_value() && workspace->is_cuda() && workspace->scalar_type() == at::kByte &&
-                       static_cast<size_t>(workspace->numel()) >= ws_bytes;
-    at::Tensor ws = given ? *workspace : empty({static_cast<int64_t>(ws_bytes)}, v, at::kByte);
-    a.workspace = ws.data_ptr();
-    a.workspace_bytes = ws_bytes;
+    const bool usable = workspace.has_value() && workspace->is_cuda() && workspace->scalar_type() == at::kByte;
+    const bool given = usable && static_cast<size_t>(workspace->numel()) >= ws_bytes;
     a.stage_events = nullptr;
     a.is_qk_norm = is_qk_norm ? 1 : 0;
-    check(gdn_chunked_forward(&a, stream), "chunked_forward");
+    // a given buffer below the fastest plan's size may hold a plan of fewer segments: the library says
+    int rc = GDN_ERR_WORKSPACE;
+    if (usable && !given && workspace->device() == v.device() && workspace->is_contiguous()) {
+        a.workspace = workspace->data_ptr();
+        a.workspace_bytes = static_cast<size_t>(workspace->numel());
+        rc = gdn_chunked_forward(&a, stream);
+    }
+    at::Tensor ws;
+    if (rc == GDN_ERR_WORKSPACE) {
+        ws = given ? *workspace : empty({static_cast<int64_t>(ws_bytes)}, v, at::kByte);
+        a.workspace = ws.data_ptr();
+        a.workspace_bytes = ws_bytes;
+        rc = gdn_chunked_forward(&a, stream);
+    }
+    check(rc, "chunked_forward");
     if (d != D) {
         out = out.narrow(-1, 0, d);
         fin = fin.narrow(-1, 0, d).narrow(-2, 0, d);

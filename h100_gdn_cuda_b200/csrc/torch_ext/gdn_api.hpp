@@ -25,8 +25,8 @@ std::pair<at::Tensor, at::Tensor> chunked_forward(at::Tensor& query, at::Tensor&
                                                   std::optional<int> total_chunks, cudaStream_t stream,
                                                   bool is_qk_norm = false);  // last argument: extension, see gdn_b200.h
 
-// chunked_forward with the gate optional (no decay without it) and, when `workspace` is large enough, that buffer
-// instead of one allocated for the call.
+// chunked_forward with the gate optional (no decay without it) and, when `workspace` is large enough for the call (with fewer
+// segments than the fastest plan has, if need be), that buffer instead of one allocated for the call.
 std::pair<at::Tensor, at::Tensor> chunked_forward_ext(const at::Tensor& query, const at::Tensor& key, const at::Tensor& value,
                                                       const at::Tensor& beta, const std::optional<at::Tensor>& gate,
                                                       std::optional<float> scale, const std::optional<at::Tensor>& initial_state,

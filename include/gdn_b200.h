@@ -245,8 +245,9 @@ int gdn_compute_o(const GdnComputeOArgs* args, gdn_stream_t stream);
  * Replaces gdn_cuda::chunked_forward (csrc/apis/gdn_forward.cpp:18-132): raw (pre-cumsum)
  * fp32 or bf16 gate, token-major beta; writes `out` (like v) and final_state.  The per-chunk
  * state tensor of the reference is never materialised.  `workspace` is caller-provided device
- * memory of at least gdn_chunked_forward_workspace_bytes(&shape) bytes, 256-byte aligned; its
- * contents need not be initialised and are garbage afterwards.  It holds one 24 KiB block per
+ * memory of gdn_chunked_forward_workspace_bytes(&shape) bytes or more, 256-byte aligned; its
+ * contents need not be initialised and are garbage afterwards.  (Less is taken where the sequences
+ * run in segments and it has room for fewer of them; GDN_ERR_WORKSPACE otherwise.)  It holds one 24 KiB block per
  * 64-token chunk and v-head (the WY/UT transform folded into a 64 x 128 and a 64 x 64 bf16
  * matrix that the state kernel consumes) and, when few long sequences (padded, or packed with
  * at most 64 sequences) are propagated in segments, three fp32 states (192 KiB) per (sequence,

@@ -143,3 +143,28 @@ def test_counts_and_modes_as_int_takes_them(api):
     d = _cuda(synthetic.decode_inputs(1, 2, 1, 1, 64, seed=1))
     for mode in (2.0, torch.tensor(2), api.SpecVerify):
         assert api.recurrent_forward(d["q"], d["k"], d["v"], d["state"], d["b"], inference_mode=mode)[1].dim() == 5
+
+
+@pytest.mark.parametrize("front", ["extension", "ctypes"])
+@pytest.mark.parametrize("B,T,kh,vh", [(1, 2500, 2, 4), (1, 7919, 2, 8)])
+def test_given_workspace_with_room_for_fewer_segments(api, monkeypatch, front, B, T, kh, vh):
+    """Few chains ask for more scratch than their longer segments did: a buffer laid out for those is used (fewer segments, other roundings of the
+    state between them), not passed over for a new one of the full size; below what the call can do with, one is allocated."""
+    if front == "ctypes":
+        monkeypatch.setattr(api, "_ext", False)
+    p = _cuda(synthetic.prefill_inputs(B, T, kh, vh, 128, seed=T, mild_gate=True))
+    run = lambda ws: api.chunked_forward(p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], _workspace=ws)
+    full = api.chunked_forward_workspace_bytes(B, T, vh, num_k_heads=kh)
+    ref = [t.float() for t in run(None)]
+    unit = B * vh * 3 * 128 * 128 * 4
+    base = B * ((T + 63) // 64) * (vh * 24576 + kh * 512)
+    for n, used in ((full, True), (full - unit, True), (base // 2, False)):
+        ws = torch.full((n,), 255, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocated_bytes.all.allocated"]
+        got = run(ws)
+        grown = torch.cuda.memory_stats()["allocated_bytes.all.allocated"] - before
+        assert (grown < base // 2 + sum(t.nbytes for t in got)) == used
+        assert bool((ws != 255).any()) == used
+        for x, y in zip(ref, got):
+            assert torch.isfinite(y.float()).all() and ((x - y.float()).norm() / x.norm()).item() <= 1e-2
