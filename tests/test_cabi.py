@@ -90,7 +90,8 @@ def test_workspace_bytes(lib):
 
 
 def test_segment_plan_heuristic():
-    """Host-side choice of the number of segments for the state propagation (heuristics.hpp)."""
+    """Number of segments for the state propagation (heuristics.hpp): the rule of sequences of more than 640 chunks.  (Shorter ones have
+    prefill_segments_short, see test_heuristics_cpu.py; for them this rule says from what scratch on a call is taken.)"""
     import subprocess, tempfile, textwrap
     src = textwrap.dedent('''
         #include <cstdio>
@@ -135,27 +136,22 @@ def test_segment_plan_heuristic():
     assert rows[13][0] == 1              # four equal sequences would already run side by side
 
 
-def test_short_sequences_of_many_chains_stay_whole():
-    """24 to 48 chains: measured uncut at 75 .. 100 chunks (cut it took up to 16 % longer), cut at 400."""
-    import subprocess, tempfile, textwrap
-    src = textwrap.dedent('''
-        #include <cstdio>
-        #include "heuristics.hpp"
-        int main() {
-            for (int chains : {24, 32, 40, 48})
-                for (int chunks : {75, 90, 400})
-                    std::printf("%d %d\\n", gdn::prefill_segments(chains, chunks, false).num_segments,
-                                gdn::prefill_segments_packed(1, chains, chunks).num_segments);
-            return 0;
-        }''')
-    with tempfile.TemporaryDirectory() as d:
-        c = os.path.join(d, "h.cpp")
-        open(c, "w").write(src)
-        exe = os.path.join(d, "h")
-        subprocess.check_call(["g++", "-std=c++17", "-I", os.path.join(ROOT, "h100_gdn_cuda_b200", "csrc"), c, "-o", exe])
-        rows = [l.split() for l in subprocess.check_output([exe]).decode().splitlines()]
-    for i, row in enumerate(rows):
-        assert all((int(n) > 1) == (i % 3 == 2) for n in row), (i, row)
+def test_dispatched_segments(lib):
+    """Segments of a call as gdn_chunked_forward cuts it, from the scratch it asks for: 192 KB per (sequence, v-head) and segment (256 bytes or so for the order of a packed batch).  Few chains of up
+    to 640 chunks by the short plan, cut where that was measured to be faster and whole where not; longer ones by the other."""
+    from h100_gdn_cuda_b200 import api
+
+    def segments(B, T, vh, packed=False):
+        chunks = B * ((T + 63) // 64)
+        n = api.chunked_forward_workspace_bytes(B, 0 if packed else T, vh, total_tokens=B * T, total_chunks=chunks if packed else 0, packed=packed, num_k_heads=1)
+        extra = n - (chunks * (vh * 24576 + 512) + 256)
+        return 1 if extra <= 512 else (extra - 256) / (B * vh * 3 * 128 * 128 * 4)
+
+    for B, chunks, vh, cut in ((1, 16, 4, False), (1, 32, 4, True), (1, 40, 8, True), (1, 64, 16, True), (1, 75, 24, True), (1, 90, 32, True), (1, 100, 32, True),
+                               (1, 256, 48, True), (1, 313, 49, False), (2, 640, 32, False), (4, 64, 32, False)):
+        assert (segments(B, 64 * chunks, vh) > 1) == cut, (B, chunks, vh)
+    assert segments(2, 131072, 4) == 18
+    assert segments(4, 4000, 4, packed=True) > 1 and segments(16, 2048, 32, packed=True) == 1 and segments(65, 6000, 1, packed=True) == 1
 
 
 @pytest.mark.parametrize("B,T,vh,packed", [(1, 50048, 2, False), (1, 65536, 2, False), (1, 16384, 8, False), (4, 8000, 4, True)])

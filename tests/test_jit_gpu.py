@@ -52,12 +52,12 @@ def test_jit_recurrent_equals_prebuilt(gdn, monkeypatch, tmp_path, use_nvrtc):
 
 @pytest.mark.parametrize("d,lens,suffix", [(128, None, "block"), (64, None, "block"), (192, [27, 40, 300], "block_packed"), (256, [1, 70, 0, 22, 23] + [2] * 20, "block_walk")])
 @pytest.mark.parametrize("use_nvrtc", ["1", "0"])
-def test_jit_token_blocks_equal_prebuilt(gdn, monkeypatch, tmp_path, d, lens, suffix, use_nvrtc):
+def test_jit_token_blocks_equal_prebuilt(gdn, monkeypatch, tmp_path, d, lens, suffix, use_nvrtc, vh=2):
     """long runs: the same kernel, and the same bits, as an ahead-of-time launch of the call takes"""
     if lens is None:
-        p = synthetic.prefill_inputs(2, 50, 1, 2, d, seed=7, mild_gate=True)
+        p = synthetic.prefill_inputs(2, 50, 1, vh, d, seed=7, mild_gate=True)
     else:
-        p = synthetic.varlen_inputs(lens, 1, 2, d, seed=7, mild_gate=True)
+        p = synthetic.varlen_inputs(lens, 1, vh, d, seed=7, mild_gate=True)
     pd = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
     run = lambda: gdn.recurrent_forward(pd["q"], pd["k"], pd["v"], pd["state"], pd["beta"], pd["g"], pd.get("cu_seqlens"), inference_mode=1)
     o_ref, s_ref = run()
@@ -72,6 +72,14 @@ def test_jit_token_blocks_equal_prebuilt(gdn, monkeypatch, tmp_path, d, lens, su
     finally:
         monkeypatch.delenv("GDN_JIT_RECURRENT")
         gdn.init(ROOT, cuda_home)
+
+
+@pytest.mark.parametrize("d,vh,lens,suffix", [(256, 6, None, "block"), (192, 6, [27, 40, 300], "block_packed"), (256, 6, [33] + [1] * 30, "block_walk")])
+def test_jit_two_groups_of_rows_equal_prebuilt(gdn, monkeypatch, tmp_path, d, vh, lens, suffix):
+    """more tiles of 16 rows than SMs (192 to 216): CTAs of 32 rows, compiled with as many groups, threads and as much shared memory"""
+    test_jit_token_blocks_equal_prebuilt(gdn, monkeypatch, tmp_path, d, lens, suffix, "1", vh)
+    src = [open(os.path.join(tmp_path, f, "kernel.cu")).read() for f in os.listdir(tmp_path) if f.startswith("kernel.recurrent_dk%d.%s." % (d, suffix))]
+    assert len(src) == 1 and "__launch_bounds__(384, 1)" in src[0]
 
 
 def test_head_dim_without_prebuilt_kernel(gdn):

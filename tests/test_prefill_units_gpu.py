@@ -172,3 +172,68 @@ def test_short_segments_back_to_back(lens, kh, vh, norm, state):
 
     a, b = chain(True), chain(False)
     assert torch.equal(a[1], b[1]) and all(torch.equal(x, y) for x, y in zip(a[0], b[0]))
+
+
+# padded short segments: 4 to 8 chains of 34 to 47 chunks, ragged ends, head dims below 128, two sequences
+PADDED = [(1, 2500, 2, 4, 128, False), (1, 2177, 4, 8, 64, True), (2, 2200, 1, 2, 96, False), (1, 3008, 2, 4, 40, True), (3, 2176, 1, 1, 128, True)]
+
+
+@pytest.mark.parametrize("B,T,kh,vh,d,norm", PADDED)
+@pytest.mark.parametrize("state", [False, True])
+def test_padded_short_segments(B, T, kh, vh, d, norm, state):
+    """against the oracle, and cut it is: the scratch has room for the segments' states"""
+    import h100_gdn_cuda_b200 as gdn
+    from h100_gdn_cuda_b200 import api
+    from oracle import gdn_oracle as O
+    assert api.chunked_forward_workspace_bytes(B, T, vh, num_k_heads=kh) > B * ((T + 63) // 64) * (vh * 24576 + kh * 512) + 3 * B * vh * 196608
+    p = synthetic.prefill_inputs(B, T, kh, vh, d, seed=T + d, mild_gate=True)
+    if norm:
+        p["q"], p["k"] = (3 * p["q"].float()).bfloat16(), (0.2 * p["k"].float()).bfloat16()
+    s0 = p["state"] if state else None
+    o_ref, s_ref = O.recurrent_ref(*(p[k].float() for k in ("q", "k", "v", "beta")), p["g"], s0.float() if state else None, is_qk_norm=norm)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in p.items()}
+    o, s = gdn.chunked_forward(c["q"], c["k"], c["v"], c["beta"], c["g"], None, c["state"] if state else None, is_qk_norm=norm)
+    for x, ref in ((o, o_ref), (s, s_ref)):
+        assert O.rel_fro(x.float().cpu(), ref) <= 1e-2 and O.max_abs_over_max(x.float().cpu(), ref) <= 5e-2
+
+
+@pytest.mark.parametrize("B,T,kh,vh,d,norm", PADDED[:3])
+def test_short_segments_in_a_graph(B, T, kh, vh, d, norm):
+    """The five launches of the call, three of which run beside the one before, recorded and replayed without a pause: the bits of a call
+    by itself, also after other inputs have been copied into the buffers."""
+    import h100_gdn_cuda_b200 as gdn
+    ps = [{k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.prefill_inputs(B, T, kh, vh, d, seed=s, mild_gate=True).items()} for s in (1, 2)]
+    run = lambda p: gdn.chunked_forward(p["q"], p["k"], p["v"], p["beta"], p["g"], None, p["state"], is_qk_norm=norm)
+    refs = [run(p) for p in ps]
+    buf = {k: (v.clone() if torch.is_tensor(v) else v) for k, v in ps[0].items()}
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o, s = run(buf)
+    for i in (0, 1, 0):
+        for k, v in ps[i].items():
+            if torch.is_tensor(v):
+                buf[k].copy_(v)
+        o.zero_(), s.zero_()
+        for _ in range(5):
+            graph.replay()
+        assert torch.equal(o, refs[i][0]) and torch.equal(s, refs[i][1])
+
+
+@pytest.mark.parametrize("B,T,kh,vh,d,norm", PADDED[:3])
+def test_short_segments_final_state_over_the_initial_one(B, T, kh, vh, d, norm):
+    """the first segments read the state that the last ones write, in another launch"""
+    import ctypes as C
+    from h100_gdn_cuda_b200 import _cabi as cabi, api
+    p = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in synthetic.prefill_inputs(B, T, kh, vh, d, seed=5, mild_gate=True).items()}
+    lib, outs = cabi.load(), []
+    n = api.chunked_forward_workspace_bytes(B, T, vh, num_k_heads=kh)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    for over in (False, True):
+        s0 = p["state"].clone()
+        out, final = torch.empty_like(p["v"]), s0 if over else torch.empty_like(s0)
+        a = cabi.ChunkedArgs(api._shape(B, T, B * T, kh, vh, d, d), *(api._token_tensor(t, False) for t in (p["q"], p["k"], p["v"], out)),
+                             api._token_scalar(p["beta"], False), api._token_scalar(p["g"], False), api._state_desc(s0), api._state_desc(final),
+                             d ** -0.5, ws.data_ptr(), n, None, int(norm))
+        assert lib.gdn_chunked_forward(C.byref(a), torch.cuda.current_stream().cuda_stream) == 0, lib.gdn_last_error()
+        outs.append((out, final))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
