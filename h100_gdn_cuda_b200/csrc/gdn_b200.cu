@@ -571,7 +571,7 @@ int gdn_recurrent_forward(const GdnRecurrentArgs* a, gdn_stream_t stream) {
     GDN_REQUIRE(p.num_tiles < (1ll << 31), "gdn_recurrent_forward: too many state tiles");
     p.status = d->status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    
+
     if (g_ring_min.load(std::memory_order_relaxed) < 0) read_env_switches();
     const int ring_min = g_ring_min.load(std::memory_order_relaxed);
     const int force_jit = g_force_jit.load(std::memory_order_relaxed);

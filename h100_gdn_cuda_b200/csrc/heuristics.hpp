@@ -94,16 +94,14 @@ constexpr long long kNoLimit = std::numeric_limits<long long>::max();
 // chunk of the state kernel" (1.25 us): a CTA costs its chunks plus about 3 for start-up and pipeline
 // fill, a chunk of the transition kernel 1.2 (1.5 us for both of its runs).  Every boundary between two segments of a chain
 // costs kBoundary on top: its composite and start state move 0.4 MB, and it is one more product of a kernel that runs 9 chains
-// at a time.  Without that term 20 to 48 chains of 75 to 200 chunks were cut although it cost time (B=1, d=128: 48 v-heads
-// of 100 chunks 200 us against 179 uncut, 32 of 75 130 against 121); with it all shapes measured (2 to 72 chains, 75 to 400
-// chunks, padded and packed) are within the noise of the better of cut and uncut.  Plans whose launches need more than one wave measured worse
-// than the model and are not made.
+// at a time.  (Fitted when this plan decided for shorter sequences too, at 2 to 72 chains of 75 to 400 chunks.)  Plans whose launches need more
+// than one wave measured worse than the model and are not made.  Sequences of up to kShortChunks chunks have the plan further down; for them
+// this one only says from what scratch on a call is taken (gdn_prefill.cu, segment_plan_in).
 constexpr int kFixed = 3;
 constexpr double kPasses = 2.2, kBoundary = 0.15, kMargin = 0.85;
-// Shortest segments.  With 16 chains of 90, 100, 125 chunks at least 20 gives 103, 103, 113 us, 25 117, 112, 119 and 32 121, 128,
-// 151; but 66 chunks are slower cut in three (94 us against 92), 32 chains of 66 by 11 %.  Packed sequences of unequal
-// lengths each end in a shorter one, hence the larger figure there (equal ones gain from 25: one of 100 chunks on 16 heads 129
-// -> 112 us).
+// Shortest segments, from measurements of 16 chains of 66 to 125 chunks, which the plan further down decides by now.  Above kShortChunks
+// they bind little (padded: at most 32 segments, so only below 800 chunks).  Packed sequences of unequal lengths each end in a shorter
+// one, hence the larger figure there.
 constexpr int kMinSegment = 25, kMinSegmentPacked = 32;
 inline long long waves(long long ctas) { return (ctas + kSms - 1) / kSms; }
 }  // namespace plan_detail
@@ -168,6 +166,7 @@ inline SegmentPlan prefill_segments_packed(int num_seqs, int num_v_heads, long l
 // us: 4 chains of 32 chunks 44.8 : 41.4, of 64 76.8 : 53.1, of 100 115 : 62.6, of 256 277 : 89.1; 16 of 64 88 : 75, of 256 322 : 170; 32 of 100 155 : 140,
 // of 256 384 : 289; 48 of 256 433 : 376.  Against the plan above, whose segments have 25 chunks and more and whose first ones are found like the
 // others: 1 sequence of 7919 tokens on 32 v-heads 177 : 161, 2 of 7344 on 8 125 : 101, 1 of 22109 on 4 121 : 103, packed 4 of 4000 on 4 165 : 82.
+// 49 chains (7 sequences on 7 v-heads) stay whole: 172 chunks 339 us, cut so 355, 250 491 : 492, 625 1196 : 1144, in three by the plan above 350, 541, 1274.
 // Longer sequences are bound by what the launches move, and a launch more costs them 1 % (4 chains of 1024 chunks in 32 segments 195 : 198): they
 // keep the plans above.
 constexpr int kShortChunks = 640, kManyChains = 48;

@@ -6,7 +6,7 @@
 // A run is a chain of dependent steps that leaves the tensor pipe idle 80 % of the time and the schedulers 60 %; two runs
 // on the same tiles fill each other's gaps and read K, Z and the gates once.  Each run has 8 state warps of its own, the
 // first MMA's accumulator shares the columns of the second's (it is dead once R is published), so both fit tensor memory.
-// B=2, T=131072, 4 v-heads (128 CTAs of 114 chunks): replaces two waves of one run per CTA, see gdn_chunked_forward.
+// B=2, T=131072, 4 v-heads (136 CTAs of 114 chunks): replaces two waves of one run per CTA, see gdn_chunked_forward.
 #pragma once
 #include <cuda.h>
 

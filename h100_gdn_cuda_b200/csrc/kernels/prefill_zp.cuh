@@ -211,8 +211,8 @@ struct TeamTiles {
 // same matrices (tokens i and r, r and j): neither is infinite unless the exact result is.
 // `tm_kq`: column of K K^T (lanes 0-63) and Q K^T (64-127).
 // A loop, block by block.  Written out (ten copies of a block, and three of row_blocks) the kernel was 67 KB of code, now 55, and waited for
-// instructions in 0.60 of 9.3 warp cycles per issue, now 0.31: B=4 T=4096, 32 v-heads 208.4 -> 206.8 us a call, 16 packed sequences of
-// 32768 tokens 443.7 -> 438.3.
+// instructions in 0.60 of 9.3 warp cycles per issue, now 0.31: B=4 T=4096, 32 v-heads 208.4 -> 206.8 us a call, B=2 T=1000 41.1 -> 40.5 (two runs of
+// one side differ by 0.1 to 0.3 %); 16 packed sequences of 32768 tokens 443.7 -> 438.3, within what two runs there differ by (2.5 %).
 template <bool kNorm>
 __device__ __forceinline__ void ap_pass(uint32_t tm_kq, const TeamTiles& t, int tw, int lane, int n, float g_mine, const float* b_mine,
                                         float p_scale) {
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(zp::kThreads, 2) gdn_zp_kernel(const __grid_co
                 //      64 columns j)
                 {
                     const uint32_t aa = smem_u32(tiles.a), ia = smem_u32(tiles.diag);
-const int row = 16 * rblk + g;
+                    const int row = 16 * rblk + g;
                     const float d0 = kNorm ? sD[row] * sRn[row] : sD[row], d1 = kNorm ? sD[row + 8] * sRn[row + 8] : sD[row + 8];
                     const f2 dd[2] = {pk(d0, d0), pk(d1, d1)};
                     const uint32_t tile = smem_u32(sT);
