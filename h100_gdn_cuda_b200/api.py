@@ -394,21 +394,20 @@ def chunked_forward(query, key, value, beta, gate, scale: Optional[float] = None
     ev = None
     if _stage_events is not None:  # three torch.cuda.Event(enable_timing=True), already recorded once
         ev = (C.c_void_p * 3)(*[e.cuda_event for e in _stage_events])
-
-    def run(ws, nbytes):
-        args = cabi.ChunkedArgs(shape, _token_tensor(q, varlen), _token_tensor(k, varlen), _token_tensor(v, varlen),
-                                _token_tensor(out, varlen), _token_scalar(beta, varlen), _token_scalar(gate, varlen),
-                                _state_desc(s_in), _state_desc(final), float(scale), ws.data_ptr(), nbytes,
-                                ev, int(bool(is_qk_norm)))
-        return lib.gdn_chunked_forward(C.byref(args), _stream())
-
+    args = cabi.ChunkedArgs(shape, _token_tensor(q, varlen), _token_tensor(k, varlen), _token_tensor(v, varlen),
+                            _token_tensor(out, varlen), _token_scalar(beta, varlen), _token_scalar(gate, varlen),
+                            _state_desc(s_in), _state_desc(final), float(scale), None, 0,
+                            ev, int(bool(is_qk_norm)))
     # a given buffer below the fastest plan's size may hold a plan of fewer segments: the library says
-    given = _workspace if _workspace is not None and _workspace.numel() >= ws_bytes else None
+    ws = _workspace if _workspace is not None and _workspace.numel() >= ws_bytes else None
     rc = cabi.GDN_ERR_WORKSPACE
-    if given is None and _workspace is not None and _workspace.device == q.device and _workspace.dtype == torch.uint8 and _workspace.is_contiguous():
-        rc = run(_workspace, _workspace.numel())
+    if ws is None and _workspace is not None and _workspace.device == q.device and _workspace.dtype == torch.uint8 and _workspace.is_contiguous():
+        args.workspace, args.workspace_bytes = _workspace.data_ptr(), _workspace.numel()
+        rc = lib.gdn_chunked_forward(C.byref(args), _stream())
     if rc == cabi.GDN_ERR_WORKSPACE:
-        rc = run(torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if given is None else given, ws_bytes)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws is None else ws
+        args.workspace, args.workspace_bytes = ws.data_ptr(), ws_bytes
+        rc = lib.gdn_chunked_forward(C.byref(args), _stream())
     cabi.check(rc, "chunked_forward")
     if d != D:
         out, final = out[..., :d], final[..., :d, :d]
