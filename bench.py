@@ -107,8 +107,8 @@ def seq_kernel_bytes_per_unit(kh: int, vh: int, d: int, c: int = CHUNK) -> float
 #   gdn_fused_seq_kernel : same capture, 4096 units
 #   gdn_recurrent_kernel : B=128 capture (gating fused), 128 sequence-tokens
 # (written data still in L2 when a launch ends is not counted by the DRAM counters)
-NCU_ZP_TRAFFIC_PER_UNIT = (68.8e6 + 38.8e6) / 4096
-NCU_FUSED_TRAFFIC_PER_UNIT = (239e6 + 35.1e6) / 4096
+NCU_ZP_TRAFFIC_PER_UNIT = (68.7e6 + 41.0e6) / 4096
+NCU_FUSED_TRAFFIC_PER_UNIT = (239.4e6 + 38.9e6) / 4096
 NCU_DECODE_TRAFFIC_PER_TOKEN = (136.373248e6 + 84.418816e6) / 128
 
 
